@@ -126,6 +126,169 @@ int launch_out(const void* x, const void* w, const void* bias, int bias_dtype, v
     BL_FAIL("bl_gemm_plain: unknown output dtype %d", out_dtype);
 }
 
+// ---- the 32-bit product with tiles in flight ---------------------------------------------------------------------------
+// The same sums (one accumulator an output, ascending k, so the same bits as the kernel above and independent of the tile)
+// for 32-bit x and W whose rows are whole 16-byte pieces: BK values of k of a tile's rows come by cp.async into a ring of
+// three stages as they lie in memory, rows padded by 16 bytes so that the eight rows that lanes of a quarter warp read
+// fall on different banks; a thread's TR x TC outputs lie (rows, columns of threads) apart, so its operands are 16-byte
+// loads of four k each. With SWIGLU the tile's upper half of W rows are the up rows, and a thread holds both sums of a unit.
+// Bound by the FMA pipes for many rows (74 TFLOP/s), by W's bytes for few.
+template <int BM, int BN, int TR, int TC, int EPI>
+__global__ void __launch_bounds__((BM / TR) * (BN / TC))
+gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, const void* __restrict__ bias, int bias_dtype,
+                float* __restrict__ out, int M, int N, int K, int ldx) {
+    constexpr int THREADS = (BM / TR) * (BN / TC), BK = 32, LD = BK + 4, STAGES = 3, GR = BM / TR, GC = BN / TC;
+    constexpr bool GLU = EPI == BL_EPI_SWIGLU;
+    constexpr int COLS = GLU ? BN / 2 : BN;               // outputs a row of the tile
+    static_assert(GC % 8 == 0 && GR % 4 == 0, "a warp is 4 rows of 8 threads");
+    extern __shared__ __align__(16) float ring[];         // [STAGES][BM + BN][LD]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tx = (warp % (GC / 8)) * 8 + (lane & 7), ty = (warp / (GC / 8)) * 4 + (lane >> 3);
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * COLS;
+    bl_pdl_wait();
+    auto fetch = [&](int k0, float* stage) {
+#pragma unroll 4
+        for (int c = tid; c < (BM + BN) * (BK / 4); c += THREADS) {
+            const int row = c / (BK / 4), k = k0 + (c % (BK / 4)) * 4;
+            const float* src;
+            bool ok = k < K;
+            if (row < BM) {
+                ok = ok && m0 + row < M;
+                src = x + (size_t)(ok ? m0 + row : 0) * ldx + (ok ? k : 0);
+            } else {
+                const int j = row - BM, n = n0 + (GLU && j >= COLS ? j - COLS : j);
+                ok = ok && n < N;
+                src = w + (size_t)(ok ? (GLU && j >= COLS ? N + n : n) : 0) * K + (ok ? k : 0);
+            }
+            const unsigned dst = (unsigned)__cvta_generic_to_shared(stage + row * LD + (c % (BK / 4)) * 4);
+            const int bytes = ok ? 16 : 0;                // 0: the piece is filled with zeros
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" :: "r"(dst), "l"(src), "r"(bytes));
+        }
+        asm volatile("cp.async.commit_group;\n" ::);
+    };
+    float acc[TR][TC];
+#pragma unroll
+    for (int i = 0; i < TR; ++i)
+#pragma unroll
+        for (int j = 0; j < TC; ++j) acc[i][j] = 0.f;
+    const int steps = (K + BK - 1) / BK;
+    fetch(0, ring);
+    if (steps > 1) fetch(BK, ring + (BM + BN) * LD);
+    else asm volatile("cp.async.commit_group;\n" ::);
+    for (int s = 0; s < steps; ++s) {
+        asm volatile("cp.async.wait_group 1;\n" ::);
+        __syncthreads();                                  // stage s has landed; everybody is through with stage s - 1
+        if (s + 2 < steps) fetch((s + 2) * BK, ring + (s + 2) % STAGES * (BM + BN) * LD);
+        else asm volatile("cp.async.commit_group;\n" ::);
+        const float* xs = ring + s % STAGES * (BM + BN) * LD + ty * LD;
+        const float* ws = ring + s % STAGES * (BM + BN) * LD + (BM + tx) * LD;
+#pragma unroll
+        for (int k = 0; k < BK; k += 4) {
+            float4 a[TR];
+#pragma unroll
+            for (int i = 0; i < TR; ++i) a[i] = *reinterpret_cast<const float4*>(xs + i * GR * LD + k);
+#pragma unroll
+            for (int j = 0; j < TC; ++j) {
+                const float4 b = *reinterpret_cast<const float4*>(ws + j * GC * LD + k);
+#pragma unroll
+                for (int i = 0; i < TR; ++i) {
+                    acc[i][j] = fmaf(a[i].x, b.x, acc[i][j]);
+                    acc[i][j] = fmaf(a[i].y, b.y, acc[i][j]);
+                    acc[i][j] = fmaf(a[i].z, b.z, acc[i][j]);
+                    acc[i][j] = fmaf(a[i].w, b.w, acc[i][j]);
+                }
+            }
+        }
+    }
+    bl_pdl_trigger();
+    const BlGluArgs glu = bl_glu_args(GLU ? bias : nullptr);
+#pragma unroll
+    for (int i = 0; i < TR; ++i) {
+        const int m = m0 + ty + i * GR;
+        if (m >= M) continue;
+#pragma unroll
+        for (int j = 0; j < (GLU ? TC / 2 : TC); ++j) {
+            const int n = n0 + tx + j * GC;
+            if (n >= N) continue;
+            float* dst = out + (size_t)m * N + n;
+            float v = acc[i][j];
+            if (EPI == BL_EPI_BIAS) v += bl_load_any(bias, bias_dtype, n);
+            if (EPI == BL_EPI_RESIDUAL) {
+                if (bias) v += bl_load_any(bias, bias_dtype, n);
+                v += *dst;
+            }
+            if (GLU) {
+                float u = acc[i][GLU ? j + TC / 2 : j];
+                if (glu.bias) { v += glu.bias[n]; u += glu.bias[N + n]; }
+                v = bl_glu(glu.kind, v, u, glu.limit);
+            }
+            *dst = v;
+        }
+    }
+}
+
+template <int BM, int BN, int TR, int TC>
+int launch_f32(const float* x, const float* w, const void* bias, int bias_dtype, float* out, int M, int N, int K, int ldx, int epi,
+               cudaStream_t s) {
+    const int cols = epi == BL_EPI_SWIGLU ? BN / 2 : BN;
+    const dim3 grid((N + cols - 1) / cols, (M + BM - 1) / BM), block((BM / TR) * (BN / TC));
+    constexpr size_t bytes = (size_t)3 * (BM + BN) * 36 * sizeof(float);
+#define BL_GO(E) do { \
+        static thread_local bool allowed = false; \
+        if (!allowed) { BL_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<BM, BN, TR, TC, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)); allowed = true; } \
+        BL_CUDA(bl_launch_dependent(gemm_f32_kernel<BM, BN, TR, TC, E>, grid, block, bytes, s, x, w, bias, bias_dtype, out, M, N, K, ldx)); } while (0)
+    switch (epi) {
+        case BL_EPI_NONE: BL_GO(BL_EPI_NONE); break;
+        case BL_EPI_BIAS: BL_GO(BL_EPI_BIAS); break;
+        case BL_EPI_RESIDUAL: BL_GO(BL_EPI_RESIDUAL); break;
+        default: BL_GO(BL_EPI_SWIGLU); break;
+    }
+#undef BL_GO
+    BL_CHECK_LAUNCH("bl_gemm_plain (32-bit tiles)");
+    return 0;
+}
+
+// Which tile: the least of ceil(blocks / SMs) blocks in a row at a tile's pace, but no less than one block alone takes
+// (microseconds for 896 values of k, measured at 1 to 2,048 rows of six products; the ratio of K scales both). Few rows
+// are bound by a block's chain of stages, many by the FMA pipes: 366 rows of 896 x 4,864 take 145 us in 32 x 32 tiles,
+// 188 in 64 x 32 (the kernel above: 914); 2,048 rows of 11,008 + 11,008 x 2,048 4.5 ms in 64 x 32, 5.8 in 32 x 32
+// (8.0; 41 TFLOP/s of the 59 that dependent FMAs with three operands reach here); one row of 151,936 x 896 101 us in
+// 4 x 64 (860; 5.4 TB/s). Tiles of 64 x 64, 128 x 64 and 128 x 128 were no faster at any of these sizes.
+// A successor is let in when the sums are done: let in at the start, its waiting blocks pile up on the SMs that this launch
+// leaves empty and it runs at the pace of those (366 rows of 896 x 4,864: 193 us).
+struct F32Tile { int bm, bn; float alone, pace; };
+constexpr F32Tile F32_TILES[] = {{64, 32, 18.5f, 13.2f}, {32, 32, 11.8f, 8.3f}, {16, 64, 12.8f, 9.4f},
+                                 {16, 32, 9.3f, 6.4f}, {4, 64, 11.8f, 5.9f}, {4, 16, 6.8f, 1.95f}};
+constexpr int F32_SMS = 148;
+
+int launch_f32_tiles(const float* x, const float* w, const void* bias, int bias_dtype, float* out, int M, int N, int K, int ldx, int epi,
+                     cudaStream_t s) {
+    int best = 0;
+    float best_us = 0.f;
+    for (int v = 0; v < (int)(sizeof(F32_TILES) / sizeof(F32_TILES[0])); ++v) {
+        const F32Tile& t = F32_TILES[v];
+        const int cols = epi == BL_EPI_SWIGLU ? t.bn / 2 : t.bn;
+        const long long down = (M + t.bm - 1) / t.bm, blocks = (long long)((N + cols - 1) / cols) * down;
+        if (down > 65535) continue;
+        const float us = fmaxf(t.alone, (float)((blocks + F32_SMS - 1) / F32_SMS) * t.pace);
+        if (best_us == 0.f || us < best_us) { best = v; best_us = us; }
+    }
+    switch (best) {
+        case 0: return launch_f32<64, 32, 4, 4>(x, w, bias, bias_dtype, out, M, N, K, ldx, epi, s);
+        case 1: return launch_f32<32, 32, 4, 2>(x, w, bias, bias_dtype, out, M, N, K, ldx, epi, s);
+        case 2: return launch_f32<16, 64, 4, 2>(x, w, bias, bias_dtype, out, M, N, K, ldx, epi, s);
+        case 3: return launch_f32<16, 32, 2, 2>(x, w, bias, bias_dtype, out, M, N, K, ldx, epi, s);
+        case 4: return launch_f32<4, 64, 1, 2>(x, w, bias, bias_dtype, out, M, N, K, ldx, epi, s);
+        default: return launch_f32<4, 16, 1, 2>(x, w, bias, bias_dtype, out, M, N, K, ldx, epi, s);
+    }
+}
+
+// 32-bit rows of whole 16-byte pieces; everything else, bfloat16 and the decays' epilogues take the kernel above.
+bool f32_tiles_fit(const void* x, const void* w, int K, int ldx, int epi, int out_dtype) {
+    return out_dtype == BL_F32 && K % 4 == 0 && ldx % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0 &&
+           (epi == BL_EPI_NONE || epi == BL_EPI_BIAS || epi == BL_EPI_RESIDUAL || epi == BL_EPI_SWIGLU);
+}
+
 }  // namespace
 
 extern "C" int bl_gemm_plain(const void* x, int x_dtype, const void* w, int w_dtype, const void* bias,
@@ -144,6 +307,8 @@ extern "C" int bl_gemm_plain_ld(const void* x, int x_dtype, int ldx, const void*
     if (epilogue == BL_EPI_BIAS && bias_dtype != BL_F32 && bias_dtype != BL_BF16)
         BL_FAIL("bl_gemm_plain: unknown bias dtype %d", bias_dtype);
     cudaStream_t s = (cudaStream_t)stream;
+    if (x_dtype == BL_F32 && w_dtype == BL_F32 && f32_tiles_fit(x, w, K, ldx, epilogue, out_dtype))
+        return launch_f32_tiles((const float*)x, (const float*)w, bias, bias_dtype, (float*)out, M, N, K, ldx, epilogue, s);
     if (x_dtype == BL_F32 && w_dtype == BL_F32)
         return launch_out<float, float>(x, w, bias, bias_dtype, out, out_dtype, M, N, K, ldx, epilogue, s);
     if (x_dtype == BL_BF16 && w_dtype == BL_BF16)
