@@ -16,14 +16,16 @@ namespace {
 constexpr int MAX_DH = 256;
 constexpr int WARPS = 4;
 
-template <typename TT>
+// VEC: 32-bit keys whose rows are whole 16-byte pieces are read a piece at a time (the dot product stays one chain in
+// ascending d). NV: 32-column groups of the values, so that a lane does not walk groups the head does not have.
+template <typename TT, bool VEC, int NV>
 __global__ void __launch_bounds__(WARPS * 32)
 attention_plain_kernel(const TT* __restrict__ q, const TT* __restrict__ kc, const TT* __restrict__ vc,
                        const int* __restrict__ tok_req, const int* __restrict__ cu_q,
                        const int* __restrict__ ctx_len, const int* __restrict__ block_table, int max_pages,
                        TT* __restrict__ out, int T, int H, int KV, int dh, int dv, int page_size, int window,
                        float scale, const void* __restrict__ sinks, int sink_dtype, const float* gate, int ld_gate, int gate_dim, float softcap) {
-    __shared__ float qs[WARPS][MAX_DH];
+    __shared__ __align__(16) float qs[WARPS][MAX_DH];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int item = blockIdx.x * WARPS + warp;
     if (item >= T * H) return;                 // whole warps leave together; no block-wide barrier below
@@ -40,18 +42,28 @@ attention_plain_kernel(const TT* __restrict__ q, const TT* __restrict__ kc, cons
     const size_t head_off = (size_t)kvh * page_size * dh, v_head_off = (size_t)kvh * page_size * dv;
     const size_t page_stride = (size_t)KV * page_size * dh, v_page_stride = (size_t)KV * page_size * dv;
     float m = -INFINITY, l = 0.f;
-    float acc[MAX_DH / 32];
+    float acc[NV];
 #pragma unroll
-    for (int i = 0; i < MAX_DH / 32; ++i) acc[i] = 0.f;
+    for (int i = 0; i < NV; ++i) acc[i] = 0.f;
     for (int base = lo; base <= pos; base += 32) {
         const int j = base + lane;
         const bool valid = j <= pos;
         float s = -INFINITY;
+        unsigned long long vrow = 0;                   // where the values of this lane's key lie
         if (valid) {
-            const int page = bt[j / page_size];
-            const TT* krow = kc + (size_t)page * page_stride + head_off + (size_t)(j % page_size) * dh;
+            const int page = bt[j / page_size], at = j % page_size;
+            vrow = (size_t)page * v_page_stride + v_head_off + (size_t)at * dv;
+            const TT* krow = kc + (size_t)page * page_stride + head_off + (size_t)at * dh;
             float dot = 0.f;
-            for (int d = 0; d < dh; ++d) dot = fmaf(qs[warp][d], bl_load(krow + d), dot);
+            if constexpr (VEC) {
+#pragma unroll 8
+                for (int d = 0; d < dh; d += 4) {
+                    const float4 a = *reinterpret_cast<const float4*>(&qs[warp][d]), b = *reinterpret_cast<const float4*>(krow + d);
+                    dot = fmaf(a.x, b.x, dot); dot = fmaf(a.y, b.y, dot); dot = fmaf(a.z, b.z, dot); dot = fmaf(a.w, b.w, dot);
+                }
+            } else {
+                for (int d = 0; d < dh; ++d) dot = fmaf(qs[warp][d], bl_load(krow + d), dot);
+            }
             s = dot * scale;
             if (softcap > 0.f) s = softcap * tanhf(s / softcap);
         }
@@ -60,17 +72,23 @@ attention_plain_kernel(const TT* __restrict__ q, const TT* __restrict__ kc, cons
         const float alpha = expf(m - m_new);           // first chunk: exp(-inf) = 0
         l = l * alpha + bl_warp_sum(p);
 #pragma unroll
-        for (int i = 0; i < MAX_DH / 32; ++i) acc[i] *= alpha;
+        for (int i = 0; i < NV; ++i) acc[i] *= alpha;
         const int n = min(32, pos - base + 1);
-        for (int jj = 0; jj < n; ++jj) {
-            const float pj = __shfl_sync(0xffffffffu, p, jj);
-            const int key = base + jj;
-            const int page = bt[key / page_size];
-            const TT* vrow = vc + (size_t)page * v_page_stride + v_head_off + (size_t)(key % page_size) * dv;
+        for (int j0 = 0; j0 < n; j0 += 8) {            // eight keys' values in flight, added in ascending position
+            float v[8][NV];
 #pragma unroll
-            for (int i = 0; i < MAX_DH / 32; ++i) {
-                const int d = lane + 32 * i;
-                if (d < dv) acc[i] = fmaf(pj, bl_load(vrow + d), acc[i]);
+            for (int u = 0; u < 8; ++u) {
+                const unsigned long long row = __shfl_sync(0xffffffffu, vrow, j0 + u);
+#pragma unroll
+                for (int i = 0; i < NV; ++i)
+                    if (j0 + u < n && lane + 32 * i < dv) v[u][i] = bl_load(vc + row + lane + 32 * i);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const float pj = __shfl_sync(0xffffffffu, p, j0 + u);
+#pragma unroll
+                for (int i = 0; i < NV; ++i)
+                    if (j0 + u < n && lane + 32 * i < dv) acc[i] = fmaf(pj, v[u][i], acc[i]);
             }
         }
         m = m_new;
@@ -81,14 +99,14 @@ attention_plain_kernel(const TT* __restrict__ q, const TT* __restrict__ kc, cons
         const float alpha = expf(m - m_new);
         l = l * alpha + expf(sk - m_new);
 #pragma unroll
-        for (int i = 0; i < MAX_DH / 32; ++i) acc[i] *= alpha;
+        for (int i = 0; i < NV; ++i) acc[i] *= alpha;
     }
     TT* orow = out + ((size_t)t * H + h) * dv;
     float inv = l > 0.f ? 1.0f / l : 0.f;
     if (gate && gate_dim == 0) inv *= bl_sigmoid(gate[(size_t)t * ld_gate + h]);
     const float* crow = gate && gate_dim ? gate + (size_t)t * ld_gate + (size_t)h * gate_dim : nullptr;
 #pragma unroll
-    for (int i = 0; i < MAX_DH / 32; ++i) {
+    for (int i = 0; i < NV; ++i) {
         const int d = lane + 32 * i;
         if (d < dv) bl_store(orow + d, crow ? acc[i] * inv * bl_sigmoid(crow[d]) : acc[i] * inv);
     }
@@ -128,16 +146,18 @@ extern "C" int bl_attention_plain_cap(const void* q, const void* k_cache, const 
     if (page_size <= 0 || max_pages <= 0 || window < 0) BL_FAIL("bl_attention_plain: bad page size, table width or window");
     cudaStream_t s = (cudaStream_t)stream;
     const int blocks = (T * H + WARPS - 1) / WARPS;
-    if (dtype == BL_F32)
-        attention_plain_kernel<float><<<blocks, WARPS * 32, 0, s>>>((const float*)q, (const float*)k_cache,
-            (const float*)v_cache, tok_req, cu_q, ctx_len, block_table, max_pages, (float*)out, T, H, KV, dh, dv,
-            page_size, window, scale, sinks, sink_dtype, gate, ld_gate, gate_dim, softcap);
-    else if (dtype == BL_BF16)
-        attention_plain_kernel<__nv_bfloat16><<<blocks, WARPS * 32, 0, s>>>((const __nv_bfloat16*)q,
-            (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, tok_req, cu_q, ctx_len, block_table,
-            max_pages, (__nv_bfloat16*)out, T, H, KV, dh, dv, page_size, window, scale, sinks, sink_dtype, gate, ld_gate, gate_dim, softcap);
+    const bool vec = dtype == BL_F32 && dh % 4 == 0 && ((uintptr_t)k_cache & 15) == 0;
+#define BL_GO(TT, VEC, NV) attention_plain_kernel<TT, VEC, NV><<<blocks, WARPS * 32, 0, s>>>((const TT*)q, (const TT*)k_cache, \
+            (const TT*)v_cache, tok_req, cu_q, ctx_len, block_table, max_pages, (TT*)out, T, H, KV, dh, dv, \
+            page_size, window, scale, sinks, sink_dtype, gate, ld_gate, gate_dim, softcap)
+#define BL_GO_NV(TT, VEC) do { if (dv <= 64) BL_GO(TT, VEC, 2); else if (dv <= 128) BL_GO(TT, VEC, 4); else BL_GO(TT, VEC, 8); } while (0)
+    if (dtype == BL_F32 && vec) BL_GO_NV(float, true);
+    else if (dtype == BL_F32) BL_GO_NV(float, false);
+    else if (dtype == BL_BF16) BL_GO_NV(__nv_bfloat16, false);
     else
         BL_FAIL("bl_attention_plain: unknown dtype %d", dtype);
+#undef BL_GO_NV
+#undef BL_GO
     BL_CHECK_LAUNCH("bl_attention_plain");
     return 0;
 }
