@@ -204,11 +204,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     volatile int* give_up = reinterpret_cast<volatile int*>(smem + OFF_BARS + 112);
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + OFF_BARS + 120);
     float* xch = reinterpret_cast<float*>(smem + OFF_XCH);               // [2 groups][maximum, sum][128 rows]
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     constexpr int ROW_WARPS = GROUPS * ROWS / 32;                        // one thread per row in each group
     // after the row warps: the issuer of the first product (it also owns the tensor memory), two copy warps, the
-    // issuer of the second product. One thread issuing both was the kernel's bottleneck: twelve MMAs, two commits and
-    // three waits a key block took it 1,800 cycles, as long as a group of row warps needs for the block's softmax.
+    // issuer of the second product: twelve MMAs, two commits and three waits a key block are too much for one thread
+    // beside a group of row warps' softmax of the block.
     const bool issuer = warp == ROW_WARPS, issuer_pv = warp == ROW_WARPS + 3;
 
     // Blocks start in the order of their index: all heads of the list's last tile, then all heads of the tile before.
@@ -238,9 +238,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         for (int i = 0; i < GROUPS; ++i) mbar_init(o_final0 + 8 * i, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // q, the newest keys and values, the output buffer and the tensor memory of the SM belong to the kernels before
-    // this one until here; the block's preamble above may run while they finish
-    bl_pdl_wait();
+    // Tensor memory is taken before the wait for the kernel before: whoever on this stream uses it triggers its successor
+    // only behind its own allocation, so an allocation that has to wait here waits for a block that needs nothing from us.
     if (issuer) {
         __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -251,15 +250,17 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    // q, the newest keys and values and the output buffer belong to the kernels before this one until here; the block's
+    // preamble above may run while they finish
+    bl_pdl_wait();
     bl_pdl_trigger();                                                    // the next kernel may start its own preamble (it waits before it touches data)
     // tensor memory: scores of block i in columns 128 (i % 3) .., its P over the upper 64 of them, its share of the
     // output in columns 384 + 64 (i & 1) .. (head size 128: 384 ..)
     bool ok = !*give_up;
 
     if (warp == ROW_WARPS + 1 || warp == ROW_WARPS + 2) {
-        // ================= two warps: the copies of the keys (and q) and of the values, a page per lane 0..7.
-        // Issuing a box costs its lane about 0.1 us, one lane after the other: two warps keep the sixteen boxes of a
-        // block off the path of the MMAs.
+        // ================= two warps: the copies of the keys (and q) and of the values; lanes 0..7 look up a page each,
+        // one thread issues the boxes.
         const bool keys = warp == ROW_WARPS + 1;
         const CUtensorMap* map = keys ? &map_k : &map_v;
         const uint32_t full0 = keys ? full_k0 : full_v0, off = keys ? OFF_K : OFF_V;
@@ -270,7 +271,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         };
         int loads[2] = {0, 0};                                           // copies started per stage
         ok = __all_sync(0xffffffffu, ok);
-        if (ok && keys && lane == 0 && nb > 0) {                         // (a tile without rows copies nothing and waits for nothing)
+        if (ok && keys && nb > 0 && elect_one()) {                         // (a tile without rows copies nothing and waits for nothing)
             mbar_expect_tx(full_q, Q_BYTES);
 #pragma unroll
             for (int a = 0; a < ATOMS; ++a)
@@ -289,14 +290,18 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             }
             const uint32_t bar = full0 + 8 * st, dst = base + off + st * KV_BYTES;
             const unsigned have = __ballot_sync(0xffffffffu, lane < PAGES && page >= 0);
-            if (lane == 0) {
-                if (have) mbar_expect_tx(bar, (uint32_t)__popc(have) * PAGE_BYTES); else mbar_arrive(bar);
-            }
-            __syncwarp();
-            if (lane < PAGES && page >= 0) {
+            int pages[PAGES];
 #pragma unroll
-                for (int a = 0; a < ATOMS; ++a)                         // 16 keys x 64 dimensions a box
-                    tma_load_2d(dst + a * ATOM_BYTES + lane * (PAGE * 128), map, bar, a * 64, (page * p.KV + kvh) * PAGE);
+            for (int pg = 0; pg < PAGES; ++pg) pages[pg] = __shfl_sync(0xffffffffu, page, pg);
+            if (elect_one()) {
+                if (have) mbar_expect_tx(bar, (uint32_t)__popc(have) * PAGE_BYTES); else mbar_arrive(bar);
+#pragma unroll
+                for (int pg = 0; pg < PAGES; ++pg) {
+                    if (pages[pg] < 0) continue;
+#pragma unroll
+                    for (int a = 0; a < ATOMS; ++a)                     // 16 keys x 64 dimensions a box
+                        tma_load_2d(dst + a * ATOM_BYTES + pg * (PAGE * 128), map, bar, a * 64, (pages[pg] * p.KV + kvh) * PAGE);
+                }
             }
             __syncwarp();
             ++loads[st];
@@ -309,7 +314,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 if (loads[s2] > 0) mbar_wait_plain(full0 + 8 * s2, (uint32_t)((loads[s2] - 1) & 1));
         }
     } else if (issuer) {
-        // ================= one warp: lane 0 issues the MMAs
+        // ================= one warp: one thread issues the MMAs
         auto issue_s = [&](int i) {                                      // S = Q . K^T of the i-th block of this tile
 #pragma unroll
             for (int at = 0; at < ATOMS; ++at) {                         // 64 dimensions of the head an atom, 16 a step
@@ -320,7 +325,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             }
             umma_commit(s_done0 + 8 * (i % SBUFS));
         };
-        if (lane == 0 && ok && nb > 0) {
+        if (ok && nb > 0 && elect_one()) {
             ok = mbar_wait<true>(full_q, 0, give_up, 1) && mbar_wait<true>(full_k0, 0, give_up, 2);
             if (ok) { fence_after_sync(); issue_s(0); }
             if (ok && nb > 1) {
@@ -342,9 +347,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
         __syncwarp();
     } else if (issuer_pv) {
-        // ================= one warp: lane 0 issues O_i = P . V once the group has written P of block i (and has taken
+        // ================= one warp: one thread issues O_i = P . V once the group has written P of block i (and has taken
         // the share of its block before out of the columns that this one goes to)
-        if (lane == 0 && ok) {
+        if (ok && elect_one()) {
             for (int i = 0; ok && i < nb; ++i) {
                 const int st = i & 1, buf = i % SBUFS;
                 ok = mbar_wait(full_v0 + 8 * st, (uint32_t)((i >> 1) & 1), give_up, 5) &&       // copied long before P is there

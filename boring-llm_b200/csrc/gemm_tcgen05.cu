@@ -66,7 +66,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     volatile int* give_up = reinterpret_cast<volatile int*>(aligned + STAGES * STAGE_BYTES + 128);
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(aligned + STAGES * STAGE_BYTES + 136);
     const uint32_t full0 = bars, empty0 = bars + 8 * STAGES, accum = bars + 16 * STAGES;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int n_tile = blockIdx.x, m0 = blockIdx.y * BM;
     const int n0 = n_tile * (GLU ? BN / 2 : BN);                              // first output column of the tile
     const int kblocks = (K + BK - 1) / BK;
@@ -92,33 +92,41 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             tma_load_2d(b_dst, &map_b, full0 + 8 * s, kb * BK, w_row0 + n0);
         }
     };
-    int early = 0;
-    if (tile_expert == nullptr && warp == 0 && lane == 0) {                     // (which matrix a grouped tile reads is the predecessor's result)
-        for (; early < STAGES && early < kblocks; ++early) {
-            mbar_expect_tx(full0 + 8 * early, STAGE_BYTES);
-            load_w(early, early);
+    // Tensor memory, too, is taken before the wait: whoever on this stream uses it triggers its successor only behind its
+    // own allocation, so an allocation that has to wait here waits for a block that needs nothing from this one.
+    auto take_tmem = [&]() {
+        if (warp == 0) {
+            __syncwarp();
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                         :: "r"(smem_u32((const void*)tmem_slot)), "r"(TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
+        fence_before_sync();
+        __syncthreads();
+        fence_after_sync();
+    };
+    const int early = tile_expert == nullptr ? min(STAGES, kblocks) : 0;        // (which matrix a grouped tile reads is the predecessor's result)
+    if (early > 0) {
+        if (warp == 0 && elect_one()) {
+            for (int j = 0; j < early; ++j) {
+                mbar_expect_tx(full0 + 8 * j, STAGE_BYTES);
+                load_w(j, j);
+            }
+        }
+        __syncwarp();
+        take_tmem();
     }
-    __syncwarp();
-    bl_pdl_wait();                                                              // x, out and the SM's tensor memory belong to the predecessor until here
+    bl_pdl_wait();                                                              // x and out belong to the predecessor until here
     if (tile_expert != nullptr) {
         const int e = tile_expert[blockIdx.y];
         if (e < 0) return;                                                      // the whole block: nothing allocated, no copy in flight
         w_row0 = e * expert_rows;
     }
-    if (warp == 0) {
-        __syncwarp();
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     :: "r"(smem_u32((const void*)tmem_slot)), "r"(TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    fence_before_sync();
-    __syncthreads();
-    fence_after_sync();
+    if (tile_expert != nullptr) take_tmem();
     const uint32_t tmem = *tmem_slot;
     bl_pdl_trigger();                                                           // the next kernel may start its preamble (it waits before it touches data)
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // loader: wait until the MMAs that read a stage are done, then refill it
         int issued = early;
         for (int kb = 0; kb < kblocks; ++kb) {
@@ -134,7 +142,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (*give_up)                                                           // let our own copies land before leaving
             for (int kb = max(0, issued - STAGES); kb < issued; ++kb)
                 mbar_wait(full0 + 8 * (kb % STAGES), (kb / STAGES) & 1, give_up, 0);
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         // issuer: four K = 16 MMAs per stage; the accumulator starts from zero at the first of them
         for (int kb = 0; kb < kblocks; ++kb) {
             const int s = kb % STAGES;

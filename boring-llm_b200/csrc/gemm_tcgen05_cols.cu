@@ -86,7 +86,7 @@ gemm_tc_cols_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                    acc_full0 = full_x + 8, acc_empty0 = acc_full0 + 16;
     volatile int* give_up = reinterpret_cast<volatile int*>(smem + bars_off + 16 * MAX_STAGES + 48);
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + bars_off + 16 * MAX_STAGES + 56);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int n_tiles = (N + BN - 1) / BN;
     const int my_tiles = blockIdx.x < n_tiles ? (n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
     const int total = my_tiles * kblocks;                                     // k blocks of W this block streams
@@ -101,18 +101,18 @@ gemm_tc_cols_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     }
     __syncthreads();
     // W does not depend on the kernel before this one: the first round of the ring is requested before the wait
-    int early = 0;
-    if (warp == 0 && lane == 0 && !*give_up) {
-        for (; early < stages && early < total; ++early) {
-            const int t = blockIdx.x + (early / kblocks) * gridDim.x, kb = early % kblocks;
-            mbar_expect_tx(full0 + 8 * early, W_BYTES);
-            tma_load_2d(ring + early * W_BYTES, &map_w, full0 + 8 * early, kb * BK, t * BN);
+    const int early = *give_up ? 0 : min(stages, total);
+    if (warp == 0 && early > 0 && elect_one()) {
+        for (int j = 0; j < early; ++j) {
+            const int t = blockIdx.x + (j / kblocks) * gridDim.x, kb = j % kblocks;
+            mbar_expect_tx(full0 + 8 * j, W_BYTES);
+            tma_load_2d(ring + j * W_BYTES, &map_w, full0 + 8 * j, kb * BK, t * BN);
         }
     }
     __syncwarp();
-    bl_pdl_wait();                                                            // x, out and the SM's tensor memory belong to the predecessor until here
+    // Tensor memory, too, is taken before the wait: whoever on this stream uses it triggers its successor only behind its
+    // own allocation, so an allocation that has to wait here waits for a block that needs nothing from this one.
     if (warp == 1) {
-        __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      :: "r"(smem_u32((const void*)tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -121,10 +121,11 @@ gemm_tc_cols_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    bl_pdl_wait();                                                            // x and out belong to the predecessor until here
     bl_pdl_trigger();
 
     if (warp == 0) {
-        if (lane == 0 && !*give_up) {
+        if (!*give_up && elect_one()) {
             // x: every k block as its own swizzled tile (rows past M arrive as zeros)
             mbar_expect_tx(full_x, (uint32_t)x_bytes);
             for (int kb = 0; kb < kblocks; ++kb) tma_load_2d(base + kb * X_TILE, &map_x, full_x, kb * BK, 0);
@@ -144,7 +145,7 @@ gemm_tc_cols_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && !*give_up && my_tiles > 0) {
+        if (!*give_up && my_tiles > 0 && elect_one()) {
             bool ok = mbar_wait(full_x, 0, give_up, 2);
             int it = 0;
             for (int local = 0; ok && local < my_tiles; ++local) {

@@ -133,7 +133,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     volatile int* give_up = reinterpret_cast<volatile int*>(aligned + RING_BYTES + STAGING_BYTES + 192);
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(aligned + RING_BYTES + STAGING_BYTES + 200);
     const uint32_t full0 = bars, empty0 = bars + 8 * MAX_STAGES, acc_full0 = bars + 16 * MAX_STAGES, acc_empty0 = acc_full0 + 16;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const bool leader = rank == 0;
@@ -147,39 +147,38 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         for (int b = 0; b < 2; ++b) { mbar_init(acc_full0 + 8 * b, 1); mbar_init(acc_empty0 + 8 * b, 2 * EPI_WARPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    __syncthreads();
-    cluster_sync();                                                  // both blocks' barriers exist before anyone signals them
-    // W does not depend on the kernel before this one: the loader starts this block's half of W for the first ring of
-    // k blocks before the dependent-launch wait, so that those copies (the first touch of this layer's weights) run
-    // while the predecessor finishes. The stage's barrier expects the bytes of x and W together; x follows after the wait.
-    int early = 0;                                                   // loader: k blocks whose W is already on its way
-    if (warp == 0 && lane == 0 && pair < total_tiles) {
-        const int n0 = (pair / m_pairs) * COLS;
-        const int w_row0 = GLU ? (int)rank * N + n0 : n0 + (int)rank * (BN / 2);
-        for (; early < STAGES && early < kblocks; ++early) {
-            if (leader) mbar_expect_tx(full0 + 8 * early, 2 * STAGE_BYTES);   // the bytes of both blocks
-#pragma unroll
-            for (int u = 0; u < KS; ++u)
-                tma_load_2d_pair(base + early * STAGE_BYTES + KS * A_BYTES + u * B_BYTES, &map_b, full0 + 8 * early, (early * KS + u) * BK, w_row0);
-        }
-    }
-    __syncwarp();
-    bl_pdl_wait();                                                   // x, the residual stream and tensor memory belong to the predecessor until here
+    // Tensor memory is taken before the wait for the kernel before: whoever on this stream uses it triggers its successor
+    // only behind its own allocation, so an allocation that has to wait here waits for a block that needs nothing from us.
     if (warp == 0) {
-        __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
                      :: "r"(smem_u32((const void*)tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     fence_before_sync();
     __syncthreads();
-    cluster_sync();                                                  // both blocks hold their tensor memory before the leader writes into it
+    cluster_sync();                                                  // both blocks' barriers and tensor memory exist before anyone uses them
     fence_after_sync();
+    // W does not depend on the kernel before this one: the loader starts this block's half of W for the first ring of
+    // k blocks before the dependent-launch wait, so that those copies (the first touch of this layer's weights) run
+    // while the predecessor finishes. The stage's barrier expects the bytes of x and W together; x follows after the wait.
+    const int early = min(STAGES, kblocks);                          // loader: steps whose W is already on its way
+    if (warp == 0 && pair < total_tiles && elect_one()) {
+        const int n0 = (pair / m_pairs) * COLS;
+        const int w_row0 = GLU ? (int)rank * N + n0 : n0 + (int)rank * (BN / 2);
+        for (int j = 0; j < early; ++j) {
+            if (leader) mbar_expect_tx(full0 + 8 * j, 2 * STAGE_BYTES);   // the bytes of both blocks
+#pragma unroll
+            for (int u = 0; u < KS; ++u)
+                tma_load_2d_pair(base + j * STAGE_BYTES + KS * A_BYTES + u * B_BYTES, &map_b, full0 + 8 * j, (j * KS + u) * BK, w_row0);
+        }
+    }
+    __syncwarp();
     const uint32_t tmem = *tmem_slot;
+    bl_pdl_wait();                                                   // x and the residual stream belong to the predecessor until here
     bl_pdl_trigger();                                                // the next kernel may start its own preamble (it waits before it touches data)
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int it = 0;                                              // k blocks loaded so far, over all tiles
             for (int t = pair; t < total_tiles && !*give_up; t += n_pairs) {
                 const int m0 = ((t % m_pairs) * 2 + (int)rank) * BM;
@@ -201,7 +200,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
         }
     } else if (warp == 1) {
-        if (leader && lane == 0) {
+        if (leader && elect_one()) {
             int it = 0, local = 0;
             for (int t = pair; t < total_tiles && !*give_up; t += n_pairs, ++local) {
                 const int buf = local & 1;
@@ -510,7 +509,7 @@ int launch_bn(const void* x, const void* w, const void* bias, int bias_dtype, vo
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    // The block waits (griddepcontrol.wait) before it allocates tensor memory or touches x and out, so it may be
+    // The block waits (griddepcontrol.wait) before it touches x and out, so it may be
     // launched while its predecessor still runs: its preamble and the first copies of W overlap the predecessor's tail.
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = bl_pdl_enabled() ? 1 : 0;

@@ -11,8 +11,8 @@
 // the epilogue (bias, residual add into the 32-bit stream, or SwiGLU over a tile whose first BN/2 columns are gate
 // rows of W and last BN/2 the matching up rows) and writes its band. The partial sums never touch global memory.
 //
-// The kernel takes part in programmatic dependent launch: barriers and the first ring of W before the wait, tensor
-// memory, x and out after it. Every wait on an mbarrier is bounded: when a bound runs out the block records a code
+// The kernel takes part in programmatic dependent launch: barriers, tensor memory and the first ring of W before the wait,
+// x and out after it. Every wait on an mbarrier is bounded: when a bound runs out the block records a code
 // in a status word and stops computing, but still meets its cluster at both cluster barriers (they are hardware
 // barriers: every block of the cluster arrives), frees its tensor memory and returns; bl_gemm_tc_splitk_status()
 // reports it on the host and the launch's results are invalid.
@@ -80,7 +80,7 @@ gemm_tc_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     volatile int* give_up = reinterpret_cast<volatile int*>(aligned + RING_BYTES + 192);
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(aligned + RING_BYTES + 200);
     const uint32_t full0 = bars, empty0 = bars + 8 * MAX_STAGES, accum = bars + 16 * MAX_STAGES;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     uint32_t rank, split;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(split));
@@ -108,17 +108,17 @@ gemm_tc_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             tma_load_2d(b_dst, &map_b, full0 + 8 * s, kb * BK, n0);
         }
     };
-    int early = 0;
-    if (warp == 0 && lane == 0) {
-        for (; early < STAGES && early < nkb; ++early) {
-            mbar_expect_tx(full0 + 8 * early, STAGE_BYTES);
-            load_w(early, kb0 + early);
+    const int early = min(STAGES, nkb);
+    if (warp == 0 && elect_one()) {
+        for (int j = 0; j < early; ++j) {
+            mbar_expect_tx(full0 + 8 * j, STAGE_BYTES);
+            load_w(j, kb0 + j);
         }
     }
     __syncwarp();
-    bl_pdl_wait();                                                              // x, out and the SM's tensor memory belong to the predecessor until here
+    // Tensor memory, too, is taken before the wait: whoever on this stream uses it triggers its successor only behind its
+    // own allocation, so an allocation that has to wait here waits for a block that needs nothing from this one.
     if (warp == 0) {
-        __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      :: "r"(smem_u32((const void*)tmem_slot)), "r"(BN) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -127,9 +127,10 @@ gemm_tc_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    bl_pdl_wait();                                                              // x and out belong to the predecessor until here
     bl_pdl_trigger();                                                           // the next kernel may start its preamble (it waits before it touches data)
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // loader: wait until the MMAs that read a stage are done, then refill it
         int issued = early;
         for (int j = 0; j < nkb; ++j) {
@@ -145,7 +146,7 @@ gemm_tc_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         if (*give_up)                                                           // let our own copies land before the ring is reused
             for (int j = max(0, issued - STAGES); j < issued; ++j)
                 mbar_wait(full0 + 8 * (j % STAGES), (j / STAGES) & 1, give_up, 0);
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         // issuer: four K = 16 MMAs per stage; the accumulator starts from zero at the first of them
         for (int j = 0; j < nkb; ++j) {
             const int s = j % STAGES;
@@ -321,7 +322,7 @@ int launch(const void* x, const void* w, const void* bias, int bias_dtype, void*
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    // a block waits (griddepcontrol.wait) before it allocates tensor memory or touches x and out, so it may be launched
+    // a block waits (griddepcontrol.wait) before it touches x and out, so it may be launched
     // while its predecessor still runs
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = bl_pdl_enabled() ? 1 : 0;
