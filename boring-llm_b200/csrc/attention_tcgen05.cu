@@ -655,7 +655,7 @@ int launch(const void* q, const void* k_cache, const void* v_cache, const Params
         BL_CUDA(cudaFuncSetAttribute(attention_tc_kernel<S, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM_BYTES));
         configured = true;
     }
-    // A block waits (griddepcontrol.wait) before it allocates tensor memory or touches data, so it may be launched
+    // A block waits (griddepcontrol.wait) before it touches data, so it may be launched
     // while the kernel before it still runs.
     BL_CUDA(bl_launch_dependent(attention_tc_kernel<S, CAP>, dim3(n_tiles * p.H, 1, 1), dim3(S::THREADS), (size_t)S::SMEM_BYTES, stream,
                                 mq, mk, mv, p));

@@ -268,7 +268,7 @@ int launch_stages(const CUtensorMap& a, const CUtensorMap& b, const void* bias, 
         BL_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<EPI, TO, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(STAGES)));
         configured = true;
     }
-    // a block waits (griddepcontrol.wait) before it allocates tensor memory or touches x and out, so it may be launched
+    // a block waits (griddepcontrol.wait) before it touches x and out, so it may be launched
     // while its predecessor still runs
     BL_CUDA(bl_launch_dependent(gemm_tc_kernel<EPI, TO, STAGES>, grid, dim3(128), (size_t)smem_bytes(STAGES), s, a, b, bias, bias_dtype, (TO*)out, M, N, K,
                                 tile_expert, expert_rows));

@@ -55,8 +55,8 @@ constexpr uint32_t PEER_BIT_MASK = 0xFEFFFFFFu;      // clears the bit that sele
 
 __device__ int g_status2 = 0;
 
-// An epilogue of this file only: the joined q/k/v product of an attention layer, finished in place. A tile of 128
-// columns is whole heads (head size 64 or 128); the accumulator gets its bias, q and k heads are rotated by the
+// An epilogue of this file only: the joined q/k/v product of an attention layer, finished in place. A tile's columns
+// are whole heads (head size 64 or 128); the accumulator gets its bias, q and k heads are rotated by the
 // token's position (pairs j, j + head size / 2; cos and sin from the step's table), and the bfloat16 results go
 // where the attention kernels read them: q rows, and the key and value pages of the token's request.
 constexpr int EPI_QKV_ROPE = 100;
@@ -263,13 +263,17 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 }
             };
             if (EPI == EPI_QKV_ROPE) {
-                // This lane's row of the accumulator is one token. The tile's 128 columns are 128 / dh heads; an item is
-                // 32 columns of a head's first half with the 32 that turn with them (dh / 2 further on); the two warps
-                // of a quarter take an item each. Everything that does not depend on the product (where the row goes,
-                // its cosines and sines, the bias) is asked for before the accumulator is waited for.
+                // This lane's row of the accumulator is one token. The tile's columns are whole heads; an item is 32 columns
+                // of a head's first half with the 32 that turn with them (dh / 2 further on); the two warps of a quarter
+                // take items in turn. Everything that does not depend on the product (where the row goes, its cosines and
+                // sines, the bias) is asked for before the accumulator is waited for.
                 const int dh = qo.dh, half_cols = dh >> 1;
                 const int m = m0 + quarter * 32 + lane;
-                const int c_lo = dh == 64 ? 2 * half : half, c_hi = c_lo + (dh >> 6);     // 32-column chunks of the tile
+                bool landed = true;
+#pragma unroll 1
+                for (int turn_no = 0; turn_no < BN / 128; ++turn_no) {
+                const int item = half + 2 * turn_no;
+                const int c_lo = dh == 64 ? 2 * item : 4 * (item >> 1) + (item & 1), c_hi = c_lo + (dh >> 6);   // 32-column chunks of the tile
                 const int n_lo = n0 + c_lo * 32;                                          // first column of the item's low half
                 const int head = n_lo / dh;                                               // q heads, then k heads, then v heads
                 const int j0 = n_lo % dh;                                                 // first pair of the item (0, or 32 for dh 128)
@@ -310,8 +314,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     bh4[i] = b16 ? reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(bias) + n_lo + half_cols)[i] : make_uint4(0u, 0u, 0u, 0u);
                 }
                 const bool b32 = bias != nullptr && bias_dtype == BL_F32 && n_lo < N;
-                if (!mbar_wait(acc_full0 + 8 * buf, (local / 2) & 1, give_up, 3)) break;
-                fence_after_sync();
+                if (turn_no == 0) {
+                    landed = mbar_wait(acc_full0 + 8 * buf, (local / 2) & 1, give_up, 3);
+                    if (!landed) break;
+                    fence_after_sync();
+                }
                 const uint32_t lane_addr = tmem + buf * 256 + ((uint32_t)(quarter * 32) << 16);
                 uint32_t lo[32], hi[32];
                 tmem_ld32(lane_addr + c_lo * 32, lo);
@@ -361,6 +368,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     *reinterpret_cast<uint4*>(dst) = v;
                 }
                 __syncwarp();
+                }
+                if (!landed) break;
                 fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive_leader(acc_empty0 + 8 * buf);
@@ -477,7 +486,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     __syncwarp();
     fence_before_sync();
     __syncthreads();
-    cluster_sync();                                                  // neither block leaves while the other may still read its memory
+    // neither block leaves while the other's MMAs may still read its memory (they are done: the epilogue has seen them;
+    // nothing is published here, so this barrier does not wait for the stores on their way)
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (warp == 0) {
         fence_after_sync();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(TMEM_COLS) : "memory");
@@ -529,15 +540,22 @@ int sm_count() {
     return n;
 }
 
-// 256-column tiles unless they would leave SM pairs without a tile while 128-column tiles would not.
+// Columns of a tile: 256, or 128 where that is over sooner. A launch takes rounds of one tile a pair, and a round of 128-wide
+// tiles takes two thirds of a round of 256-wide ones (376 cycles a k block against 560: half the arithmetic, three quarters of
+// the bytes). 2,048 rows of 896 columns are one round either way; of 2,048 columns two rounds of 128 or one of 256 (K 11,008:
+// 2,001 rows 87 us against 68).
+int tile_columns(int M, int N, bool glu) {
+    const int pairs = sm_count() / 2, m_pairs = (M + 2 * BM - 1) / (2 * BM);
+    auto rounds = [&](int cols) { return ((long long)m_pairs * ((N + cols - 1) / cols) + pairs - 1) / pairs; };
+    const int cols = glu ? 128 : 256;
+    return 2 * rounds(cols / 2) < 3 * rounds(cols) ? 128 : 256;
+}
+
 template <int EPI, typename TO>
 int launch(const void* x, const void* w, const void* bias, int bias_dtype, void* out, int M, int N, int K, cudaStream_t s,
            const NormLink& nl = NormLink()) {
     const int sms = sm_count();
-    const int cols256 = EPI == BL_EPI_SWIGLU ? 128 : 256;
-    const int m_pairs = (M + 2 * BM - 1) / (2 * BM);
-    const int tiles256 = m_pairs * ((N + cols256 - 1) / cols256);
-    if (tiles256 < sms / 2) return launch_bn<EPI, TO, 128>(x, w, bias, bias_dtype, out, M, N, K, sms, s, QkvOut(), nl);
+    if (tile_columns(M, N, EPI == BL_EPI_SWIGLU) == 128) return launch_bn<EPI, TO, 128>(x, w, bias, bias_dtype, out, M, N, K, sms, s, QkvOut(), nl);
     return launch_bn<EPI, TO, 256>(x, w, bias, bias_dtype, out, M, N, K, sms, s, QkvOut(), nl);
 }
 
@@ -575,9 +593,7 @@ extern "C" int bl_gemm_tc_pair(const void* x, const void* w, const void* bias, i
 
 // Values per row that bl_gemm_tc_pair_residual_norm writes into `ss` for these sizes (two per tile of columns).
 extern "C" int bl_gemm_tc_pair_norm_parts(int M, int N) {
-    const int sms = sm_count();
-    const int m_pairs = (M + 2 * BM - 1) / (2 * BM);
-    const int cols = m_pairs * ((N + 255) / 256) < sms / 2 ? 128 : 256;
+    const int cols = tile_columns(M, N, false);
     return 2 * ((N + cols - 1) / cols);
 }
 
@@ -638,7 +654,10 @@ extern "C" int bl_gemm_tc_pair_qkv_rope(const void* x, const void* w, const void
     qo.H = H; qo.KV = KV; qo.dh = dh;
     NormLink nl = NormLink();                     // x may be rows whose norm is pending (ss != null): see bl_gemm_tc_pair_residual_norm
     if (ss != nullptr) { nl.ss_in = ss; nl.parts_in = parts; nl.inv_dim = inv_dim; nl.eps = eps; }
-    return launch_bn<EPI_QKV_ROPE, __nv_bfloat16, 128>(x, w, bias, bias_dtype, nullptr, M, (H + 2 * KV) * dh, K, sm_count(), (cudaStream_t)stream, qo, nl);
+    const int N = (H + 2 * KV) * dh;
+    if (tile_columns(M, N, false) == 128)
+        return launch_bn<EPI_QKV_ROPE, __nv_bfloat16, 128>(x, w, bias, bias_dtype, nullptr, M, N, K, sm_count(), (cudaStream_t)stream, qo, nl);
+    return launch_bn<EPI_QKV_ROPE, __nv_bfloat16, 256>(x, w, bias, bias_dtype, nullptr, M, N, K, sm_count(), (cudaStream_t)stream, qo, nl);
 }
 
 extern "C" int bl_gemm_tc_pair_status(int* status) {

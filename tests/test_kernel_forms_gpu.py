@@ -1,0 +1,83 @@
+"""Forms of the kernels that only some sizes reach: each against the kernels it stands in for, or a 64-bit restatement."""
+import numpy as np
+import pytest
+import torch
+
+import plain_model as plain
+from test_kernels_gpu import close, data, ops, paged_setup
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+BF = torch.bfloat16
+
+
+@pytest.mark.parametrize("H,KV,dh", [(36, 2, 64), (16, 2, 128), (33, 3, 64), (17, 1, 128)])
+def test_qkv_rope_in_tiles_of_256_columns(H, KV, dh):
+    """2,001 rows of about 2,500 columns run in 256-wide tiles, whose epilogue takes two items of a head a warp (the last
+    tile of 33 + 6 or 17 + 2 heads overhangs the columns): q, keys and values against the kernels it replaces."""
+    o = ops()
+    page, d = 16, 72
+    ctx_lens, q_lens = [1400, 900, 301], [1000, 700, 301]
+    s = paged_setup(ctx_lens, q_lens, KV, dh, page, BF, 9)
+    s2 = paged_setup(ctx_lens, q_lens, KV, dh, page, BF, 9)
+    T = s["T"]
+    x = (data((T, d), 41) * 0.5).to(BF)
+    w = (data(((H + 2 * KV) * dh, d), 43) * 0.2).to(BF)
+    b = (data(((H + 2 * KV) * dh,), 44) * 0.5).to(BF)
+    j = np.arange(dh // 2, dtype=np.float32)
+    inv = torch.from_numpy(np.float32(1.0) / np.power(np.float32(1.0e4), (np.float32(2.0) * j) / np.float32(dh), dtype=np.float32)).to(DEV)
+    qkv = torch.empty(T, (H + 2 * KV) * dh, device=DEV)
+    o.gemm_plain(x, w, qkv, b, o.EPI_BIAS)
+    q_ref = torch.empty(T, H * dh, dtype=BF, device=DEV)
+    o.rope_kv_write(qkv, s["positions"], s["tok_req"], s["table"], inv, dh // 2, 1.0, q_ref, s["kc"], s["vc"], H, KV, dh, 0)
+    cs, sn = o.rope_table(s2["positions"], inv, dh // 2, 1.0)
+    q = torch.full((T, H * dh), float("nan"), dtype=BF, device=DEV)
+    o.qkv_rope_tc(x, w, b, s2["positions"], s2["tok_req"], s2["table"], cs, sn, q, s2["kc"], s2["vc"], H, KV, dh)
+    o.check_status()
+    close(q, q_ref.double(), BF, "q")
+    pos, req = torch.from_numpy(s["positions_np"]).long(), torch.from_numpy(s["tok_req_np"]).long()
+    pages = torch.from_numpy(s["table_np"]).long()[req, pos // page].to(DEV)
+    rows = (pos % page).to(DEV)
+    for name in ("kc", "vc"):
+        close(s2[name][pages, :, rows], s[name][pages, :, rows].double(), BF, name)
+
+
+@pytest.mark.parametrize("M,N", [(2001, 2048), (1793, 2052), (2304, 2304)])
+def test_residual_norm_in_tiles_of_256_columns(M, N):
+    """One round of 256-wide tiles where 128-wide ones would take two: the stream, the rows of the pending norm and their
+    sums of squares (one part per tile and half)."""
+    o = ops()
+    K = 72
+    x = (data((M, K), 51) * 0.5).to(BF)
+    w = (data((N, K), 52) * 0.2).to(BF)
+    stream = data((M, N), 53) * 2
+    nw = (data((N,), 54) * 0.25 + 1).to(BF)
+    want = stream.double().cpu() + x.double().cpu() @ w.double().cpu().T
+    out = stream.clone()
+    hw, ss = o.gemm_residual_norm(x, w, out, nw)
+    o.check_status()
+    assert ss.shape[1] == 2 * (-(-N // 256))
+    close(out, want, torch.float32, "stream")
+    close(hw, want * nw.double().cpu(), BF, "stream times weight")
+    close(ss.sum(dim=1), (want * want).sum(dim=1), torch.float32, "sums of squares")
+
+
+@pytest.mark.parametrize("d", [4, 508, 516, 1024, 1028, 2048, 2052, 4096])
+def test_layer_end_chain_at_the_widths_where_its_registers_change(d):
+    """The chain of norms at the edges of its forms, against the kernels it stands in for (bit for bit)."""
+    o = ops()
+    rows, n = 5, 3
+    streams = data((n + 1, rows, d), 61) * 2
+    sub, gate, gb = data((rows, d), 62), data((rows, d), 63), (data((d,), 64)).to(BF)
+    pw, pb, tw, tb = ((data((d,), 65 + i) * 0.25 + 1).to(BF) for i in range(4))
+    c = data((n,), 70)
+    ref = streams.clone()
+    o.gated_norm_residual(ref[n - 1], sub, gate, pw, pb, 1e-6, gb)
+    o.depth_mix(ref, c, n, ref[n])
+    y_ref = torch.empty(rows, d, dtype=BF, device=DEV)
+    o.layernorm(ref[n], tw, tb, 1e-5, y_ref)
+    y = torch.empty_like(y_ref)
+    o.norm_chain(streams[n - 1], sub, gate, gb, (pw, pb, 1e-6), streams=streams, coeffs=c, n=n, mix_out=streams[n],
+                 then=(tw, tb, 1e-5), y=y)
+    assert torch.equal(streams, ref) and torch.equal(y, y_ref)
