@@ -162,6 +162,10 @@ int bl_norm_qkv_rope(const float* x, const void* norm_w, int norm_w_dtype, float
                      const int* block_table, int max_pages, const float* inv_freq, float mscale,
                      void* q_out, void* k_cache, void* v_cache, int M, int K, int H, int KV, int dh,
                      int page_size, int pair_layout, void* stream);
+int bl_qkv_rope_normed(const void* normed, const void* w_qkv, const void* bias, int bias_dtype, const int* positions,
+                       const int* tok_req, const int* block_table, int max_pages, const float* inv_freq, float mscale,
+                       void* q_out, void* k_cache, void* v_cache, int M, int K, int H, int KV, int dh, int page_size,
+                       int pair_layout, void* stream);
 // Programmatic dependent launch for the small kernels of a step (on by default): 0 launches them the ordinary way.
 void bl_set_dependent_launch(int on);
 

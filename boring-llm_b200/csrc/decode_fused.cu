@@ -23,6 +23,7 @@ constexpr int WARPS = 8;
 constexpr int MODE_PLAIN = 0, MODE_SWIGLU = 1, MODE_QKV = 2;
 
 struct FusedParams {
+    const __nv_bfloat16* normed;      // rows that are normed already ([M, K]; null: x, and the norm is part of the kernel)
     const float* x; const int* row_idx; const void* norm_w; int norm_w_dtype; float eps;
     const __nv_bfloat16* w; const void* bias; int bias_dtype;
     void* out;                        // PLAIN: float [M, N]; SWIGLU: bfloat16 [M, N]; QKV: bfloat16 q [M, H * dh]
@@ -43,16 +44,21 @@ __device__ __forceinline__ uint4 ld16(const __nv_bfloat16* p, bool ok) {
     return ok ? __ldg(reinterpret_cast<const uint4*>(p)) : make_uint4(0u, 0u, 0u, 0u);
 }
 
-template <int MT, int MODE>
-__global__ void __launch_bounds__(WARPS * 32, MT == 1 ? (MODE == MODE_SWIGLU ? 3 : 2) : 1)
+// PRE: the rows come normed, from a norm kernel of its own: they are read as they are needed, from L2, and the block
+// keeps nothing of them in shared memory. For more than a few rows: there every block's norm of all its rows is longer
+// than its product, and the normed rows of a block leave an SM room for one block. 16 rows of 3,584 by
+// 4,608 columns 27.5 us with the norm inside, 17.8 with a norm of its own; 64 rows of 896 by 1,152 7.4 and 5.2.
+template <int MT, int MODE, bool PRE>
+__global__ void __launch_bounds__(WARPS * 32, PRE ? (MT <= 2 ? 2 : 1) : MT == 1 ? (MODE == MODE_SWIGLU ? 3 : 2) : 1)
 fused_norm_gemm_kernel(const FusedParams p) {
+    static_assert(!PRE || MODE == MODE_QKV, "only the q/k/v product takes normed rows");
     constexpr bool GLU = MODE == MODE_SWIGLU;
     constexpr int TOK = MT * 8;
-    constexpr int UNROLL = (GLU || MT > 2) ? 2 : 4;    // fewer registers where two matrices stream: three blocks fit an SM
+    constexpr int UNROLL = (GLU || MT > 2 || PRE) ? 2 : 4;    // fewer registers where two matrices stream: three blocks fit an SM
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int K = p.K, XROW = K + 8;
     __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(smem_raw);                       // [TOK][K + 8]
-    float* red = reinterpret_cast<float*>(smem_raw + (((size_t)TOK * XROW * 2 + 15) & ~(size_t)15));   // [GLU?2:1][WARPS][16][TOK + 1]
+    float* red = reinterpret_cast<float*>(smem_raw + (PRE ? 0 : (((size_t)TOK * XROW * 2 + 15) & ~(size_t)15)));   // [GLU?2:1][WARPS][16][TOK + 1]
     float* nws = red + (size_t)(GLU ? 2 : 1) * WARPS * 16 * (TOK + 1);                    // [K] norm weights, 32-bit
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int tile = blockIdx.x / p.m_groups;
@@ -76,6 +82,26 @@ fused_norm_gemm_kernel(const FusedParams p) {
     const __nv_bfloat16* u_hi = p.w + (size_t)(p.N + r_hi) * K;
 
     uint4 a_lo[UNROLL], a_hi[UNROLL], g_lo[GLU ? UNROLL : 1], g_hi[GLU ? UNROLL : 1];
+    uint4 a2_lo[PRE ? UNROLL : 1], a2_hi[PRE ? UNROLL : 1], b1[PRE ? UNROLL : 1][MT], b2[PRE ? UNROLL : 1][MT];    // PRE: two batches in flight
+    auto fetch_pre_w = [&](uint4 (&lo)[PRE ? UNROLL : 1], uint4 (&hi)[PRE ? UNROLL : 1], int kc0) {
+#pragma unroll
+        for (int u = 0; u < (PRE ? UNROLL : 1); ++u) {
+            const int k = kc0 + u * WARPS * 32 + 8 * t;
+            lo[u] = ld16(w_lo + k, lo_ok && k < K);
+            hi[u] = ld16(w_hi + k, hi_ok && k < K);
+        }
+    };
+    auto fetch_pre_x = [&](uint4 (&b)[PRE ? UNROLL : 1][MT], int kc0) {
+#pragma unroll
+        for (int u = 0; u < (PRE ? UNROLL : 1); ++u) {
+            const int k = kc0 + u * WARPS * 32 + 8 * t;
+#pragma unroll
+            for (int j = 0; j < MT; ++j) {
+                const int m = m0 + 8 * j + g;
+                b[u][j] = (m < p.M && k < K) ? *reinterpret_cast<const uint4*>(p.normed + (size_t)m * K + k) : make_uint4(0u, 0u, 0u, 0u);
+            }
+        }
+    };
     auto fetch = [&](int kc0) {
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u) {
@@ -99,7 +125,8 @@ fused_norm_gemm_kernel(const FusedParams p) {
     }
     // everything that no earlier kernel of the step writes is fetched before the wait: the norm's weights, and for
     // the q/k/v epilogue each thread's bias pair, position, page and rotation
-    for (int k = threadIdx.x; k < K; k += WARPS * 32) nws[k] = bl_load_any(p.norm_w, p.norm_w_dtype, k);
+    if (!PRE)
+        for (int k = threadIdx.x; k < K; k += WARPS * 32) nws[k] = bl_load_any(p.norm_w, p.norm_w_dtype, k);
     float e_b0 = 0.f, e_b1 = 0.f, e_cs = 1.f, e_sn = 0.f;
     int e_pos = 0, e_page = -1;
     if (MODE == MODE_QKV && threadIdx.x < 8 * TOK) {
@@ -117,8 +144,10 @@ fused_norm_gemm_kernel(const FusedParams p) {
                 e_page = p.block_table[(size_t)p.tok_req[m] * p.max_pages + e_pos / p.page_size];
         }
     }
+    if (PRE) fetch_pre_w(a2_lo, a2_hi, warp * 32 + UNROLL * WARPS * 32);
     bl_pdl_wait();                                     // from here on the residual stream may be read
 
+    if (!PRE) {
     __syncthreads();                                   // the norm weights are in shared memory
     // normalise this block's rows into shared memory: warp w takes rows w, w + 8, ...
     constexpr int NB = 8;                              // 16-byte words per lane that hold a row of up to 1,024 values
@@ -206,6 +235,7 @@ fused_norm_gemm_kernel(const FusedParams p) {
         }
     }
     __syncthreads();
+    }
 
     float acc[MT][4], acu[GLU ? MT : 1][4];
 #pragma unroll
@@ -213,6 +243,27 @@ fused_norm_gemm_kernel(const FusedParams p) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) { acc[j][i] = 0.f; if (GLU) acu[j][i] = 0.f; }
     // warp-uniform loop bounds: the MMA needs all 32 lanes
+    if constexpr (PRE) {
+        constexpr int STEP = UNROLL * WARPS * 32;
+        auto multiply = [&](uint4 (&lo)[UNROLL], uint4 (&hi)[UNROLL], uint4 (&b)[UNROLL][MT]) {
+#pragma unroll
+            for (int u = 0; u < UNROLL; ++u)
+#pragma unroll
+                for (int j = 0; j < MT; ++j) {
+                    mma_bf16(acc[j], lo[u].x, hi[u].x, lo[u].y, hi[u].y, b[u][j].x, b[u][j].y);
+                    mma_bf16(acc[j], lo[u].z, hi[u].z, lo[u].w, hi[u].w, b[u][j].z, b[u][j].w);
+                }
+        };
+        fetch_pre_x(b1, warp * 32);
+        fetch_pre_x(b2, warp * 32 + STEP);
+        for (int kc0 = warp * 32; kc0 < K; kc0 += 2 * STEP) {
+            multiply(a_lo, a_hi, b1);
+            if (kc0 + 2 * STEP < K) { fetch(kc0 + 2 * STEP); fetch_pre_x(b1, kc0 + 2 * STEP); }
+            if (kc0 + STEP >= K) break;
+            multiply(a2_lo, a2_hi, b2);
+            if (kc0 + 3 * STEP < K) { fetch_pre_w(a2_lo, a2_hi, kc0 + 3 * STEP); fetch_pre_x(b2, kc0 + 3 * STEP); }
+        }
+    } else
     for (int kc0 = warp * 32; kc0 < K; kc0 += UNROLL * WARPS * 32) {
         uint4 b[UNROLL][MT];
 #pragma unroll
@@ -295,28 +346,38 @@ fused_norm_gemm_kernel(const FusedParams p) {
     }
 }
 
-size_t smem_bytes(int mt, int K, bool glu) {
+size_t smem_bytes(int mt, int K, bool glu, bool pre = false) {
     const size_t tok = (size_t)mt * 8;
+    if (pre) return (size_t)WARPS * 16 * (tok + 1) * sizeof(float);
     const size_t xs = (tok * (K + 8) * 2 + 15) & ~(size_t)15;
     return xs + (glu ? 2 : 1) * (size_t)WARPS * 16 * (tok + 1) * sizeof(float) + (size_t)K * sizeof(float);
 }
 constexpr size_t SMEM_LIMIT = 200 * 1024;
 
-template <int MT, int MODE>
+template <int MT, int MODE, bool PRE = false>
 int launch(const FusedParams& p, int tiles, cudaStream_t s) {
     static size_t configured = 0;
-    const size_t bytes = smem_bytes(MT, p.K, MODE == MODE_SWIGLU);
+    const size_t bytes = smem_bytes(MT, p.K, MODE == MODE_SWIGLU, PRE);
     if (bytes > configured) {
-        BL_CUDA(cudaFuncSetAttribute(fused_norm_gemm_kernel<MT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT));
+        BL_CUDA(cudaFuncSetAttribute(fused_norm_gemm_kernel<MT, MODE, PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT));
         configured = SMEM_LIMIT;
     }
-    BL_CUDA(bl_launch_dependent(fused_norm_gemm_kernel<MT, MODE>, dim3(tiles * p.m_groups), dim3(WARPS * 32), bytes, s, p));
+    BL_CUDA(bl_launch_dependent(fused_norm_gemm_kernel<MT, MODE, PRE>, dim3(tiles * p.m_groups), dim3(WARPS * 32), bytes, s, p));
     BL_CHECK_LAUNCH("bl_norm_gemm");
     return 0;
 }
 
 template <int MODE>
 int dispatch(FusedParams& p, int tiles, cudaStream_t s) {
+    if constexpr (MODE == MODE_QKV) {
+        if (p.normed != nullptr) {
+            const int mt = p.M <= 8 ? 1 : p.M <= 16 ? 2 : 4;
+            p.m_groups = (p.M + mt * 8 - 1) / (mt * 8);
+            if (mt == 1) return launch<1, MODE, true>(p, tiles, s);
+            if (mt == 2) return launch<2, MODE, true>(p, tiles, s);
+            return launch<4, MODE, true>(p, tiles, s);
+        }
+    }
     // the largest row group whose normalised rows fit shared memory
     int mt = p.M <= 8 ? 1 : p.M <= 16 ? 2 : 4;
     while (mt > 1 && smem_bytes(mt, p.K, MODE == MODE_SWIGLU) > SMEM_LIMIT) mt /= 2;
@@ -365,22 +426,23 @@ extern "C" int bl_norm_gemm(const float* x, const int* row_idx, const void* norm
     return dispatch<MODE_PLAIN>(p, tiles, (cudaStream_t)stream);
 }
 
-// q, k, v = rmsnorm(x) . Wqkv^T (+ bias); q and k rotated by position; k, v written to the pages of each token's
-// request (k_cache / v_cache may be null: q only). Every dimension of a head rotates (n_rot = head size).
-extern "C" int bl_norm_qkv_rope(const float* x, const void* norm_w, int norm_w_dtype, float eps, const void* w_qkv,
-                                const void* bias, int bias_dtype, const int* positions, const int* tok_req,
-                                const int* block_table, int max_pages, const float* inv_freq, float mscale,
-                                void* q_out, void* k_cache, void* v_cache, int M, int K, int H, int KV, int dh,
-                                int page_size, int pair_layout, void* stream) {
+namespace {
+
+int qkv_rope(const void* normed, const float* x, const void* norm_w, int norm_w_dtype, float eps, const void* w_qkv,
+             const void* bias, int bias_dtype, const int* positions, const int* tok_req, const int* block_table, int max_pages,
+             const float* inv_freq, float mscale, void* q_out, void* k_cache, void* v_cache, int M, int K, int H, int KV, int dh,
+             int page_size, int pair_layout, void* stream) {
     if (M <= 0) return 0;
     if (pair_layout != BL_PAIRS_HALVES && pair_layout != BL_PAIRS_INTERLEAVED)
         BL_FAIL("bl_norm_qkv_rope: unknown pair layout %d (0: (j, j + head/2), 1: (2j, 2j + 1))", pair_layout);
     if (check_common("bl_norm_qkv_rope", x, w_qkv, M, K, norm_w_dtype)) return 1;
+    if ((uintptr_t)normed & 15) BL_FAIL("bl_norm_qkv_rope: the normed rows must be 16-byte aligned");
     if (H <= 0 || KV <= 0 || dh <= 0 || dh % 16 != 0) BL_FAIL("bl_norm_qkv_rope: head size %d must be a multiple of 16", dh);
     if (page_size <= 0 || max_pages <= 0) BL_FAIL("bl_norm_qkv_rope: bad page size or table width");
     if ((k_cache == nullptr) != (v_cache == nullptr)) BL_FAIL("bl_norm_qkv_rope: key and value cache must both be given or both be null");
     if (bias != nullptr && bias_dtype != BL_F32 && bias_dtype != BL_BF16) BL_FAIL("bl_norm_qkv_rope: unknown bias dtype %d", bias_dtype);
     FusedParams p = {};
+    p.normed = (const __nv_bfloat16*)normed;
     p.x = x; p.norm_w = norm_w; p.norm_w_dtype = norm_w_dtype; p.eps = eps; p.w = (const __nv_bfloat16*)w_qkv;
     p.bias = bias; p.bias_dtype = bias_dtype; p.out = q_out; p.M = M; p.N = (H + 2 * KV) * dh; p.K = K;
     p.positions = positions; p.tok_req = tok_req; p.block_table = block_table; p.max_pages = max_pages;
@@ -388,4 +450,27 @@ extern "C" int bl_norm_qkv_rope(const float* x, const void* norm_w, int norm_w_d
     p.H = H; p.KV = KV; p.dh = dh; p.page_size = page_size; p.pair_layout = pair_layout;
     const int heads = k_cache ? H + 2 * KV : H;
     return dispatch<MODE_QKV>(p, heads * (dh / 16), (cudaStream_t)stream);
+}
+
+}  // namespace
+
+// q, k, v = rmsnorm(x) . Wqkv^T (+ bias); q and k rotated by position; k, v written to the pages of each token's
+// request (k_cache / v_cache may be null: q only). Every dimension of a head rotates (n_rot = head size).
+extern "C" int bl_norm_qkv_rope(const float* x, const void* norm_w, int norm_w_dtype, float eps, const void* w_qkv,
+                                const void* bias, int bias_dtype, const int* positions, const int* tok_req,
+                                const int* block_table, int max_pages, const float* inv_freq, float mscale,
+                                void* q_out, void* k_cache, void* v_cache, int M, int K, int H, int KV, int dh,
+                                int page_size, int pair_layout, void* stream) {
+    return qkv_rope(nullptr, x, norm_w, norm_w_dtype, eps, w_qkv, bias, bias_dtype, positions, tok_req, block_table, max_pages,
+                    inv_freq, mscale, q_out, k_cache, v_cache, M, K, H, KV, dh, page_size, pair_layout, stream);
+}
+
+// The same of rows that are normed already (bfloat16 [M, K], 16-byte aligned).
+extern "C" int bl_qkv_rope_normed(const void* normed, const void* w_qkv, const void* bias, int bias_dtype, const int* positions,
+                                  const int* tok_req, const int* block_table, int max_pages, const float* inv_freq, float mscale,
+                                  void* q_out, void* k_cache, void* v_cache, int M, int K, int H, int KV, int dh,
+                                  int page_size, int pair_layout, void* stream) {
+    if (M > 0 && normed == nullptr) BL_FAIL("bl_qkv_rope_normed: no rows");
+    return qkv_rope(normed, nullptr, nullptr, BL_F32, 0.f, w_qkv, bias, bias_dtype, positions, tok_req, block_table, max_pages,
+                    inv_freq, mscale, q_out, k_cache, v_cache, M, K, H, KV, dh, page_size, pair_layout, stream);
 }

@@ -93,12 +93,13 @@ __global__ void rmsnorm_kernel(const float* x /* written by the kernel before: n
         bl_store(y + (size_t)r * d + i, x[src + i] * inv * bl_load_any(w, w_dtype, i));
 }
 
-// The same with one warp per row and 16-byte loads, for widths that are a multiple of 4: a row of up to 1,024
-// values stays in registers between the sum of squares and the scaling; nothing is shared between warps, so
-// there is no barrier. A lane adds its squares in index order and the warp's sum is a fixed butterfly: the
-// result of a row depends only on d.
+// The same with one warp per row and 16-byte loads, for widths that are a multiple of 4: a row of up to NB * 128
+// values stays in registers between the sum of squares and the scaling, all its words on their way at once; nothing
+// is shared between warps, so there is no barrier. A lane adds its squares in index order and the warp's sum is a
+// fixed butterfly: the result of a row depends only on d (and not on NB). Bound by trips to L2 for few rows: 16 rows of
+// 3,584 in batches of 1,024, read twice, took 15.5 us of a decode step's chain; 8 rows of 3,584 alone take 3.9 us now (2,048: 2.5).
 constexpr int NORM_ROWS_PER_BLOCK = 2;      // small blocks: a few hundred rows still spread over every SM
-template <typename TY>
+template <typename TY, int NB>
 __global__ void __launch_bounds__(32 * NORM_ROWS_PER_BLOCK)
 rmsnorm_rows_kernel(const float* x /* written by the kernel before: no read-only cache */,
                     const int* __restrict__ row_idx, const void* __restrict__ w, int w_dtype, TY* __restrict__ y,
@@ -106,14 +107,22 @@ rmsnorm_rows_kernel(const float* x /* written by the kernel before: no read-only
     bl_pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int r = blockIdx.x * NORM_ROWS_PER_BLOCK + (threadIdx.x >> 5);
-    constexpr int NB = 8;
-    // the norm's weights do not depend on the kernel before: a row of up to NB * 128 values has them in registers
-    // before the wait
+    // the norm's weights do not depend on the kernel before: they are in registers before the wait (of a row of more than
+    // 1,024 values as the bfloat16 words they are; 32-bit ones are then read behind the sum)
     const bool single = d <= NB * 128;
-    float4 wv[NB];
-    if (single) {
+    constexpr int NW = NB == 8 ? NB : 1, NR = NB > 8 ? NB : 1;
+    float4 wv[NW];
+    uint2 wr[NR];
+    if (NB > 8 && w_dtype == BL_BF16) {                // (w is 16-byte aligned)
 #pragma unroll
-        for (int j = 0; j < NB; ++j) {
+        for (int j = 0; j < NR; ++j) {
+            const int k = j * 128 + lane * 4;
+            wr[j] = k < d ? *reinterpret_cast<const uint2*>((const __nv_bfloat16*)w + k) : make_uint2(0u, 0u);
+        }
+    }
+    if (NB == 8 && single) {
+#pragma unroll
+        for (int j = 0; j < NW; ++j) {
             const int k = j * 128 + lane * 4;
             wv[j] = k < d ? make_float4(bl_load_any(w, w_dtype, k), bl_load_any(w, w_dtype, k + 1), bl_load_any(w, w_dtype, k + 2),
                                         bl_load_any(w, w_dtype, k + 3)) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -130,6 +139,11 @@ rmsnorm_rows_kernel(const float* x /* written by the kernel before: no read-only
             v[j] = k < d ? *reinterpret_cast<const float4*>(src + k) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
+    auto weight4 = [&](uint2 u, int k) {
+        if (w_dtype == BL_F32) return *reinterpret_cast<const float4*>((const float*)w + k);
+        const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&u.x), b = *reinterpret_cast<const __nv_bfloat162*>(&u.y);
+        return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
+    };
     float ss = 0.f;
     for (int k0 = 0; k0 < d; k0 += NB * 128) {
         load_batch(k0);
@@ -145,8 +159,9 @@ rmsnorm_rows_kernel(const float* x /* written by the kernel before: no read-only
         for (int j = 0; j < NB; ++j) {
             const int k = k0 + j * 128 + lane * 4;
             if (k >= d) continue;
-            const float4 ww = single ? wv[j] : make_float4(bl_load_any(w, w_dtype, k), bl_load_any(w, w_dtype, k + 1),
-                                                              bl_load_any(w, w_dtype, k + 2), bl_load_any(w, w_dtype, k + 3));
+            const float4 ww = NB > 8 ? weight4(wr[NB > 8 ? j : 0], k) : single ? wv[NB == 8 ? j : 0] :
+                              make_float4(bl_load_any(w, w_dtype, k), bl_load_any(w, w_dtype, k + 1),
+                                          bl_load_any(w, w_dtype, k + 2), bl_load_any(w, w_dtype, k + 3));
             const float o0 = v[j].x * inv * ww.x, o1 = v[j].y * inv * ww.y;
             const float o2 = v[j].z * inv * ww.z, o3 = v[j].w * inv * ww.w;
             if (sizeof(TY) == 4) {
@@ -169,14 +184,18 @@ extern "C" int bl_rmsnorm(const float* x, const int* row_idx, const void* w, int
     if (y_dtype != BL_F32 && y_dtype != BL_BF16) BL_FAIL("bl_rmsnorm: unknown output dtype %d", y_dtype);
     cudaStream_t s = (cudaStream_t)stream;
     const bool wide = d % 4 == 0 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0;      // 16-byte loads and stores of whole rows
-    if (wide && y_dtype == BL_F32)
-        BL_CUDA(bl_launch_dependent(rmsnorm_rows_kernel<float>, dim3((rows + NORM_ROWS_PER_BLOCK - 1) / NORM_ROWS_PER_BLOCK), dim3(32 * NORM_ROWS_PER_BLOCK), 0, s, x, row_idx, w, w_dtype, (float*)y, rows, d, eps));
-    else if (wide)
-        BL_CUDA(bl_launch_dependent(rmsnorm_rows_kernel<__nv_bfloat16>, dim3((rows + NORM_ROWS_PER_BLOCK - 1) / NORM_ROWS_PER_BLOCK), dim3(32 * NORM_ROWS_PER_BLOCK), 0, s, x, row_idx, w, w_dtype, (__nv_bfloat16*)y, rows, d, eps));
+    const int nb = d <= 1024 || d > 4096 || ((uintptr_t)w & 15) ? 8 : d <= 2048 ? 16 : 32;
+#define BL_NORM_ROWS(TY, NB) BL_CUDA(bl_launch_dependent(rmsnorm_rows_kernel<TY, NB>, dim3((rows + NORM_ROWS_PER_BLOCK - 1) / NORM_ROWS_PER_BLOCK), \
+        dim3(32 * NORM_ROWS_PER_BLOCK), 0, s, x, row_idx, w, w_dtype, (TY*)y, rows, d, eps))
+#define BL_NORM_ROWS_NB(TY) do { if (nb == 8) BL_NORM_ROWS(TY, 8); else if (nb == 16) BL_NORM_ROWS(TY, 16); else BL_NORM_ROWS(TY, 32); } while (0)
+    if (wide && y_dtype == BL_F32) BL_NORM_ROWS_NB(float);
+    else if (wide) BL_NORM_ROWS_NB(__nv_bfloat16);
     else if (y_dtype == BL_F32)
         BL_CUDA(bl_launch_dependent(rmsnorm_kernel<float>, dim3(rows), dim3(128), 0, s, x, row_idx, w, w_dtype, (float*)y, d, eps));
     else
         BL_CUDA(bl_launch_dependent(rmsnorm_kernel<__nv_bfloat16>, dim3(rows), dim3(128), 0, s, x, row_idx, w, w_dtype, (__nv_bfloat16*)y, d, eps));
+#undef BL_NORM_ROWS_NB
+#undef BL_NORM_ROWS
     BL_CHECK_LAUNCH("bl_rmsnorm");
     return 0;
 }

@@ -811,11 +811,20 @@ def norm_gemm(x: torch.Tensor, norm_w: torch.Tensor, eps: float, w: torch.Tensor
           _dt(bias) if bias is not None else 0, _p(out), M, N, K, epilogue, _stream())
 
 
+def norm_inside_qkv(M: int, K: int) -> bool:
+    """Whether the norm in front of the q/k/v product is part of it (each block norms all its rows) or a launch of its own.
+    Inside up to 8 rows (of 3,584 values by 4,608 columns: 14.2 us against 15.3) and up to 16 where a row is one batch of
+    loads (896 by 1,152: 3.7 against 3.9; 3,584 by 4,608: 27.5 against 17.8); apart for more (32 rows of 896 by 1,152: 6.4
+    against 4.8, 64 rows 7.4 against 5.2, of 3,584 by 4,608 106 against 40)."""
+    return M <= 8 or (M <= 16 and K <= 1024)
+
+
 def norm_qkv_rope(x: torch.Tensor, norm_w: torch.Tensor, eps: float, w_qkv: torch.Tensor, bias: Optional[torch.Tensor],
                   positions: torch.Tensor, tok_req: torch.Tensor, block_table: torch.Tensor, inv_freq: torch.Tensor,
                   mscale: float, q_out: torch.Tensor, k_cache: Optional[torch.Tensor], v_cache: Optional[torch.Tensor],
                   H: int, KV: int, dh: int, pair_layout: int = 0) -> None:
-    """rmsnorm -> joined q/k/v product (+ bias) -> rotation of q and k -> k, v into the pages, q out, in one launch."""
+    """rmsnorm -> joined q/k/v product (+ bias) -> rotation of q and k -> k, v into the pages, q out, in one launch (or, where
+    `norm_inside_qkv` says so, in two)."""
     M, K = x.shape
     _need(x, "x", torch.float32); _need(norm_w, "norm_w", None, (K,)); _need(w_qkv, "w_qkv", torch.bfloat16, ((H + 2 * KV) * dh, K))
     _need(positions, "positions", torch.int32, (M,)); _need(tok_req, "tok_req", torch.int32, (M,))
@@ -829,6 +838,13 @@ def norm_qkv_rope(x: torch.Tensor, norm_w: torch.Tensor, eps: float, w_qkv: torc
         if k_cache.shape[1] != KV or k_cache.shape[3] != dh:
             raise KernelError(f"k_cache: shape {tuple(k_cache.shape)} does not hold {KV} heads of {dh}")
         page_size = k_cache.shape[2]
+    if not norm_inside_qkv(M, K):
+        normed = torch.empty((M, K), dtype=torch.bfloat16, device=x.device)
+        rmsnorm(x, norm_w, eps, normed)
+        _call(_lib().bl_qkv_rope_normed, _p(normed), _p(w_qkv), _p(bias), _dt(bias) if bias is not None else 0, _p(positions),
+              _p(tok_req), _p(block_table), block_table.shape[1], _p(inv_freq), ctypes.c_float(mscale), _p(q_out), _p(k_cache),
+              _p(v_cache), M, K, H, KV, dh, page_size, pair_layout, _stream())
+        return
     _call(_lib().bl_norm_qkv_rope, _p(x), _p(norm_w), _dt(norm_w), ctypes.c_float(eps), _p(w_qkv), _p(bias),
           _dt(bias) if bias is not None else 0, _p(positions), _p(tok_req), _p(block_table), block_table.shape[1],
           _p(inv_freq), ctypes.c_float(mscale), _p(q_out), _p(k_cache), _p(v_cache), M, K, H, KV, dh, page_size,

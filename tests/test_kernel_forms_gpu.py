@@ -81,3 +81,52 @@ def test_layer_end_chain_at_the_widths_where_its_registers_change(d):
     o.norm_chain(streams[n - 1], sub, gate, gb, (pw, pb, 1e-6), streams=streams, coeffs=c, n=n, mix_out=streams[n],
                  then=(tw, tb, 1e-5), y=y)
     assert torch.equal(streams, ref) and torch.equal(y, y_ref)
+
+
+@pytest.mark.parametrize("d", [1020, 1024, 1028, 2048, 2052, 4092, 4096, 4100])
+@pytest.mark.parametrize("wdtype", [torch.float32, BF])
+def test_rms_norm_at_the_widths_where_its_registers_change(d, wdtype):
+    o = ops()
+    x = data((7, d), 2) * 3
+    w = (data((d,), 3) * 0.25 + 1).to(wdtype)
+    for ydtype in (torch.float32, BF):
+        y = torch.empty(7, d, dtype=ydtype, device=DEV)
+        o.rmsnorm(x, w, 1e-5, y)
+        close(y, plain.rms_norm(x.double().cpu(), w.double().cpu(), 1e-5), ydtype, "rmsnorm")
+
+
+@pytest.mark.parametrize("M,H,KV,dh,d", [(1, 2, 1, 64, 72), (9, 14, 2, 64, 1032), (16, 4, 2, 128, 3584), (17, 6, 2, 32, 520),
+                                         (33, 14, 2, 64, 896), (64, 2, 2, 16, 2056)])
+@pytest.mark.parametrize("layout", [0, 1])
+def test_qkv_rope_of_rows_that_are_normed_already(M, H, KV, dh, d, layout):
+    """The q/k/v product of a decode step that reads normed rows, at the edges of its row groups and with K that is no multiple of
+    its batches, against the kernels it replaces (product with bias, rotation and cache write)."""
+    o = ops()
+    page = 16
+    ctx_lens, q_lens = [3 + 5 * (i % 40) for i in range(M)], [1] * M
+    s = paged_setup(ctx_lens, q_lens, KV, dh, page, BF, 9)
+    s2 = paged_setup(ctx_lens, q_lens, KV, dh, page, BF, 9)
+    x = data((M, d), 41) * 2
+    nw = (data((d,), 42) * 0.25 + 1).to(BF)
+    w = (data(((H + 2 * KV) * dh, d), 43) * 0.2).to(BF)
+    b = (data(((H + 2 * KV) * dh,), 44) * 0.5).to(BF)
+    inv = torch.from_numpy(np.float32(1.0e4) ** (-np.arange(dh // 2, dtype=np.float32) * 2 / dh)).to(DEV)
+    h = torch.empty(M, d, dtype=BF, device=DEV)
+    o.rmsnorm(x, nw, 1e-6, h)
+    qkv = torch.empty(M, (H + 2 * KV) * dh, device=DEV)
+    o.gemm_plain(h, w, qkv, b, o.EPI_BIAS)
+    q_ref = torch.empty(M, H * dh, dtype=BF, device=DEV)
+    o.rope_kv_write(qkv, s["positions"], s["tok_req"], s["table"], inv, dh // 2, 1.0, q_ref, s["kc"], s["vc"], H, KV, dh, layout)
+    q = torch.full((M, H * dh), float("nan"), dtype=BF, device=DEV)
+    inside = o.norm_inside_qkv
+    o.norm_inside_qkv = lambda M, K: False
+    try:
+        o.norm_qkv_rope(x, nw, 1e-6, w, b, s2["positions"], s2["tok_req"], s2["table"], inv, 1.0, q, s2["kc"], s2["vc"], H, KV, dh, layout)
+    finally:
+        o.norm_inside_qkv = inside
+    close(q, q_ref.double(), BF, "q")
+    pos, req = torch.from_numpy(s["positions_np"]).long(), torch.from_numpy(s["tok_req_np"]).long()
+    pages = torch.from_numpy(s["table_np"]).long()[req, pos // page].to(DEV)
+    rows = (pos % page).to(DEV)
+    for name in ("kc", "vc"):
+        close(s2[name][pages, :, rows], s[name][pages, :, rows].double(), BF, name)
