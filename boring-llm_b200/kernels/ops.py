@@ -631,6 +631,9 @@ def gemm_tc_cols(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
 SKINNY_MAX_ROWS = 64                  # up to here W streams through registers (faster than 128-row tcgen05 tiles at 64 rows)
 TC_MIN_COLUMNS_FEW_ROWS = 4096        # 17..64 rows: wide products have enough 128-column tiles for TMA to stream W at full rate
 TC_MIN_COLUMNS_VERY_FEW_ROWS = 32768  # an output head: up to 64 rows take the kernel made for it; without it 128-row tiles win from 9 rows
+COLS_MIN_COLUMNS = 9473               # up to 32 rows the output head's kernel takes all products of more column blocks than the kernel that streams
+                                      # W through registers keeps in flight (8 rows, 13,056 columns, K 2,048: 11.5 us against 31; 12,288 columns, K 1,024:
+                                      # 7.1 against 14.5; 5,760 columns, K 896: 5.3 against 4.2)
 PAIR_MIN_ROWS = 256                   # from here on pairs of SMs share 256 x 256 tiles (tcgen05 cta_group::2)
 SPLITK_MIN_ROWS, SPLITK_MAX_ROWS = 32, 640   # products with few tiles in this range of rows are cut along K over clusters ...
 SPLITK_VERY_LONG_K = 16384            # ... or, below 32 rows, very long (K 18,944 by N 3,584 at 8 rows: 43 us against 72 us through registers)
@@ -673,8 +676,8 @@ def gemm_kernel(x: torch.Tensor, w: torch.Tensor, N: int, bias: Optional[torch.T
     M, K = x.shape
     few_rows_tc = ((M > 16 and N >= TC_MIN_COLUMNS_FEW_ROWS) or (M > 8 and N >= TC_MIN_COLUMNS_VERY_FEW_ROWS)
                    or gemm_streams_better(w))
-    if (N >= TC_MIN_COLUMNS_VERY_FEW_ROWS and bias is None and epilogue == EPI_NONE and M <= 64
-            and gemm_tc_cols_supported(x, w)):
+    if ((N >= TC_MIN_COLUMNS_VERY_FEW_ROWS or (N >= COLS_MIN_COLUMNS and M <= 32)) and bias is None and epilogue == EPI_NONE
+            and M <= 64 and gemm_tc_cols_supported(x, w)):
         return "cols"
     if (epilogue != EPI_SWIGLU and M <= SPLITK_MAX_ROWS and (M >= SPLITK_MIN_ROWS or K >= SPLITK_VERY_LONG_K)
             and (K >= SPLITK_LONG_K or 64 < M <= 128) and gemm_tc_splitk_split(M, N, K, epilogue) >= 2):
