@@ -22,8 +22,8 @@ constexpr int WARPS = 4;
 constexpr int RKMAX = 16;          // rows of a column that one lane holds
 constexpr int MAX_TAPS = 16;
 constexpr int SCAN_SMEM_BYTES = 40 * 1024;
-constexpr int SCAN_VEC_ROWS = 16;
-constexpr int SCAN_SPLIT_MIN = 256;  // tokens of a request in one step from which its portion is cut into parts that run side by side  // rows a lane holds in the kernel with 16-byte fetches, where the key size allows
+constexpr int SCAN_VEC_ROWS = 16;    // rows a lane holds in the kernel with 16-byte fetches, where the key size allows
+constexpr int SCAN_SPLIT_MIN = 256;  // tokens of a request in one step from which its portion is cut into parts that run side by side
 
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
 
@@ -182,36 +182,37 @@ recurrent_scan_kernel(const float* q, int ldq, const float* k, int ldk, const fl
 
 // The same walk for key sizes that split evenly: a lane holds RK4 * 4 CONSECUTIVE rows of its column (dk = KS * RK4 * 4),
 // so a token's q, k and decays reach its registers as 16-byte loads at fixed offsets, two tokens' registers take turns
-// (no copies), and the dot products run in two chains. A warp has no other warp on its scheduler to hide latencies
-// behind (a request gives H * dv / (WARPS * CW) blocks): what counts is the number of instructions per token.
-template <int RULE, int RK4>
-__global__ void __launch_bounds__(WARPS * 32)
+// (no copies), and the dot products run in two chains. Where a launch has few blocks a warp has no other warp on its
+// scheduler to hide latencies behind (a request gives H * dv / (WARPS * CW) blocks): what counts is the number of
+// instructions per token. DENSE: for launches of more blocks than two an SM: one token's registers instead of two, so that
+// four blocks fit an SM and hide each other's latencies. The order of every sum is the same in both.
+// QUIET: the first pass over a portion that was cut: no read-out. With four blocks an SM, up to 32 parts instead of 16 and
+// the folds' loads in flight, a Fezopel prefill of 2,048 tokens (0.5B sizes, six recurrent layers) 2,629 -> 2,090 us.
+template <int RULE, int RK4, bool DENSE, bool QUIET>
+__global__ void __launch_bounds__(WARPS * 32, DENSE ? 4 : 1)
 recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, const float* z, int ldz,
                           const float* beta, int ldb, float q_scale,
                           float* state, size_t slot_stride, const int* __restrict__ slots, const int* __restrict__ cu_q,
                           float* out, int H, int G, int dk, int dv, int KS, int chunk, int vec,
-                          int nc, int pass, float* part_s, float* part_p, const float* part_start) {
+                          int nc, float* part_s, float* part_p, const float* part_start) {
     bl_pdl_trigger();
     bl_pdl_wait();
     extern __shared__ __align__(16) float sm[];
     constexpr bool DELTA = RULE == BL_RULE_DELTA, BONUS = RULE == BL_RULE_BONUS;
     constexpr int RK = RK4 * 4;
-    // A long portion of a request may be cut into nc parts that run side by side (linear attention only: its recurrence is
-    // linear in S with a diagonal transition). pass 1: every part from a ZERO state, leaving its own contribution S_part and
-    // the product P of its decays; pass 2: a part starts from the request's state folded through the parts before it
-    // (S <- P o S + S_part) and writes the outputs; a small kernel then folds all parts into the slot. The delta rule's
-    // transition is a matrix: its fold (S <- P S + S_part, a small product) runs between the passes, leaves every part's
-    // start state in scratch and the final state in the slot. Short portions
-    // (and nc 1) take one block per (request, head, columns) through pass 0 / 2 as before.
+    // A long portion of a request may be cut into nc parts that run side by side (the recurrence is linear in S). First pass
+    // (QUIET): every part from a ZERO state, leaving its own contribution S_part and its transition P (a product of decays a
+    // row; of the delta rule a matrix). Between the passes a fold (S <- P S + S_part) leaves every part's start state in
+    // scratch and the final state in the slot. Second pass: a part runs from its start state and writes the outputs. Short
+    // portions (and nc 1) take one block per (request, head, columns) through the second pass alone.
     const int r = blockIdx.z / nc, part = blockIdx.z % nc, h = blockIdx.y;
     const int n_all = cu_q[r + 1] - cu_q[r];
     if (n_all <= 0) return;
     const bool split = nc > 1 && n_all >= SCAN_SPLIT_MIN;
-    if (!split && (part != 0 || pass == 1)) return;
-    const int part_len = split ? (n_all + nc - 1) / nc : n_all;
-    const int t_first = split ? part * part_len : 0;
-    const int t0 = cu_q[r] + t_first, n = min(n_all - t_first, part_len);
-    if (n <= 0) return;
+    if (!split && (part != 0 || QUIET)) return;
+    // (of more parts than tokens some are empty: they leave a zero state and the identity)
+    const int t_first = split ? (int)((long long)part * n_all / nc) : 0;
+    const int t0 = cu_q[r] + t_first, n = (split ? (int)((long long)(part + 1) * n_all / nc) : n_all) - t_first;
     const int gh = h / (H / G);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int CW = 32 / KS, cols_blk = WARPS * CW;
@@ -219,7 +220,7 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
     const int c = (blockIdx.x * WARPS + warp) * CW + cc;
     // The delta rule's transition over a part is a key x key matrix: pass 1 makes it in dk further columns that start as
     // the identity and see values of zero (column dv + j ends as the part's transition applied to unit vector j).
-    const int n_cols = dv + (DELTA && split && pass == 1 ? dk : 0);
+    const int n_cols = dv + (DELTA && QUIET ? dk : 0);
     const bool col_ok = c < n_cols;
     const int per_tok = 3 * dk + cols_blk + 4;
     const int buf_floats = chunk * per_tok;
@@ -238,11 +239,13 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
             const float* gz = z + tok * ldz + h * dk;
             if (vec) {
                 for (int d = lane * 4; d < dk; d += 128) {
-                    cp_async16(dst + d, gq + d); cp_async16(dst + dk + d, gk + d); cp_async16(dst + 2 * dk + d, gz + d);
+                    if (!QUIET) cp_async16(dst + d, gq + d);
+                    cp_async16(dst + dk + d, gk + d); cp_async16(dst + 2 * dk + d, gz + d);
                 }
             } else {
                 for (int d = lane; d < dk; d += 32) {
-                    cp_async4(dst + d, gq + d); cp_async4(dst + dk + d, gk + d); cp_async4(dst + 2 * dk + d, gz + d);
+                    if (!QUIET) cp_async4(dst + d, gq + d);
+                    cp_async4(dst + dk + d, gk + d); cp_async4(dst + 2 * dk + d, gz + d);
                 }
             }
             const float* gv = v + tok * ldv + h * dv + col0;
@@ -256,33 +259,26 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
     };
 
     issue(0, sm);
-    float st[RK], pr[RK];
+    float st[RK], pr[QUIET && !DELTA ? RK : 1];
     const size_t part_base = ((size_t)r * nc) * H + h;           // + p * H for part p
 #pragma unroll
     for (int i = 0; i < RK; ++i) {
-        if (split && pass == 1) st[i] = (DELTA && c >= dv && row0 + i == c - dv) ? 1.f : 0.f;
-        else if (DELTA && split) st[i] = col_ok ? part_start[((part_base + (size_t)part * H) * dk + row0 + i) * dv + c] : 0.f;
+        if (QUIET) st[i] = (DELTA && c >= dv && row0 + i == c - dv) ? 1.f : 0.f;
+        else if (split) st[i] = col_ok ? part_start[((part_base + (size_t)part * H) * dk + row0 + i) * dv + c] : 0.f;
         else st[i] = col_ok ? S[(size_t)(row0 + i) * dv + c] : 0.f;
-        pr[i] = 1.f;
+        if (QUIET && !DELTA) pr[QUIET && !DELTA ? i : 0] = 1.f;
     }
-    if (!DELTA && split && pass == 2) {
-        for (int p = 0; p < part; ++p) {
-            const float* ps = part_s + (part_base + (size_t)p * H) * dk * dv;
-            const float* pp = part_p + (part_base + (size_t)p * H) * dk;
-#pragma unroll
-            for (int i = 0; i < RK; ++i)
-                st[i] = col_ok ? fmaf(pp[row0 + i], st[i], ps[(size_t)(row0 + i) * dv + c]) : 0.f;
-        }
-    }
-    const bool quiet = split && pass == 1;                       // no outputs yet
     const int v_off = 3 * dk + warp * CW + cc, b_off = 3 * dk + cols_blk;
     const int dk4 = dk >> 2;
 
-    struct Tok { float4 q[RK4], k[RK4], d[RK4]; float v, b; };
+    struct Tok { float4 q[QUIET ? 1 : RK4], k[RK4], d[RK4]; float v, b; };
     auto fetch = [&](const float* tokp, Tok& t) {
         const float4* p4 = reinterpret_cast<const float4*>(tokp + row0);
 #pragma unroll
-        for (int j = 0; j < RK4; ++j) { t.q[j] = p4[j]; t.k[j] = p4[dk4 + j]; t.d[j] = p4[2 * dk4 + j]; }
+        for (int j = 0; j < RK4; ++j) {
+            if (!QUIET) t.q[QUIET ? 0 : j] = p4[j];
+            t.k[j] = p4[dk4 + j]; t.d[j] = p4[2 * dk4 + j];
+        }
         t.v = tokp[v_off];
         t.b = (DELTA || BONUS) ? tokp[b_off] : 0.f;
     };
@@ -295,14 +291,14 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
             float o0 = 0.f, o1 = 0.f;
 #pragma unroll
             for (int i = 0; i < RK; i += 2) {
-                if (BONUS) { o0 = fmaf(st[i], tq[i], o0); o1 = fmaf(st[i + 1], tq[i + 1], o1); }       // the state before the write
+                if (BONUS && !QUIET) { o0 = fmaf(st[i], tq[i], o0); o1 = fmaf(st[i + 1], tq[i + 1], o1); }       // the state before the write
                 st[i] = fmaf(td[i], st[i], tk[i] * t.v);
                 st[i + 1] = fmaf(td[i + 1], st[i + 1], tk[i + 1] * t.v);
-                if (!BONUS) { o0 = fmaf(st[i], tq[i], o0); o1 = fmaf(st[i + 1], tq[i + 1], o1); }
+                if (!BONUS && !QUIET) { o0 = fmaf(st[i], tq[i], o0); o1 = fmaf(st[i + 1], tq[i + 1], o1); }
             }
-            if (quiet) {
+            if (QUIET) {
 #pragma unroll
-                for (int i = 0; i < RK; ++i) pr[i] *= td[i];
+                for (int i = 0; i < (QUIET && !DELTA ? RK : 1); ++i) pr[i] *= td[i];
                 return;
             }
             o = o0 + o1;
@@ -315,21 +311,25 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
                 st[i] *= td[i];
                 st[i + 1] *= td[i + 1];
                 sk0 = fmaf(st[i], tk[i], sk0); sk1 = fmaf(st[i + 1], tk[i + 1], sk1);
-                sq0 = fmaf(st[i], tq[i], sq0); sq1 = fmaf(st[i + 1], tq[i + 1], sq1);
-                kq0 = fmaf(tk[i], tq[i], kq0); kq1 = fmaf(tk[i + 1], tq[i + 1], kq1);
+                if (!QUIET) {
+                    sq0 = fmaf(st[i], tq[i], sq0); sq1 = fmaf(st[i + 1], tq[i + 1], sq1);
+                    kq0 = fmaf(tk[i], tq[i], kq0); kq1 = fmaf(tk[i + 1], tq[i + 1], kq1);
+                }
             }
             float sk_ = sk0 + sk1, sq_ = sq0 + sq1, kq = kq0 + kq1;
             for (int x = 16; x >= CW; x >>= 1) {
                 sk_ += __shfl_xor_sync(0xffffffffu, sk_, x);
-                sq_ += __shfl_xor_sync(0xffffffffu, sq_, x);
-                kq += __shfl_xor_sync(0xffffffffu, kq, x);
+                if (!QUIET) {
+                    sq_ += __shfl_xor_sync(0xffffffffu, sq_, x);
+                    kq += __shfl_xor_sync(0xffffffffu, kq, x);
+                }
             }
             const float u = t.b * (t.v - sk_);
 #pragma unroll
             for (int i = 0; i < RK; ++i) st[i] = fmaf(tk[i], u, st[i]);
             o = fmaf(kq, u, sq_);
         }
-        if (s == 0 && col_ok && !quiet) out[tok * H * dv + h * dv + c] = o * q_scale;
+        if (!QUIET && s == 0 && col_ok) out[tok * H * dv + h * dv + c] = o * q_scale;
     };
 
     int which = 0;
@@ -346,10 +346,19 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
             }
             __syncthreads();
         }
-        Tok ta, tb;
-        fetch(buf, ta);
         const size_t tok0 = (size_t)(t0 + base);
         int tt = 0;
+        if (DENSE) {
+            for (; tt < m; ++tt) {
+                Tok t;
+                fetch(buf + (size_t)tt * per_tok, t);
+                step(t, tok0 + tt);
+            }
+            __syncthreads();
+            continue;
+        }
+        Tok ta, tb;
+        fetch(buf, ta);
         for (; tt + 1 < m; tt += 2) {
             fetch(buf + (size_t)(tt + 1) * per_tok, tb);
             step(ta, tok0 + tt);
@@ -360,7 +369,7 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
         __syncthreads();                               // the buffer is free for the chunk after next
     }
     if (split) {
-        if (pass == 1 && DELTA) {
+        if (QUIET && DELTA) {
             float* ps = part_s + (part_base + (size_t)part * H) * dk * dv;
             float* pm = part_p + (part_base + (size_t)part * H) * dk * dk;      // [row][unit vector]
 #pragma unroll
@@ -368,16 +377,16 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
                 if (c < dv) ps[(size_t)(row0 + i) * dv + c] = st[i];
                 else if (col_ok) pm[(size_t)(row0 + i) * dk + (c - dv)] = st[i];
             }
-        } else if (pass == 1) {
+        } else if (QUIET) {
             float* ps = part_s + (part_base + (size_t)part * H) * dk * dv;
             float* pp = part_p + (part_base + (size_t)part * H) * dk;
 #pragma unroll
             for (int i = 0; i < RK; ++i) {
                 if (col_ok) ps[(size_t)(row0 + i) * dv + c] = st[i];
-                if (blockIdx.x == 0 && warp == 0 && cc == 0) pp[row0 + i] = pr[i];
+                if (blockIdx.x == 0 && warp == 0 && cc == 0) pp[row0 + i] = pr[QUIET && !DELTA ? i : 0];
             }
         }
-        return;                                        // the slot is written by the fold behind pass 2
+        return;                                        // the slot is written by the fold
     }
 #pragma unroll
     for (int i = 0; i < RK; ++i)
@@ -386,8 +395,9 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
 
 // Between the two passes of a cut portion of the delta rule: start[0] = the slot's state, start[p + 1] = P_p start[p] +
 // S_part_p (P_p a key x key matrix), the last one into the slot. A block owns FOLD_COLS columns of one (request, head) and
-// keeps the current state's columns in shared memory, two buffers taking turns.
-constexpr int FOLD_COLS = 32, FOLD_MAX_DK = 128;
+// keeps the current state's columns in shared memory, two buffers taking turns. The parts follow one another, so a part's
+// time is a chain of trips to L2: few columns a block (more blocks), P in 16-byte pieces, a row's pieces in flight together.
+constexpr int FOLD_COLS = 8, FOLD_MAX_DK = 128;
 __global__ void __launch_bounds__(256)
 scan_fold_matrix_kernel(float* state, size_t slot_stride, const int* __restrict__ slots, const int* __restrict__ cu_q,
                         const float* part_s, const float* part_pm, float* part_start, int H, int dk, int dv, int nc) {
@@ -398,9 +408,10 @@ scan_fold_matrix_kernel(float* state, size_t slot_stride, const int* __restrict_
     if (cu_q[r + 1] - cu_q[r] < SCAN_SPLIT_MIN) return;
     float* S = state + (size_t)slots[r] * slot_stride + (size_t)h * dk * dv;
     const size_t base = ((size_t)r * nc) * H + h;
-    const int col = threadIdx.x % FOLD_COLS, rg = threadIdx.x / FOLD_COLS;      // 8 row groups
+    const int col = threadIdx.x % FOLD_COLS, rg = threadIdx.x / FOLD_COLS;
+    constexpr int GROUPS = 256 / FOLD_COLS;                                     // row groups
     const bool ok = c0 + col < dv;
-    for (int row = rg; row < dk; row += 8) {
+    for (int row = rg; row < dk; row += GROUPS) {
         const float x = ok ? S[(size_t)row * dv + c0 + col] : 0.f;
         cur[0][row][col] = x;
         if (ok) part_start[((base + 0) * dk + row) * dv + c0 + col] = x;
@@ -410,10 +421,15 @@ scan_fold_matrix_kernel(float* state, size_t slot_stride, const int* __restrict_
     for (int p = 0; p < nc; ++p, w ^= 1) {
         const float* pm = part_pm + (base + (size_t)p * H) * dk * dk;
         const float* ps = part_s + (base + (size_t)p * H) * dk * dv;
-        for (int row = rg; row < dk; row += 8) {
+        for (int row = rg; row < dk; row += GROUPS) {
             float acc = ok ? ps[(size_t)row * dv + c0 + col] : 0.f;
-            const float* prow = pm + (size_t)row * dk;
-            for (int j = 0; j < dk; ++j) acc = fmaf(prow[j], cur[w][j][col], acc);
+            const float4* prow = reinterpret_cast<const float4*>(pm + (size_t)row * dk);    // dk is a multiple of 4
+#pragma unroll 8
+            for (int j = 0; j < dk >> 2; ++j) {
+                const float4 a = prow[j];
+                acc = fmaf(a.x, cur[w][4 * j][col], acc); acc = fmaf(a.y, cur[w][4 * j + 1][col], acc);
+                acc = fmaf(a.z, cur[w][4 * j + 2][col], acc); acc = fmaf(a.w, cur[w][4 * j + 3][col], acc);
+            }
             cur[w ^ 1][row][col] = acc;
             if (ok) {
                 if (p + 1 < nc) part_start[((base + (size_t)(p + 1) * H) * dk + row) * dv + c0 + col] = acc;
@@ -424,9 +440,10 @@ scan_fold_matrix_kernel(float* state, size_t slot_stride, const int* __restrict_
     }
 }
 
-// Behind the two passes of a cut portion: the request's state folded through all parts, into its slot.
+// The same where the transition is a decay per row: start[p + 1] = P_p o start[p] + S_part_p. Every part's start takes the
+// place of its contribution in part_s.
 __global__ void scan_fold_kernel(float* state, size_t slot_stride, const int* __restrict__ slots, const int* __restrict__ cu_q,
-                                 const float* part_s, const float* part_p, int H, int dk, int dv, int nc) {
+                                 float* part_s, const float* part_p, int H, int dk, int dv, int nc) {
     bl_pdl_trigger();
     bl_pdl_wait();
     const int r = blockIdx.z, h = blockIdx.y;
@@ -437,9 +454,21 @@ __global__ void scan_fold_kernel(float* state, size_t slot_stride, const int* __
     if (e >= dk * dv) return;
     const int row = e / dv;
     float sv = S[e];
-#pragma unroll 4
-    for (int p = 0; p < nc; ++p)
-        sv = fmaf(part_p[(base + (size_t)p * H) * dk + row], sv, part_s[(base + (size_t)p * H) * dk * dv + e]);
+    for (int p0 = 0; p0 < nc; p0 += 8) {               // eight parts' values in flight
+        float add[8], mul[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (p0 + i < nc) {
+                mul[i] = part_p[(base + (size_t)(p0 + i) * H) * dk + row];
+                add[i] = part_s[(base + (size_t)(p0 + i) * H) * dk * dv + e];
+            }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (p0 + i < nc) {
+                part_s[(base + (size_t)(p0 + i) * H) * dk * dv + e] = sv;
+                sv = fmaf(mul[i], sv, add[i]);
+            }
+    }
     S[e] = sv;
 }
 
@@ -763,6 +792,16 @@ gated_group_norm_kernel(const float* o, const float* x, int ld_x, const void* __
         bl_store(y + (size_t)t * width + c0 + i, value(c0 + i) * inv * (w ? bl_load_any(w, w_dtype, c0 + i) : 1.f));
 }
 
+int scan_sms() {
+    static int sms = 0;                                                         // (of the current device at the first call)
+    if (sms == 0) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+            sms = 148;
+    }
+    return sms;
+}
+
 }  // namespace
 
 extern "C" int bl_recurrent_scan(int rule, const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
@@ -830,15 +869,25 @@ extern "C" int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const 
         const bool dl = rule == BL_RULE_DELTA;
         float* part_s = scratch;                                                 // [R, nc, H, dk, dv]
         float* part_p = scratch ? scratch + (size_t)R * nc * H * dk * dv : nullptr;   // [R, nc, H, dk] or, delta rule, [R, nc, H, dk, dk]
-        float* part_start = (scratch && dl) ? part_p + (size_t)R * nc * H * dk * dk : nullptr;   // delta rule: [R, nc, H, dk, dv]
-#define BL_SCAN(D, R4, PASS) BL_CUDA(bl_launch_dependent(recurrent_scan_vec_kernel<D, R4>, (D == BL_RULE_DELTA && PASS == 1) ? grid_wide : grid, dim3(WARPS * 32), smem, s, \
-        q, ldq, k, ldk, v, ldv, z, ldz, beta, ldb, q_scale, state, (size_t)slot_stride, slots, cu_q, out, H, G, dk, dv, KS, chunk, vec, nc, PASS, \
+        // [R, nc, H, dk, dv]; a fold with a decay per row leaves the starts in part_s
+        float* part_start = scratch == nullptr ? nullptr : dl ? part_p + (size_t)R * nc * H * dk * dk : part_s;
+        const int two_an_sm = 2 * scan_sms();
+#define BL_SCAN_Q(D, R4, DENSE, QUIET, GRID) BL_CUDA(bl_launch_dependent(recurrent_scan_vec_kernel<D, R4, DENSE, QUIET>, GRID, dim3(WARPS * 32), smem, s, \
+        q, ldq, k, ldk, v, ldv, z, ldz, beta, ldb, q_scale, state, (size_t)slot_stride, slots, cu_q, out, H, G, dk, dv, KS, chunk, vec, nc, \
         part_s, part_p, (const float*)part_start))
+#define BL_SCAN(D, R4, PASS) do { \
+        const dim3 g = (D == BL_RULE_DELTA && PASS == 1) ? grid_wide : grid; \
+        const bool dense = (long long)g.x * g.y * g.z > two_an_sm; \
+        if (PASS == 1) { if (dense) BL_SCAN_Q(D, R4, true, true, g); else BL_SCAN_Q(D, R4, false, true, g); } \
+        else if (dense) BL_SCAN_Q(D, R4, true, false, g); else BL_SCAN_Q(D, R4, false, false, g); } while (0)
         for (int pass = (nc > 1 ? 1 : 2); pass <= 2; ++pass) {
             if (pass == 2 && nc > 1 && dl)
                 BL_CUDA(bl_launch_dependent(scan_fold_matrix_kernel, dim3((dv + FOLD_COLS - 1) / FOLD_COLS, H, R), dim3(256), 0, s, state,
                                             (size_t)slot_stride, slots, cu_q, (const float*)part_s, (const float*)part_p, part_start,
                                             H, dk, dv, nc));
+            if (pass == 2 && nc > 1 && !dl)
+                BL_CUDA(bl_launch_dependent(scan_fold_kernel, dim3((dk * dv + 255) / 256, H, R), dim3(256), 0, s, state, (size_t)slot_stride,
+                                            slots, cu_q, part_s, (const float*)part_p, H, dk, dv, nc));
             switch (rk4) {
 #define BL_SCAN_RULE(R4) do { if (dl) BL_SCAN(BL_RULE_DELTA, R4, pass); else if (rule == BL_RULE_BONUS) BL_SCAN(BL_RULE_BONUS, R4, pass); \
                                   else BL_SCAN(BL_RULE_GLA, R4, pass); } while (0)
@@ -850,9 +899,7 @@ extern "C" int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const 
             }
         }
 #undef BL_SCAN
-        if (nc > 1 && !dl)
-            BL_CUDA(bl_launch_dependent(scan_fold_kernel, dim3((dk * dv + 255) / 256, H, R), dim3(256), 0, s, state, (size_t)slot_stride, slots, cu_q,
-                                        (const float*)part_s, (const float*)part_p, H, dk, dv, nc));
+#undef BL_SCAN_Q
         BL_CHECK_LAUNCH("bl_recurrent_scan");
         return 0;
     }

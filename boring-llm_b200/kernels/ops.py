@@ -975,9 +975,10 @@ def gemm_plain_decay(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tens
           _p(coef), group, ctypes.c_float(sign), _stream())
 
 
-SCAN_MAX_PARTS = 16               # most parts a long portion of a request is cut into
+SCAN_MAX_PARTS = 32               # most parts a long portion of a request is cut into
 SCAN_PART_MIN_TOKENS = 256        # requests with fewer tokens in a step are walked in one piece (the kernel's own rule)
-SCAN_BLOCKS_PER_SM = 2            # blocks of the scan kernel that an SM holds (its registers)
+SCAN_BLOCKS_PER_SM = 4            # blocks of the scan kernel that an SM holds (its registers)
+SCAN_MAX_SCRATCH_PARTS = 1024     # parts x requests of a step that scratch is taken for
 
 
 def recurrent_scan_parts(rule: int, H: int, dk: int, dv: int, n_long: int) -> int:
@@ -1016,6 +1017,7 @@ def recurrent_scan(rule: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     _need(out, "out", torch.float32, (T, H * dv))
     if not state.is_cuda or state.dtype != torch.float32 or state.dim() != 2 or state.stride(1) != 1 or state.shape[1] < H * dk * dv:
         raise KernelError("state: must be 32-bit [slots, >= H * dk * dv] with contiguous rows")
+    parts = min(parts, max(8, SCAN_MAX_SCRATCH_PARTS // max(1, R)))
     if parts > 1:
         lib = _lib()
         lib.bl_recurrent_scan_parts_scratch.restype = ctypes.c_longlong

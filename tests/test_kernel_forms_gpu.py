@@ -130,3 +130,51 @@ def test_qkv_rope_of_rows_that_are_normed_already(M, H, KV, dh, d, layout):
     rows = (pos % page).to(DEV)
     for name in ("kc", "vc"):
         close(s2[name][pages, :, rows], s[name][pages, :, rows].double(), BF, name)
+
+
+def _scan64(rule, q, k, v, a, b, scale, S, H):
+    """The recurrence of one request in 64 bits: rows q, k, a [n, H, dk], v [n, H, dv], b [n, H]; S [H, dk, dv] is left updated."""
+    o = ops()
+    out = torch.zeros_like(v)
+    for t in range(q.shape[0]):
+        if rule == o.RULE_BONUS:
+            out[t] = (torch.einsum("hkv,hk->hv", S, q[t]) + b[t][:, None] * v[t]) * scale
+        S *= a[t][:, :, None]
+        u = v[t] if rule != o.RULE_DELTA else torch.sigmoid(b[t])[:, None] * (v[t] - torch.einsum("hkv,hk->hv", S, k[t]))
+        S += k[t][:, :, None] * u[:, None]
+        if rule != o.RULE_BONUS:
+            out[t] = torch.einsum("hkv,hk->hv", S, q[t]) * scale
+    return out
+
+
+@pytest.mark.parametrize("rule", ["RULE_GLA", "RULE_DELTA", "RULE_BONUS"])
+@pytest.mark.parametrize("H,dk,dv,lens", [(2, 64, 128, [257, 5, 0, 700]), (3, 128, 40, [256, 255]), (1, 16, 33, [300]), (5, 32, 256, [1, 512, 3, 9, 1, 1])])
+@pytest.mark.parametrize("parts", [1, 2, 9, 32, 300])
+def test_scan_in_parts(rule, H, dk, dv, lens, parts):
+    """Portions cut into parts (more parts than tokens among them) beside short ones and requests without tokens, few blocks and
+    many (the two forms of the kernel): outputs and states against 64 bits, and slots that no request owns stay as they are."""
+    o = ops()
+    rule = getattr(o, rule)
+    T, R = sum(lens), len(lens)
+    g = torch.Generator().manual_seed(T + parts)
+    rnd = lambda *n: torch.randn(*n, generator=g)
+    q, k, v, b = rnd(T, H * dk) * 0.3, rnd(T, H * dk), rnd(T, H * dv), rnd(T, H)
+    k = (k.view(T, H, dk) / k.view(T, H, dk).norm(dim=-1, keepdim=True)).reshape(T, H * dk)
+    a = torch.sigmoid(rnd(T, H * dk) + 3.0)
+    state = rnd(R + 2, H * dk * dv)
+    slots = torch.arange(R, 0, -1, dtype=torch.int32)
+    cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).to(torch.int32)
+    dev = lambda t: t.to(DEV)
+    st = dev(state.clone())
+    out = torch.full((T, H * dv), float("nan"), device=DEV)
+    o.recurrent_scan(rule, dev(q), dev(k), dev(v), dev(a), None if rule == o.RULE_GLA else dev(b), 0.5, st, dev(slots), dev(cu), out,
+                     H, H, dk, dv, parts=parts)
+    want_state = state.double().clone()
+    for r in range(R):
+        lo, hi = int(cu[r]), int(cu[r + 1])
+        S = want_state[int(slots[r])].view(H, dk, dv)
+        w = _scan64(rule, *(x[lo:hi].double().view(hi - lo, H, -1) for x in (q, k, v, a)), b[lo:hi].double(), 0.5, S, H)
+        if hi > lo:
+            close(out[lo:hi], w.reshape(hi - lo, -1), torch.float32, f"outputs of request {r}")
+    close(st, want_state, torch.float32, "states")
+    assert torch.equal(st[0].cpu(), state[0]) and torch.equal(st[R + 1].cpu(), state[R + 1])
