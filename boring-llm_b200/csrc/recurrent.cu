@@ -662,52 +662,50 @@ conv_silu_unit_kernel(const float* x, int ld, const float* __restrict__ taps, in
 
 // The same for four taps, channels in groups of four with 16-byte accesses: the unit heads' values stay in shared memory
 // between the convolution and the norm (the kernel above writes, reads and writes them again, and reads each tap of a
-// channel by itself). per_block tokens a block one after the other: a token's inputs are its neighbours', too, and come
-// from L1 then. Sums in the order of the kernel above. MEASURED_CONV
+// channel by itself). Sums in the order of the kernel above. Bound by trips to L2 for few tokens (8 of 4,096 channels
+// 21 -> 5.2 us) and by the rows' bytes for many (2,048 of 1,792 channels 30 -> 19 us; several tokens a block, for their
+// common inputs in L1, are slower: 21).
 constexpr int CONV4_THREADS = 256;
 __global__ void __launch_bounds__(CONV4_THREADS)
 conv4_silu_unit_kernel(const float* x, int ld, const float4* __restrict__ taps, const float* tail, size_t slot_stride,
                        const int* __restrict__ slots, const int* __restrict__ tok_req, const int* __restrict__ cu_q, float* y,
-                       int T, int C, int unit_heads, int scaled_heads, int dk, float q_scale, float unit_eps, const void* __restrict__ bias,
-                       int bias_dtype, int per_block) {
+                       int C, int unit_heads, int scaled_heads, int dk, float q_scale, float unit_eps, const void* __restrict__ bias,
+                       int bias_dtype) {
     bl_pdl_trigger();
     bl_pdl_wait();
     extern __shared__ __align__(16) float units[];               // [unit_heads * dk]
     const int lane = threadIdx.x & 31, unit_cols = unit_heads * dk;
-    const int t_end = min(T, (int)(blockIdx.x + 1) * per_block);
-    for (int t = blockIdx.x * per_block; t < t_end; ++t) {
-        const int r = tok_req[t];
-        const int j = t - cu_q[r];
-        const float* tl = tail + (size_t)slots[r] * slot_stride;
-        for (int ch = threadIdx.x * 4; ch < C; ch += CONV4_THREADS * 4) {
-            float4 in[4], tp[4];
+    const int t = blockIdx.x;
+    const int r = tok_req[t];
+    const int j = t - cu_q[r];
+    const float* tl = tail + (size_t)slots[r] * slot_stride;
+    for (int ch = threadIdx.x * 4; ch < C; ch += CONV4_THREADS * 4) {
+        float4 in[4], tp[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int off = j - 3 + i;
-                in[i] = *reinterpret_cast<const float4*>(off >= 0 ? x + (size_t)(t - j + off) * ld + ch : tl + (size_t)(3 + off) * C + ch);
-                tp[i] = taps[ch + i];                            // the four taps of channel ch + i
-            }
-            float acc[4];
+        for (int i = 0; i < 4; ++i) {
+            const int off = j - 3 + i;
+            in[i] = *reinterpret_cast<const float4*>(off >= 0 ? x + (size_t)(t - j + off) * ld + ch : tl + (size_t)(3 + off) * C + ch);
+            tp[i] = taps[ch + i];                            // the four taps of channel ch + i
+        }
+        float acc[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                float a = bias ? bl_load_any(bias, bias_dtype, ch + e) : 0.f;
-                a = fmaf(tp[e].x, reinterpret_cast<const float*>(&in[0])[e], a);
-                a = fmaf(tp[e].y, reinterpret_cast<const float*>(&in[1])[e], a);
-                a = fmaf(tp[e].z, reinterpret_cast<const float*>(&in[2])[e], a);
-                a = fmaf(tp[e].w, reinterpret_cast<const float*>(&in[3])[e], a);
-                acc[e] = bl_silu(a);
-            }
-            *reinterpret_cast<float4*>(ch < unit_cols ? units + ch : y + (size_t)t * C + ch) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        for (int e = 0; e < 4; ++e) {
+            float a = bias ? bl_load_any(bias, bias_dtype, ch + e) : 0.f;
+            a = fmaf(tp[e].x, reinterpret_cast<const float*>(&in[0])[e], a);
+            a = fmaf(tp[e].y, reinterpret_cast<const float*>(&in[1])[e], a);
+            a = fmaf(tp[e].z, reinterpret_cast<const float*>(&in[2])[e], a);
+            a = fmaf(tp[e].w, reinterpret_cast<const float*>(&in[3])[e], a);
+            acc[e] = bl_silu(a);
         }
-        __syncthreads();
-        for (int hh = threadIdx.x >> 5; hh < unit_heads; hh += CONV4_THREADS / 32) {
-            const float* p = units + (size_t)hh * dk;
-            float ss = 0.f;
-            for (int d = lane; d < dk; d += 32) ss += p[d] * p[d];
-            const float inv = (hh < scaled_heads ? q_scale : 1.f) / sqrtf(bl_warp_sum(ss) + unit_eps);
-            for (int d = lane; d < dk; d += 32) y[(size_t)t * C + (size_t)hh * dk + d] = p[d] * inv;
-        }
-        if (per_block > 1) __syncthreads();
+        *reinterpret_cast<float4*>(ch < unit_cols ? units + ch : y + (size_t)t * C + ch) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    }
+    __syncthreads();
+    for (int hh = threadIdx.x >> 5; hh < unit_heads; hh += CONV4_THREADS / 32) {
+        const float* p = units + (size_t)hh * dk;
+        float ss = 0.f;
+        for (int d = lane; d < dk; d += 32) ss += p[d] * p[d];
+        const float inv = (hh < scaled_heads ? q_scale : 1.f) / sqrtf(bl_warp_sum(ss) + unit_eps);
+        for (int d = lane; d < dk; d += 32) y[(size_t)t * C + (size_t)hh * dk + d] = p[d] * inv;
     }
 }
 
@@ -1060,10 +1058,9 @@ extern "C" int bl_conv_silu_unit_bias(const float* x, int ld, const float* taps,
     const int unit_cols = unit_heads * dk;
     if (n_taps == 4 && C % 4 == 0 && ld % 4 == 0 && slot_stride % 4 == 0 && unit_cols % 4 == 0 && unit_cols <= 8192 &&
         (((uintptr_t)x | (uintptr_t)taps | (uintptr_t)tail | (uintptr_t)y) & 15) == 0) {
-        const int per_block = T > 8 * scan_sms() ? 4 : 1;        // (one a block while the blocks fit the device at once)
-        BL_CUDA(bl_launch_dependent(conv4_silu_unit_kernel, dim3((T + per_block - 1) / per_block), dim3(CONV4_THREADS), (size_t)unit_cols * sizeof(float),
-                                    (cudaStream_t)stream, x, ld, (const float4*)taps, tail, (size_t)slot_stride, slots, tok_req, cu_q, y, T, C,
-                                    unit_heads, scaled_heads, dk, q_scale, unit_eps, bias, bias_dtype, per_block));
+        BL_CUDA(bl_launch_dependent(conv4_silu_unit_kernel, dim3(T), dim3(CONV4_THREADS), (size_t)unit_cols * sizeof(float),
+                                    (cudaStream_t)stream, x, ld, (const float4*)taps, tail, (size_t)slot_stride, slots, tok_req, cu_q, y, C,
+                                    unit_heads, scaled_heads, dk, q_scale, unit_eps, bias, bias_dtype));
         BL_CHECK_LAUNCH("bl_conv_silu_unit");
         return 0;
     }
