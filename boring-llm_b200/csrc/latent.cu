@@ -36,10 +36,74 @@ latent_prep_kernel(const float* proj, int ld, int off_q, int q_rank, int off_kv,
                    int max_pages, int page_size, const float* __restrict__ inv_freq, float mscale, TT* __restrict__ cq,
                    TT* __restrict__ cache) {
     bl_pdl_trigger();
-    bl_pdl_wait();
     __shared__ float part[4];
     const int t = blockIdx.x;
     const float* row = proj + (size_t)t * ld;
+    // Rows that fit the threads' registers (PREP_KEEP values each of the query and of the key/value latent): both are asked for
+    // at once, the norms' weights, the token's page and its rotation even before the wait, and nothing is read twice. Sums in
+    // the order of the loops below. 8 rows of 384 + 288 values took 4.8 us of a decode step's chain read piece by piece.
+    constexpr int PREP_KEEP = 8;
+    if (q_rank <= PREP_KEEP * THREADS && rank <= PREP_KEEP * THREADS && rot_dim <= THREADS) {
+        float wq[PREP_KEEP], wk[PREP_KEEP], zq[PREP_KEEP], zk[PREP_KEEP];
+        const int j = threadIdx.x;
+        float c = 1.f, sn = 0.f;
+        TT* dst = nullptr;
+#pragma unroll
+        for (int i = 0; i < PREP_KEEP; ++i) {
+            const int e = threadIdx.x + i * THREADS;
+            wq[i] = cq && e < q_rank ? bl_load_any(qw, qw_dtype, e) : 0.f;
+            wk[i] = cache && e < rank ? bl_load_any(kw, kw_dtype, e) : 0.f;
+        }
+        if (cache) {
+            const int pos = positions[t];
+            const int page = block_table[(size_t)tok_req[t] * max_pages + pos / page_size];
+            dst = cache + ((size_t)page * page_size + pos % page_size) * (rank + rot_dim);
+            if (j < rot_half) {
+                const float a = (float)pos * inv_freq[j];
+                c = cosf(a) * mscale; sn = sinf(a) * mscale;
+            }
+        }
+        bl_pdl_wait();
+        float rot_u = 0.f, rot_v = 0.f;
+#pragma unroll
+        for (int i = 0; i < PREP_KEEP; ++i) {
+            const int e = threadIdx.x + i * THREADS;
+            zq[i] = cq && e < q_rank ? row[off_q + e] : 0.f;
+            zk[i] = cache && e < rank ? row[off_kv + e] : 0.f;
+        }
+        if (cache && j < rot_half) { rot_u = row[off_kv + rank + j]; rot_v = row[off_kv + rank + rot_half + j]; }
+        else if (cache && j >= 2 * rot_half && j < rot_dim) rot_u = row[off_kv + rank + j];
+        if (cq) {
+            float s = 0.f;
+#pragma unroll
+            for (int i = 0; i < PREP_KEEP; ++i) if (threadIdx.x + i * THREADS < q_rank) s += zq[i] * zq[i];
+            const float inv = 1.0f / sqrtf(block_sum(s, part) / (float)q_rank + eps);
+#pragma unroll
+            for (int i = 0; i < PREP_KEEP; ++i) {
+                const int e = threadIdx.x + i * THREADS;
+                if (e < q_rank) bl_store(cq + (size_t)t * q_rank + e, zq[i] * inv * wq[i]);
+            }
+        }
+        if (cache) {
+            float s = 0.f;
+#pragma unroll
+            for (int i = 0; i < PREP_KEEP; ++i) if (threadIdx.x + i * THREADS < rank) s += zk[i] * zk[i];
+            const float inv = 1.0f / sqrtf(block_sum(s, part) / (float)rank + eps);
+#pragma unroll
+            for (int i = 0; i < PREP_KEEP; ++i) {
+                const int e = threadIdx.x + i * THREADS;
+                if (e < rank) bl_store(dst + e, zk[i] * inv * wk[i]);
+            }
+            if (j < rot_half) {
+                bl_store(dst + rank + j, rot_u * c - rot_v * sn);
+                bl_store(dst + rank + rot_half + j, rot_v * c + rot_u * sn);
+            } else if (j >= 2 * rot_half && j < rot_dim) {
+                bl_store(dst + rank + j, rot_u);                                   // not rotated
+            }
+        }
+        return;
+    }
+    bl_pdl_wait();
     if (cq) {
         const float* z = row + off_q;
         float s = 0.f;
@@ -97,11 +161,12 @@ __global__ void __launch_bounds__(THREADS)
 rope_heads_kernel(const float* q, size_t ld, size_t head_stride, int off, const int* __restrict__ positions,
                   const float* __restrict__ inv_freq, int n, int rot_half, float mscale, TO* __restrict__ out, size_t ld_out,
                   size_t out_head, int out_off, int H, const float* lead, int n_lead, TO* __restrict__ lead_out, size_t ld_lead,
-                  size_t lead_head) {
+                  size_t lead_head, int lead4) {
     bl_pdl_trigger();
-    bl_pdl_wait();
     extern __shared__ float cs[];                      // cos [rot_half], sin [rot_half]
     const int t = blockIdx.x;
+    // blocks of a token take its heads in equal shares (few tokens: more blocks, each a trip to L2 long)
+    const int h_first = (int)((long long)blockIdx.y * H / gridDim.y), heads = (int)((long long)(blockIdx.y + 1) * H / gridDim.y) - h_first;
     const int pos = positions[t];
     for (int j = threadIdx.x; j < rot_half; j += THREADS) {
         const float a = (float)pos * inv_freq[j];
@@ -109,8 +174,9 @@ rope_heads_kernel(const float* q, size_t ld, size_t head_stride, int off, const 
         cs[rot_half + j] = sinf(a) * mscale;
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < H * rot_half; e += THREADS) {
-        const int h = e / rot_half, j = e % rot_half;
+    bl_pdl_wait();                                     // (positions are the step's own index array)
+    for (int e = threadIdx.x; e < heads * rot_half; e += THREADS) {
+        const int h = h_first + e / rot_half, j = e % rot_half;
         const float* src = q + (size_t)t * ld + (size_t)h * head_stride + off;
         TO* dst = out + (size_t)t * ld_out + (size_t)h * out_head + out_off;
         const float u = src[j], v = src[rot_half + j];
@@ -118,13 +184,29 @@ rope_heads_kernel(const float* q, size_t ld, size_t head_stride, int off, const 
         bl_store(dst + rot_half + j, v * cs[j] + u * cs[rot_half + j]);
     }
     const int rest = n - 2 * rot_half;                 // values of a head's slice that are not rotated
-    for (int e = threadIdx.x; e < H * rest; e += THREADS) {
-        const int h = e / rest, d = 2 * rot_half + e % rest;
+    for (int e = threadIdx.x; e < heads * rest; e += THREADS) {
+        const int h = h_first + e / rest, d = 2 * rot_half + e % rest;
         bl_store(out + (size_t)t * ld_out + (size_t)h * out_head + out_off + d, q[(size_t)t * ld + (size_t)h * head_stride + off + d]);
     }
     // another slice of every head (the part of q that is not rotated), strided as q, cast into a tensor of its own
-    for (int e = threadIdx.x; e < H * n_lead; e += THREADS) {
-        const int h = e / n_lead, d = e % n_lead;
+    if (lead4) {                                       // four values a thread: whole 16-byte pieces
+        const int n4 = n_lead >> 2;
+#pragma unroll 4
+        for (int e = threadIdx.x; e < heads * n4; e += THREADS) {
+            const int h = h_first + e / n4, d = (e % n4) * 4;
+            const float4 v = *reinterpret_cast<const float4*>(lead + (size_t)t * ld + (size_t)h * head_stride + d);
+            TO* dst = lead_out + (size_t)t * ld_lead + (size_t)h * lead_head + d;
+            if constexpr (sizeof(TO) == 4) {
+                *reinterpret_cast<float4*>(dst) = v;
+            } else {
+                __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+                *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<unsigned*>(&a), *reinterpret_cast<unsigned*>(&b));
+            }
+        }
+        return;
+    }
+    for (int e = threadIdx.x; e < heads * n_lead; e += THREADS) {
+        const int h = h_first + e / n_lead, d = e % n_lead;
         bl_store(lead_out + (size_t)t * ld_lead + (size_t)h * lead_head + d, lead[(size_t)t * ld + (size_t)h * head_stride + d]);
     }
 }
@@ -226,6 +308,36 @@ __global__ void heads_gate_rows_kernel(const float* __restrict__ hv, const float
     }
 }
 
+// The same, four values a thread: N and the gate's row stride multiples of 4, 16-byte aligned. 2,000 rows of 16 x 128: 20 us of a
+// prefill's chain a value at a time (four 64-bit divisions each).
+template <typename TO>
+__global__ void heads_gate_rows4_kernel(const float* __restrict__ hv, const float* gate, size_t ld_gate, TO* __restrict__ out, int T, int H,
+                                        int N4, size_t Tp, int gate_heads) {
+    bl_pdl_trigger();
+    bl_pdl_wait();
+    const int t = blockIdx.x;
+    const float* gr = gate ? gate + (size_t)t * ld_gate : nullptr;
+#pragma unroll 2
+    for (int e = threadIdx.x; e < H * N4; e += blockDim.x) {
+        const int h = e / N4, n = (e % N4) * 4;
+        float4 v = *reinterpret_cast<const float4*>(hv + ((size_t)h * Tp + t) * N4 * 4 + n);
+        if (gate) {
+            float4 g;
+            if (gate_heads) { const float x = gr[h]; g = make_float4(x, x, x, x); }
+            else g = *reinterpret_cast<const float4*>(gr + 4 * (size_t)e);
+            v.x *= 1.0f / (1.0f + expf(-g.x)); v.y *= 1.0f / (1.0f + expf(-g.y));
+            v.z *= 1.0f / (1.0f + expf(-g.z)); v.w *= 1.0f / (1.0f + expf(-g.w));
+        }
+        TO* dst = out + ((size_t)t * H * N4 + e) * 4;
+        if constexpr (sizeof(TO) == 4) {
+            *reinterpret_cast<float4*>(dst) = v;
+        } else {
+            __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+            *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<unsigned*>(&a), *reinterpret_cast<unsigned*>(&b));
+        }
+    }
+}
+
 }  // namespace
 
 extern "C" int bl_head_tiles(int* tile, int n_heads, int per, void* stream) {
@@ -241,6 +353,13 @@ extern "C" int bl_heads_gate_rows(const float* hv, const float* gate, long long 
     if (T <= 0) return 0;
     if (H <= 0 || N <= 0 || Tp < T) BL_FAIL("bl_heads_gate_rows: bad sizes T=%d H=%d N=%d Tp=%d", T, H, N, Tp);
     cudaStream_t s = (cudaStream_t)stream;
+    if (N % 4 == 0 && (!gate || gate_heads || ld_gate % 4 == 0) && (((uintptr_t)hv | (uintptr_t)out | (gate_heads ? 0 : (uintptr_t)gate)) & 15) == 0 &&
+        (out_dtype == BL_F32 || out_dtype == BL_BF16) && (long long)H * N < (1LL << 30)) {
+        if (out_dtype == BL_F32) BL_CUDA(bl_launch_dependent(heads_gate_rows4_kernel<float>, dim3(T), dim3(256), 0, s, hv, gate, (size_t)ld_gate, (float*)out, T, H, N / 4, (size_t)Tp, gate_heads));
+        else BL_CUDA(bl_launch_dependent(heads_gate_rows4_kernel<__nv_bfloat16>, dim3(T), dim3(256), 0, s, hv, gate, (size_t)ld_gate, (__nv_bfloat16*)out, T, H, N / 4, (size_t)Tp, gate_heads));
+        BL_CHECK_LAUNCH("bl_heads_gate_rows");
+        return 0;
+    }
     const long long total = (long long)T * H * N;
     const int g = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
     if (out_dtype == BL_F32) BL_CUDA(bl_launch_dependent(heads_gate_rows_kernel<float>, dim3(g), dim3(256), 0, s, hv, gate, (size_t)ld_gate, (float*)out, T, H, N, (size_t)Tp, gate_heads));
@@ -302,9 +421,12 @@ extern "C" int bl_rope_heads(const float* q, long long ld, long long head_stride
     if (H <= 0 || off < 0 || out_off < 0 || rot_half < 0 || 2 * rot_half > n) BL_FAIL("bl_rope_heads: bad sizes H=%d n=%d pairs=%d offsets %d, %d", H, n, rot_half, off, out_off);
     cudaStream_t s = (cudaStream_t)stream;
     const size_t smem = (size_t)(2 * rot_half + 1) * sizeof(float);
-#define BL_GO(TO) BL_CUDA(bl_launch_dependent(rope_heads_kernel<TO>, dim3(T), dim3(THREADS), smem, s, q, (size_t)ld, (size_t)head_stride, off, \
+    const int shares = T <= 256 ? (H < 8 ? H : 8) : 1;             // (a launch of a few hundred blocks fills the device)
+    const int lead4 = n_lead > 0 && n_lead % 4 == 0 && ld % 4 == 0 && head_stride % 4 == 0 && ld_lead % 4 == 0 && lead_head % 4 == 0 &&
+                      (((uintptr_t)lead | (uintptr_t)lead_out) & 15) == 0;
+#define BL_GO(TO) BL_CUDA(bl_launch_dependent(rope_heads_kernel<TO>, dim3(T, shares), dim3(THREADS), smem, s, q, (size_t)ld, (size_t)head_stride, off, \
         positions, inv_freq, n, rot_half, mscale, (TO*)out, (size_t)ld_out, (size_t)out_head, out_off, H, lead, n_lead, (TO*)lead_out, \
-        (size_t)ld_lead, (size_t)lead_head))
+        (size_t)ld_lead, (size_t)lead_head, lead4))
     if (out_dtype == BL_F32) BL_GO(float);
     else if (out_dtype == BL_BF16) BL_GO(__nv_bfloat16);
     else BL_FAIL("bl_rope_heads: unknown dtype %d", out_dtype);

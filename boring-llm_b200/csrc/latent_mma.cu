@@ -308,26 +308,64 @@ latent_attention_mma_kernel(const LatentParams p) {
 }
 
 // The slices of one (request, head): out = sum_s o_s 2^(m_s - M) / (sum_s l_s 2^(m_s - M) + 2^(sink - M)), in slice order.
+// Bound by trips to L2: a lane holds a slice's maximum and sum, and a thread asks for its first column of up to MERGE_AHEAD
+// slices before it needs them. 8 requests of 14 heads in 16 slices took 7.6 us of a decode step's chain with one load after
+// the other (this, the latent rows' norms and the rotation of the heads together: a Miforax decode of 8 rows 730 -> 648 us).
+constexpr int MERGE_AHEAD = 16;
 __global__ void __launch_bounds__(128)
 latent_merge_kernel(const LatentParams p) {
     bl_pdl_trigger();
-    bl_pdl_wait();
     const int item = blockIdx.x / p.H, head = blockIdx.x % p.H;
     const int r = p.work[item];
     const int q_begin = p.cu_q[r];
-    if (p.cu_q[r + 1] - q_begin <= 0) return;
+    const bool live = p.cu_q[r + 1] - q_begin > 0;
+    float sk = -INFINITY;
+    if (p.sinks) sk = bl_load_any(p.sinks, p.sink_dtype, head) * 1.4426950408889634f;
+    bl_pdl_wait();
+    if (!live) return;
     const size_t prow = ((size_t)item * p.H + head) * p.n_splits;
+    __nv_bfloat16* dst = p.out + ((size_t)head * p.Tp + q_begin) * p.rank;
+    if (p.n_splits <= MERGE_AHEAD && p.rank <= 4 * 128) {
+        const int lane = threadIdx.x & 31;
+        float2 ml = make_float2(-INFINITY, 0.f);
+        if (lane < p.n_splits) ml = *reinterpret_cast<const float2*>(p.part_ml + 2 * (prow + lane));
+        float o[MERGE_AHEAD];
+        auto fetch = [&](int c) {
+#pragma unroll
+            for (int s = 0; s < MERGE_AHEAD; ++s) o[s] = s < p.n_splits && c < p.rank ? p.part_o[(prow + s) * p.rank + c] : 0.f;
+        };
+        fetch(threadIdx.x);
+        const float mm = fmaxf(bl_warp_max(ml.x), sk);
+        const float w = ml.x != -INFINITY ? exp2f(ml.x - mm) : 0.f;
+        float den = p.sinks ? exp2f(sk - mm) : 0.f;
+        float ws[MERGE_AHEAD];
+#pragma unroll
+        for (int s = 0; s < MERGE_AHEAD; ++s) {
+            ws[s] = __shfl_sync(0xffffffffu, w, s);
+            const float ls = __shfl_sync(0xffffffffu, ml.y, s), ms = __shfl_sync(0xffffffffu, ml.x, s);
+            if (s < p.n_splits && ms != -INFINITY) den += ls * ws[s];
+            else ws[s] = 0.f;
+        }
+        const float inv = den > 0.f ? 1.0f / den : 0.f;
+        for (int c = threadIdx.x; c < p.rank; c += 128) {
+            float acc = 0.f;
+#pragma unroll
+            for (int s = 0; s < MERGE_AHEAD; ++s)
+                if (ws[s] != 0.f) acc += o[s] * ws[s];     // (a slice without keys may hold anything)
+            dst[c] = __float2bfloat16_rn(acc * inv);
+            fetch(c + 128);
+        }
+        return;
+    }
     float mm = -INFINITY;
     for (int s = 0; s < p.n_splits; ++s) mm = fmaxf(mm, p.part_ml[2 * (prow + s)]);
-    float sk = -INFINITY;
-    if (p.sinks) { sk = bl_load_any(p.sinks, p.sink_dtype, head) * 1.4426950408889634f; mm = fmaxf(mm, sk); }
+    mm = fmaxf(mm, sk);
     float den = p.sinks ? exp2f(sk - mm) : 0.f;
     for (int s = 0; s < p.n_splits; ++s) {
         const float ms = p.part_ml[2 * (prow + s)];
         if (ms != -INFINITY) den += p.part_ml[2 * (prow + s) + 1] * exp2f(ms - mm);
     }
     const float inv = den > 0.f ? 1.0f / den : 0.f;
-    __nv_bfloat16* dst = p.out + ((size_t)head * p.Tp + q_begin) * p.rank;
     for (int c = threadIdx.x; c < p.rank; c += blockDim.x) {
         float acc = 0.f;
         for (int s = 0; s < p.n_splits; ++s) {

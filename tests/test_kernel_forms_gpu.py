@@ -179,3 +179,65 @@ def test_scan_in_parts(rule, H, dk, dv, lens, parts):
         close(out[lo:hi], w.reshape(hi - lo, -1), torch.float32, f"outputs of request {r}")
     close(st, want_state, torch.float32, "states")
     assert torch.equal(st[0].cpu(), state[0]) and torch.equal(st[R + 1].cpu(), state[R + 1])
+
+
+@pytest.mark.parametrize("taps,C,unit,dk", [(4, 96, 4, 16), (4, 2052, 2, 130), (4, 8200, 8, 1024), (3, 96, 4, 16), (4, 90, 4, 16)])
+def test_short_convolution_forms(taps, C, unit, dk):
+    """Four taps of channels in groups of four, and what does not fit that form, against 64 bits: requests that begin here,
+    go on from a slot's tail, have one token or none."""
+    o = ops()
+    lens = [5, 1, 0, 2, 40]
+    T, R = sum(lens), len(lens)
+    ld = C + 12
+    x, tail = data((T, ld), 3), data((R + 1, (taps - 1) * C + 4), 5)
+    w, bias = data((C, taps), 7), data((C,), 8)
+    slots = torch.tensor([4, 2, 0, 1, 3], dtype=torch.int32, device=DEV)
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32)
+    req = torch.repeat_interleave(torch.arange(R), torch.tensor(lens)).to(torch.int32)
+    for b in (None, bias):
+        y = torch.full((T, C), float("nan"), device=DEV)
+        o.conv_silu_unit(x, w, tail, slots, req.to(DEV), cu.to(DEV), y, unit, 1, dk, 0.25, 1e-6, bias=b)
+        for r in range(R):
+            lo, hi = int(cu[r]), int(cu[r + 1])
+            if lo == hi:
+                continue
+            rows = torch.cat([tail[int(slots[r]), :(taps - 1) * C].view(taps - 1, C), x[lo:hi, :C]]).double().cpu()
+            z = sum(rows[i:i + hi - lo] * w[:, i].double().cpu() for i in range(taps)) + (0 if b is None else b.double().cpu())
+            z = z * torch.sigmoid(z)
+            u = z[:, :unit * dk].reshape(hi - lo, unit, dk)
+            u = u / torch.sqrt((u * u).sum(-1, keepdim=True) + 1e-6)
+            u[:, 0] *= 0.25
+            z[:, :unit * dk] = u.reshape(hi - lo, -1)
+            close(y[lo:hi], z, torch.float32, f"request {r}")
+
+
+@pytest.mark.parametrize("H,N,T,gate_heads", [(3, 20, 5, False), (2, 128, 300, True), (3, 18, 4, False), (1, 4, 1, None)])
+def test_gated_head_rows_forms(H, N, T, gate_heads):
+    o = ops()
+    Tp = T + 3
+    hv = data((H, Tp, N), 3)
+    gate = None if gate_heads is None else data((T, (H if gate_heads else H * N) + 4), 4)
+    out = torch.empty(T, H * N, dtype=BF, device=DEV)
+    o.heads_gate_rows(hv, None if gate is None else gate[:, :(H if gate_heads else H * N)], out, gate_heads=bool(gate_heads))
+    want = hv[:, :T].double().cpu().permute(1, 0, 2)
+    if gate is not None:
+        g = torch.sigmoid(gate.double().cpu())
+        want = want * (g[:, :H, None] if gate_heads else g[:, :H * N].view(T, H, N))
+    close(out, want.reshape(T, H * N), BF, "gated rows")
+
+
+@pytest.mark.parametrize("d,top", [(4, 1), (36, 3), (2052, 2), (30, 2), (1028, 9)])
+@pytest.mark.parametrize("add", [False, True])
+def test_combined_expert_rows_forms(d, top, add):
+    o = ops()
+    T = 7
+    y, x = data((T * top + 5, d), 3), data((T, d), 4).to(BF)
+    pos = (torch.arange(T * top, dtype=torch.int32) * 3) % (T * top + 5)
+    pos[::4] = -1                                             # pairs without a row: the token's own
+    wts, out = data((T, top), 6), data((T, d), 7)
+    want = out.double().cpu() if add else torch.zeros(T, d, dtype=torch.float64)
+    for p in range(T * top):
+        row = x[p // top] if pos[p] < 0 else y[int(pos[p])]
+        want[p // top] += wts[p // top, p % top].double().cpu() * row.double().cpu()
+    o.moe_combine_rows(y, pos.to(DEV), wts, out, add=add, x=x)
+    close(out, want, torch.float32, "combined rows")
