@@ -176,6 +176,7 @@ int bl_stamp(unsigned long long* buf, int slot, void* stream);
 // arithmetic per byte loaded into shared memory. Same contract as bl_gemm_tc.
 int bl_gemm_tc_pair(const void* x, const void* w, const void* bias, int bias_dtype, void* out, int out_dtype,
                     int M, int N, int K, int epilogue, void* stream);
+int bl_gemm_tc_pair_act(const void* x, const void* w, void* y, float* rest, int M, int N, int n_act, int K, int act, void* stream);
 int bl_gemm_tc_pair_status(int* status);
 
 // The same product for shapes with few output tiles: a cluster of up to eight blocks shares a tile of 128 rows and

@@ -1080,6 +1080,12 @@ def linear_act(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: int, fa
     rows_w = w.shape[0]
     if rows_w < N:
         raise KernelError("linear_act: w has fewer rows than out has columns")
+    if (out.dtype == torch.bfloat16 and out.is_contiguous() and out.data_ptr() % 16 == 0 and rows_w % 4 == 0 and N % 4 == 0
+            and gemm_kernel(x, w, rows_w, None, EPI_NONE, fast) == "pair"):      # many rows: the activation in the product's epilogue
+        _need(x, "x", torch.bfloat16, (M, w.shape[1])); _need(w, "w", torch.bfloat16)
+        rest = torch.empty((M, rows_w - N), dtype=torch.float32, device=x.device) if rows_w > N else None
+        _call(_lib().bl_gemm_tc_pair_act, _p(x), _p(w), _p(out), _p(rest), M, rows_w, N, w.shape[1], act, _stream())
+        return rest
     sums = torch.empty((M, rows_w), dtype=torch.float32, device=x.device)
     gemm(x, w, sums, None, EPI_NONE, fast=fast)
     activation(sums[:, :N], out, act)

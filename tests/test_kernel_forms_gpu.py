@@ -241,3 +241,42 @@ def test_combined_expert_rows_forms(d, top, add):
         want[p // top] += wts[p // top, p % top].double().cpu() * row.double().cpu()
     o.moe_combine_rows(y, pos.to(DEV), wts, out, add=add, x=x)
     close(out, want, torch.float32, "combined rows")
+
+
+@pytest.mark.parametrize("M,N,n_act,K", [(256, 8, 4, 64), (300, 200, 200, 72), (700, 1000, 620, 136), (2048, 5760, 4864, 64), (257, 300, 36, 8)])
+@pytest.mark.parametrize("act", [0, 1, 2])
+def test_activation_in_the_epilogue_of_the_product_on_pairs(M, N, n_act, K, act):
+    """The activated columns and the further 32-bit columns behind them equal the product and the activation in launches of their
+    own, bit for bit; widths that cut a chunk of 32 columns, tiles of 128 and of 256, no further columns."""
+    o = ops()
+    x, w = (data((M, K), 1) * 0.5).to(BF), (data((N, K), 2) * 0.3).to(BF)
+    sums = torch.empty(M, N, device=DEV)
+    o.gemm_tc_pair(x, w, sums)
+    want = torch.empty(M, n_act, dtype=BF, device=DEV)
+    o.activation(sums[:, :n_act], want, act)
+    y = torch.full((M, n_act), float("nan"), dtype=BF, device=DEV)
+    assert o.gemm_kernel(x, w, N, None, o.EPI_NONE) == "pair"
+    rest = o.linear_act(x, w, y, act)
+    o.check_status()
+    assert torch.equal(y, want)
+    assert (rest is None) == (N == n_act) and (rest is None or torch.equal(rest, sums[:, n_act:]))
+
+
+@pytest.mark.parametrize("K", [4, 28, 32, 36, 896])
+@pytest.mark.parametrize("M,N", [(1, 16), (3, 70), (17, 33), (65, 100), (366, 257)])
+def test_32_bit_product_does_not_depend_on_the_rows_beside_a_row(M, N, K):
+    """The 32-bit tiles (chosen by the number of rows) at edges of rows, columns and stages, with rows of x that lie further apart
+    than they are long: 64 bits, and the same bits for a row alone."""
+    o = ops()
+    full = data((M, K + 8), 1)
+    x, w, b = full[:, :K], data((N, K), 2) * 0.3, data((N,), 3)
+    out = torch.empty(M, N, device=DEV)
+    xc = x.contiguous()
+    o.gemm_plain(xc, w, out, b, o.EPI_BIAS)
+    close(out, xc.double().cpu() @ w.double().cpu().T + b.double().cpu(), torch.float32, "product")
+    one = torch.empty(1, N, device=DEV)
+    o.gemm_plain(xc[M // 2:M // 2 + 1], w, one, b, o.EPI_BIAS)
+    assert torch.equal(one[0], out[M // 2])
+    strided = torch.empty(M, N, device=DEV)
+    o.gemm_plain(x, w, strided, b, o.EPI_BIAS)
+    assert torch.equal(strided, out)
