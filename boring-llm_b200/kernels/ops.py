@@ -637,6 +637,9 @@ COLS_MIN_COLUMNS = 9473               # up to 32 rows the output head's kernel t
 PAIR_MIN_ROWS = 256                   # from here on pairs of SMs share 256 x 256 tiles (tcgen05 cta_group::2)
 SPLITK_MIN_ROWS, SPLITK_MAX_ROWS = 32, 640   # products with few tiles in this range of rows are cut along K over clusters ...
 SPLITK_VERY_LONG_K = 16384            # ... or, below 32 rows, very long (K 18,944 by N 3,584 at 8 rows: 43 us against 72 us through registers)
+SPLITK_FEW_ROWS_K = 8192              # ... or, from 9 rows, this long (16 rows of K 11,008 by N 2,048: 12.9 us against 23.6 through registers, of 8,960 by
+                                      # 1,536 10.3 against 14.8; of 4,864 by 896 7.1 against 4.8), from 17 rows
+SPLITK_MORE_ROWS_K = 4096             # ... this long (24 rows of 4,864 by 896: 7.1 against 12.3, of 4,096 by 1,024 6.8 against 10.2; of 2,048 by 2,048 7.4 against 5.4)
 STREAM_MIN_BYTES = 128 << 20          # matrices from this size on stream faster through TMA and tcgen05 than through registers, at any number of rows
 SPLITK_LONG_K = 2048                  # ... when K is long (measured: K 4,864 by N 896 gains 2x at 128 rows, 1.25x at 512; K 896 gains only up to 128 rows)
 
@@ -679,7 +682,8 @@ def gemm_kernel(x: torch.Tensor, w: torch.Tensor, N: int, bias: Optional[torch.T
     if ((N >= TC_MIN_COLUMNS_VERY_FEW_ROWS or (N >= COLS_MIN_COLUMNS and M <= 32)) and bias is None and epilogue == EPI_NONE
             and M <= 64 and gemm_tc_cols_supported(x, w)):
         return "cols"
-    if (epilogue != EPI_SWIGLU and M <= SPLITK_MAX_ROWS and (M >= SPLITK_MIN_ROWS or K >= SPLITK_VERY_LONG_K)
+    if (epilogue != EPI_SWIGLU and M <= SPLITK_MAX_ROWS
+            and (M >= SPLITK_MIN_ROWS or K >= SPLITK_VERY_LONG_K or (M > 8 and K >= SPLITK_FEW_ROWS_K) or (M > 16 and K >= SPLITK_MORE_ROWS_K))
             and (K >= SPLITK_LONG_K or 64 < M <= 128) and gemm_tc_splitk_split(M, N, K, epilogue) >= 2):
         return "splitk"
     if M <= SKINNY_MAX_ROWS and not few_rows_tc:

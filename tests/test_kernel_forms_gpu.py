@@ -280,3 +280,19 @@ def test_32_bit_product_does_not_depend_on_the_rows_beside_a_row(M, N, K):
     strided = torch.empty(M, N, device=DEV)
     o.gemm_plain(x, w, strided, b, o.EPI_BIAS)
     assert torch.equal(strided, out)
+
+
+@pytest.mark.parametrize("M,N,K,kind", [(8, 256, 8192, "skinny"), (9, 256, 8192, "splitk"), (16, 200, 8200, "splitk"), (16, 256, 8184, "skinny"),
+                                        (17, 136, 4096, "splitk"), (31, 1024, 4104, "splitk"), (16, 256, 4096, "skinny"),
+                                        (32, 9473, 72, "cols"), (1, 9480, 520, "cols"), (8, 9472, 72, "skinny")])
+def test_products_of_few_rows_at_the_lines_between_their_kernels(M, N, K, kind):
+    """The kernel that the dispatch takes on either side of a line, and its result against 64 bits."""
+    o = ops()
+    x, w = (data((M, K), 1) * 0.5).to(BF), (data((N, K), 2) * 0.2).to(BF)
+    epi = o.EPI_NONE if kind == "cols" or N == 9472 else o.EPI_RESIDUAL
+    out = data((M, N), 3)
+    want = x.double().cpu() @ w.double().cpu().T + (out.double().cpu() if epi == o.EPI_RESIDUAL else 0.0)
+    assert o.gemm_kernel(x, w, N, None, epi) == kind
+    o.gemm(x, w, out, None, epi)
+    o.check_status()
+    close(out, want, BF, "product")
