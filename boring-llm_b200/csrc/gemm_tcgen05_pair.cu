@@ -208,6 +208,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     for (int u = 0; u < KS; ++u) tma_load_2d_pair(a_dst + u * A_BYTES, &map_a, full0 + 8 * s, (kb * KS + u) * BK, m0);
                 }
             }
+            // the commits on the stages of the last round, which no refill waits for (done when the last tile is)
+            for (int j = max(0, it - STAGES); j < it; ++j)
+                if (!mbar_wait(empty0 + 8 * (j % STAGES), (j / STAGES) & 1, give_up, 1)) break;
         }
     } else if (warp == 1) {
         if (leader && elect_one()) {
@@ -382,7 +385,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 if (!landed) break;
                 fence_before_sync();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_leader(acc_empty0 + 8 * buf);
+                if (lane == 0 && t + 2 * n_pairs < total_tiles) mbar_arrive_leader(acc_empty0 + 8 * buf);
                 continue;
             }
             if (PRELOAD && half < CHUNKS) preload(half);
@@ -508,18 +511,22 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     if ((lane & 7) == 0 && m < M) nl.ss_out[(size_t)m * parts + part] = q;
                 }
             }
-            // this warp is done with the buffer: tell the issuer (in the leader block)
+            // this warp is done with the buffer: tell the issuer (in the leader block), if a tile is left that waits for it
             fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive_leader(acc_empty0 + 8 * buf);
+            if (lane == 0 && t + 2 * n_pairs < total_tiles) mbar_arrive_leader(acc_empty0 + 8 * buf);
         }
     }
     __syncwarp();
     fence_before_sync();
     __syncthreads();
-    // neither block leaves while the other's MMAs may still read its memory (they are done: the epilogue has seen them;
-    // nothing is published here, so this barrier does not wait for the stores on their way)
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    // Neither block leaves while the other, or an arrival on its way, may still reach into its memory. By here nothing is on its
+    // way: the epilogues have seen every tile's MMAs done, the issuer has waited for every arrival on acc_empty and the loaders
+    // for every commit on empty. So the barrier orders nothing, and it does not wait for the stores on their way either (with
+    // a release a launch of 256 x 256 x 64 takes 4.2 us instead of 4.0, one of 2,048 x 896 x 896 8.7 instead of 8.1). Where a
+    // wait gave up, arrivals may be under way, and it releases.
+    if (*give_up) cluster_sync();
+    else asm volatile("barrier.cluster.arrive.relaxed.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (warp == 0) {
         fence_after_sync();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(TMEM_COLS) : "memory");

@@ -296,3 +296,20 @@ def test_products_of_few_rows_at_the_lines_between_their_kernels(M, N, K, kind):
     o.gemm(x, w, out, None, epi)
     o.check_status()
     close(out, want, BF, "product")
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 256, 64), (300, 19000, 72), (513, 40000, 136), (2048, 896, 896)])
+def test_products_on_pairs_one_behind_the_other(M, N, K):
+    """One to five tiles a pair, launch upon launch (the next one's blocks move in as the last one's leave): the same bits
+    every time, and those are the product's."""
+    o = ops()
+    x, w = (data((M, K), 1) * 0.5).to(BF), (data((N, K), 2) * 0.2).to(BF)
+    outs = [torch.full((M, N), float("nan"), device=DEV) for _ in range(4)]
+    for i in range(40):
+        o.gemm_tc_pair(x, w, outs[i % 4])
+        if i % 4 == 3:
+            assert all(torch.equal(outs[0], t) for t in outs[1:])
+    o.check_status()
+    want = torch.empty(M, N, device=DEV)
+    o.gemm_plain(x, w, want)
+    close(outs[0], want.double(), torch.float32, "product")
