@@ -160,6 +160,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // Tensor memory is taken before the wait for the kernel before: whoever on this stream uses it triggers its successor
     // only behind its own allocation, so an allocation that has to wait here waits for a block that needs nothing from us.
     if (warp == 0) {
+        __syncwarp();                                                // (its first lane comes from setting up the barriers)
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
                      :: "r"(smem_u32((const void*)tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");

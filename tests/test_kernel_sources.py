@@ -55,3 +55,14 @@ def test_every_arrival_in_the_product_on_pairs_is_waited_for(n_pairs, stages):
                 tail = [(j, (j // stages) & 1) for j in range(max(0, it - stages), it)]
                 assert [w for w, _ in refills + tail] == list(range(it))
                 assert all(parity == (w // stages) & 1 for w, parity in refills + tail)
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
+def test_warps_meet_before_they_take_or_free_tensor_memory(path):
+    """tcgen05.alloc and dealloc are for a whole warp at once: behind code of one thread (setting up barriers, first copies) the
+    warp's lanes meet before them."""
+    text = code(path)
+    for at in [m.start() for m in re.finditer(r"tcgen05\.(?:de)?alloc\b", text)]:
+        before = text[:at]
+        alone = max(before.rfind(s) for s in ("threadIdx.x == 0", "lane == 0", "elect_one()"))
+        assert alone >= 0 and re.search(r"__syncwarp\(\)|__syncthreads\(\)", before[alone:])
