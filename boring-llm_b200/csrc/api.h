@@ -297,17 +297,17 @@ int bl_gemm_plain_decay(const float* x, int ldx, const void* w, int w_dtype, con
 int bl_recurrent_scan(int rule, const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
                       const float* a, int lda, const float* beta, int ldb, float q_scale, float* state, long long slot_stride, const int* slots, const int* cu_q, int R,
                       float* out, int H, int G, int dk, int dv, void* stream);
-// The same with long portions cut into nc parts that run side by side (requests with 256 tokens or more in the step;
-// linear attention with key sizes that bl_recurrent_scan_can_split takes): every part first runs from a zero state, then
-// from the request's state folded through the parts before it, and a fold leaves the slot (the delta rule's fold, a
-// product with the part's key x key transition, runs between the passes). scratch: bl_recurrent_scan_parts_scratch
-// floats. nc 1: bl_recurrent_scan.
-long long bl_recurrent_scan_parts_scratch(int rule, int R, int nc, int H, int dk, int dv);
+// The same with long portions cut into nc parts that run side by side (of the first n_cut requests with 256 tokens or more
+// in the step; key sizes that bl_recurrent_scan_can_split takes): every part first runs from a zero state, a fold takes the
+// request's state through the parts (by a decay per row, or, delta rule, by the part's key x key transition) and leaves the
+// slot and every part's start, then every part runs from its start. scratch: bl_recurrent_scan_parts_scratch floats. nc 1:
+// bl_recurrent_scan.
+long long bl_recurrent_scan_parts_scratch(int rule, int n_cut, int nc, int H, int dk, int dv);
 int bl_recurrent_scan_can_split(int rule, int H, int dk, int dv);   // 0, or the blocks one request's portion runs on
 int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
                             const float* a, int lda, const float* beta, int ldb, float q_scale, float* state,
                             long long slot_stride, const int* slots, const int* cu_q, int R, float* out, int H, int G,
-                            int dk, int dv, int nc, float* scratch, void* stream);
+                            int dk, int dv, int nc, int n_cut, float* scratch, void* stream);
 // y[t, h, :] = o[t, h, :] / sqrt(mean(o^2) + eps) * w[:] * gate(g[t * ld_gate + h * dv + :]) (gate null: none).
 #define BL_GATE_SIGMOID 0
 #define BL_GATE_SILU 1

@@ -180,6 +180,17 @@ recurrent_scan_kernel(const float* q, int ldq, const float* k, int ldk, const fl
     }
 }
 
+// Of the requests whose portions are long enough to be cut, how many stand before r: its place in the scratch, which holds the
+// cut requests only (not the running ones beside them). All threads of the block come here.
+__device__ __forceinline__ int scan_cut_place(const int* __restrict__ cu_q, int r) {
+    int n = 0;
+    for (int i0 = 0; i0 < r; i0 += blockDim.x) {
+        const int i = i0 + threadIdx.x;
+        n += __syncthreads_count(i < r && cu_q[i + 1] - cu_q[i] >= SCAN_SPLIT_MIN);
+    }
+    return n;
+}
+
 // The same walk for key sizes that split evenly: a lane holds RK4 * 4 CONSECUTIVE rows of its column (dk = KS * RK4 * 4),
 // so a token's q, k and decays reach its registers as 16-byte loads at fixed offsets, two tokens' registers take turns
 // (no copies), and the dot products run in two chains. Where a launch has few blocks a warp has no other warp on its
@@ -194,7 +205,7 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
                           const float* beta, int ldb, float q_scale,
                           float* state, size_t slot_stride, const int* __restrict__ slots, const int* __restrict__ cu_q,
                           float* out, int H, int G, int dk, int dv, int KS, int chunk, int vec,
-                          int nc, float* part_s, float* part_p, const float* part_start) {
+                          int nc, int n_cut, float* part_s, float* part_p, const float* part_start) {
     bl_pdl_trigger();
     bl_pdl_wait();
     extern __shared__ __align__(16) float sm[];
@@ -204,11 +215,13 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
     // (QUIET): every part from a ZERO state, leaving its own contribution S_part and its transition P (a product of decays a
     // row; of the delta rule a matrix). Between the passes a fold (S <- P S + S_part) leaves every part's start state in
     // scratch and the final state in the slot. Second pass: a part runs from its start state and writes the outputs. Short
-    // portions (and nc 1) take one block per (request, head, columns) through the second pass alone.
+    // portions (and nc 1, and long ones past the n_cut that scratch is there for) take one block per (request, head, columns)
+    // through the second pass alone.
     const int r = blockIdx.z / nc, part = blockIdx.z % nc, h = blockIdx.y;
     const int n_all = cu_q[r + 1] - cu_q[r];
     if (n_all <= 0) return;
-    const bool split = nc > 1 && n_all >= SCAN_SPLIT_MIN;
+    const int place = nc > 1 && n_all >= SCAN_SPLIT_MIN ? scan_cut_place(cu_q, r) : n_cut;
+    const bool split = place < n_cut;
     if (!split && (part != 0 || QUIET)) return;
     // (of more parts than tokens some are empty: they leave a zero state and the identity)
     const int t_first = split ? (int)((long long)part * n_all / nc) : 0;
@@ -260,7 +273,7 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
 
     issue(0, sm);
     float st[RK], pr[QUIET && !DELTA ? RK : 1];
-    const size_t part_base = ((size_t)r * nc) * H + h;           // + p * H for part p
+    const size_t part_base = ((size_t)place * nc) * H + h;       // + p * H for part p
 #pragma unroll
     for (int i = 0; i < RK; ++i) {
         if (QUIET) st[i] = (DELTA && c >= dv && row0 + i == c - dv) ? 1.f : 0.f;
@@ -400,14 +413,17 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
 constexpr int FOLD_COLS = 8, FOLD_MAX_DK = 128;
 __global__ void __launch_bounds__(256)
 scan_fold_matrix_kernel(float* state, size_t slot_stride, const int* __restrict__ slots, const int* __restrict__ cu_q,
-                        const float* part_s, const float* part_pm, float* part_start, int H, int dk, int dv, int nc) {
+                        const float* part_s, const float* part_pm, float* part_start, int H, int dk, int dv, int nc,
+                        int n_cut) {
     bl_pdl_trigger();
     bl_pdl_wait();
     __shared__ float cur[2][FOLD_MAX_DK][FOLD_COLS];
     const int r = blockIdx.z, h = blockIdx.y, c0 = blockIdx.x * FOLD_COLS;
     if (cu_q[r + 1] - cu_q[r] < SCAN_SPLIT_MIN) return;
+    const int place = scan_cut_place(cu_q, r);
+    if (place >= n_cut) return;
     float* S = state + (size_t)slots[r] * slot_stride + (size_t)h * dk * dv;
-    const size_t base = ((size_t)r * nc) * H + h;
+    const size_t base = ((size_t)place * nc) * H + h;
     const int col = threadIdx.x % FOLD_COLS, rg = threadIdx.x / FOLD_COLS;
     constexpr int GROUPS = 256 / FOLD_COLS;                                     // row groups
     const bool ok = c0 + col < dv;
@@ -443,13 +459,15 @@ scan_fold_matrix_kernel(float* state, size_t slot_stride, const int* __restrict_
 // The same where the transition is a decay per row: start[p + 1] = P_p o start[p] + S_part_p. Every part's start takes the
 // place of its contribution in part_s.
 __global__ void scan_fold_kernel(float* state, size_t slot_stride, const int* __restrict__ slots, const int* __restrict__ cu_q,
-                                 float* part_s, const float* part_p, int H, int dk, int dv, int nc) {
+                                 float* part_s, const float* part_p, int H, int dk, int dv, int nc, int n_cut) {
     bl_pdl_trigger();
     bl_pdl_wait();
     const int r = blockIdx.z, h = blockIdx.y;
     if (cu_q[r + 1] - cu_q[r] < SCAN_SPLIT_MIN) return;
+    const int place = scan_cut_place(cu_q, r);
+    if (place >= n_cut) return;
     float* S = state + (size_t)slots[r] * slot_stride + (size_t)h * dk * dv;
-    const size_t base = ((size_t)r * nc) * H + h;
+    const size_t base = ((size_t)place * nc) * H + h;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= dk * dv) return;
     const int row = e / dv;
@@ -857,7 +875,7 @@ extern "C" int bl_recurrent_scan(int rule, const float* q, int ldq, const float*
                                  const float* z, int ldz, const float* beta, int ldb, float q_scale, float* state, long long slot_stride, const int* slots, const int* cu_q, int R,
                                  float* out, int H, int G, int dk, int dv, void* stream) {
     return bl_recurrent_scan_parts(rule, q, ldq, k, ldk, v, ldv, z, ldz, beta, ldb, q_scale, state, slot_stride, slots, cu_q, R, out,
-                                   H, G, dk, dv, 1, nullptr, stream);
+                                   H, G, dk, dv, 1, 0, nullptr, stream);
 }
 
 // Whether bl_recurrent_scan_parts can cut long portions of this rule and key size (else it runs them in one piece):
@@ -874,18 +892,18 @@ extern "C" int bl_recurrent_scan_can_split(int rule, int H, int dk, int dv) {
     return 0;
 }
 
-// Floats of scratch that bl_recurrent_scan_parts needs.
-extern "C" long long bl_recurrent_scan_parts_scratch(int rule, int R, int nc, int H, int dk, int dv) {
+// Floats of scratch that bl_recurrent_scan_parts needs to cut n_cut requests.
+extern "C" long long bl_recurrent_scan_parts_scratch(int rule, int n_cut, int nc, int H, int dk, int dv) {
     const long long per = rule == BL_RULE_DELTA ? (long long)dk * (2 * dv + dk) : (long long)dk * (dv + 1);
-    return (long long)R * nc * H * per;
+    return (long long)n_cut * nc * H * per;
 }
 
 extern "C" int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
                                        const float* z, int ldz, const float* beta, int ldb, float q_scale, float* state,
                                        long long slot_stride, const int* slots, const int* cu_q, int R, float* out, int H, int G,
-                                       int dk, int dv, int nc, float* scratch, void* stream) {
+                                       int dk, int dv, int nc, int n_cut, float* scratch, void* stream) {
     if (R <= 0) return 0;
-    if (nc < 1 || (nc > 1 && (scratch == nullptr || !bl_recurrent_scan_can_split(rule, H, dk, dv) || (long long)R * nc > 65535)))
+    if (nc < 1 || (nc > 1 && (n_cut < 1 || n_cut > R || scratch == nullptr || !bl_recurrent_scan_can_split(rule, H, dk, dv) || (long long)R * nc > 65535)))
         BL_FAIL("bl_recurrent_scan_parts: %d parts for rule %d, %d key channels, %d requests", nc, rule, dk, R);
     if (H <= 0 || G <= 0 || H % G != 0 || dk <= 0 || dv <= 0) BL_FAIL("bl_recurrent_scan: bad sizes H=%d G=%d dk=%d dv=%d", H, G, dk, dv);
     if (dk > RKMAX * 32) BL_FAIL("bl_recurrent_scan: %d key channels, at most %d", dk, RKMAX * 32);
@@ -916,13 +934,13 @@ extern "C" int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const 
     if (rule != BL_RULE_GLA && rule != BL_RULE_DELTA && rule != BL_RULE_BONUS) BL_FAIL("bl_recurrent_scan: unknown rule %d", rule);
     if (rk4 > 0) {                                     // a lane's rows are whole groups of four
         const bool dl = rule == BL_RULE_DELTA;
-        float* part_s = scratch;                                                 // [R, nc, H, dk, dv]
-        float* part_p = scratch ? scratch + (size_t)R * nc * H * dk * dv : nullptr;   // [R, nc, H, dk] or, delta rule, [R, nc, H, dk, dk]
-        // [R, nc, H, dk, dv]; a fold with a decay per row leaves the starts in part_s
-        float* part_start = scratch == nullptr ? nullptr : dl ? part_p + (size_t)R * nc * H * dk * dk : part_s;
+        float* part_s = scratch;                                                 // [n_cut, nc, H, dk, dv]
+        float* part_p = scratch ? scratch + (size_t)n_cut * nc * H * dk * dv : nullptr;   // [n_cut, nc, H, dk] or, delta rule, [n_cut, nc, H, dk, dk]
+        // [n_cut, nc, H, dk, dv]; a fold with a decay per row leaves the starts in part_s
+        float* part_start = scratch == nullptr ? nullptr : dl ? part_p + (size_t)n_cut * nc * H * dk * dk : part_s;
         const int two_an_sm = 2 * scan_sms();
 #define BL_SCAN_Q(D, R4, DENSE, QUIET, GRID) BL_CUDA(bl_launch_dependent(recurrent_scan_vec_kernel<D, R4, DENSE, QUIET>, GRID, dim3(WARPS * 32), smem, s, \
-        q, ldq, k, ldk, v, ldv, z, ldz, beta, ldb, q_scale, state, (size_t)slot_stride, slots, cu_q, out, H, G, dk, dv, KS, chunk, vec, nc, \
+        q, ldq, k, ldk, v, ldv, z, ldz, beta, ldb, q_scale, state, (size_t)slot_stride, slots, cu_q, out, H, G, dk, dv, KS, chunk, vec, nc, n_cut, \
         part_s, part_p, (const float*)part_start))
 #define BL_SCAN(D, R4, PASS) do { \
         const dim3 g = (D == BL_RULE_DELTA && PASS == 1) ? grid_wide : grid; \
@@ -933,10 +951,10 @@ extern "C" int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const 
             if (pass == 2 && nc > 1 && dl)
                 BL_CUDA(bl_launch_dependent(scan_fold_matrix_kernel, dim3((dv + FOLD_COLS - 1) / FOLD_COLS, H, R), dim3(256), 0, s, state,
                                             (size_t)slot_stride, slots, cu_q, (const float*)part_s, (const float*)part_p, part_start,
-                                            H, dk, dv, nc));
+                                            H, dk, dv, nc, n_cut));
             if (pass == 2 && nc > 1 && !dl)
                 BL_CUDA(bl_launch_dependent(scan_fold_kernel, dim3((dk * dv + 255) / 256, H, R), dim3(256), 0, s, state, (size_t)slot_stride,
-                                            slots, cu_q, part_s, (const float*)part_p, H, dk, dv, nc));
+                                            slots, cu_q, part_s, (const float*)part_p, H, dk, dv, nc, n_cut));
             switch (rk4) {
 #define BL_SCAN_RULE(R4) do { if (dl) BL_SCAN(BL_RULE_DELTA, R4, pass); else if (rule == BL_RULE_BONUS) BL_SCAN(BL_RULE_BONUS, R4, pass); \
                                   else BL_SCAN(BL_RULE_GLA, R4, pass); } while (0)

@@ -982,7 +982,6 @@ def gemm_plain_decay(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tens
 SCAN_MAX_PARTS = 32               # most parts a long portion of a request is cut into
 SCAN_PART_MIN_TOKENS = 256        # requests with fewer tokens in a step are walked in one piece (the kernel's own rule)
 SCAN_BLOCKS_PER_SM = 4            # blocks of the scan kernel that an SM holds (its registers)
-SCAN_MAX_SCRATCH_PARTS = 1024     # parts x requests of a step that scratch is taken for
 
 
 def recurrent_scan_parts(rule: int, H: int, dk: int, dv: int, n_long: int) -> int:
@@ -1004,14 +1003,15 @@ def recurrent_scan_parts(rule: int, H: int, dk: int, dv: int, n_long: int) -> in
 
 def recurrent_scan(rule: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, beta: Optional[torch.Tensor],
                    q_scale: float, state: torch.Tensor, slots: torch.Tensor, cu_q: torch.Tensor, out: torch.Tensor,
-                   H: int, G: int, dk: int, dv: int, parts: int = 1) -> None:
+                   H: int, G: int, dk: int, dv: int, parts: int = 1, n_long: Optional[int] = None) -> None:
     """A linear recurrence over a matrix state per head and request (`RULE_GLA`, `RULE_DELTA`, `RULE_BONUS`, whose beta is
     a given number per token and head, see `bonus_dot`; see `bl_recurrent_scan`).
     q, k [T, G * dk], v [T, H * dv], decay [T, H * dk] (in (0, 1], see `gemm_plain_decay`), beta [T, H] (logits): 32-bit
     rows, possibly column ranges of a wider matrix. state: [slots, >= H * dk * dv] 32-bit, the matrix state first in each
     slot. out [T, H * dv] 32-bit, already times q_scale. `parts` > 1 (`recurrent_scan_parts`): portions of 256 tokens and
     more are cut into that many parts, which run side by side (twice the arithmetic on `parts` times the blocks; the
-    results differ from the walk in one piece by rounding only)."""
+    results differ from the walk in one piece by rounding only). `n_long`: how many requests that are (None: any may be);
+    scratch is taken for so many, and the first so many are cut."""
     T = out.shape[0]
     R = cu_q.shape[0] - 1
     ldq, ldk, ldv, ldz = (_rows32(q, "q", T, G * dk), _rows32(k, "k", T, G * dk), _rows32(v, "v", T, H * dv),
@@ -1021,14 +1021,14 @@ def recurrent_scan(rule: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     _need(out, "out", torch.float32, (T, H * dv))
     if not state.is_cuda or state.dtype != torch.float32 or state.dim() != 2 or state.stride(1) != 1 or state.shape[1] < H * dk * dv:
         raise KernelError("state: must be 32-bit [slots, >= H * dk * dv] with contiguous rows")
-    parts = min(parts, max(8, SCAN_MAX_SCRATCH_PARTS // max(1, R)))
-    if parts > 1:
+    n_cut = R if n_long is None else min(n_long, R)
+    if parts > 1 and n_cut > 0:
         lib = _lib()
         lib.bl_recurrent_scan_parts_scratch.restype = ctypes.c_longlong
-        scratch = torch.empty(int(lib.bl_recurrent_scan_parts_scratch(rule, R, parts, H, dk, dv)), dtype=torch.float32, device=out.device)
+        scratch = torch.empty(int(lib.bl_recurrent_scan_parts_scratch(rule, n_cut, parts, H, dk, dv)), dtype=torch.float32, device=out.device)
         _call(_lib().bl_recurrent_scan_parts, rule, _p(q), ldq, _p(k), ldk, _p(v), ldv, _p(decay), ldz, _p(beta), ldb,
               ctypes.c_float(q_scale), _p(state), ctypes.c_longlong(state.stride(0)), _p(slots), _p(cu_q), R,
-              _p(out), H, G, dk, dv, parts, _p(scratch), _stream())
+              _p(out), H, G, dk, dv, parts, n_cut, _p(scratch), _stream())
         return
     _call(_lib().bl_recurrent_scan, rule, _p(q), ldq, _p(k), ldk, _p(v), ldv, _p(decay), ldz, _p(beta), ldb,
           ctypes.c_float(q_scale), _p(state), ctypes.c_longlong(state.stride(0)), _p(slots), _p(cu_q), R,

@@ -37,26 +37,31 @@ class _StateMixer(Mixer):
 
     RULE = None                      # ops.RULE_GLA or ops.RULE_DELTA
 
-    def _parts(self, q_lens) -> int:
+    def _cut(self, q_lens) -> dict:
+        """Into how many parts a step's long portions are cut (they run side by side), and how many requests have one."""
         n_long = sum(1 for n in q_lens if n >= ops.SCAN_PART_MIN_TOKENS)
-        return ops.recurrent_scan_parts(self.RULE, self.H, self.dk, self.dv, n_long) if n_long else 1
+        parts = ops.recurrent_scan_parts(self.RULE, self.H, self.dk, self._value_columns(), n_long) if n_long else 1
+        return {"parts": parts, "n_long": n_long if parts > 1 else 0}
+
+    def _value_columns(self) -> int:
+        return self.dv                  # columns of a head's state
 
     def plan_step(self, q_lens, ctx_lens, filler=None):
-        """Into how many parts this step's long portions are cut (they run side by side): a launch shape, so part of what
-        names a captured step."""
-        parts = self._parts(q_lens)
-        return self._plan_key(), StepPlan(host={"parts": parts}, shape=(parts,))
+        """How the scan is launched: part of what names a captured step."""
+        cut = self._cut(q_lens)
+        return self._plan_key(), StepPlan(host=cut, shape=tuple(cut.values()))
 
     def _plan_key(self) -> str:
-        return f"recurrence parts {self.RULE} {self.H}x{self.dk}x{self.dv}"       # layers of equal sizes share the plan
+        return f"recurrence parts {self.RULE} {self.H}x{self.dk}x{self._value_columns()}"       # layers of equal sizes share the plan
 
-    def _step_parts(self, ctx) -> int:
+    def _step_cut(self, ctx) -> dict:
+        """The arguments of `recurrent_scan` that say how long portions are cut."""
         if not ctx.fast:
-            return 1
+            return {}
         plan = ctx.plans.get(self._plan_key())
         if plan is not None:
-            return plan.host["parts"]
-        return self._parts(ctx.q_lens) if ctx.q_lens else 1       # a step put together without asking the parts
+            return plan.host
+        return self._cut(ctx.q_lens) if ctx.q_lens else {}       # a step put together without asking the parts
 
     @staticmethod
     def _check(write_cache):
@@ -117,7 +122,7 @@ class GatedLinearAttention(_StateMixer):
         o = ctx.empty((T, H * dv), torch.float32)
         ops.recurrent_scan(ops.RULE_GLA, proj[:, :self.off_k], proj[:, self.off_k:self.off_v], proj[:, self.off_v:self.off_g],
                            decay, None, dk ** -0.5, ctx.state(cache_layer), ctx.slots, ctx.cu_q, o, H, H, dk, dv,
-                           parts=self._step_parts(ctx))
+                           **self._step_cut(ctx))
         y = ctx.empty((T, H * dv))
         ops.head_norm_gate(o, self.norm, proj[:, self.off_g:self.off_a], ops.GATE_SILU, self.eps, y, H, dv)
         linear(ctx, y, self.wo, out, None, epilogue)
@@ -196,7 +201,7 @@ class ChannelDeltaRule(_StateMixer):
         o = ctx.empty((T, H * dv), torch.float32)
         ops.recurrent_scan(ops.RULE_DELTA, qkv[:, :G * dk], qkv[:, G * dk:2 * G * dk], qkv[:, 2 * G * dk:], decay,
                            proj[:, self.off_b:self.off_a], 1.0, state, ctx.slots, ctx.cu_q, o, H, G, dk, dv,
-                           parts=self._step_parts(ctx))
+                           **self._step_cut(ctx))
         y = ctx.empty((T, H * dv))
         ops.head_norm_gate(o, self.norm, glog, ops.GATE_SIGMOID, self.eps, y, H, dv)
         linear(ctx, y, self.wo, out, None, epilogue)
@@ -245,12 +250,8 @@ class MatrixMemory(_StateMixer):
     def cache_spec(self):
         return StateSpec((self.H * self.dk * (self.dv + 1) + self.H,), "float32")
 
-    def _parts(self, q_lens) -> int:
-        n_long = sum(1 for n in q_lens if n >= ops.SCAN_PART_MIN_TOKENS)
-        return ops.recurrent_scan_parts(self.RULE, self.H, self.dk, self.dv + 1, n_long) if n_long else 1
-
-    def _plan_key(self) -> str:
-        return f"recurrence parts {self.RULE} {self.H}x{self.dk}x{self.dv + 1}"
+    def _value_columns(self) -> int:
+        return self.dv + 1
 
     def _run(self, ctx, h, out, cache_layer, write_cache, epilogue):
         self._check(write_cache)
@@ -263,7 +264,7 @@ class MatrixMemory(_StateMixer):
                                                       self.cap, state, self.off_m, ctx.slots, ctx.cu_q, H, dk, dv)
         o = ctx.empty((T, H * (dv + 1)), torch.float32)      # a head's last column: n . q
         ops.recurrent_scan(ops.RULE_GLA, proj[:, :self.off_k], keys, values, decay, None, dk ** -0.5, state, ctx.slots, ctx.cu_q, o,
-                           H, H, dk, dv + 1, parts=self._step_parts(ctx))
+                           H, H, dk, dv + 1, **self._step_cut(ctx))
         y = ctx.empty((T, H * dv))
         ops.head_norm_gate_ext(o, self.norm, proj[:, self.off_g:self.off_i], ops.GATE_SIGMOID, self.eps, y, H, dv, floor=floor)
         linear(ctx, y, self.wo, out, None, epilogue)
@@ -335,7 +336,7 @@ class ShiftedDecayRecurrence(_StateMixer):
         ops.bonus_dot(r, k, self.u, bonus, H, dk)
         o = ctx.empty((T, H * dk), torch.float32)
         ops.recurrent_scan(ops.RULE_BONUS, r, k, v, decay, bonus, 1.0, state, ctx.slots, ctx.cu_q, o, H, H, dk, dk,
-                           parts=self._step_parts(ctx))
+                           **self._step_cut(ctx))
         y = ctx.empty((T, H * dk))
         ops.head_norm_gate_ext(o, self.norm, g, ops.GATE_SILU, self.eps, y, H, dk)
         linear(ctx, y, self.wo, out, None, epilogue)
@@ -395,7 +396,7 @@ class Retention(_StateMixer):
                                           rot.rot_half if rot is not None else 0, self.head_decay, dk ** -0.5, H, dk)
         o = ctx.empty((T, H * dv), torch.float32)
         ops.recurrent_scan(ops.RULE_GLA, q, k, proj[:, self.off_v:self.off_g], decay, None, 1.0, ctx.state(cache_layer), ctx.slots,
-                           ctx.cu_q, o, H, H, dk, dv, parts=self._step_parts(ctx))
+                           ctx.cu_q, o, H, H, dk, dv, **self._step_cut(ctx))
         y = ctx.empty((T, H * dv))
         ops.head_norm_gate(o, None, proj[:, self.off_g:self.off_g + H * dv], ops.GATE_SILU, self.eps, y, H, dv)
         linear(ctx, y, self.wo, out, None, epilogue)
@@ -466,7 +467,7 @@ class StateSpaceDuality(_StateMixer):
         decay, v = ops.ssd_prep(proj[:, self.off_dt:self.off_dt + H], self.dt_bias, self.rate, x, H, N, dv)
         o = ctx.empty((T, inner), torch.float32)
         ops.recurrent_scan(ops.RULE_GLA, xbc[:, inner + G * N:], xbc[:, inner:inner + G * N], v, decay, None, 1.0, state, ctx.slots,
-                           ctx.cu_q, o, H, G, N, dv, parts=self._step_parts(ctx))
+                           ctx.cu_q, o, H, G, N, dv, **self._step_cut(ctx))
         y = ctx.empty((T, inner))
         ops.gated_group_norm(o, x, self.skip, dv, proj[:, :inner], self.norm, self.norm_groups, self.eps, y)
         linear(ctx, y, self.wo, out, None, epilogue)

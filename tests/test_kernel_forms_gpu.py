@@ -181,6 +181,41 @@ def test_scan_in_parts(rule, H, dk, dv, lens, parts):
     assert torch.equal(st[0].cpu(), state[0]) and torch.equal(st[R + 1].cpu(), state[R + 1])
 
 
+@pytest.mark.parametrize("rule", ["RULE_GLA", "RULE_DELTA", "RULE_BONUS"])
+@pytest.mark.parametrize("lens,n_long", [([3, 300, 1, 0, 257, 1], 2), ([1] * 130 + [256, 1, 400], 2), ([300, 270, 1, 290], 1), ([1, 260], 0)])
+def test_scan_keeps_scratch_for_the_requests_that_are_cut(rule, lens, n_long):
+    """Long portions among short ones: scratch by long request and not by request; long portions past the number given (the last
+    two cases) are walked in one piece. Outputs and states against 64 bits."""
+    o = ops()
+    rule = getattr(o, rule)
+    H, dk, dv, parts = 2, 32, 40, 6
+    T, R = sum(lens), len(lens)
+    g = torch.Generator().manual_seed(T)
+    rnd = lambda *n: torch.randn(*n, generator=g)
+    q, k, v, b = rnd(T, H * dk) * 0.3, rnd(T, H * dk), rnd(T, H * dv), rnd(T, H)
+    k = (k.view(T, H, dk) / k.view(T, H, dk).norm(dim=-1, keepdim=True)).reshape(T, H * dk)
+    a = torch.sigmoid(rnd(T, H * dk) + 3.0)
+    state = rnd(R, H * dk * dv)
+    cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).to(torch.int32)
+    args = [t.to(DEV) for t in (q, k, v, a)] + [None if rule == o.RULE_GLA else b.to(DEV), 0.5]
+    st, out = state.to(DEV), torch.full((T, H * dv), float("nan"), device=DEV)
+    slots, cud = torch.arange(R, dtype=torch.int32, device=DEV), cu.to(DEV)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    o.recurrent_scan(rule, *args, st, slots, cud, out, H, H, dk, dv, parts=parts, n_long=n_long)
+    per = dk * (2 * dv + dk) if rule == o.RULE_DELTA else dk * (dv + 1)
+    assert torch.cuda.max_memory_allocated() - before <= n_long * parts * H * per * 4 + 512
+    want_state = state.double()
+    for r in range(R):
+        lo, hi = int(cu[r]), int(cu[r + 1])
+        if hi > lo:
+            w = _scan64(rule, *(x[lo:hi].double().view(hi - lo, H, -1) for x in (q, k, v, a)), b[lo:hi].double(), 0.5,
+                        want_state[r].view(H, dk, dv), H)
+            close(out[lo:hi], w.reshape(hi - lo, -1), torch.float32, f"outputs of request {r}")
+    close(st, want_state, torch.float32, "states")
+
+
 @pytest.mark.parametrize("taps,C,unit,dk", [(4, 96, 4, 16), (4, 2052, 2, 130), (4, 8200, 8, 1024), (3, 96, 4, 16), (4, 90, 4, 16)])
 def test_short_convolution_forms(taps, C, unit, dk):
     """Four taps of channels in groups of four, and what does not fit that form, against 64 bits: requests that begin here,
