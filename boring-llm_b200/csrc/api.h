@@ -302,7 +302,7 @@ int bl_recurrent_scan(int rule, const float* q, int ldq, const float* k, int ldk
 // request's state through the parts (by a decay per row, or, delta rule, by the part's key x key transition) and leaves the
 // slot and every part's start, then every part runs from its start. scratch: bl_recurrent_scan_parts_scratch floats. nc 1:
 // bl_recurrent_scan.
-long long bl_recurrent_scan_parts_scratch(int rule, int n_cut, int nc, int H, int dk, int dv);
+long long bl_recurrent_scan_parts_scratch(int rule, int R, int n_cut, int nc, int H, int dk, int dv);
 int bl_recurrent_scan_can_split(int rule, int H, int dk, int dv);   // 0, or the blocks one request's portion runs on
 int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
                             const float* a, int lda, const float* beta, int ldb, float q_scale, float* state,

@@ -205,7 +205,7 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
                           const float* beta, int ldb, float q_scale,
                           float* state, size_t slot_stride, const int* __restrict__ slots, const int* __restrict__ cu_q,
                           float* out, int H, int G, int dk, int dv, int KS, int chunk, int vec,
-                          int nc, int n_cut, float* part_s, float* part_p, const float* part_start) {
+                          int nc, int n_cut, int* places, float* part_s, float* part_p, const float* part_start) {
     bl_pdl_trigger();
     bl_pdl_wait();
     extern __shared__ __align__(16) float sm[];
@@ -220,8 +220,18 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
     const int r = blockIdx.z / nc, part = blockIdx.z % nc, h = blockIdx.y;
     const int n_all = cu_q[r + 1] - cu_q[r];
     if (n_all <= 0) return;
-    const int place = nc > 1 && n_all >= SCAN_SPLIT_MIN ? scan_cut_place(cu_q, r) : n_cut;
-    const bool split = place < n_cut;
+    // The first pass counts out a request's place in the scratch (-1: not cut) and leaves it for the launches behind it;
+    // where scratch is there for all requests, it is r. (Counted
+    // in the second pass too, it cost the walk in one piece its registers: 188 -> 204, 8 heads of 128 x 256 385 -> 436 us.)
+    int place = 0;
+    if (QUIET) {
+        place = n_all < SCAN_SPLIT_MIN ? -1 : places ? scan_cut_place(cu_q, r) : r;
+        if (place >= n_cut) place = -1;
+        if (places && blockIdx.x == 0 && h == 0 && part == 0 && threadIdx.x == 0) places[r] = place;
+    } else if (nc > 1) {
+        place = places ? places[r] : n_all >= SCAN_SPLIT_MIN ? r : -1;
+    }
+    const bool split = nc > 1 && place >= 0;
     if (!split && (part != 0 || QUIET)) return;
     // (of more parts than tokens some are empty: they leave a zero state and the identity)
     const int t_first = split ? (int)((long long)part * n_all / nc) : 0;
@@ -413,15 +423,14 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
 constexpr int FOLD_COLS = 8, FOLD_MAX_DK = 128;
 __global__ void __launch_bounds__(256)
 scan_fold_matrix_kernel(float* state, size_t slot_stride, const int* __restrict__ slots, const int* __restrict__ cu_q,
-                        const float* part_s, const float* part_pm, float* part_start, int H, int dk, int dv, int nc,
-                        int n_cut) {
+                        const int* places, const float* part_s, const float* part_pm, float* part_start, int H, int dk, int dv, int nc) {
     bl_pdl_trigger();
     bl_pdl_wait();
     __shared__ float cur[2][FOLD_MAX_DK][FOLD_COLS];
     const int r = blockIdx.z, h = blockIdx.y, c0 = blockIdx.x * FOLD_COLS;
     if (cu_q[r + 1] - cu_q[r] < SCAN_SPLIT_MIN) return;
-    const int place = scan_cut_place(cu_q, r);
-    if (place >= n_cut) return;
+    const int place = places ? places[r] : r;
+    if (place < 0) return;
     float* S = state + (size_t)slots[r] * slot_stride + (size_t)h * dk * dv;
     const size_t base = ((size_t)place * nc) * H + h;
     const int col = threadIdx.x % FOLD_COLS, rg = threadIdx.x / FOLD_COLS;
@@ -459,13 +468,13 @@ scan_fold_matrix_kernel(float* state, size_t slot_stride, const int* __restrict_
 // The same where the transition is a decay per row: start[p + 1] = P_p o start[p] + S_part_p. Every part's start takes the
 // place of its contribution in part_s.
 __global__ void scan_fold_kernel(float* state, size_t slot_stride, const int* __restrict__ slots, const int* __restrict__ cu_q,
-                                 float* part_s, const float* part_p, int H, int dk, int dv, int nc, int n_cut) {
+                                 const int* places, float* part_s, const float* part_p, int H, int dk, int dv, int nc) {
     bl_pdl_trigger();
     bl_pdl_wait();
     const int r = blockIdx.z, h = blockIdx.y;
     if (cu_q[r + 1] - cu_q[r] < SCAN_SPLIT_MIN) return;
-    const int place = scan_cut_place(cu_q, r);
-    if (place >= n_cut) return;
+    const int place = places ? places[r] : r;
+    if (place < 0) return;
     float* S = state + (size_t)slots[r] * slot_stride + (size_t)h * dk * dv;
     const size_t base = ((size_t)place * nc) * H + h;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -892,10 +901,10 @@ extern "C" int bl_recurrent_scan_can_split(int rule, int H, int dk, int dv) {
     return 0;
 }
 
-// Floats of scratch that bl_recurrent_scan_parts needs to cut n_cut requests.
-extern "C" long long bl_recurrent_scan_parts_scratch(int rule, int n_cut, int nc, int H, int dk, int dv) {
+// Floats of scratch that bl_recurrent_scan_parts needs to cut n_cut of a step's R requests.
+extern "C" long long bl_recurrent_scan_parts_scratch(int rule, int R, int n_cut, int nc, int H, int dk, int dv) {
     const long long per = rule == BL_RULE_DELTA ? (long long)dk * (2 * dv + dk) : (long long)dk * (dv + 1);
-    return (long long)n_cut * nc * H * per;
+    return (R + 3) / 4 * 4 + (long long)n_cut * nc * H * per;
 }
 
 extern "C" int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
@@ -934,13 +943,14 @@ extern "C" int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const 
     if (rule != BL_RULE_GLA && rule != BL_RULE_DELTA && rule != BL_RULE_BONUS) BL_FAIL("bl_recurrent_scan: unknown rule %d", rule);
     if (rk4 > 0) {                                     // a lane's rows are whole groups of four
         const bool dl = rule == BL_RULE_DELTA;
-        float* part_s = scratch;                                                 // [n_cut, nc, H, dk, dv]
-        float* part_p = scratch ? scratch + (size_t)n_cut * nc * H * dk * dv : nullptr;   // [n_cut, nc, H, dk] or, delta rule, [n_cut, nc, H, dk, dk]
+        int* places = n_cut < R ? reinterpret_cast<int*>(scratch) : nullptr;     // [R], up to a multiple of 16 bytes; null: r is r's place
+        float* part_s = scratch ? scratch + (R + 3) / 4 * 4 : nullptr;           // [n_cut, nc, H, dk, dv]
+        float* part_p = scratch ? part_s + (size_t)n_cut * nc * H * dk * dv : nullptr;   // [n_cut, nc, H, dk] or, delta rule, [n_cut, nc, H, dk, dk]
         // [n_cut, nc, H, dk, dv]; a fold with a decay per row leaves the starts in part_s
         float* part_start = scratch == nullptr ? nullptr : dl ? part_p + (size_t)n_cut * nc * H * dk * dk : part_s;
         const int two_an_sm = 2 * scan_sms();
 #define BL_SCAN_Q(D, R4, DENSE, QUIET, GRID) BL_CUDA(bl_launch_dependent(recurrent_scan_vec_kernel<D, R4, DENSE, QUIET>, GRID, dim3(WARPS * 32), smem, s, \
-        q, ldq, k, ldk, v, ldv, z, ldz, beta, ldb, q_scale, state, (size_t)slot_stride, slots, cu_q, out, H, G, dk, dv, KS, chunk, vec, nc, n_cut, \
+        q, ldq, k, ldk, v, ldv, z, ldz, beta, ldb, q_scale, state, (size_t)slot_stride, slots, cu_q, out, H, G, dk, dv, KS, chunk, vec, nc, n_cut, places, \
         part_s, part_p, (const float*)part_start))
 #define BL_SCAN(D, R4, PASS) do { \
         const dim3 g = (D == BL_RULE_DELTA && PASS == 1) ? grid_wide : grid; \
@@ -950,11 +960,11 @@ extern "C" int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const 
         for (int pass = (nc > 1 ? 1 : 2); pass <= 2; ++pass) {
             if (pass == 2 && nc > 1 && dl)
                 BL_CUDA(bl_launch_dependent(scan_fold_matrix_kernel, dim3((dv + FOLD_COLS - 1) / FOLD_COLS, H, R), dim3(256), 0, s, state,
-                                            (size_t)slot_stride, slots, cu_q, (const float*)part_s, (const float*)part_p, part_start,
-                                            H, dk, dv, nc, n_cut));
+                                            (size_t)slot_stride, slots, cu_q, (const int*)places, (const float*)part_s, (const float*)part_p, part_start,
+                                            H, dk, dv, nc));
             if (pass == 2 && nc > 1 && !dl)
                 BL_CUDA(bl_launch_dependent(scan_fold_kernel, dim3((dk * dv + 255) / 256, H, R), dim3(256), 0, s, state, (size_t)slot_stride,
-                                            slots, cu_q, part_s, (const float*)part_p, H, dk, dv, nc, n_cut));
+                                            slots, cu_q, (const int*)places, part_s, (const float*)part_p, H, dk, dv, nc));
             switch (rk4) {
 #define BL_SCAN_RULE(R4) do { if (dl) BL_SCAN(BL_RULE_DELTA, R4, pass); else if (rule == BL_RULE_BONUS) BL_SCAN(BL_RULE_BONUS, R4, pass); \
                                   else BL_SCAN(BL_RULE_GLA, R4, pass); } while (0)

@@ -1025,7 +1025,7 @@ def recurrent_scan(rule: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     if parts > 1 and n_cut > 0:
         lib = _lib()
         lib.bl_recurrent_scan_parts_scratch.restype = ctypes.c_longlong
-        scratch = torch.empty(int(lib.bl_recurrent_scan_parts_scratch(rule, n_cut, parts, H, dk, dv)), dtype=torch.float32, device=out.device)
+        scratch = torch.empty(int(lib.bl_recurrent_scan_parts_scratch(rule, R, n_cut, parts, H, dk, dv)), dtype=torch.float32, device=out.device)
         _call(_lib().bl_recurrent_scan_parts, rule, _p(q), ldq, _p(k), ldk, _p(v), ldv, _p(decay), ldz, _p(beta), ldb,
               ctypes.c_float(q_scale), _p(state), ctypes.c_longlong(state.stride(0)), _p(slots), _p(cu_q), R,
               _p(out), H, G, dk, dv, parts, n_cut, _p(scratch), _stream())
