@@ -301,13 +301,14 @@ int bl_recurrent_scan(int rule, const float* q, int ldq, const float* k, int ldk
 // in the step; key sizes that bl_recurrent_scan_can_split takes): every part first runs from a zero state, a fold takes the
 // request's state through the parts (by a decay per row, or, delta rule, by the part's key x key transition) and leaves the
 // slot and every part's start, then every part runs from its start. scratch: bl_recurrent_scan_parts_scratch floats. nc 1:
-// bl_recurrent_scan.
+// bl_recurrent_scan. busy: how many requests' portions are under way for most of the launch (it decides how many blocks an SM
+// takes; any value gives the same bits).
 long long bl_recurrent_scan_parts_scratch(int rule, int R, int n_cut, int nc, int H, int dk, int dv);
 int bl_recurrent_scan_can_split(int rule, int H, int dk, int dv);   // 0, or the blocks one request's portion runs on
 int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
                             const float* a, int lda, const float* beta, int ldb, float q_scale, float* state,
                             long long slot_stride, const int* slots, const int* cu_q, int R, float* out, int H, int G,
-                            int dk, int dv, int nc, int n_cut, float* scratch, void* stream);
+                            int dk, int dv, int nc, int n_cut, int busy, float* scratch, void* stream);
 // y[t, h, :] = o[t, h, :] / sqrt(mean(o^2) + eps) * w[:] * gate(g[t * ld_gate + h * dv + :]) (gate null: none).
 #define BL_GATE_SIGMOID 0
 #define BL_GATE_SILU 1

@@ -884,7 +884,7 @@ extern "C" int bl_recurrent_scan(int rule, const float* q, int ldq, const float*
                                  const float* z, int ldz, const float* beta, int ldb, float q_scale, float* state, long long slot_stride, const int* slots, const int* cu_q, int R,
                                  float* out, int H, int G, int dk, int dv, void* stream) {
     return bl_recurrent_scan_parts(rule, q, ldq, k, ldk, v, ldv, z, ldz, beta, ldb, q_scale, state, slot_stride, slots, cu_q, R, out,
-                                   H, G, dk, dv, 1, 0, nullptr, stream);
+                                   H, G, dk, dv, 1, 0, R, nullptr, stream);
 }
 
 // Whether bl_recurrent_scan_parts can cut long portions of this rule and key size (else it runs them in one piece):
@@ -910,7 +910,7 @@ extern "C" long long bl_recurrent_scan_parts_scratch(int rule, int R, int n_cut,
 extern "C" int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
                                        const float* z, int ldz, const float* beta, int ldb, float q_scale, float* state,
                                        long long slot_stride, const int* slots, const int* cu_q, int R, float* out, int H, int G,
-                                       int dk, int dv, int nc, int n_cut, float* scratch, void* stream) {
+                                       int dk, int dv, int nc, int n_cut, int busy, float* scratch, void* stream) {
     if (R <= 0) return 0;
     if (nc < 1 || (nc > 1 && (n_cut < 1 || n_cut > R || scratch == nullptr || !bl_recurrent_scan_can_split(rule, H, dk, dv) || (long long)R * nc > 65535)))
         BL_FAIL("bl_recurrent_scan_parts: %d parts for rule %d, %d key channels, %d requests", nc, rule, dk, R);
@@ -948,13 +948,17 @@ extern "C" int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const 
         float* part_p = scratch ? part_s + (size_t)n_cut * nc * H * dk * dv : nullptr;   // [n_cut, nc, H, dk] or, delta rule, [n_cut, nc, H, dk, dk]
         // [n_cut, nc, H, dk, dv]; a fold with a decay per row leaves the starts in part_s
         float* part_start = scratch == nullptr ? nullptr : dl ? part_p + (size_t)n_cut * nc * H * dk * dk : part_s;
+        // Two an SM, or the build for four: by the blocks that work side by side for most of the launch, not by those of a few
+        // tokens beside a long portion that leave at once (2,000 tokens beside 31 running requests, in one piece: 7 heads of
+        // 64 x 128 640 us counted by all, 507 so; 8 of 128 x 256 1,115 and 824; the delta rule 778 and 613, 1,215 and 934).
         const int two_an_sm = 2 * scan_sms();
+        const long long at_once[2] = {(long long)n_cut * nc, nc > 1 ? (long long)n_cut * nc + (busy > n_cut ? busy - n_cut : 0) : busy};
 #define BL_SCAN_Q(D, R4, DENSE, QUIET, GRID) BL_CUDA(bl_launch_dependent(recurrent_scan_vec_kernel<D, R4, DENSE, QUIET>, GRID, dim3(WARPS * 32), smem, s, \
         q, ldq, k, ldk, v, ldv, z, ldz, beta, ldb, q_scale, state, (size_t)slot_stride, slots, cu_q, out, H, G, dk, dv, KS, chunk, vec, nc, n_cut, places, \
         part_s, part_p, (const float*)part_start))
 #define BL_SCAN(D, R4, PASS) do { \
         const dim3 g = (D == BL_RULE_DELTA && PASS == 1) ? grid_wide : grid; \
-        const bool dense = (long long)g.x * g.y * g.z > two_an_sm; \
+        const bool dense = at_once[PASS - 1] * g.x * g.y > two_an_sm; \
         if (PASS == 1) { if (dense) BL_SCAN_Q(D, R4, true, true, g); else BL_SCAN_Q(D, R4, false, true, g); } \
         else if (dense) BL_SCAN_Q(D, R4, true, false, g); else BL_SCAN_Q(D, R4, false, false, g); } while (0)
         for (int pass = (nc > 1 ? 1 : 2); pass <= 2; ++pass) {

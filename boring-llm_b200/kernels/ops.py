@@ -1003,7 +1003,7 @@ def recurrent_scan_parts(rule: int, H: int, dk: int, dv: int, n_long: int) -> in
 
 def recurrent_scan(rule: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, beta: Optional[torch.Tensor],
                    q_scale: float, state: torch.Tensor, slots: torch.Tensor, cu_q: torch.Tensor, out: torch.Tensor,
-                   H: int, G: int, dk: int, dv: int, parts: int = 1, n_long: Optional[int] = None) -> None:
+                   H: int, G: int, dk: int, dv: int, parts: int = 1, n_long: Optional[int] = None, busy: Optional[int] = None) -> None:
     """A linear recurrence over a matrix state per head and request (`RULE_GLA`, `RULE_DELTA`, `RULE_BONUS`, whose beta is
     a given number per token and head, see `bonus_dot`; see `bl_recurrent_scan`).
     q, k [T, G * dk], v [T, H * dv], decay [T, H * dk] (in (0, 1], see `gemm_plain_decay`), beta [T, H] (logits): 32-bit
@@ -1011,7 +1011,8 @@ def recurrent_scan(rule: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     slot. out [T, H * dv] 32-bit, already times q_scale. `parts` > 1 (`recurrent_scan_parts`): portions of 256 tokens and
     more are cut into that many parts, which run side by side (twice the arithmetic on `parts` times the blocks; the
     results differ from the walk in one piece by rounding only). `n_long`: how many requests that are (None: any may be);
-    scratch is taken for so many, and the first so many are cut."""
+    scratch is taken for so many, and the first so many are cut. `busy`: how many requests' portions are under way for most
+    of the launch (None: all); it decides how many blocks an SM takes and changes no bit."""
     T = out.shape[0]
     R = cu_q.shape[0] - 1
     ldq, ldk, ldv, ldz = (_rows32(q, "q", T, G * dk), _rows32(k, "k", T, G * dk), _rows32(v, "v", T, H * dv),
@@ -1022,17 +1023,16 @@ def recurrent_scan(rule: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     if not state.is_cuda or state.dtype != torch.float32 or state.dim() != 2 or state.stride(1) != 1 or state.shape[1] < H * dk * dv:
         raise KernelError("state: must be 32-bit [slots, >= H * dk * dv] with contiguous rows")
     n_cut = R if n_long is None else min(n_long, R)
+    scratch = None
     if parts > 1 and n_cut > 0:
         lib = _lib()
         lib.bl_recurrent_scan_parts_scratch.restype = ctypes.c_longlong
         scratch = torch.empty(int(lib.bl_recurrent_scan_parts_scratch(rule, R, n_cut, parts, H, dk, dv)), dtype=torch.float32, device=out.device)
-        _call(_lib().bl_recurrent_scan_parts, rule, _p(q), ldq, _p(k), ldk, _p(v), ldv, _p(decay), ldz, _p(beta), ldb,
-              ctypes.c_float(q_scale), _p(state), ctypes.c_longlong(state.stride(0)), _p(slots), _p(cu_q), R,
-              _p(out), H, G, dk, dv, parts, n_cut, _p(scratch), _stream())
-        return
-    _call(_lib().bl_recurrent_scan, rule, _p(q), ldq, _p(k), ldk, _p(v), ldv, _p(decay), ldz, _p(beta), ldb,
+    else:
+        parts, n_cut = 1, 0
+    _call(_lib().bl_recurrent_scan_parts, rule, _p(q), ldq, _p(k), ldk, _p(v), ldv, _p(decay), ldz, _p(beta), ldb,
           ctypes.c_float(q_scale), _p(state), ctypes.c_longlong(state.stride(0)), _p(slots), _p(cu_q), R,
-          _p(out), H, G, dk, dv, _stream())
+          _p(out), H, G, dk, dv, parts, n_cut, R if busy is None else busy, _p(scratch), _stream())
 
 
 def head_norm_gate(o: torch.Tensor, weight: Optional[torch.Tensor], gate: Optional[torch.Tensor], gate_kind: int, eps: float,

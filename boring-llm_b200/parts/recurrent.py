@@ -38,10 +38,11 @@ class _StateMixer(Mixer):
     RULE = None                      # ops.RULE_GLA or ops.RULE_DELTA
 
     def _cut(self, q_lens) -> dict:
-        """Into how many parts a step's long portions are cut (they run side by side), and how many requests have one."""
+        """Into how many parts a step's long portions are cut (they run side by side), how many requests have one, and how many
+        portions are under way for most of the scan (the tokens over those of the longest)."""
         n_long = sum(1 for n in q_lens if n >= ops.SCAN_PART_MIN_TOKENS)
         parts = ops.recurrent_scan_parts(self.RULE, self.H, self.dk, self._value_columns(), n_long) if n_long else 1
-        return {"parts": parts, "n_long": n_long if parts > 1 else 0}
+        return {"parts": parts, "n_long": n_long if parts > 1 else 0, "busy": max(1, round(sum(q_lens) / max(1, max(q_lens))))}
 
     def _value_columns(self) -> int:
         return self.dv                  # columns of a head's state
@@ -55,7 +56,7 @@ class _StateMixer(Mixer):
         return f"recurrence parts {self.RULE} {self.H}x{self.dk}x{self._value_columns()}"       # layers of equal sizes share the plan
 
     def _step_cut(self, ctx) -> dict:
-        """The arguments of `recurrent_scan` that say how long portions are cut."""
+        """The arguments of `recurrent_scan` that say how it is launched."""
         if not ctx.fast:
             return {}
         plan = ctx.plans.get(self._plan_key())

@@ -216,6 +216,29 @@ def test_scan_keeps_scratch_for_the_requests_that_are_cut(rule, lens, n_long):
     close(st, want_state, torch.float32, "states")
 
 
+@pytest.mark.parametrize("rule", ["RULE_GLA", "RULE_DELTA", "RULE_BONUS"])
+def test_scan_takes_blocks_by_the_portions_under_way(rule):
+    """The requests of a few tokens beside a long portion are not counted as if they kept the launch busy, and both builds
+    of the kernel give the same bits."""
+    from boring_llm_b200.parts.recurrent import GatedLinearAttention
+    o = ops()
+    rule = getattr(o, rule)
+    H, dk, dv, lens = 4, 64, 256, [200] + [1] * 40
+    mixer = GatedLinearAttention(64, H, dk, dv, 16.0, 1e-6, {})
+    assert [mixer._cut(x)["busy"] for x in ([2000] + [1] * 31, [1] * 64, [200, 100] + [50] * 12, [0, 0])] == [1, 64, 4, 1]
+    T, R = sum(lens), len(lens)
+    q, k, v, b = data((T, H * dk), 1) * 0.3, data((T, H * dk), 2) * 0.1, data((T, H * dv), 3), data((T, H), 4)
+    a = torch.sigmoid(data((T, H * dk), 5) + 3.0)
+    cu = torch.tensor([0] + lens, device=DEV).cumsum(0).to(torch.int32)
+    got = []
+    for busy in (1, R, None):
+        st, out = data((R, H * dk * dv), 6), torch.full((T, H * dv), float("nan"), device=DEV)
+        o.recurrent_scan(rule, q, k, v, a, None if rule == o.RULE_GLA else b, 0.5, st, torch.arange(R, dtype=torch.int32, device=DEV), cu, out,
+                         H, H, dk, dv, busy=busy)
+        got.append((out, st))
+    assert all(torch.equal(x, y) for other in got[1:] for x, y in zip(got[0], other))
+
+
 @pytest.mark.parametrize("taps,C,unit,dk", [(4, 96, 4, 16), (4, 2052, 2, 130), (4, 8200, 8, 1024), (3, 96, 4, 16), (4, 90, 4, 16)])
 def test_short_convolution_forms(taps, C, unit, dk):
     """Four taps of channels in groups of four, and what does not fit that form, against 64 bits: requests that begin here,
