@@ -239,6 +239,17 @@ def test_scan_takes_blocks_by_the_portions_under_way(rule):
     assert all(torch.equal(x, y) for other in got[1:] for x, y in zip(got[0], other))
 
 
+def test_scans_are_cut_where_that_was_measured_to_pay():
+    """One long portion at two sizes: a cut of linear attention pays at both (few parts at the larger, where every further round
+    of blocks costs), of the delta rule only at the smaller, whose fold is short; several long portions fill the device."""
+    o = ops()
+    parts = o.recurrent_scan_parts
+    assert parts(o.RULE_DELTA, 8, 128, 256, 1) == 1
+    assert 4 <= parts(o.RULE_GLA, 8, 128, 256, 1) <= 12
+    assert 8 <= parts(o.RULE_DELTA, 7, 64, 128, 1) <= 12 and 16 <= parts(o.RULE_GLA, 7, 64, 128, 1) <= 21
+    assert parts(o.RULE_GLA, 8, 128, 256, 2) == 1 and parts(o.RULE_GLA, 7, 64, 128, 8) == 1 and parts(o.RULE_GLA, 7, 64, 128, 0) == 1
+
+
 @pytest.mark.parametrize("taps,C,unit,dk", [(4, 96, 4, 16), (4, 2052, 2, 130), (4, 8200, 8, 1024), (3, 96, 4, 16), (4, 90, 4, 16)])
 def test_short_convolution_forms(taps, C, unit, dk):
     """Four taps of channels in groups of four, and what does not fit that form, against 64 bits: requests that begin here,
