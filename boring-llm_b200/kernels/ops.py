@@ -1112,13 +1112,14 @@ def conv_tail_update(x: torch.Tensor, n_taps: int, tail: torch.Tensor, slots: to
 
 def linear_act(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: int, fast: bool = True):
     """out = act((x @ w.T)[:, :N]), N = out's columns, the activation evaluated in 32-bit on the product's 32-bit sums.
-    w may have more rows than out has columns: the sums of those further rows are returned as they are (a 32-bit view
-    [M, rows - N]; None when there are none)."""
+    w may have more rows than out has columns: the sums of those further rows are returned as they are ([M, rows - N] in 32 bits,
+    contiguous or a range of columns; None when there are none). out may be x."""
     M, N = out.shape
     rows_w = w.shape[0]
     if rows_w < N:
         raise KernelError("linear_act: w has fewer rows than out has columns")
     if (out.dtype == torch.bfloat16 and out.is_contiguous() and out.data_ptr() % 16 == 0 and rows_w % 4 == 0 and N % 4 == 0
+            and out.untyped_storage().data_ptr() != x.untyped_storage().data_ptr()   # (a tile is written while others still read their x)
             and gemm_kernel(x, w, rows_w, None, EPI_NONE, fast) == "pair"):      # many rows: the activation in the product's epilogue
         _need(x, "x", torch.bfloat16, (M, w.shape[1])); _need(w, "w", torch.bfloat16)
         rest = torch.empty((M, rows_w - N), dtype=torch.float32, device=x.device) if rows_w > N else None

@@ -331,6 +331,31 @@ def test_activation_in_the_epilogue_of_the_product_on_pairs(M, N, n_act, K, act)
     assert (rest is None) == (N == n_act) and (rest is None or torch.equal(rest, sums[:, n_act:]))
 
 
+@pytest.mark.parametrize("M", [64, 300])
+def test_activated_product_over_its_own_rows(M):
+    """out in the place of x: no tile is written while another still reads, so the product has a launch of its own."""
+    o = ops()
+    x, w = (data((M, 1024), 1) * 0.5).to(BF), (data((1024, 1024), 2) * 0.05).to(BF)
+    want = torch.empty(M, 1024, dtype=BF, device=DEV)
+    seen = []
+    call = o._call
+
+    def spy(fn, *a):
+        seen.append(fn.__name__)
+        return call(fn, *a)
+    o._call = spy
+    try:
+        assert o.linear_act(x, w, want, 1) is None
+        assert ("bl_gemm_tc_pair_act" in seen) == (M >= 256)
+        seen.clear()
+        assert o.linear_act(x, w, x, 1) is None
+        assert "bl_gemm_tc_pair_act" not in seen
+    finally:
+        o._call = call
+    o.check_status()
+    assert torch.equal(x, want)
+
+
 @pytest.mark.parametrize("K", [4, 28, 32, 36, 896])
 @pytest.mark.parametrize("M,N", [(1, 16), (3, 70), (17, 33), (65, 100), (366, 257)])
 def test_32_bit_product_does_not_depend_on_the_rows_beside_a_row(M, N, K):
