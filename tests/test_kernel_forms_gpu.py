@@ -407,3 +407,104 @@ def test_products_on_pairs_one_behind_the_other(M, N, K):
     want = torch.empty(M, N, device=DEV)
     o.gemm_plain(x, w, want)
     close(outs[0], want.double(), torch.float32, "product")
+
+
+@pytest.mark.parametrize("rank,rot", [(8, 8), (128, 32), (136, 8), (504, 16), (512, 64)])
+@pytest.mark.parametrize("window,contexts", [(0, [1100, 70, 1]), (130, [1100, 129, 40])])
+def test_slices_of_a_token_with_a_long_context(rank, rot, window, contexts):
+    """A token's keys in 15, 16 and 17 slices (the merge holds up to 16 in a thread's registers, 128 columns at a time) and in more
+    slices than there are key blocks: slices without keys leave their sums of earlier memory, which is NaN here, alone."""
+    import plain_miforax as pm
+    o = ops()
+    if not o.latent_attention_mma_supported(BF, rank, rot, 16):
+        pytest.skip("sizes that the kernel does not take")
+    H, R, dk, scale = 3, len(contexts), rank + rot, 0.3
+    g = torch.Generator().manual_seed(rank + window)
+    rows = [(torch.randn(n, dk, generator=g, dtype=torch.float64) * 0.5).to(BF).double() for n in contexts]
+    q = (torch.randn(R, H, dk, generator=g, dtype=torch.float64) * 0.5).to(BF).double()
+    sinks = torch.randn(H, generator=g, dtype=torch.float64)
+    width = -(-max(contexts) // 16)
+    cache = torch.full((R * width, 1, 16, dk), float("nan"), dtype=BF)
+    table = torch.arange(R * width, dtype=torch.int32).flip(0).reshape(R, width)
+    want = torch.empty(H, R, rank, dtype=torch.float64)
+    for r, n in enumerate(contexts):
+        for j in range(n):
+            cache[table[r, j // 16], 0, j % 16] = rows[r][j].to(BF)
+        k = rows[r][None].expand(H, n, dk)
+        seen = torch.arange(n) >= (n - window if window else 0)
+        want[:, r] = pm.sink_softmax_attention(q[r][:, None], k, k[:, :, :rank], scale, sinks, seen[None])[:, 0]
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device=DEV)
+    head_major = lambda t: t.permute(1, 0, 2).to(BF).contiguous().to(DEV)
+    args = (head_major(q[:, :, :rank]), head_major(q[:, :, rank:]), cache.to(DEV), i32(list(range(R + 1))), i32(contexts), table.to(DEV), i32(list(range(R))))
+    for splits in (1, 15, 16, 17, 40):
+        poison = torch.full((4, H * R * splits * max(rank, 2)), float("nan"), device=DEV)
+        torch.cuda.synchronize()
+        del poison                                            # what the scratch is taken from
+        out = torch.full((H, R, rank), float("nan"), dtype=BF, device=DEV)
+        o.latent_attention_mma(*args, True, out, window, scale, sinks.float().to(DEV), splits)
+        assert torch.isfinite(out).all()
+        close(out, want, BF, f"{splits} slices")              # (weights and results of 8 bits, as the kernels' other tests take them)
+
+
+@pytest.mark.parametrize("q_rank,rank,rot_dim,dims", [(127, 129, 8, 8), (128, 128, 16, 12), (1024, 1024, 64, 64), (1025, 40, 8, 8), (40, 1025, 8, 4),
+                                                      (129, 520, 128, 128), (24, 16, 130, 130)])
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+def test_latent_rows_at_the_widths_where_their_form_changes(q_rank, rank, rot_dim, dims, dtype):
+    """Both norms, the rotation and the cache row with all values in registers (up to 1,024 a norm, 128 of the shared key part) and
+    read in loops; either result left out. NaN in what a form must not read."""
+    o = ops()
+    T, eps, mscale = 5, 1e-5, 1.25
+    positions = [37, 5, 16, 0, 31]
+    proj = data((T, q_rank + rank + rot_dim + 9), 1)
+    off_q, off_kv = 3, q_rank + 5
+    qw, kw = (data((q_rank,), 2) * 0.25 + 1).to(dtype), (data((rank,), 3) * 0.25 + 1).to(dtype)
+    inv = torch.tensor([100.0 ** (-2.0 * j / dims) for j in range(dims // 2)], device=DEV)
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device=DEV)
+    table = i32([[4, 7, 2], [6, 1, 0], [3, 5, 8]])
+    req = [0, 1, 2, 2, 1]
+    p = proj.double().cpu()
+    zq, zk, zr = p[:, off_q:off_q + q_rank], p[:, off_kv:off_kv + rank], p[:, off_kv + rank:off_kv + rank + rot_dim]
+    a = torch.tensor(positions, dtype=torch.float64)[:, None] * inv.double().cpu()
+    u, v, h = zr[:, :dims // 2], zr[:, dims // 2:dims], zr[:, dims:]
+    turned = torch.cat([(u * a.cos() - v * a.sin()) * mscale, (v * a.cos() + u * a.sin()) * mscale, h], 1)
+    want_q = plain.rms_norm(zq, qw.double().cpu(), eps)
+    want_row = torch.cat([plain.rms_norm(zk, kw.double().cpu(), eps), turned], 1)
+    for with_q, with_row in ((True, True), (True, False), (False, True)):
+        x = proj.clone()
+        if not with_q:
+            x[:, off_q:off_q + q_rank] = float("nan")
+        if not with_row:
+            x[:, off_kv:] = float("nan")
+        cq = torch.full((T, q_rank), float("nan"), dtype=dtype, device=DEV) if with_q else None
+        cache = torch.full((9, 1, 16, rank + rot_dim), float("nan"), dtype=dtype, device=DEV) if with_row else None
+        o.latent_prep(x, off_q, q_rank, off_kv, rank, rot_dim, dims // 2, qw if with_q else None, kw if with_row else None, eps,
+                      i32(positions), i32(req), table, inv, mscale, cq, cache)
+        if with_q:
+            close(cq, want_q, dtype, "query latent")
+        if with_row:
+            at = [(int(table[r, t // 16]), t % 16) for r, t in zip(req, positions)]
+            close(torch.stack([cache[pg, 0, s] for pg, s in at]), want_row, dtype, "cache rows")
+            assert int(torch.isfinite(cache).all(-1).sum()) == T
+
+
+@pytest.mark.parametrize("T,H", [(1, 3), (256, 9), (257, 9), (256, 8), (300, 2), (2, 17)])
+@pytest.mark.parametrize("n,rot_half,n_lead,gap", [(32, 16, 64, 0), (32, 12, 62, 2), (8, 4, 4, 1), (10, 5, 0, 0), (64, 32, 128, 4)])
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+def test_turned_heads_in_shares(T, H, n, rot_half, n_lead, gap, dtype):
+    """Up to 256 tokens a token's heads lie on several blocks, of unequal shares where eight do not divide them; the other slice in
+    16-byte pieces where sizes and strides allow, else value by value."""
+    o = ops()
+    width = n_lead + n + gap
+    x = data((T, H * width), 1).view(T, H, width)
+    lead, q = (x[:, :, :n_lead] if n_lead else None), x[:, :, n_lead:n_lead + n]
+    positions = torch.arange(T, dtype=torch.int32, device=DEV) * 3 % 97
+    inv = torch.tensor([50.0 ** (-j / rot_half) for j in range(rot_half)], device=DEV)
+    out = torch.full((T, H, n), float("nan"), dtype=dtype, device=DEV)
+    lead_out = torch.full((T, H, n_lead), float("nan"), dtype=dtype, device=DEV) if n_lead else None
+    o.rope_heads(q, positions, inv, rot_half, 0.75, out, lead, lead_out)
+    a = (positions.double().cpu()[:, None] * inv.double().cpu())[:, None]
+    c, s, z = a.cos() * 0.75, a.sin() * 0.75, q.double().cpu()
+    u, v = z[:, :, :rot_half], z[:, :, rot_half:2 * rot_half]
+    close(out, torch.cat([u * c - v * s, v * c + u * s, z[:, :, 2 * rot_half:]], 2), dtype, "turned heads")
+    if n_lead:
+        assert torch.equal(lead_out, lead.to(dtype))
