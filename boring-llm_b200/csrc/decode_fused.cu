@@ -370,23 +370,22 @@ int launch(const FusedParams& p, int tiles, cudaStream_t s) {
 template <int MODE>
 int dispatch(FusedParams& p, int tiles, cudaStream_t s) {
     if constexpr (MODE == MODE_QKV) {
-        if (p.normed != nullptr) {
-            const int mt = p.M <= 8 ? 1 : p.M <= 16 ? 2 : 4;
+        if (p.normed != nullptr) {                     // (the callers norm up to 8 rows inside)
+            const int mt = p.M <= 16 ? 2 : 4;
             p.m_groups = (p.M + mt * 8 - 1) / (mt * 8);
-            if (mt == 1) return launch<1, MODE, true>(p, tiles, s);
-            if (mt == 2) return launch<2, MODE, true>(p, tiles, s);
-            return launch<4, MODE, true>(p, tiles, s);
+            return mt == 2 ? launch<2, MODE, true>(p, tiles, s) : launch<4, MODE, true>(p, tiles, s);
         }
     }
-    // the largest row group whose normalised rows fit shared memory
-    int mt = p.M <= 8 ? 1 : p.M <= 16 ? 2 : 4;
+    // the largest row group whose normalised rows fit shared memory (q/k/v: the callers have more than 16 rows normed before)
+    int mt = p.M <= 8 ? 1 : p.M <= 16 || MODE == MODE_QKV ? 2 : 4;
     while (mt > 1 && smem_bytes(mt, p.K, MODE == MODE_SWIGLU) > SMEM_LIMIT) mt /= 2;
     if (smem_bytes(mt, p.K, MODE == MODE_SWIGLU) > SMEM_LIMIT)
         BL_FAIL("bl_norm_gemm: rows of %d values do not fit shared memory; run the norm and the product separately", p.K);
     p.m_groups = (p.M + mt * 8 - 1) / (mt * 8);
     if (mt == 1) return launch<1, MODE>(p, tiles, s);
-    if (mt == 2) return launch<2, MODE>(p, tiles, s);
-    return launch<4, MODE>(p, tiles, s);
+    if constexpr (MODE != MODE_QKV)
+        if (mt == 4) return launch<4, MODE>(p, tiles, s);
+    return launch<2, MODE>(p, tiles, s);
 }
 
 int check_common(const char* who, const void* x, const void* w, int M, int K, int norm_w_dtype) {

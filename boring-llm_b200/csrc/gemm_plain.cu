@@ -132,7 +132,8 @@ int launch_out(const void* x, const void* w, const void* bias, int bias_dtype, v
 // three stages as they lie in memory, rows padded by 16 bytes so that the eight rows that lanes of a quarter warp read
 // fall on different banks; a thread's TR x TC outputs lie (rows, columns of threads) apart, so its operands are 16-byte
 // loads of four k each. With SWIGLU the tile's upper half of W rows are the up rows, and a thread holds both sums of a unit.
-// Bound by the FMA pipes for many rows (74 TFLOP/s), by W's bytes for few.
+// Bound by the FMA pipes for many rows (41 TFLOP/s at 2,048 rows; FMAs with three register operands reach 59 of the pipes'
+// 74), by W's bytes for few.
 template <int BM, int BN, int TR, int TC, int EPI>
 __global__ void __launch_bounds__((BM / TR) * (BN / TC))
 gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, const void* __restrict__ bias, int bias_dtype,
@@ -259,18 +260,26 @@ int launch_f32(const float* x, const float* w, const void* bias, int bias_dtype,
 struct F32Tile { int bm, bn; float alone, pace; };
 constexpr F32Tile F32_TILES[] = {{64, 32, 18.5f, 13.2f}, {32, 32, 11.8f, 8.3f}, {16, 64, 12.8f, 9.4f},
                                  {16, 32, 9.3f, 6.4f}, {4, 64, 11.8f, 5.9f}, {4, 16, 6.8f, 1.95f}};
-constexpr int F32_SMS = 148;
+
+int f32_sms() {
+    static const int sms = [] {
+        int dev = 0, n = 0;
+        return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
+    }();
+    return sms;
+}
 
 int launch_f32_tiles(const float* x, const float* w, const void* bias, int bias_dtype, float* out, int M, int N, int K, int ldx, int epi,
                      cudaStream_t s) {
     int best = 0;
     float best_us = 0.f;
+    const int sms = f32_sms();
     for (int v = 0; v < (int)(sizeof(F32_TILES) / sizeof(F32_TILES[0])); ++v) {
         const F32Tile& t = F32_TILES[v];
         const int cols = epi == BL_EPI_SWIGLU ? t.bn / 2 : t.bn;
         const long long down = (M + t.bm - 1) / t.bm, blocks = (long long)((N + cols - 1) / cols) * down;
         if (down > 65535) continue;
-        const float us = fmaxf(t.alone, (float)((blocks + F32_SMS - 1) / F32_SMS) * t.pace);
+        const float us = fmaxf(t.alone, (float)((blocks + sms - 1) / sms) * t.pace);
         if (best_us == 0.f || us < best_us) { best = v; best_us = us; }
     }
     switch (best) {

@@ -869,12 +869,10 @@ gated_group_norm_kernel(const float* o, const float* x, int ld_x, const void* __
 }
 
 int scan_sms() {
-    static int sms = 0;                                                         // (of the current device at the first call)
-    if (sms == 0) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-            sms = 148;
-    }
+    static const int sms = [] {                                                 // (of the current device at the first call)
+        int dev = 0, n = 0;
+        return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
+    }();
     return sms;
 }
 

@@ -832,7 +832,7 @@ def norm_qkv_rope(x: torch.Tensor, norm_w: torch.Tensor, eps: float, w_qkv: torc
                   mscale: float, q_out: torch.Tensor, k_cache: Optional[torch.Tensor], v_cache: Optional[torch.Tensor],
                   H: int, KV: int, dh: int, pair_layout: int = 0) -> None:
     """rmsnorm -> joined q/k/v product (+ bias) -> rotation of q and k -> k, v into the pages, q out, in one launch (or, where
-    `norm_inside_qkv` says so, in two)."""
+    `norm_inside_qkv` says that the norm stays apart, in two)."""
     M, K = x.shape
     _need(x, "x", torch.float32); _need(norm_w, "norm_w", None, (K,)); _need(w_qkv, "w_qkv", torch.bfloat16, ((H + 2 * KV) * dh, K))
     _need(positions, "positions", torch.int32, (M,)); _need(tok_req, "tok_req", torch.int32, (M,))
