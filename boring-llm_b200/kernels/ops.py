@@ -983,7 +983,6 @@ def gemm_plain_decay(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tens
 SCAN_MAX_PARTS = 32               # most parts a long portion of a request is cut into
 SCAN_PART_MIN_TOKENS = 256        # requests with fewer tokens in a step are walked in one piece (the kernel's own rule)
 SCAN_BLOCKS_PER_SM = 4            # blocks of the scan kernel that an SM holds (its registers)
-SCAN_TYPICAL_TOKENS = 1024        # the portion that a cut is chosen for
 
 
 def _scan_rounds(blocks: int) -> float:
@@ -997,42 +996,46 @@ def _scan_rounds(blocks: int) -> float:
     return 1.3 * full + (0.0 if rest == 0 else 0.7 if 2 * rest <= room else 1.1)
 
 
-def _scan_cost(rule: int, H: int, dk: int, dv: int, n_long: int, parts: int, first_blocks: int, blocks: int) -> float:
-    """Microseconds of a scan of `n_long` portions of SCAN_TYPICAL_TOKENS. A token's chain takes 0.25 us at 64 key channels
+def _scan_cost(rule: int, H: int, dk: int, dv: int, n_long: int, tokens: int, parts: int, first_blocks: int, blocks: int) -> float:
+    """Microseconds of a scan of `n_long` portions of so many tokens. A token's chain takes 0.25 us at 64 key channels
     and 0.37 at 128 (a fifth more for the delta rule). Cut: both passes, the launches, the parts' states to and fro through
     L2 and, for the delta rule, a fold that is a chain of matrix products, 3 us a part at 64 key channels and 27 at 128 (8
     heads of 256)."""
     token = 0.254 * (dk / 64) ** 0.56 * (1.2 if rule == RULE_DELTA else 1.0)
     if parts == 1:
-        return SCAN_TYPICAL_TOKENS * token * _scan_rounds(blocks * n_long)
+        return tokens * token * _scan_rounds(blocks * n_long)
     between = 9.0 + parts * 16.0 * H * n_long * dk * dv / 3e6
     if rule == RULE_DELTA:
         between += 3.0 * parts * (dk / 64) ** 2 * max(1.0, H * n_long * -(-dv // 8) / _sms())
-    return SCAN_TYPICAL_TOKENS / parts * token * (_scan_rounds(first_blocks * n_long * parts) + _scan_rounds(blocks * n_long * parts)) + between
+    return tokens / parts * token * (_scan_rounds(first_blocks * n_long * parts) + _scan_rounds(blocks * n_long * parts)) + between
 
 
 @functools.lru_cache(maxsize=1024)                    # (asked by every layer of every step)
-def recurrent_scan_parts(rule: int, H: int, dk: int, dv: int, n_long: int) -> int:
-    """How many parts `recurrent_scan` should cut the portions of a step's `n_long` long requests into (1: none). Cutting
+def recurrent_scan_parts(rule: int, H: int, dk: int, dv: int, n_long: int, tokens: int = 1024) -> int:
+    """How many parts `recurrent_scan` should cut the portions of a step's `n_long` long requests into (1: none), the longest of
+    about `tokens` tokens (a power of two: the number of parts names captured steps). Cutting
     runs every token twice, on `parts` times the blocks; the delta rule's first pass has as many columns more as the key size
     (its transition over a part is a matrix). It pays while a request's blocks leave much of the device idle: the fewest parts
-    within 2 % of the least time by `_scan_cost`, if that is 0.8 of the walk in one piece or less. Microseconds in one piece
+    within 2 % of the least time by `_scan_cost`, if that is 0.9 of the walk in one piece or less. Microseconds in one piece
     and as chosen, one portion of 2,048 / 1,024 / 256 tokens:
         linear attention, 7 heads of  64 x 128    520 / 260 / 68    21 parts   85 /  50 / 24
                           8 heads of 128 x 256    770 / 389 / 99     9 parts  445 / 235 / 78   (23 parts 454 / 249 / 97)
-        the delta rule,   7 heads of  64 x 128    626 / 314 / 81    10 parts  198 / 134 / 78   (14 parts 242 / 174 / 122)
-                          8 heads of 128 x 256    886 / 445 / 114   one piece                  (3 parts 894 / 492 / 189)
-    and four portions of 512 tokens: linear attention, 7 heads of 64 x 128, 150 in one piece, 96 in 10 parts."""
+        the delta rule,   7 heads of  64 x 128    626 / 314 / 81    14, 10 and 6 parts 242 / 134 / 61   (14 parts 242 / 174 / 122)
+                          8 heads of 128 x 256    886 / 445 / 114   6 parts 901, one piece     (3 parts 894 / 492 / 189)
+    and four portions of 512 tokens: linear attention, 7 heads of 64 x 128, 150 in one piece, 88 in 5 parts. (Alone. Between the
+    other kernels of a model 14 parts are the better ones for 2,048 tokens of the delta rule, 2,055 us a step against 2,069 in 10:
+    they fill the device, so no later launch's blocks wait where the fold's would run. So are 6 parts at the larger size: 6,687 us
+    a step against 6,813 in one piece.)"""
     if n_long <= 0:
         return 1
     first = int(library.load().bl_recurrent_scan_can_split(rule, H, dk, dv))
     if first <= 0:
         return 1
     blocks = int(library.load().bl_recurrent_scan_can_split(RULE_GLA, H, dk, dv))     # of a pass without further columns
-    cost = {p: _scan_cost(rule, H, dk, dv, n_long, p, first, blocks) for p in range(1, SCAN_MAX_PARTS + 1)}
+    cost = {p: _scan_cost(rule, H, dk, dv, n_long, tokens, p, first, blocks) for p in range(1, SCAN_MAX_PARTS + 1)}
     least = min(cost[p] for p in cost if p > 1)
     best = min(p for p in cost if p > 1 and cost[p] <= 1.02 * least)
-    return best if cost[best] <= 0.8 * cost[1] else 1
+    return best if cost[best] <= 0.9 * cost[1] else 1
 
 
 def recurrent_scan(rule: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, beta: Optional[torch.Tensor],

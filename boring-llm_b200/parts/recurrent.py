@@ -7,6 +7,7 @@ State, decays, gates and every sum of the recurrences are 32-bit in both engine 
 """
 from __future__ import annotations
 
+import math
 from typing import Dict, Optional
 
 import torch
@@ -41,7 +42,7 @@ class _StateMixer(Mixer):
         """Into how many parts a step's long portions are cut (they run side by side), how many requests have one, and how many
         portions are under way for most of the scan (the tokens over those of the longest)."""
         n_long = sum(1 for n in q_lens if n >= ops.SCAN_PART_MIN_TOKENS)
-        parts = ops.recurrent_scan_parts(self.RULE, self.H, self.dk, self._value_columns(), n_long) if n_long else 1
+        parts = ops.recurrent_scan_parts(self.RULE, self.H, self.dk, self._value_columns(), n_long, 1 << round(math.log2(max(q_lens)))) if n_long else 1
         return {"parts": parts, "n_long": n_long if parts > 1 else 0, "busy": max(1, round(sum(q_lens) / max(1, max(q_lens))))}
 
     def _value_columns(self) -> int:

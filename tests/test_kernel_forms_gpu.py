@@ -247,6 +247,7 @@ def test_scans_are_cut_where_that_was_measured_to_pay():
     assert parts(o.RULE_DELTA, 8, 128, 256, 1) == 1
     assert 4 <= parts(o.RULE_GLA, 8, 128, 256, 1) <= 12
     assert 8 <= parts(o.RULE_DELTA, 7, 64, 128, 1) <= 12 and 16 <= parts(o.RULE_GLA, 7, 64, 128, 1) <= 21
+    assert 4 <= parts(o.RULE_DELTA, 7, 64, 128, 1, 256) <= 8 and parts(o.RULE_DELTA, 7, 64, 128, 1, 2048) == 14
     assert parts(o.RULE_GLA, 8, 128, 256, 2) == 1 and parts(o.RULE_GLA, 7, 64, 128, 8) == 1 and parts(o.RULE_GLA, 7, 64, 128, 0) == 1
 
 
