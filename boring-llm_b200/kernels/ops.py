@@ -633,14 +633,17 @@ SKINNY_MAX_ROWS = 64                  # up to here W streams through registers (
 TC_MIN_COLUMNS_FEW_ROWS = 4096        # 17..64 rows: wide products have enough 128-column tiles for TMA to stream W at full rate
 TC_MIN_COLUMNS_VERY_FEW_ROWS = 32768  # an output head: up to 64 rows take the kernel made for it; without it 128-row tiles win from 9 rows
 COLS_MIN_COLUMNS = 9473               # up to 32 rows the output head's kernel takes all products of more column blocks than the kernel that streams
-                                      # W through registers keeps in flight (8 rows, 13,056 columns, K 2,048: 11.5 us against 31; 12,288 columns, K 1,024:
-                                      # 7.1 against 14.5; 5,760 columns, K 896: 5.3 against 4.2)
+                                      # W through registers keeps in flight: the faster at every number of rows from 1 to 32 (13,056 columns, K 2,048, 1, 16
+                                      # and 32 rows: 12.6, 12.1 and 13.0 us, the next best kernel 19.2, 19.0 and 13.2; 9,480 columns, K 520: 4.8, 5.0 and 5.4
+                                      # against 6.3, 6.8 and 7.3), but not below (8 rows of 5,760 columns, K 896: 5.3 against 4.2)
 PAIR_MIN_ROWS = 256                   # from here on pairs of SMs share 256 x 256 tiles (tcgen05 cta_group::2)
 SPLITK_MIN_ROWS, SPLITK_MAX_ROWS = 32, 640   # products with few tiles in this range of rows are cut along K over clusters ...
 SPLITK_VERY_LONG_K = 16384            # ... or, below 32 rows, very long (K 18,944 by N 3,584 at 8 rows: 43 us against 72 us through registers)
-SPLITK_FEW_ROWS_K = 8192              # ... or, from 9 rows, this long (16 rows of K 11,008 by N 2,048: 12.9 us against 23.6 through registers, of 8,960 by
-                                      # 1,536 10.3 against 14.8; of 4,864 by 896 7.1 against 4.8), from 17 rows
-SPLITK_MORE_ROWS_K = 4096             # ... this long (24 rows of 4,864 by 896: 7.1 against 12.3, of 4,096 by 1,024 6.8 against 10.2; of 2,048 by 2,048 7.4 against 5.4)
+SPLITK_FEW_ROWS_K = 8192              # ... or, from 9 rows, this long (9 and 16 rows of K 11,008 by N 2,048: 13.4 and 13.3 us against 20.1 and 23.5 through
+                                      # registers, of 8,960 by 1,536 10.2 and 10.4 against 12.3 and 14.8; of few columns it may lose a microsecond: 12,288 by
+                                      # 1,024 10.8 and 10.9 against 9.3 and 11.0, 8,192 by 256 6.8 against 5.6 and 6.6; 16 rows of 4,864 by 896 7.1 against 4.8),
+SPLITK_MORE_ROWS_K = 4096             # ... or, from 17 rows, this long (17 and 31 rows of 4,864 by 896: 7.1 and 7.3 us against 9.9 and 12.0, of 4,096 by 2,048 8.0
+                                      # and 8.3 against 8.4 and 10.4, by 136 5.2 and 5.3 against 6.0 and 7.8; 24 rows of 2,048 by 2,048 7.4 against 5.4)
 STREAM_MIN_BYTES = 128 << 20          # matrices from this size on stream faster through TMA and tcgen05 than through registers, at any number of rows
 SPLITK_LONG_K = 2048                  # ... when K is long (measured: K 4,864 by N 896 gains 2x at 128 rows, 1.25x at 512; K 896 gains only up to 128 rows)
 
