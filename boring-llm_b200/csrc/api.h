@@ -516,6 +516,16 @@ int bl_latent_attention_mma(const void* q_lat, const void* q_rot, const void* ca
                             const int* block_table, int max_pages, const int* work, int n_work, int single, void* out, int H, int Tp,
                             int rank, int rot, int page_size, int window, float scale, const void* sinks, int sink_dtype, int n_splits,
                             float* part_o, float* part_ml, void* stream);
+// Every head's own keys and values made for the step. bl_latent_rows: rows 16 i .. 16 i + 15 of latent [., rank] and shared [., 64]
+// (its first `rot` columns) = the cached rows of the 16 keys from work[i][1] on of request work[i][0], zeros where there are none (latent.cu).
+// bl_attention_rows_tc: the tcgen05 attention (attention_tcgen05.cu) over q [T, H, own + rot], kv [L, H * own + H * dv] (all heads'
+// own parts of the keys, then all heads' values) and the keys' shared part rot_rows [L, 64]; key j of request r is row key_row[r] + j.
+int bl_latent_rows(const void* cache, const int* work, int n_work, const int* cu_q, const int* ctx_len, const int* block_table,
+                   int max_pages, int rank, int rot, void* latent, void* shared, void* stream);
+int bl_attention_rows_tc_supported(int own, int rot, int dv);
+int bl_attention_rows_tc(const void* q, const void* kv, const void* rot_rows, const int* key_row, const int* cu_q, const int* ctx_len,
+                         const int* tiles, int n_tiles, void* out, int T, int L, int H, int own, int rot, int dv, int window,
+                         float scale, const void* sinks, int sink_dtype, const float* gate, int ld_gate, int gate_dim, void* stream);
 // tile[i] = i / per for n_heads * per tiles; out[t, h * N + n] = hv[h, t, n] (* sigmoid(gate[t, h * N + n])) with hv [H, Tp, N] (latent.cu).
 int bl_head_tiles(int* tile, int n_heads, int per, void* stream);
 int bl_heads_gate_rows(const float* hv, const float* gate, long long ld_gate, void* out, int out_dtype, int T, int H, int N, int Tp,

@@ -31,6 +31,7 @@
 // scores are scaled after the dot product (src/math.br:319-322); a key j is visible to a query at position p
 // when j <= p and, with a window, j + window > p (:327-328).
 #include "tcgen05.cuh"
+#include <atomic>
 
 namespace {
 
@@ -52,20 +53,26 @@ constexpr uint32_t WAIT_LIMIT = 1u << 22;
 // thread's registers; twice the tensor-core work per score leaves the single group less to wait for), one share of
 // the output of 128 columns, written by block i + 1 only after block i's has been taken (the row warps take it before
 // they post P of block i + 1). Keys, values and q lie as DH / 64 atoms of 64 dimensions.
-template <int DH_, int GROUPS_>
+//
+// Keys of DH values with values of DV, both of them rows of matrices instead of pages (ROT > 0; attention over cached latents whose
+// keys and values have been made for this step): a key is DH - ROT values of its head's own, a column range of the matrix
+// `map_k`, and ROT that all heads share, the matrix `map_v`; the values are another column range of `map_k`. A key block is then one
+// box of 128 rows per atom. 128 + 64 with values of 128 as the head size 128, 64 + 32 with values of 64 as the head size 64.
+template <int DH_, int GROUPS_, int DV_ = DH_, int ROT_ = 0>
 struct Shape {
-    static constexpr int DH = DH_, GROUPS = GROUPS_;
-    static constexpr int ATOMS = DH / 64;
+    static constexpr int DH = DH_, GROUPS = GROUPS_, DV = DV_, ROT = ROT_;
+    static constexpr int ATOMS = (DH + 63) / 64, V_ATOMS = DV / 64, STEPS = DH / 16;     // atoms of a key row and of a value row, MMAs of the first product
     static constexpr int PAGE_BYTES = PAGE * DH * 2;
     static constexpr int THREADS = GROUPS * ROWS + 128;  // the row warps, a warp that issues S = Q K^T, two that copy, one that issues O = P V
-    static constexpr int Q_BYTES = ROWS * DH * 2, KV_BYTES = KBLK * DH * 2;
-    static constexpr int MERGE_ROW = DH / 2 + 1;                          // half of a group's output at the merge, rows padded by one float
+    static constexpr int Q_BYTES = ATOMS * ATOM_BYTES, K_BYTES = ATOMS * ATOM_BYTES, V_BYTES = V_ATOMS * ATOM_BYTES;
+    static constexpr int MERGE_ROW = DV / 2 + 1;                          // half of a group's output at the merge, rows padded by one float
     static constexpr int MERGE_BYTES = GROUPS == 2 ? ROWS * MERGE_ROW * 4 : 0;
-    static constexpr int OFF_Q = 0, OFF_K = Q_BYTES, OFF_V = OFF_K + 2 * KV_BYTES, OFF_MERGE = OFF_V + 2 * KV_BYTES;
+    static constexpr int OFF_Q = 0, OFF_K = Q_BYTES, OFF_V = OFF_K + 2 * K_BYTES, OFF_MERGE = OFF_V + 2 * V_BYTES;
     static constexpr int OFF_XCH = OFF_MERGE + 2 * MERGE_BYTES;          // the groups' maxima and sums at the merge: 4 x 128 floats
     static constexpr int OFF_BARS = OFF_XCH + 4 * ROWS * 4;
     static constexpr int SMEM_BYTES = OFF_BARS + 256;
-    static_assert(DH % 64 == 0 && COL_O + GROUPS * DH <= TMEM_COLS && SMEM_BYTES <= 227 * 1024, "shape does not fit an SM");
+    static_assert(COL_O + GROUPS * DV <= TMEM_COLS && SMEM_BYTES <= 227 * 1024, "shape does not fit an SM");
+    static_assert(ROT > 0 ? (DH - ROT) % 64 == 0 && ROT % 16 == 0 && ROT <= 64 : DH % 64 == 0 && DV == DH, "atoms of 64 values");
 };
 
 __device__ int g_status = 0;           // 0 = fine; else the code of the first wait that ran out
@@ -77,6 +84,7 @@ struct Params {
     int H, KV, window; float scale_log2;
     BlAttnTail tail;                   // a sink per head and a gate per (token, head), or nulls
     float cap_log2;                    // the kernel with a cap on the scores: the cap times log2 e (s <- cap tanh(s / cap) on the scaled score)
+    const int* key_row;                // keys in matrices: the row of a request's key 0 (its key j is row key_row[r] + j)
 };
 
 // Bounded wait. False when the bound ran out or another thread of the block has given up. SLEEP: the waiter is one
@@ -183,8 +191,9 @@ template <class S, bool CAP = false>
 __global__ void __launch_bounds__(S::THREADS, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const Params p) {
-    constexpr int DH = S::DH, GROUPS = S::GROUPS, ATOMS = S::ATOMS, PAGE_BYTES = S::PAGE_BYTES;
-    constexpr int Q_BYTES = S::Q_BYTES, KV_BYTES = S::KV_BYTES, MERGE_BYTES = S::MERGE_BYTES, MERGE_ROW = S::MERGE_ROW;
+    constexpr int DH = S::DH, DV = S::DV, GROUPS = S::GROUPS, ATOMS = S::ATOMS, V_ATOMS = S::V_ATOMS, PAGE_BYTES = S::PAGE_BYTES;
+    constexpr bool MATRIX = S::ROT > 0;                                  // keys and values in matrices
+    constexpr int Q_BYTES = S::Q_BYTES, K_BYTES = S::K_BYTES, V_BYTES = S::V_BYTES, MERGE_BYTES = S::MERGE_BYTES, MERGE_ROW = S::MERGE_ROW;
     constexpr int OFF_Q = S::OFF_Q, OFF_K = S::OFF_K, OFF_V = S::OFF_V, OFF_MERGE = S::OFF_MERGE, OFF_XCH = S::OFF_XCH;
     constexpr int OFF_BARS = S::OFF_BARS;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -218,7 +227,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const int r = p.tiles[2 * tile], tok0 = p.tiles[2 * tile + 1];
     const int head = blockIdx.x % p.H, kvh = head / (p.H / p.KV);
     const int q_begin = p.cu_q[r], q_len = p.cu_q[r + 1] - q_begin, ctx = p.ctx_len[r];
-    const int* table = p.block_table + (size_t)r * p.max_pages;
+    const int* table = MATRIX ? nullptr : p.block_table + (size_t)r * p.max_pages;
     const int rows_here = min(ROWS, q_len - tok0);                       // <= 0 only for the padding entries of a replayed step's list
     const int p_first = ctx - q_len + tok0, p_last = p_first + rows_here - 1;
     const int lo = p.window > 0 ? max(0, p_first - p.window + 1) : 0, hi = p_last;
@@ -277,10 +286,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             for (int a = 0; a < ATOMS; ++a)
                 tma_load_2d(base + OFF_Q + a * ATOM_BYTES, &map_q, full_q, head * DH + a * 64, q_begin + tok0);
         }
-        int page = lane < PAGES && nb > 0 ? page_of(b_begin, lane) : -1;
+        const int row0 = MATRIX && nb > 0 ? p.key_row[r] : 0;
+        int page = !MATRIX && lane < PAGES && nb > 0 ? page_of(b_begin, lane) : -1;
         for (int i = 0; ok && i < nb; ++i) {
             const int st = i & 1;
-            const int page_next = lane < PAGES && i + 1 < nb ? page_of(b_begin + i + 1, lane) : -1;   // on its way during this block's copies
+            const int page_next = !MATRIX && lane < PAGES && i + 1 < nb ? page_of(b_begin + i + 1, lane) : -1;   // on its way during this block's copies
             if (i >= 2) {                                                // the stage is free once block i - 2 has been multiplied
                 if (lane == 0)
                     ok = keys ? mbar_wait<true>(s_done0 + 8 * ((i - 2) % SBUFS), (uint32_t)(((i - 2) / SBUFS) & 1), give_up, 3)
@@ -288,7 +298,25 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
             }
-            const uint32_t bar = full0 + 8 * st, dst = base + off + st * KV_BYTES;
+            const uint32_t bar = full0 + 8 * st, dst = base + off + st * (keys ? K_BYTES : V_BYTES);
+            if constexpr (MATRIX) {                                      // 128 keys x 64 values a box; rows past the matrix arrive as zeros
+                if (elect_one()) {
+                    constexpr int OWN = (DH - S::ROT) / 64;              // atoms of the head's own part of a key
+                    const int row = row0 + (b_begin + i) * KBLK;
+                    mbar_expect_tx(bar, keys ? K_BYTES : V_BYTES);
+                    if (keys) {
+#pragma unroll
+                        for (int a = 0; a < OWN; ++a) tma_load_2d(dst + a * ATOM_BYTES, &map_k, bar, head * (DH - S::ROT) + a * 64, row);
+                        tma_load_2d(dst + OWN * ATOM_BYTES, &map_v, bar, 0, row);
+                    } else {
+#pragma unroll
+                        for (int a = 0; a < V_ATOMS; ++a) tma_load_2d(dst + a * ATOM_BYTES, &map_k, bar, p.H * (DH - S::ROT) + head * DV + a * 64, row);
+                    }
+                }
+                __syncwarp();
+                ++loads[st];
+                continue;
+            }
             const unsigned have = __ballot_sync(0xffffffffu, lane < PAGES && page >= 0);
             int pages[PAGES];
 #pragma unroll
@@ -319,9 +347,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
             for (int at = 0; at < ATOMS; ++at) {                         // 64 dimensions of the head an atom, 16 a step
                 const uint64_t a = smem_desc(base + OFF_Q + at * ATOM_BYTES);
-                const uint64_t b = smem_desc(base + OFF_K + (i & 1) * KV_BYTES + at * ATOM_BYTES);
+                const uint64_t b = smem_desc(base + OFF_K + (i & 1) * K_BYTES + at * ATOM_BYTES);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) umma_bf16(tmem + (i % SBUFS) * KBLK, a + 2 * k, b + 2 * k, IDESC_S, (at | k) != 0);
+                for (int k = 0; k < 4 && 4 * at + k < S::STEPS; ++k) umma_bf16(tmem + (i % SBUFS) * KBLK, a + 2 * k, b + 2 * k, IDESC_S, (at | k) != 0);
             }
             umma_commit(s_done0 + 8 * (i % SBUFS));
         };
@@ -357,11 +385,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 if (!ok) break;
                 fence_after_sync();
 #pragma unroll
-                for (int at = 0; at < ATOMS; ++at) {                     // 64 dimensions of the head at a time
-                    const uint64_t bv = smem_desc(base + OFF_V + st * KV_BYTES + at * ATOM_BYTES);
+                for (int at = 0; at < V_ATOMS; ++at) {                   // 64 dimensions of the head at a time
+                    const uint64_t bv = smem_desc(base + OFF_V + st * V_BYTES + at * ATOM_BYTES);
 #pragma unroll
                     for (int kk = 0; kk < KBLK / 16; ++kk)              // 16 keys a step: 8 columns of P, two 8-row groups of V
-                        umma_bf16_ts(tmem + COL_O + (GROUPS == 2 ? st * DH : 0) + at * 64, tmem + buf * KBLK + COL_P + kk * 8,
+                        umma_bf16_ts(tmem + COL_O + (GROUPS == 2 ? st * DV : 0) + at * 64, tmem + buf * KBLK + COL_P + kk * 8,
                                      bv + (uint64_t)(kk * (2048 >> 4)), IDESC_PV, (kk == 0 && i < GROUPS) ? 0u : 1u);   // the group's first block starts its sum
                 }
                 umma_commit(o_done0 + 8 * st);
@@ -387,7 +415,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // accumulated output (load, scale, store), which after a row's first blocks is rare.
         constexpr float RESCALE = 8.f;
         float m = -INFINITY, l = 0.f;
-        const uint32_t t_o = tmem + COL_O + (GROUPS == 2 ? grp * DH : 0) + lane_off;
+        const uint32_t t_o = tmem + COL_O + (GROUPS == 2 ? grp * DV : 0) + lane_off;
         // Waits until the second product of block `blk` has been added. A wait on a barrier's phase is valid only
         // while the barrier is at most one phase behind the one asked for (phases are told apart by parity alone).
         // The group does not look at every one of these phases; what keeps it in step is the rotation of the score
@@ -460,7 +488,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 if (last >= 0) {                                          // what has been added so far moves to the new reference
                     if (!output_done(last)) { ok = false; break; }
 #pragma unroll
-                    for (int h = 0; h < DH / 32; ++h) {
+                    for (int h = 0; h < DV / 32; ++h) {
                         uint32_t v[32];
                         tmem_ld32(t_o + h * 32, v);
                         tmem_ld_wait(v);
@@ -528,20 +556,20 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             l = l * alpha + ((s_a + s_b) + (s_c + s_d));
             // the values of this block: rows that were not copied, or that lie past the last key, become zeros
             // (their P is 0, and 0 times whatever an old request left in a page must stay 0)
-            if (k0 + KBLK - 1 > hi || k0 < lo) {
+            if (k0 + KBLK - 1 > hi || (!MATRIX && k0 < lo)) {
                 // (once the product before has been added, the values of two blocks ago have been copied: the
                 // barrier of this block's values is one phase behind at most)
                 if (last >= 0 && !output_done(last)) { ok = false; break; }
                 ok = mbar_wait(full_v, par, give_up, 10) && ok;
                 if (ok) {
                     // (atom, key row, 16-byte chunk); the swizzle keeps a row's chunks in the row
-                    for (int idx = threadIdx.x & (ROWS - 1); idx < ATOMS * KBLK * 8; idx += ROWS) {
+                    for (int idx = threadIdx.x & (ROWS - 1); idx < V_ATOMS * KBLK * 8; idx += ROWS) {
                         const int in_atom = idx % (KBLK * 8);
                         const int key = k0 + (in_atom >> 3);
                         const int first = key / PAGE * PAGE;
-                        const bool copied = !(first > hi || first + PAGE - 1 < lo) && table[first / PAGE] >= 0;
+                        const bool copied = MATRIX || (!(first > hi || first + PAGE - 1 < lo) && table[first / PAGE] >= 0);
                         if (!copied || key > hi)
-                            *reinterpret_cast<uint4*>(smem + OFF_V + st * KV_BYTES + (idx / (KBLK * 8)) * ATOM_BYTES + (in_atom << 4)) = make_uint4(0u, 0u, 0u, 0u);
+                            *reinterpret_cast<uint4*>(smem + OFF_V + st * V_BYTES + (idx / (KBLK * 8)) * ATOM_BYTES + (in_atom << 4)) = make_uint4(0u, 0u, 0u, 0u);
                     }
                 }
             }
@@ -552,16 +580,16 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             last = i;
         }
         ok = __all_sync(0xffffffffu, ok);
-        float o[DH];                                                     // the row's output against m, not yet divided by l
+        float o[DV];                                                     // the row's output against m, not yet divided by l
 #pragma unroll
-        for (int j = 0; j < DH; ++j) o[j] = 0.f;
+        for (int j = 0; j < DV; ++j) o[j] = 0.f;
         if (ok && last >= 0) {
             ok = mbar_wait(o_final0 + 8 * grp, 0, give_up, 13);
             ok = __all_sync(0xffffffffu, ok);
             if (ok) fence_after_sync();
             if (ok) {
 #pragma unroll
-                for (int h = 0; h < DH / 32; ++h) {
+                for (int h = 0; h < DV / 32; ++h) {
                     uint32_t v[32];
                     tmem_ld32(t_o + h * 32, v);
                     tmem_ld_wait(v);
@@ -575,11 +603,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             ok = __all_sync(0xffffffffu, ok);
             if (ok && valid) {
                 const float inv = bl_attn_tail(p.tail, m, l, (size_t)(q_begin + tok0 + row), head);
-                __nv_bfloat16* dst = p.out + ((size_t)(q_begin + tok0 + row) * p.H + head) * DH;
+                __nv_bfloat16* dst = p.out + ((size_t)(q_begin + tok0 + row) * p.H + head) * DV;
                 // (the row's channel gate, if there is one, in a loop of its own: 16 channels at a time keep the registers as they were)
                 if (p.tail.gate_dim) {
 #pragma unroll
-                    for (int c = 0; c < DH; c += 16) {
+                    for (int c = 0; c < DV; c += 16) {
                         asm volatile("" ::: "memory");
 #pragma unroll
                         for (int j = c; j < c + 16; j += 4) {
@@ -589,7 +617,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     }
                 }
 #pragma unroll
-                for (int j = 0; j < DH; j += 8)
+                for (int j = 0; j < DV; j += 8)
                     *reinterpret_cast<uint4*>(dst + j) = make_uint4(pack_bf16(o[j] * inv, o[j + 1] * inv), pack_bf16(o[j + 2] * inv, o[j + 3] * inv),
                                                                     pack_bf16(o[j + 4] * inv, o[j + 5] * inv), pack_bf16(o[j + 6] * inv, o[j + 7] * inv));
             }
@@ -599,7 +627,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             float* mine = reinterpret_cast<float*>(smem + OFF_MERGE + grp * MERGE_BYTES);          // [row][MERGE_ROW]
             const float* theirs = reinterpret_cast<const float*>(smem + OFF_MERGE + (grp ^ 1) * MERGE_BYTES);
 #pragma unroll
-            for (int j = 0; j < DH / 2; ++j) mine[row * MERGE_ROW + j] = grp ? o[j] : o[DH / 2 + j];
+            for (int j = 0; j < DV / 2; ++j) mine[row * MERGE_ROW + j] = grp ? o[j] : o[DV / 2 + j];
             xch[(grp * 2) * ROWS + row] = m;
             xch[(grp * 2 + 1) * ROWS + row] = l;
             mbar_arrive(l_ready);
@@ -612,19 +640,19 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 const float total = l * a + l_o * a_o;
                 const float inv = bl_attn_tail(p.tail, mm, total, (size_t)(q_begin + tok0 + row), head);
                 const float wa = a * inv, wo = a_o * inv;
-                float r[DH / 2];
+                float r[DV / 2];
 #pragma unroll
-                for (int j = 0; j < DH / 2; ++j) r[j] = (grp ? o[DH / 2 + j] : o[j]) * wa + theirs[row * MERGE_ROW + j] * wo;
+                for (int j = 0; j < DV / 2; ++j) r[j] = (grp ? o[DV / 2 + j] : o[j]) * wa + theirs[row * MERGE_ROW + j] * wo;
                 if (p.tail.gate_dim) {
 #pragma unroll
-                    for (int j = 0; j < DH / 2; j += 4) {
-                        const float4 cg = bl_gate4(p.tail, (size_t)(q_begin + tok0 + row), head, grp * (DH / 2) + j);
+                    for (int j = 0; j < DV / 2; j += 4) {
+                        const float4 cg = bl_gate4(p.tail, (size_t)(q_begin + tok0 + row), head, grp * (DV / 2) + j);
                         r[j] *= cg.x; r[j + 1] *= cg.y; r[j + 2] *= cg.z; r[j + 3] *= cg.w;
                     }
                 }
-                __nv_bfloat16* dst = p.out + ((size_t)(q_begin + tok0 + row) * p.H + head) * DH + grp * (DH / 2);
+                __nv_bfloat16* dst = p.out + ((size_t)(q_begin + tok0 + row) * p.H + head) * DV + grp * (DV / 2);
 #pragma unroll
-                for (int j = 0; j < DH / 2; j += 8)
+                for (int j = 0; j < DV / 2; j += 8)
                     *reinterpret_cast<uint4*>(dst + j) = make_uint4(pack_bf16(r[j], r[j + 1]), pack_bf16(r[j + 2], r[j + 3]),
                                                                     pack_bf16(r[j + 4], r[j + 5]), pack_bf16(r[j + 6], r[j + 7]));
             }
@@ -665,6 +693,51 @@ int launch(const void* q, const void* k_cache, const void* v_cache, const Params
 
 }  // namespace
 
+namespace {
+
+template <class S>
+int launch_matrix(const void* q, const void* kv, const void* rot, const Params& p, int n_tiles, int T, int L, cudaStream_t stream) {
+    CUtensorMap mq, mk, mr;
+    if (bl_make_map_bf16(WHO, &mq, q, T, p.H * S::DH, ROWS, 64)) return 1;
+    if (bl_make_map_bf16(WHO, &mk, kv, L, p.H * (S::DH - S::ROT + S::DV), KBLK, 64)) return 1;
+    if (bl_make_map_bf16(WHO, &mr, rot, L, 64, KBLK, 64)) return 1;
+    static std::atomic<bool> configured{false};                          // per shape
+    if (!configured) {
+        BL_CUDA(cudaFuncSetAttribute(attention_tc_kernel<S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM_BYTES));
+        configured = true;
+    }
+    BL_CUDA(bl_launch_dependent(attention_tc_kernel<S, false>, dim3(n_tiles * p.H, 1, 1), dim3(S::THREADS), (size_t)S::SMEM_BYTES, stream,
+                                mq, mk, mr, p));
+    BL_CHECK_LAUNCH("bl_attention_rows_tc");
+    return 0;
+}
+
+}  // namespace
+
+extern "C" int bl_attention_rows_tc_supported(int own, int rot, int dv) { return (own == 128 && rot == 64 && dv == 128) || (own == 64 && rot == 32 && dv == 64); }
+
+// The same attention with every head's keys and values made for the step: q [T, H, own + rot]; kv [L, H * own + H * dv], first all
+// heads' own parts of the keys, then all heads' values; rot [L, 64], the part of the keys that all heads share in its first
+// `rot` columns. Key j of request r is row key_row[r] + j, for every block of 128 keys (multiples of 128) that a new token of r sees.
+// 1,400 + 600 tokens of 16 heads of 128 + 64 with values of 128 and a window of 1,024: 38 us, where the attention over the cached
+// rows of 512 + 64 values (latent_mma.cu) takes 265.
+extern "C" int bl_attention_rows_tc(const void* q, const void* kv, const void* rot_rows, const int* key_row, const int* cu_q, const int* ctx_len,
+                                    const int* tiles, int n_tiles, void* out, int T, int L, int H, int own, int rot, int dv, int window,
+                                    float scale, const void* sinks, int sink_dtype, const float* gate, int ld_gate, int gate_dim, void* stream) {
+    if (n_tiles <= 0) return 0;
+    if (!bl_attention_rows_tc_supported(own, rot, dv)) BL_FAIL("bl_attention_rows_tc: keys of %d + %d with values of %d are not built (128 + 64 with 128, 64 + 32 with 64)", own, rot, dv);
+    if (H <= 0 || T <= 0 || L <= 0 || window < 0 || key_row == nullptr) BL_FAIL("bl_attention_rows_tc: bad sizes H=%d T=%d L=%d", H, T, L);
+    if (!(scale > 0.f)) BL_FAIL("bl_attention_rows_tc: the scale of the scores must be positive (got %g)", (double)scale);
+    if (((uintptr_t)q | (uintptr_t)kv | (uintptr_t)rot_rows | (uintptr_t)out) & 15) BL_FAIL("bl_attention_rows_tc: q, keys, values and out must be 16-byte aligned");
+    if ((long long)n_tiles * H > 2147483647LL) BL_FAIL("bl_attention_rows_tc: %d tiles x %d heads are more blocks than a launch takes", n_tiles, H);
+    if (!bl_channel_gate_ok(gate, ld_gate, gate_dim, H, dv)) BL_FAIL("%s: a gate of %d channels a head in rows of %d does not fit %d heads of %d in 16-byte pieces", "bl_attention_rows_tc", gate_dim, ld_gate, H, dv);
+    Params p{};
+    p.out = (__nv_bfloat16*)out; p.cu_q = cu_q; p.ctx_len = ctx_len; p.tiles = tiles; p.H = H; p.KV = H; p.window = window;
+    p.scale_log2 = scale * 1.4426950408889634f; p.tail = BlAttnTail{sinks, sink_dtype, gate, ld_gate, gate_dim}; p.key_row = key_row;
+    if (own == 128) return launch_matrix<Shape<192, 1, 128, 64>>(q, kv, rot_rows, p, n_tiles, T, L, (cudaStream_t)stream);
+    return launch_matrix<Shape<96, 2, 64, 32>>(q, kv, rot_rows, p, n_tiles, T, L, (cudaStream_t)stream);
+}
+
 // tiles[n_tiles][2] = (request, first token of the tile's 128 rows within the request's new tokens); the last
 // entries start first. T: rows of q and out; n_pages: pages of the cache tensors (their first dimension).
 extern "C" int bl_attention_prefill_tc(const void* q, const void* k_cache, const void* v_cache, const int* cu_q,
@@ -700,7 +773,7 @@ extern "C" int bl_attention_prefill_tc_cap(const void* q, const void* k_cache, c
     if (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out) & 15)
         BL_FAIL("bl_attention_prefill_tc: q, the caches and out must be 16-byte aligned");
     if ((long long)n_tiles * H > 2147483647LL) BL_FAIL("bl_attention_prefill_tc: %d tiles x %d heads are more blocks than a launch takes", n_tiles, H);
-    Params p;
+    Params p{};
     p.out = (__nv_bfloat16*)out; p.cu_q = cu_q; p.ctx_len = ctx_len; p.block_table = block_table; p.max_pages = max_pages;
     p.tiles = tiles; p.H = H; p.KV = KV; p.window = window; p.scale_log2 = scale * 1.4426950408889634f;
     p.tail = BlAttnTail{sinks, sink_dtype, gate, ld_gate, gate_dim};

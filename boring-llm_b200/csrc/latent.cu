@@ -338,7 +338,43 @@ __global__ void heads_gate_rows4_kernel(const float* __restrict__ hv, const floa
     }
 }
 
+// Cached rows of a step's requests side by side, for the product that makes every head's keys and values of them: block i copies
+// the page of 16 keys that starts at key work[i][1] of request work[i][0] to rows 16 i .. of latent [., rank] and of shared [., 64]
+// (its first `rot` columns). Keys past the request's last and pages that a window has given back become zeros, so that the product is
+// finite everywhere. Bound by trips: 2,000 rows of 576 values 4.5 us in a chain of kernels.
+__global__ void __launch_bounds__(THREADS)
+latent_rows_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restrict__ work, const int* __restrict__ cu_q,
+                   const int* __restrict__ ctx_len, const int* __restrict__ block_table, int max_pages, int rank, int rot,
+                   __nv_bfloat16* __restrict__ latent, __nv_bfloat16* __restrict__ shared) {
+    bl_pdl_trigger();
+    const int r = work[2 * blockIdx.x], key0 = work[2 * blockIdx.x + 1];
+    const int have = cu_q[r + 1] - cu_q[r] > 0 ? ctx_len[r] - key0 : 0;          // (padding entries name a request without tokens)
+    const int page = have > 0 ? block_table[(size_t)r * max_pages + key0 / 16] : -1;
+    const int dk = rank + rot, chunks = dk / 8, own = rank / 8;
+    const __nv_bfloat16* src = cache + (size_t)(page < 0 ? 0 : page) * 16 * dk;
+    bl_pdl_wait();
+    for (int c = threadIdx.x; c < 16 * chunks; c += THREADS) {
+        const int row = c / chunks, at = c % chunks;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (page >= 0 && row < have) v = *reinterpret_cast<const uint4*>(src + (size_t)row * dk + at * 8);
+        const size_t to = (size_t)blockIdx.x * 16 + row;
+        if (at < own) *reinterpret_cast<uint4*>(latent + to * rank + at * 8) = v;
+        else *reinterpret_cast<uint4*>(shared + to * 64 + (at - own) * 8) = v;
+    }
+}
+
 }  // namespace
+
+extern "C" int bl_latent_rows(const void* cache, const int* work, int n_work, const int* cu_q, const int* ctx_len, const int* block_table,
+                              int max_pages, int rank, int rot, void* latent, void* shared, void* stream) {
+    if (n_work <= 0) return 0;
+    if (rank <= 0 || rank % 8 != 0 || rot < 0 || rot > 64 || rot % 8 != 0 || max_pages <= 0) BL_FAIL("bl_latent_rows: rows of %d + %d values are not copied (whole 16-byte pieces, at most 64 shared values)", rank, rot);
+    if (((uintptr_t)cache | (uintptr_t)latent | (uintptr_t)shared) & 15) BL_FAIL("bl_latent_rows: cache and rows must be 16-byte aligned");
+    BL_CUDA(bl_launch_dependent(latent_rows_kernel, dim3(n_work), dim3(THREADS), 0, (cudaStream_t)stream, (const __nv_bfloat16*)cache, work,
+                                cu_q, ctx_len, block_table, max_pages, rank, rot, (__nv_bfloat16*)latent, (__nv_bfloat16*)shared));
+    BL_CHECK_LAUNCH("bl_latent_rows");
+    return 0;
+}
 
 extern "C" int bl_head_tiles(int* tile, int n_heads, int per, void* stream) {
     if (n_heads <= 0 || per <= 0) BL_FAIL("bl_head_tiles: %d heads with %d tiles each", n_heads, per);

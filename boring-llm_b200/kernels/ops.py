@@ -1656,6 +1656,42 @@ def latent_attention_mma(q_lat: torch.Tensor, q_rot: Optional[torch.Tensor], cac
           ctypes.c_float(scale), _p(sinks), _vec_dt(sinks), n_splits, _p(part_o), _p(part_ml), _stream())
 
 
+LATENT_KEY_SHAPES = ((128, 64, 128), (64, 32, 64))     # (own part of a head's key, shared part, values) that the tcgen05 kernel has
+
+
+def latent_rows(cache: torch.Tensor, work: torch.Tensor, cu_q: torch.Tensor, ctx_len: torch.Tensor, block_table: torch.Tensor,
+                latent: torch.Tensor, shared: torch.Tensor) -> None:
+    """Rows 16 i .. of latent [L, rank] and of shared [L, 64] (its first columns) are the cached rows [latent | shared part] of the 16
+    keys from work[i, 1] on (a multiple of 16) of request work[i, 0]; zeros past its last key, for pages that are gone and for requests
+    without tokens."""
+    L, rank = latent.shape
+    _need(cache, "cache", torch.bfloat16); _need(work, "work", torch.int32, (L // 16, 2))
+    _need(latent, "latent", torch.bfloat16); _need(shared, "shared", torch.bfloat16, (L, 64))
+    if cache.dim() != 4 or cache.shape[1] != 1 or cache.shape[2] != 16 or cache.shape[3] < rank:
+        raise KernelError(f"latent_rows: cache {tuple(cache.shape)} does not hold rows of {rank} and more in pages of 16")
+    _need(cu_q, "cu_q", torch.int32); _need(ctx_len, "ctx_len", torch.int32); _need(block_table, "block_table", torch.int32)
+    _call(_lib().bl_latent_rows, _p(cache), _p(work), work.shape[0], _p(cu_q), _p(ctx_len), _p(block_table), block_table.shape[1], rank,
+          cache.shape[3] - rank, _p(latent), _p(shared), _stream())
+
+
+def attention_rows_tc(q: torch.Tensor, kv: torch.Tensor, shared: torch.Tensor, key_row: torch.Tensor, cu_q: torch.Tensor,
+                      ctx_len: torch.Tensor, tiles: torch.Tensor, out: torch.Tensor, H: int, own: int, dv: int, window: int,
+                      scale: float, sinks: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, gate_dim: int = 0) -> None:
+    """Causal attention on the tcgen05 kernel over keys and values made for this step: q [T, H * (own + rot)], kv [L, H * own + H * dv]
+    (all heads' own parts of the keys, then all heads' values), shared [L, 64] (the part of the keys that all heads share, in its first
+    rot columns). Key j of request r is row key_row[r] + j; a block of 128 keys that a new token sees must lie in the rows whole or
+    end with them. out [T, H * dv]. `tiles`, `window`, `sinks` and `gate` as in `attention_prefill_tc`."""
+    T = q.shape[0]
+    L = kv.shape[0]
+    rot = q.shape[1] // H - own
+    _need(q, "q", torch.bfloat16, (T, H * (own + rot))); _need(kv, "kv", torch.bfloat16, (L, H * (own + dv)))
+    _need(shared, "shared", torch.bfloat16, (L, 64)); _need(out, "out", torch.bfloat16, (T, H * dv))
+    _need(key_row, "key_row", torch.int32); _need(cu_q, "cu_q", torch.int32); _need(ctx_len, "ctx_len", torch.int32)
+    _need(tiles, "tiles", torch.int32, (tiles.shape[0], 2))
+    _call(_lib().bl_attention_rows_tc, _p(q), _p(kv), _p(shared), _p(key_row), _p(cu_q), _p(ctx_len), _p(tiles), tiles.shape[0], _p(out),
+          T, L, H, own, rot, dv, window, ctypes.c_float(scale), *_tail(T, H, sinks, gate, gate_dim), gate_dim, _stream())
+
+
 LATENT_ROWS = 32               # rows of a block of the latent attention kernel (heads of a single token)
 LATENT_RESIDENT = 2 * 148      # its blocks that the device holds at once (two an SM up to 256 latent values)
 LATENT_MAX_SPLITS = 16

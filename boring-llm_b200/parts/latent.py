@@ -3,15 +3,69 @@ from __future__ import annotations
 
 from typing import Dict, Optional
 
+import numpy as np
 import torch
 
 from ..cache import PagedKVSpec
 from ..kernels import ops
 from ..weights import TensorSpec, MATRIX, BIAS, NORM
-from .attention import Mixer, PLAN_KEY, attention_plan
-from .base import to_device_matrix, to_device_vector
+from .attention import Mixer, attention_plan
+from .base import StepPlan, to_device_matrix, to_device_vector
 from .linear import linear, EPI_NONE, EPI_RESIDUAL
 from .rotary import RotaryTable
+
+
+KEY_BLOCK = 128                # keys that the tcgen05 attention reads at a time
+
+
+def latent_keys_plan(q_lens, ctx_lens, filler, window: int, sizes) -> Optional[StepPlan]:
+    """What a step does that makes every head's keys and values of the rows its tokens see (`LatentAttention`), or None where the
+    attention over the cached rows themselves is the faster. `work` [L / 16, 2]: the (request, first key) of each page whose rows
+    go to rows 16 i .. of the step's matrices; `key_row` [requests]: the row of a request's key 0 (key blocks start at multiples of
+    128, so every block that is read lies in the request's own rows or past its last key); `tiles` [n, 2]: the 128-token tiles, the
+    one with the fewest keys first. Requests with a single token and a long context (decoding beside prompts) would pay for all of
+    their context: such steps stay with the cached rows. The lists of a step that is replayed (`filler` given) are padded to
+    multiples of 8.
+
+    The line between the two, in microseconds (`sizes`: heads, own and shared part of a key, values, rank): the cached rows cost
+    143 TFLOP/s over 2 (2 rank + shared) operations a (query, key, head) and 150 in the products with Uk and Uv before and behind;
+    keys and values of their own 300 over 2 (own + shared + values), and their product over all rows at 700; 6 us more of launches.
+    A step of one prompt over eight layers, cached rows and own keys: 16 heads of 128 + 64 over a rank of 512, 160 tokens 1,873 and
+    1,788 us, 256 1,944 and 1,826, 512 2,311 and 2,037, 2,000 6,306 and 3,671; 14 heads of 64 + 32 over 256, 512 1,234 and 1,043,
+    1,000 1,650 and 1,236, 2,000 2,610 and 1,560."""
+    H, dn, dr, dv, rank = sizes
+    pairs, tokens, at = 0.0, 0, 0
+    key_row = [0] * len(q_lens)
+    work, tiles = [], []
+    for r, (n, c) in enumerate(zip(q_lens, ctx_lens)):
+        if n == 0:
+            continue
+        if n == 1 and c > KEY_BLOCK:
+            return None
+        start = max(0, c - n - window + 1) // KEY_BLOCK * KEY_BLOCK if window > 0 else 0
+        key_row[r] = at - start
+        pages = -(-(c - start) // 16)
+        work += [[r, start + 16 * i] for i in range(pages)]
+        at += 16 * pages
+        seen = min(window, c - 0.5 * n) if window > 0 else c - 0.5 * n
+        pairs += n * seen
+        tokens += n
+        for t0 in range(0, n, KEY_BLOCK):
+            first = c - n + t0
+            lo = max(0, first - window + 1) if window > 0 else 0
+            tiles.append([min(first + KEY_BLOCK, c) // KEY_BLOCK - lo // KEY_BLOCK, r, t0])
+    cached = pairs * H * (4 * rank + 2 * dr) / 143e6 + tokens * H * rank * 2.0 * (dn + dv) / 150e6
+    own = pairs * H * 2.0 * (dn + dr + dv) / 300e6 + at * H * rank * 2.0 * (dn + dv) / 700e6 + 6.0
+    if own >= cached:
+        return None
+    tiles.sort()
+    tiles = [t[1:] for t in tiles]
+    if filler is not None:
+        work = work + [[filler, 0]] * (-len(work) % 8)
+        tiles = [[filler, 0]] * (-len(tiles) % 8) + tiles                # the front of this list is launched last
+    return StepPlan(arrays={"work": np.asarray(work, dtype=np.int32), "key_row": np.asarray(key_row, dtype=np.int32),
+                            "tiles": np.asarray(tiles, dtype=np.int32)},
+                    host={}, shape=("keys", len(work), len(key_row), len(tiles)))
 
 
 class LatentAttention(Mixer):
@@ -32,8 +86,10 @@ class LatentAttention(Mixer):
       entry names that cache layer with `write_cache=False`); `cache_window` is then what the owner and all its readers
       agree the cache keeps (the widest of their windows, 0 if any sees everything).
 
-    Only [c | rotated part] is cached (one row of kv_rank + rot_dim values per token, `values_in_keys`). The products with
-    Uk and Uv are moved to the query's side, q' = Uk_h^T q_nope and out_h = Uv_h (sum_j p_j c_j), so every head of every
+    Only [c | rotated part] is cached (one row of kv_rank + rot_dim values per token, `values_in_keys`). Two ways from there. For a
+    step's prompts (`latent_keys_plan` says when) every head's keys and values of the rows they see are made by one product with
+    [Uk; Uv] over those rows, and the tcgen05 attention runs on them: 2 (nope_dim + rot_dim + v_dim) operations a (query, key, head)
+    instead of 2 (2 kv_rank + rot_dim). Otherwise the products with Uk and Uv are moved to the query's side, q' = Uk_h^T q_nope and out_h = Uv_h (sum_j p_j c_j), so every head of every
     token reads the same cached rows. All of the mixer's first products (Wdq, Wdkv, Wg) are ONE joined product with
     32-bit sums; both norms, the rotation and the cache write are one kernel; the gate is applied where the product with
     Uv is read. Norms, angles, scores and the softmax are 32-bit.
@@ -70,7 +126,7 @@ class LatentAttention(Mixer):
         self.off_g = self.off_kv + (pad(kv_rank + rot_dim) if self.own_kv else 0)
         self.n_gate = (n_heads if self.gate_heads else n_heads * v_dim) if self.out_gate else 0
         self.n_in = self.off_g + (pad(self.n_gate) if self.gate_heads else self.n_gate)
-        self.w_in = self.wuq = self.wuk = self.wuv = self.wo = self.dq_norm = self.dkv_norm = self.sinks = None
+        self.w_in = self.wuq = self.wkv = self.wuk = self.wuv = self.wo = self.dq_norm = self.dkv_norm = self.sinks = None
 
     def local_specs(self):
         s = {"wdq": TensorSpec((self.q_rank, self.dim), MATRIX), "dq_norm": TensorSpec((self.q_rank,), NORM),
@@ -107,10 +163,12 @@ class LatentAttention(Mixer):
         per = self.dn + self.dr
         wuq = torch.cat([self._halves(local["wuq"][h * per:(h + 1) * per], self.dn) for h in range(self.H)])
         self.wuq = to_device_matrix(wuq, dtype, device)
-        self.wuk = to_device_matrix(local["wuk"], dtype, device)              # [H * nope_dim, kv_rank] as stored
+        # [Uk; Uv], the matrix that makes all heads' keys and values of a latent
+        self.wkv = to_device_matrix(torch.cat([local["wuk"], local["wuv"]]), dtype, device)
+        self.wuk = self.wkv[:self.H * self.dn]                                # [H * nope_dim, kv_rank] as stored
         # Uk_h^T stacked [H, kv_rank, nope_dim]: the matrices of the grouped product that moves the queries into the latent's space
         self.wuk_t = to_device_matrix(local["wuk"].view(self.H, self.dn, self.rank).transpose(1, 2).contiguous(), dtype, device)
-        self.wuv = to_device_matrix(local["wuv"], dtype, device)              # [H * v_dim, kv_rank] as stored
+        self.wuv = self.wkv[self.H * self.dn:]                                # [H * v_dim, kv_rank] as stored
         self.wo = to_device_matrix(local["wo"], dtype, device)
         if self.has_sink:
             self.sinks = to_device_vector(local["sink"], dtype, device)
@@ -126,8 +184,28 @@ class LatentAttention(Mixer):
                 and self.w_in.dtype == torch.bfloat16 and -(-self.n_in // 16) <= ops.SKINNY_LINK_MAX_BLOCKS
                 and not ops.gemm_streams_better(self.w_in))
 
+    def _plan_key(self) -> str:
+        """Mixers of equal sizes and window share their plan."""
+        return "latent attention, window %d, %d heads, sizes %d %d %d %d" % (self.window, self.H, self.dn, self.dr, self.dv, self.rank)
+
+    def _makes_keys(self) -> bool:
+        """Whether steps of prompts may run on keys and values of their own."""
+        return bool((self.dn, self.dr, self.dv) in ops.LATENT_KEY_SHAPES and self.rank % 8 == 0 and self.scale > 0
+                    and self.wkv is not None and self.wkv.dtype == torch.bfloat16)
+
     def plan_step(self, q_lens, ctx_lens, filler=None):
-        return PLAN_KEY, attention_plan(q_lens, ctx_lens, filler)
+        plan = None
+        if self._makes_keys():
+            plan = latent_keys_plan(q_lens, ctx_lens, filler, self.window, (self.H, self.dn, self.dr, self.dv, self.rank))
+        return self._plan_key(), plan if plan is not None else attention_plan(q_lens, ctx_lens, filler)
+
+    def _plan(self, ctx) -> StepPlan:
+        plan = ctx.plans.get(self._plan_key())
+        if plan is None:                              # a step put together without asking the parts: plan it now
+            plan = self.plan_step(ctx.q_lens, ctx.ctx_lens)[1]
+            plan.arrays = {k: torch.from_numpy(v).to(ctx.device) for k, v in plan.arrays.items()}
+            ctx.plans[self._plan_key()] = plan
+        return plan
 
     # -- the steps of a pass, each one kernel or product ----------------------------------------------------------------
     def absorbed_queries(self, ctx, cq):
@@ -149,6 +227,30 @@ class LatentAttention(Mixer):
     def head_major(self, ctx, cache) -> bool:
         """Whether this step runs on the tensor-core kernels in the head-major layout."""
         return bool(ctx.fast and self.dn % 8 == 0 and ops.latent_attention_mma_supported(cache.dtype, self.rank, self.dr, cache.shape[2]))
+
+    def _attend_own_keys(self, ctx, cq, cache, cache_layer, table, gate, heads, plan):
+        """heads [T, H * v_dim] from the normed query latent cq, over every head's own keys and values of the cached rows."""
+        T, H = cq.shape[0], self.H
+        per = self.dn + self.dr
+        work = plan.arrays["work"]
+        key = ("latent rows", cache_layer, self._plan_key())
+        if not self.own_kv and key in ctx.memo:       # the layer that wrote the cache has read the same rows back already
+            latent, shared = ctx.memo[key]
+        else:
+            latent, shared = ctx.empty((16 * work.shape[0], self.rank)), ctx.empty((16 * work.shape[0], 64))
+            ops.latent_rows(cache, work, ctx.cu_q, ctx.ctx_len, table, latent, shared)
+            ctx.memo[key] = (latent, shared)
+        kv = ctx.empty((latent.shape[0], H * (self.dn + self.dv)))
+        linear(ctx, latent, self.wkv, kv, None, EPI_NONE)
+        q32 = ctx.empty((T, H * per), torch.float32)
+        linear(ctx, cq, self.wuq, q32, None, EPI_NONE)
+        q = ctx.empty((T, H * per))
+        q32v, qv = q32.view(T, H, per), q.view(T, H, per)
+        ops.rope_heads(q32v[:, :, self.dn:], ctx.positions, self.rotary.inv_freq, self.rotary.rot_half, self.rotary.mscale,
+                       qv[:, :, self.dn:], lead=q32v[:, :, :self.dn], lead_out=qv[:, :, :self.dn])
+        ops.attention_rows_tc(q, kv, shared, plan.arrays["key_row"], ctx.cu_q, ctx.ctx_len, plan.arrays["tiles"], heads, H, self.dn,
+                              self.dv, self.window, self.scale, self.sinks, gate,
+                              gate_dim=0 if gate is None or self.gate_heads else self.dv)
 
     def _attend_head_major(self, ctx, cq, cache, table, gate, heads):
         """heads [T, H * v_dim] from the normed query latent cq, over the cached rows, everything in between head-major."""
@@ -172,11 +274,7 @@ class LatentAttention(Mixer):
         q_lat = ctx.empty((H, Tp, self.rank))
         ops.gemm_grouped(qn.view(H * Tp, self.dn), self.wuk_t, tile_head, q_lat.view(H * Tp, self.rank), EPI_NONE)
         lat = ctx.empty((H, Tp, self.rank))
-        plan = ctx.plans.get(PLAN_KEY)
-        if plan is None:                              # a step put together without asking the parts: plan it now
-            plan = attention_plan(ctx.q_lens, ctx.ctx_lens)
-            plan.arrays = {k: torch.from_numpy(v).to(ctx.device) for k, v in plan.arrays.items()}
-            ctx.plans[PLAN_KEY] = plan
+        plan = self._plan(ctx)
         longest = plan.host["longest_single"]
         if self.window > 0:
             longest = min(longest, self.window + 64)
@@ -206,7 +304,11 @@ class LatentAttention(Mixer):
                         cache if write_cache else None)
         if self.head_major(ctx, cache):
             heads = ctx.empty((T, self.H * self.dv))
-            self._attend_head_major(ctx, cq, cache, table, self._gate(proj), heads)
+            plan = self._plan(ctx)
+            if "key_row" in plan.arrays:
+                self._attend_own_keys(ctx, cq, cache, cache_layer, table, self._gate(proj), heads, plan)
+            else:
+                self._attend_head_major(ctx, cq, cache, table, self._gate(proj), heads)
             linear(ctx, heads, self.wo, out, None, epilogue)
             return
         qa = self.absorbed_queries(ctx, cq)

@@ -509,3 +509,77 @@ def test_turned_heads_in_shares(T, H, n, rot_half, n_lead, gap, dtype):
     close(out, torch.cat([u * c - v * s, v * c + u * s, z[:, :, 2 * rot_half:]], 2), dtype, "turned heads")
     if n_lead:
         assert torch.equal(lead_out, lead.to(dtype))
+
+
+@pytest.mark.parametrize("H,own,rot,dv,rank", [(3, 128, 64, 128, 512), (2, 64, 32, 64, 72)])
+@pytest.mark.parametrize("window,gate_dim", [(0, 0), (200, 1), (128, 0), (37, 1)])
+def test_attention_over_keys_made_of_latents(H, own, rot, dv, rank, window, gate_dim):
+    """Portions that end at edges of tiles, key blocks and pages, beside single tokens of short contexts and a request without
+    tokens, pages that the window has given back missing from the table and full of NaN: the rows that are copied, bit for bit, and the
+    attention against 64 bits on the same bfloat16 operands."""
+    from boring_llm_b200.parts.latent import latent_keys_plan
+    o = ops()
+    ctx = [1, 130, 128, 700, 129, 16, 385, 128, 1]
+    q_lens = [1, 130, 127, 300, 1 if window == 0 else 2, 16, 129, 1, 0]
+    if window == 0:
+        ctx[4], q_lens[4] = 128, 1
+    R, T = len(ctx), sum(q_lens)
+    plan = latent_keys_plan(q_lens, ctx, R - 1, window, (H, own, rot, dv, 10 ** 6))
+    assert plan is not None and plan.shape == ("keys", len(plan.arrays["work"]), R, len(plan.arrays["tiles"]))
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    cu = [0]
+    for n in q_lens:
+        cu.append(cu[-1] + n)
+    dk = rank + rot
+    pages = sum(-(-c // 16) for c in ctx) + 1
+    cache = data((pages, 1, 16, dk), 1).to(BF)
+    width = max(-(-c // 16) for c in ctx) + 2
+    table, at, rows = np.full((R, width), -1, np.int32), 1, []
+    for r, (c, n) in enumerate(zip(ctx, q_lens)):
+        k = -(-c // 16)
+        first = max(0, c - max(n, 1) - window + 1) // 16 if window else 0           # the first page that a new token sees
+        got = cache[at:at + k, 0].reshape(-1, dk)[:c].clone()
+        got[:16 * first] = 0
+        cache[at:at + first] = float("nan")
+        table[r, first:k] = np.arange(at + first, at + k)
+        if c % 16:
+            cache[at + k - 1, 0, c % 16:] = float("nan")                            # what an earlier request left behind the last key
+        at += k
+        rows.append(got)
+    L = 16 * len(plan.arrays["work"])
+    latent, shared = torch.full((L, rank), 7.0, dtype=BF, device=DEV), torch.full((L, 64), 7.0, dtype=BF, device=DEV)
+    o.latent_rows(cache, i32(plan.arrays["work"]), i32(cu), i32(ctx), i32(table), latent, shared)
+    key_row = plan.arrays["key_row"]
+    starts = [max(0, c - n - window + 1) // 128 * 128 if window else 0 for c, n in zip(ctx, q_lens)]
+    for r, (c, n) in enumerate(zip(ctx, q_lens)):
+        if n:
+            to = int(key_row[r]) + starts[r]
+            assert torch.equal(latent[to:to + c - starts[r]], rows[r][starts[r]:, :rank])
+            assert torch.equal(shared[to:to + c - starts[r], :rot], rows[r][starts[r]:, rank:])
+    assert torch.isfinite(latent.float()).all()
+    kv = torch.empty(L, H * (own + dv), dtype=BF, device=DEV)
+    o.gemm(latent, (data((H * (own + dv), rank), 2) * rank ** -0.5).to(BF), kv)
+    q = data((T, H * (own + rot)), 3).to(BF)
+    sinks, gate = data((H,), 4), data((T, H * dv + 4), 5)
+    scale = 0.3
+    out = torch.full((T, H * dv), float("nan"), dtype=BF, device=DEV)
+    o.attention_rows_tc(q, kv, shared, i32(key_row), i32(cu), i32(ctx), i32(plan.arrays["tiles"]), out, H, own, dv, window, scale, sinks,
+                        gate if gate_dim else gate[:, :H], gate_dim=dv if gate_dim else 0)
+    o.check_status()
+    kv64, sh64, q64 = kv.double(), shared.double()[:, :rot], q.double().view(T, H, own + rot)
+    for r, (c, n) in enumerate(zip(ctx, q_lens)):
+        if not n:
+            continue
+        span = slice(int(key_row[r]) + starts[r], int(key_row[r]) + c)
+        i = torch.arange(c - n, c, device=DEV)[:, None]
+        j = torch.arange(starts[r], c, device=DEV)[None, :]
+        seen = (j <= i) & ((i - j < window) if window else (j >= 0))
+        for h in range(H):
+            k = torch.cat([kv64[span, h * own:(h + 1) * own], sh64[span]], dim=1)
+            v = kv64[span, H * own + h * dv:H * own + (h + 1) * dv]
+            t = slice(cu[r], cu[r + 1])
+            s = (q64[t, h] @ k.T * scale).masked_fill(~seen, float("-inf"))
+            s = torch.cat([s, sinks[h].double().expand(n, 1)], dim=1)
+            want = torch.softmax(s, dim=1)[:, :-1] @ v
+            want = want * torch.sigmoid(gate[t, h * dv:(h + 1) * dv].double() if gate_dim else gate[t, h:h + 1].double())
+            close(out[t, h * dv:(h + 1) * dv], want, BF, f"request {r} head {h}")
