@@ -1,0 +1,380 @@
+// The 32-bit product on the fifth-generation tensor cores: out[M, N] = epilogue(x[M, K] . W[N, K]^T), 32-bit operands and results.
+//
+// A 32-bit number v is split into hi, its first 11 significant bits (tf32), and lo = v - hi rounded to tf32: hi + lo is v to
+// 2^-22. A product is then hi hi' + (lo hi' + hi lo'), whose missing lo lo' is 2^-20 of it at most, 2^-22 on average. The tensor cores add
+// into a 32-bit accumulator, but they cut bits off where a register's addition rounds, an error that has a sign and grows with
+// the number of additions. So they sum 32 values of k at a time, the small products first, and threads add these segments' sums up
+// in registers, rounded to nearest, in ascending k: 28 rounded additions for K = 896 where a chain of FMAs makes 896.
+// Errors against 64 bits are no larger than such a chain's (the test of this kernel has both).
+//
+// W is the M side of the MMA (128 rows of W a tile; with SWIGLU 64 units, 16 gate rows and the 16 up rows that match in turn) and
+// NT rows of x its N side. A block: 8 warps fetch rows of W and x (16-byte loads, DEPTH segments ahead in registers), split
+// them and store both halves where the MMAs read them (128-byte swizzle); a thread of the first of them issues the 12 MMAs of the
+// segment before, into one of two accumulators (a warp of its own for that would leave 96 registers a thread, and spills); 4 or 8 warps
+// add the other one to their registers. At the end the tile passes through shared memory to the
+// epilogue. Products of few tiles cut K over the blocks of a cluster (f32_tc_spans), whose totals are added in ascending k through
+// distributed shared memory. What a result is computed from, and in which order, depends on N and K only: it is the same whatever
+// rows stand beside a row and however wide a tile is (the same promise that the kernels in gemm_plain.cu make, which keep the
+// small products).
+// A sum that is not finite (an infinity or NaN among the inputs, whose halves are NaN, or an overflow) is worked out again as
+// a chain of FMAs over the inputs themselves.
+//
+// Bound by shared memory: a segment of a 128 x 128 tile stores 64 KB and its MMAs read 96 KB, 1,280 cycles of the SM's
+// port against 830 of the tensor cores.
+// Every wait on an mbarrier is bounded; when a bound runs out the block records a code in a status word and stops computing, but
+// still meets its cluster, frees its tensor memory and returns (bl_gemm_f32_tc_status).
+#include "tcgen05.cuh"
+#include <atomic>
+
+namespace {
+
+constexpr int BM = 128;                    // rows of W a tile
+constexpr int BK = 32;                     // values of k a segment: one 128-byte row of the swizzled operand tiles
+constexpr int SPLITTERS = 256, ADDERS = 256, THREADS = SPLITTERS + ADDERS;
+constexpr int TMEM_COLS = 256;             // two accumulators of up to 128 columns
+constexpr uint32_t WAIT_LIMIT = 1u << 22;
+
+template <int NT>
+struct Tile {
+    static constexpr int W_BYTES = BM * 128, X_BYTES = NT * 128, STAGE_BYTES = 2 * (W_BYTES + X_BYTES);     // hi and lo of both
+    static constexpr int STAGES = NT >= 64 ? 3 : 5;
+    static constexpr int DEPTH = NT >= 64 ? 2 : 3;                        // segments that a splitter has in flight
+    static constexpr int HALVES = NT >= 64 ? 2 : 1;                       // the columns are dealt to one or two groups of four adder warps
+    static constexpr int COLS = NT / HALVES;
+    static constexpr int CHUNKS = 4 + (NT + 31) / 32;                     // 16-byte pieces of a segment a splitter
+    static constexpr int OFF_BARS = STAGES * STAGE_BYTES;
+    static constexpr int SMEM_BYTES = OFF_BARS + 256 + 1024;
+    static_assert(NT % 16 == 0 && COLS % 16 == 0 && BM * NT * 4 <= STAGES * STAGE_BYTES && SMEM_BYTES <= 227 * 1024, "tile");
+};
+
+__device__ int g_status = 0;               // 0 = fine; else the code of the first wait that ran out
+
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* give_up, int code) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if (*give_up) return false;
+    }
+    *give_up = 1;
+    atomicCAS(&g_status, 0, code);
+    return false;
+}
+__device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}"
+                 :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
+}
+// The halves of a number: its first 11 significant bits, and the rest rounded to 11. Integer arithmetic: the conversion instruction
+// runs at a fraction of its rate. (The first half of an infinity or a NaN is one, too.)
+__device__ __forceinline__ float first_half(float v) { return __uint_as_float(__float_as_uint(v) & 0xffffe000u); }
+__device__ __forceinline__ float second_half(float v, float first) { return __uint_as_float((__float_as_uint(v - first) + 0x1000u) & 0xffffe000u); }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+// The sum as a chain of FMAs in ascending k.
+__device__ __noinline__ float plain_dot(const float* x, const float* w, int K) {
+    float acc = 0.f;
+    for (int k = 0; k < K; ++k) acc = fmaf(x[k], w[k], acc);
+    return acc;
+}
+
+template <int EPI, int NT>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_f32_tc_kernel(const float* __restrict__ x, const float* __restrict__ w, const void* __restrict__ bias, int bias_dtype,
+                   float* __restrict__ out, int M, int N, int K, int ldx, int spans, int m_tiles) {
+    using T = Tile<NT>;
+    constexpr bool GLU = EPI == BL_EPI_SWIGLU;
+    constexpr int UNITS = GLU ? BM / 2 : BM;                              // outputs of a row of x a tile
+    constexpr int STAGES = T::STAGES, DEPTH = T::DEPTH, CHUNKS = T::CHUNKS;
+    // D 32-bit, A and B tf32 and K-major, N >> 3 at bit 17, M >> 4 at bit 24
+    constexpr uint32_t IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    unsigned char* smem = smem_raw + (base - smem_u32(smem_raw));
+    const uint32_t full0 = base + T::OFF_BARS, empty0 = full0 + 8 * STAGES, sum0 = empty0 + 8 * STAGES, taken0 = sum0 + 16;
+    volatile int* give_up = reinterpret_cast<volatile int*>(smem + T::OFF_BARS + 192);
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + T::OFF_BARS + 200);
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
+    // a cluster is the spans of one tile; the tiles of rows are neighbours, so that a tile of W is fetched from memory once
+    const int span = blockIdx.x % spans, tile = blockIdx.x / spans;
+    const int m0 = tile % m_tiles * NT, n0 = tile / m_tiles * UNITS;
+    const int all = (K + BK - 1) / BK, each = (all + spans - 1) / spans;
+    const int first = min(span * each, all), steps = min(each, all - first);
+    if (threadIdx.x == 0) {
+        *give_up = 0;
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, SPLITTERS / 32); mbar_init(empty0 + 8 * s, 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(sum0 + 8 * b, 1); mbar_init(taken0 + 8 * b, 4 * T::HALVES); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 8) {
+        __syncwarp();
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     :: "r"(smem_u32((const void*)tmem_slot)), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    const uint32_t tmem = *tmem_slot;
+    bool ok = true;
+    float* sums = reinterpret_cast<float*>(smem);                          // in the end: [column][row of the tile]
+
+    if (warp >= 8) {
+        // ================= splitters: thread (row t / 8 + 32 i, piece t % 8) of W (i < 4) and of x (i >= 4)
+        const int t = threadIdx.x - ADDERS, row = t >> 3, piece = t & 7;
+        const int unit = GLU ? n0 + (row & 15) : n0 + row;
+        constexpr int W_STEP = GLU ? 16 : 32;                              // units from one of a thread's rows of W to the next
+        const float* wp = w + (size_t)(unit + (GLU && row >= 16 ? N : 0)) * K + (size_t)first * BK + piece * 4;
+        const float* xp = x + (size_t)(m0 + row) * ldx + (size_t)first * BK + piece * 4;
+        float4 v[DEPTH][CHUNKS];
+        auto fetch = [&](int d, int i0, int i1, int step) {                // pieces i0 .. i1 of segment `step`
+            const int k = (first + step) * BK + piece * 4;
+#pragma unroll
+            for (int i = 0; i < CHUNKS; ++i) {
+                if (i < i0 || i >= i1) continue;
+                const bool is_w = i < 4;
+                bool have = step < steps && k < K;
+                if (is_w) have = have && unit + W_STEP * i < N;
+                else have = have && row + 32 * (i - 4) < NT && m0 + row + 32 * (i - 4) < M;
+                const float* p = is_w ? wp + (size_t)(W_STEP * i) * K : xp + (size_t)(32 * (i - 4)) * ldx;
+                v[d][i] = have ? *reinterpret_cast<const float4*>(p + (size_t)step * BK) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        };
+#pragma unroll
+        for (int d = 0; d < DEPTH; ++d) fetch(d, 0, 4, d);                 // W does not depend on the kernel before this one
+        bl_pdl_wait();
+        bl_pdl_trigger();
+#pragma unroll
+        for (int d = 0; d < DEPTH; ++d) fetch(d, 4, CHUNKS, d);
+        // the MMAs of segment s, by one thread of the first splitter warp
+        auto issue = [&](int s) {
+            if (warp != 8) return;
+            const int st = s % STAGES, b = s & 1;
+            ok = mbar_wait(full0 + 8 * st, (uint32_t)((s / STAGES) & 1), give_up, 2);
+            if (ok && s >= 2) ok = mbar_wait(taken0 + 8 * b, (uint32_t)((s / 2 - 1) & 1), give_up, 2);
+            ok = __all_sync(0xffffffffu, ok);
+            if (ok && elect_one()) {
+                fence_after_sync();
+                const uint32_t stage = base + st * T::STAGE_BYTES, d = tmem + b * 128;
+                const uint64_t wh = smem_desc(stage), wl = smem_desc(stage + T::W_BYTES);
+                const uint64_t xh = smem_desc(stage + 2 * T::W_BYTES), xl = smem_desc(stage + 2 * T::W_BYTES + T::X_BYTES);
+#pragma unroll
+                for (int k = 0; k < BK / 8; ++k) {                         // the small products first
+                    umma_tf32(d, wl + 2 * k, xh + 2 * k, IDESC, k != 0);
+                    umma_tf32(d, wh + 2 * k, xl + 2 * k, IDESC, 1);
+                }
+#pragma unroll
+                for (int k = 0; k < BK / 8; ++k) umma_tf32(d, wh + 2 * k, xh + 2 * k, IDESC, 1);
+                umma_commit(empty0 + 8 * st);
+                umma_commit(sum0 + 8 * b);
+            }
+            __syncwarp();
+        };
+        const uint32_t at = base + (uint32_t)row * 128 + (uint32_t)((piece ^ (row & 7)) << 4);       // (rows 32 apart swizzle alike)
+        for (int s0 = 0; ok && s0 < steps; s0 += DEPTH) {
+#pragma unroll
+            for (int d = 0; d < DEPTH; ++d) {
+                const int s = s0 + d;
+                if (s >= steps || !ok) break;
+                const int st = s % STAGES;
+                if (s >= STAGES) {
+                    ok = mbar_wait(empty0 + 8 * st, (uint32_t)((s / STAGES - 1) & 1), give_up, 1);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                }
+#pragma unroll
+                for (int i = 0; i < CHUNKS; ++i) {
+                    if (i >= 4 && row + 32 * (i - 4) >= NT) continue;
+                    const float4 a = v[d][i];
+                    const float4 h = make_float4(first_half(a.x), first_half(a.y), first_half(a.z), first_half(a.w));
+                    const float4 l = make_float4(second_half(a.x, h.x), second_half(a.y, h.y), second_half(a.z, h.z), second_half(a.w, h.w));
+                    const uint32_t to = at + st * T::STAGE_BYTES + (i < 4 ? i * 4096 : 2 * T::W_BYTES + (i - 4) * 4096);
+                    const uint32_t to_lo = to + (i < 4 ? T::W_BYTES : T::X_BYTES);
+                    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" :: "r"(to), "f"(h.x), "f"(h.y), "f"(h.z), "f"(h.w) : "memory");
+                    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" :: "r"(to_lo), "f"(l.x), "f"(l.y), "f"(l.z), "f"(l.w) : "memory");
+                }
+                fetch(d, 0, CHUNKS, s + DEPTH);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full0 + 8 * st);
+                if (s > 0) issue(s - 1);
+            }
+        }
+        if (ok && steps > 0) issue(steps - 1);
+    } else {
+        // ================= adders
+        bl_pdl_wait();
+        bl_pdl_trigger();
+        const uint32_t t_at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * T::COLS;
+        if (warp < 4 * T::HALVES) {
+            float acc[T::COLS];                                            // row 32 (warp & 3) + lane of the tile, COLS of its columns
+#pragma unroll
+            for (int j = 0; j < T::COLS; ++j) acc[j] = 0.f;
+            for (int s = 0; ok && s < steps; ++s) {
+                const int b = s & 1;
+                ok = mbar_wait(sum0 + 8 * b, (uint32_t)((s >> 1) & 1), give_up, 3);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                fence_after_sync();
+#pragma unroll
+                for (int c = 0; c < T::COLS; c += 16) {
+                    uint32_t r[16];
+                    tmem_ld16(t_at + b * 128 + c, r);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) acc[c + j] += __uint_as_float(r[j]);
+                }
+                fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(taken0 + 8 * b);
+            }
+            // the last segment's MMAs have read the operand tiles, which make room for the sums
+#pragma unroll
+            for (int j = 0; j < T::COLS; ++j) sums[((warp >> 2) * T::COLS + j) * BM + (warp & 3) * 32 + lane] = acc[j];
+        }
+    }
+    if (spans > 1) cluster_sync(); else __syncthreads();
+    const BlGluArgs glu = bl_glu_args(GLU ? bias : nullptr);
+    // the outputs of the tile, neighbours along n in neighbouring threads; a cluster's blocks take a share each
+    for (int e = span * THREADS + threadIdx.x; e < NT * UNITS; e += spans * THREADS) {
+        const int u = e % UNITS, col = e / UNITS;
+        const int m = m0 + col, n = n0 + u;
+        if (m >= M || n >= N) continue;
+        const uint32_t mine = base + (uint32_t)(col * BM + (GLU ? (u >> 4) * 32 + (u & 15) : u)) * 4;
+        float s = 0.f, up = 0.f;
+        if (spans == 1) {
+            s = *reinterpret_cast<const float*>(smem + (mine - base));
+            if (GLU) up = *reinterpret_cast<const float*>(smem + (mine - base) + 64);
+        } else {
+            for (int r = 0; r < spans; ++r) {                              // ascending k
+                uint32_t peer;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(mine), "r"(r));
+                s = r == 0 ? ld_cluster(peer) : s + ld_cluster(peer);
+                if (GLU) up = r == 0 ? ld_cluster(peer + 64) : up + ld_cluster(peer + 64);
+            }
+        }
+        if (!isfinite(s)) s = plain_dot(x + (size_t)m * ldx, w + (size_t)n * K, K);
+        if (GLU && !isfinite(up)) up = plain_dot(x + (size_t)m * ldx, w + (size_t)(N + n) * K, K);
+        float* dst = out + (size_t)m * N + n;
+        if (EPI == BL_EPI_BIAS) s += bl_load_any(bias, bias_dtype, n);
+        if (EPI == BL_EPI_RESIDUAL) {
+            if (bias) s += bl_load_any(bias, bias_dtype, n);
+            s += *dst;
+        }
+        if (GLU) {
+            if (glu.bias) { s += glu.bias[n]; up += glu.bias[N + n]; }
+            s = bl_glu(glu.kind, s, up, glu.limit);
+        }
+        *dst = s;
+    }
+    fence_before_sync();
+    if (spans > 1) cluster_sync(); else __syncthreads();                   // no block leaves while another may still read its sums
+    if (warp == 8) {
+        fence_after_sync();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(TMEM_COLS) : "memory");
+    }
+}
+
+int device_sms() {
+    static const int sms = [] {
+        int dev = 0, n = 0;
+        return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
+    }();
+    return sms;
+}
+
+template <int EPI, int NT>
+int launch(const float* x, const float* w, const void* bias, int bias_dtype, float* out, int M, int N, int K, int ldx, int spans, cudaStream_t s) {
+    static std::atomic<bool> allowed{false};
+    if (!allowed) {
+        BL_CUDA(cudaFuncSetAttribute(gemm_f32_tc_kernel<EPI, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<NT>::SMEM_BYTES));
+        allowed = true;
+    }
+    const int units = EPI == BL_EPI_SWIGLU ? BM / 2 : BM;
+    const int m_tiles = (M + NT - 1) / NT;
+    const dim3 grid((unsigned)((long long)((N + units - 1) / units) * m_tiles * spans));
+    if (spans > 1) {
+        BL_CUDA(bl_launch_dependent_clusters(gemm_f32_tc_kernel<EPI, NT>, grid, dim3(THREADS), (size_t)Tile<NT>::SMEM_BYTES, s, (unsigned)spans,
+                                             x, w, bias, bias_dtype, out, M, N, K, ldx, spans, m_tiles));
+    } else {
+        BL_CUDA(bl_launch_dependent(gemm_f32_tc_kernel<EPI, NT>, grid, dim3(THREADS), (size_t)Tile<NT>::SMEM_BYTES, s,
+                                    x, w, bias, bias_dtype, out, M, N, K, ldx, spans, m_tiles));
+    }
+    BL_CHECK_LAUNCH("bl_gemm_f32_tc");
+    return 0;
+}
+
+template <int EPI>
+int launch_width(const float* x, const float* w, const void* bias, int bias_dtype, float* out, int M, int N, int K, int ldx, int spans, cudaStream_t s) {
+    // The width of a tile: the least of rounds of blocks times a segment's cycles of the shared-memory port (16 KB and NT rows
+    // stored twice, 12 MMAs that read 128 and NT rows of 32 bytes).
+    const int units = EPI == BL_EPI_SWIGLU ? BM / 2 : BM;
+    const long long n_tiles = (N + units - 1) / units;
+    const int slots = spans > 1 ? device_sms() / spans - (spans > 2 ? 1 : 0) : device_sms();       // tiles under way at once
+    const int widths[] = {128, 96, 64, 32, 16};
+    int best = 0;
+    double least = 0.0;
+    for (int i = 0; i < 5; ++i) {
+        const int nt = widths[i];
+        const long long tiles = n_tiles * ((M + nt - 1) / nt);
+        const double cost = (double)((tiles + slots - 1) / slots) * (640 + 5 * nt);
+        if (i == 0 || cost < least) { least = cost; best = nt; }
+    }
+    switch (best) {
+        case 128: return launch<EPI, 128>(x, w, bias, bias_dtype, out, M, N, K, ldx, spans, s);
+        case 96: return launch<EPI, 96>(x, w, bias, bias_dtype, out, M, N, K, ldx, spans, s);
+        case 64: return launch<EPI, 64>(x, w, bias, bias_dtype, out, M, N, K, ldx, spans, s);
+        case 32: return launch<EPI, 32>(x, w, bias, bias_dtype, out, M, N, K, ldx, spans, s);
+        default: return launch<EPI, 16>(x, w, bias, bias_dtype, out, M, N, K, ldx, spans, s);
+    }
+}
+
+// Into how many spans K is cut, over the blocks of a cluster: four where a row of tiles fills less than a quarter of the device
+// and the spans keep four segments each. By N and K alone: which spans a sum is made of must not depend on the rows.
+int f32_tc_spans(int N, int K, int epi) {
+    const int n_tiles = (N + (epi == BL_EPI_SWIGLU ? BM / 2 : BM) - 1) / (epi == BL_EPI_SWIGLU ? BM / 2 : BM);
+    return n_tiles <= 32 && K >= 4 * 4 * BK ? 4 : 1;
+}
+
+}  // namespace
+
+// Whether the tensor cores take a product of these sizes (rows of whole 16-byte pieces): by N and K alone, see above.
+extern "C" int bl_gemm_f32_tc_supported(int N, int K, int ldx) { return N >= 128 && K >= 256 && K % 4 == 0 && ldx % 4 == 0; }
+
+extern "C" int bl_gemm_f32_tc(const float* x, int ldx, const float* w, const void* bias, int bias_dtype, float* out, int M, int N, int K,
+                              int epilogue, void* stream) {
+    if (M <= 0) return 0;
+    if (N <= 0 || K <= 0 || ldx < K || !bl_gemm_f32_tc_supported(N, K, ldx) || (((uintptr_t)x | (uintptr_t)w) & 15))
+        BL_FAIL("bl_gemm_f32_tc: N=%d K=%d ldx=%d is not what this kernel takes", N, K, ldx);
+    if (epilogue == BL_EPI_BIAS && bias == nullptr) BL_FAIL("bl_gemm_f32_tc: bias epilogue without a bias");
+    const int spans = f32_tc_spans(N, K, epilogue);
+    if ((long long)((N + 63) / 64) * ((M + 15) / 16) * spans > 0x7fffffffLL) BL_FAIL("bl_gemm_f32_tc: too many blocks");
+    cudaStream_t s = (cudaStream_t)stream;
+    switch (epilogue) {
+        case BL_EPI_NONE: return launch_width<BL_EPI_NONE>(x, w, bias, bias_dtype, out, M, N, K, ldx, spans, s);
+        case BL_EPI_BIAS: return launch_width<BL_EPI_BIAS>(x, w, bias, bias_dtype, out, M, N, K, ldx, spans, s);
+        case BL_EPI_RESIDUAL: return launch_width<BL_EPI_RESIDUAL>(x, w, bias, bias_dtype, out, M, N, K, ldx, spans, s);
+        case BL_EPI_SWIGLU: return launch_width<BL_EPI_SWIGLU>(x, w, bias, bias_dtype, out, M, N, K, ldx, spans, s);
+        default: BL_FAIL("bl_gemm_f32_tc: unknown epilogue %d", epilogue);
+    }
+}
+
+// Reads and clears the status word: 0 when no block has given up on a wait (1 a splitter, 2 the issuer, 3 an adder). Synchronises.
+extern "C" int bl_gemm_f32_tc_status(int* status) {
+    int v = 0, zero = 0;
+    BL_CUDA(cudaMemcpyFromSymbol(&v, g_status, sizeof(int)));
+    if (v != 0) BL_CUDA(cudaMemcpyToSymbol(g_status, &zero, sizeof(int)));
+    *status = v;
+    return 0;
+}

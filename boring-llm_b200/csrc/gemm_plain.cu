@@ -316,6 +316,8 @@ extern "C" int bl_gemm_plain_ld(const void* x, int x_dtype, int ldx, const void*
     if (epilogue == BL_EPI_BIAS && bias_dtype != BL_F32 && bias_dtype != BL_BF16)
         BL_FAIL("bl_gemm_plain: unknown bias dtype %d", bias_dtype);
     cudaStream_t s = (cudaStream_t)stream;
+    if (x_dtype == BL_F32 && w_dtype == BL_F32 && f32_tiles_fit(x, w, K, ldx, epilogue, out_dtype) && bl_gemm_f32_tc_supported(N, K, ldx))
+        return bl_gemm_f32_tc((const float*)x, ldx, (const float*)w, bias, bias_dtype, (float*)out, M, N, K, epilogue, stream);
     if (x_dtype == BL_F32 && w_dtype == BL_F32 && f32_tiles_fit(x, w, K, ldx, epilogue, out_dtype))
         return launch_f32_tiles((const float*)x, (const float*)w, bias, bias_dtype, (float*)out, M, N, K, ldx, epilogue, s);
     if (x_dtype == BL_F32 && w_dtype == BL_F32)

@@ -585,7 +585,10 @@ class ModelRunner:
             q_lens=q_lens, ctx_lens=ctx_lens, slot_list=slot_list, storage=self.storage, fast=self.fast)
         ctx.plans = _plans_on_device(plans, {k: take(int(arr.size)).view(arr.shape) for k, arr in plan_items})
         logits = self.model.forward(ctx)
-        self._waits_unchecked = self.fast and self.dtype == torch.bfloat16
+        if self.dtype == torch.float32:               # products on tensor cores; single tokens are looked at now and then, as replays are
+            self._waits_unchecked = self._waits_unchecked or T > R or self.steps % 256 == 0
+        else:
+            self._waits_unchecked = self.fast
         return logits
 
     # ---- captured general steps ------------------------------------------------------------------------

@@ -181,7 +181,8 @@ def _need_bias(bias: torch.Tensor, N: int, epilogue: int) -> None:
 
 def gemm_plain(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
                epilogue: int = EPI_NONE) -> None:
-    """out = epilogue(x @ w.T) on CUDA cores with 32-bit accumulation. x may be a range of columns of a wider
+    """out = epilogue(x @ w.T) on CUDA cores with 32-bit accumulation (32-bit operands with a long K: on the tensor cores, to the same
+    precision, see gemm_f32_tc.cu); a row's result does not depend on the rows beside it. x may be a range of columns of a wider
     row-major matrix (its rows `x.stride(0)` values apart)."""
     M, K = x.shape
     N = out.shape[1]
@@ -784,7 +785,7 @@ def gemm_swiglu_scaled(hw: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ss:
 
 def check_status() -> None:
     """Raises if a tensor-core block gave up on one of its bounded waits since the last check. Synchronises."""
-    for name, fn in (("bl_gemm_tc", _lib().bl_gemm_tc_status), ("bl_gemm_tc_pair", _lib().bl_gemm_tc_pair_status),
+    for name, fn in (("bl_gemm_tc", _lib().bl_gemm_tc_status), ("bl_gemm_f32_tc", _lib().bl_gemm_f32_tc_status), ("bl_gemm_tc_pair", _lib().bl_gemm_tc_pair_status),
                      ("bl_attention_prefill_tc", _lib().bl_attention_prefill_tc_status),
                      ("bl_gemm_tc_cols", _lib().bl_gemm_tc_cols_status),
                      ("bl_gemm_tc_splitk", _lib().bl_gemm_tc_splitk_status),

@@ -583,3 +583,78 @@ def test_attention_over_keys_made_of_latents(H, own, rot, dv, rank, window, gate
             want = torch.softmax(s, dim=1)[:, :-1] @ v
             want = want * torch.sigmoid(gate[t, h * dv:(h + 1) * dv].double() if gate_dim else gate[t, h:h + 1].double())
             close(out[t, h * dv:(h + 1) * dv], want, BF, f"request {r} head {h}")
+
+
+@pytest.mark.parametrize("N,K", [(128, 256), (130, 260), (896, 896), (1152, 900), (4160, 512), (896, 4864)])
+@pytest.mark.parametrize("M", [1, 16, 33, 97, 366])
+def test_32_bit_product_on_tensor_cores(M, N, K):
+    """Spans of K and none, widths of 16 to 128 rows, remainders of rows, columns and segments, every epilogue: no further from 64
+    bits than a chain of FMAs in 32 bits comes (numbers of one sign, where cut-off bits would add up, among them), and the same bits
+    for a row alone."""
+    o = ops()
+    g = torch.Generator().manual_seed(M * 7919 + N + K)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    full, w, w2, b = rnd(M, K + 4), rnd(N, K) * 0.3, rnd(2 * N, K) * 0.3, rnd(N)
+    x = full[:, :K]
+
+    def chain(x, w):                                   # fmaf in ascending k: the 48-bit product is exact in 64 bits, the sum rounded to 32
+        acc = torch.zeros(x.shape[0], w.shape[0], device=DEV)
+        for k in range(x.shape[1]):
+            acc = (acc.double() + x[:, k:k + 1].double() * w[:, k].double()).float()
+        return acc.double()
+
+    def rel(got, want):
+        return ((got.double() - want).norm() / want.norm()).item()
+
+    out = torch.empty(M, N, device=DEV)
+    for x_, w_ in ((x, w), (full.abs()[:, :K], w.abs())):
+        o.gemm_plain(x_, w_, out)
+        want = x_.double() @ w_.double().T
+        assert rel(out, want) <= rel(chain(x_, w_), want)
+        close(out, want, torch.float32, "product")
+    one = torch.empty(1, N, device=DEV)
+    o.gemm_plain(x, w, out, b, o.EPI_BIAS)
+    o.gemm_plain(x[M // 2:M // 2 + 1].contiguous(), w, one, b, o.EPI_BIAS)
+    assert torch.equal(one[0], out[M // 2])
+    res = rnd(M, N)
+    want = res.double() + x.double() @ w.double().T
+    o.gemm_plain(x, w, res, None, o.EPI_RESIDUAL)
+    close(res, want, torch.float32, "residual")
+    o.gemm_plain(x, w2, out, None, o.EPI_SWIGLU)
+    gu = x.double() @ w2.double().T
+    close(out, plain.silu(gu[:, :N]) * gu[:, N:], torch.float32, "swiglu")
+    one = torch.empty(1, N, device=DEV)
+    o.gemm_plain(x[M - 1:], w2, one, None, o.EPI_SWIGLU)
+    assert torch.equal(one[0], out[M - 1])
+    o.check_status()
+
+
+def test_32_bit_product_on_tensor_cores_of_infinities_and_extremes():
+    """Rows with an infinity, a NaN, the largest numbers and small ones: what a chain of FMAs gives, and other rows untouched."""
+    o = ops()
+    g = torch.Generator().manual_seed(5)
+    M, N, K = 70, 256, 512
+    x, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    plainly = torch.empty(M, N, device=DEV)
+    o.gemm_plain(x, w, plainly)
+    y = x.clone()
+    y[3, 7], y[5, 9], y[8, 0], y[11, 500] = float("inf"), float("nan"), -float("inf"), 3.4028234e38
+    y[20] *= 1e-30
+    y[21] *= 1e30
+    v = w.clone()
+    v[40, 7] = 0.0                                     # infinity times zero
+    v[41] = w[41].bfloat16().float()                   # numbers whose second half is zero
+    out = torch.empty(M, N, device=DEV)
+    o.gemm_plain(y, v, out)
+    want = (y.double() @ v.double().T)
+    for r in (3, 8):
+        torch.testing.assert_close(out[r].double(), want[r], rtol=0, atol=0, equal_nan=True)
+    assert out[5].isnan().all()
+    fits = torch.isfinite(want[11].float())
+    assert 0 < fits.sum() < N and torch.equal(torch.isfinite(out[11]), fits)
+    for r, n in ((11, fits), (20, slice(None)), (21, slice(None))):
+        assert ((out[r][n].double() - want[r][n]).norm() / want[r][n].norm()) < 1e-6
+    keep = [r for r in range(M) if r not in (3, 5, 8, 11, 20, 21)]
+    cols = [n for n in range(N) if n not in (40, 41)]
+    assert torch.equal(out[keep][:, cols], plainly[keep][:, cols])
+    o.check_status()
