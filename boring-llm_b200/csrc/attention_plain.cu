@@ -9,6 +9,7 @@
 // joins the softmax's denominator once, unscaled, without a value; a gate per (token, head) whose sigmoid multiplies
 // the head's output, or one per (token, head, channel); a cap c on the scores, s <- c tanh(s / c), applied to the scaled score before the softmax.
 #include "common.cuh"
+#include <atomic>
 #include "api.h"
 
 namespace {
@@ -112,6 +113,139 @@ attention_plain_kernel(const TT* __restrict__ q, const TT* __restrict__ kc, cons
     }
 }
 
+// The same for many 32-bit rows: a warp takes up to HPW heads of a token that share a key/value head, and the same sums in the same
+// order. The kernel above reads a key's row by the lane that owns the key, 32 lines a load, which is what it waits for; here a
+// chunk's keys and values pass through the warp's shared memory in whole lines (cp.async: the values arrive under the scores, the next
+// keys under the products with the values) and serve all its heads.
+template <int HPW, int NV>
+__global__ void __launch_bounds__(WARPS * 32)
+attention_plain_heads_kernel(const float* __restrict__ q, const float* __restrict__ kc, const float* __restrict__ vc,
+                             const int* __restrict__ tok_req, const int* __restrict__ cu_q, const int* __restrict__ ctx_len,
+                             const int* __restrict__ block_table, int max_pages, float* __restrict__ out, int T, int H, int KV, int dh, int dv,
+                             int page_size, int window, float scale, const void* __restrict__ sinks, int sink_dtype, const float* gate,
+                             int ld_gate, int gate_dim, float softcap) {
+    extern __shared__ __align__(16) float sm[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ldk = dh + 4;                            // padded: eight rows' pieces of 16 bytes fall on different banks
+    float* qs = sm + (size_t)warp * (HPW * dh + 32 * (ldk + dv + HPW));     // [HPW][dh]
+    float* ks = qs + HPW * dh;                         // [32][ldk]
+    float* vs = ks + 32 * ldk;                         // [32][dv]
+    float* ps = vs + 32 * dv;                          // [32][HPW]
+    const int G = H / KV, per = (G + HPW - 1) / HPW;
+    const int item = blockIdx.x * WARPS + warp;
+    bl_pdl_trigger();
+    bl_pdl_wait();
+    if (item >= T * KV * per) return;                  // whole warps leave together; no block-wide barrier below
+    const int t = item / (KV * per), kvh = item / per % KV, h0 = kvh * G + item % per * HPW;
+    const int nh = min(HPW, (kvh + 1) * G - h0);
+    const int r = tok_req[t];
+    const int q_len = cu_q[r + 1] - cu_q[r];
+    const int pos = ctx_len[r] - q_len + (t - cu_q[r]);
+    const int lo = window > 0 ? max(0, pos - window + 1) : 0;
+    for (int d = lane; d < HPW * dh; d += 32) qs[d] = d < nh * dh ? q[((size_t)t * H + h0) * dh + d] : 0.f;
+    const int* bt = block_table + (size_t)r * max_pages;
+    // Rows [base, base + 32) of a cache, those past `pos` left out, 2^n4 pieces of 16 bytes a row: a lane knows where one row lies.
+    auto copy = [&](float* dst, int ld, const float* cache, int n4, int base) {
+        const int j = min(base + lane, pos), width = 4 << n4;
+        const long long mine = ((long long)bt[j / page_size] * KV + kvh) * page_size + j % page_size;
+        const int rows = min(32, pos - base + 1), col = lane & ((1 << n4) - 1);
+#pragma unroll 4
+        for (int row0 = 0; row0 < rows; row0 += 32 >> n4) {
+            const int row = row0 + (lane >> n4);
+            const long long at = __shfl_sync(0xffffffffu, mine, row & 31);
+            if (row < rows)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n"
+                             :: "r"((unsigned)__cvta_generic_to_shared(dst + row * ld + col * 4)), "l"(cache + at * width + col * 4));
+        }
+        asm volatile("cp.async.commit_group;\n" ::);
+    };
+    const int k_log = 31 - __clz(dh >> 2), v_log = 31 - __clz(dv >> 2);
+    float m[HPW], l[HPW], acc[HPW][NV];
+#pragma unroll
+    for (int h = 0; h < HPW; ++h) {
+        m[h] = -INFINITY; l[h] = 0.f;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) acc[h][i] = 0.f;
+    }
+    copy(ks, ldk, kc, k_log, lo);
+    for (int base = lo; base <= pos; base += 32) {
+        copy(vs, dv, vc, v_log, base);
+        asm volatile("cp.async.wait_group 1;\n" ::);   // the keys
+        __syncwarp();
+        const bool valid = base + lane <= pos;
+        float s[HPW];
+#pragma unroll
+        for (int h = 0; h < HPW; ++h) s[h] = 0.f;
+#pragma unroll 4
+        for (int d = 0; d < dh; d += 4) {
+            const float4 b = *reinterpret_cast<const float4*>(ks + lane * ldk + d);
+#pragma unroll
+            for (int h = 0; h < HPW; ++h) {
+                const float4 a = *reinterpret_cast<const float4*>(qs + h * dh + d);
+                s[h] = fmaf(a.x, b.x, s[h]); s[h] = fmaf(a.y, b.y, s[h]); s[h] = fmaf(a.z, b.z, s[h]); s[h] = fmaf(a.w, b.w, s[h]);
+            }
+        }
+        __syncwarp();                                  // the keys have been read
+        if (base + 32 <= pos) copy(ks, ldk, kc, k_log, base + 32);
+        else asm volatile("cp.async.commit_group;\n" ::);
+#pragma unroll
+        for (int h = 0; h < HPW; ++h) {
+            float sc = s[h] * scale;
+            if (softcap > 0.f) sc = softcap * tanhf(sc / softcap);
+            if (!valid) sc = -INFINITY;                // (whatever the lane's row of the buffer holds)
+            const float m_new = fmaxf(m[h], bl_warp_max(sc));
+            const float p = valid ? expf(sc - m_new) : 0.f;
+            const float alpha = expf(m[h] - m_new);    // first chunk: exp(-inf) = 0
+            l[h] = l[h] * alpha + bl_warp_sum(p);
+#pragma unroll
+            for (int i = 0; i < NV; ++i) acc[h][i] *= alpha;
+            ps[lane * HPW + h] = p;
+            m[h] = m_new;
+        }
+        asm volatile("cp.async.wait_group 1;\n" ::);   // the values
+        __syncwarp();
+        const int n = min(32, pos - base + 1);
+#pragma unroll 4
+        for (int j = 0; j < n; ++j) {                  // ascending position
+            float v[NV], p[HPW];
+#pragma unroll
+            for (int i = 0; i < NV; ++i) v[i] = lane + 32 * i < dv ? vs[j * dv + lane + 32 * i] : 0.f;
+#pragma unroll
+            for (int h = 0; h < HPW; ++h) p[h] = ps[j * HPW + h];
+#pragma unroll
+            for (int h = 0; h < HPW; ++h)
+#pragma unroll
+                for (int i = 0; i < NV; ++i) acc[h][i] = fmaf(p[h], v[i], acc[h][i]);
+        }
+        __syncwarp();                                  // values and weights have been read
+    }
+#pragma unroll
+    for (int h = 0; h < HPW; ++h) {
+        if (h >= nh) continue;
+        const int head = h0 + h;
+        if (sinks) {                                   // one more term of the denominator, after the last key
+            const float sk = bl_load_any(sinks, sink_dtype, head);
+            const float m_new = fmaxf(m[h], sk);
+            const float alpha = expf(m[h] - m_new);
+            l[h] = l[h] * alpha + expf(sk - m_new);
+#pragma unroll
+            for (int i = 0; i < NV; ++i) acc[h][i] *= alpha;
+        }
+        float inv = l[h] > 0.f ? 1.0f / l[h] : 0.f;
+        if (gate && gate_dim == 0) inv *= bl_sigmoid(gate[(size_t)t * ld_gate + head]);
+        const float* crow = gate && gate_dim ? gate + (size_t)t * ld_gate + (size_t)head * gate_dim : nullptr;
+        float* orow = out + ((size_t)t * H + head) * dv;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int d = lane + 32 * i;
+            if (d < dv) orow[d] = crow ? acc[h][i] * inv * bl_sigmoid(crow[d]) : acc[h][i] * inv;
+        }
+    }
+}
+
+// Rows times heads from which warps with several heads each fill the device, heads a warp takes.
+constexpr int HEADS_MIN_ITEMS = 2048, HEADS_A_WARP = 4, HEADS_MAX_DH = 128;
+
 }  // namespace
 
 extern "C" int bl_attention_plain(const void* q, const void* k_cache, const void* v_cache, int dtype,
@@ -147,6 +281,24 @@ extern "C" int bl_attention_plain_cap(const void* q, const void* k_cache, const 
     cudaStream_t s = (cudaStream_t)stream;
     const int blocks = (T * H + WARPS - 1) / WARPS;
     const bool vec = dtype == BL_F32 && dh % 4 == 0 && ((uintptr_t)k_cache & 15) == 0;
+    // Several heads a warp: rows and values of 4, 8, .. 128 values, heads that share keys, and enough of them.
+    const auto power = [](int n) { return n >= 4 && n <= HEADS_MAX_DH && (n & (n - 1)) == 0; };
+    if (vec && H > KV && power(dh) && power(dv) && ((uintptr_t)v_cache & 15) == 0 && (long long)T * H >= HEADS_MIN_ITEMS) {
+        const int per = (H / KV + HEADS_A_WARP - 1) / HEADS_A_WARP;
+        const int grid = (T * KV * per + WARPS - 1) / WARPS;
+        const size_t smem = (size_t)WARPS * (HEADS_A_WARP * dh + 32 * (dh + 4 + dv + HEADS_A_WARP)) * sizeof(float);
+#define BL_HEADS(NV) do { \
+            static std::atomic<bool> allowed{false}; \
+            if (!allowed) { BL_CUDA(cudaFuncSetAttribute(attention_plain_heads_kernel<HEADS_A_WARP, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                (int)(WARPS * (HEADS_A_WARP * HEADS_MAX_DH + 32 * (2 * HEADS_MAX_DH + 4 + HEADS_A_WARP)) * sizeof(float)))); allowed = true; } \
+            BL_CUDA(bl_launch_dependent(attention_plain_heads_kernel<HEADS_A_WARP, NV>, dim3(grid), dim3(WARPS * 32), smem, s, (const float*)q, (const float*)k_cache, \
+                (const float*)v_cache, tok_req, cu_q, ctx_len, block_table, max_pages, (float*)out, T, H, KV, dh, dv, page_size, window, scale, sinks, \
+                sink_dtype, gate, ld_gate, gate_dim, softcap)); } while (0)
+        if (dv <= 64) BL_HEADS(2); else BL_HEADS(4);
+#undef BL_HEADS
+        BL_CHECK_LAUNCH("bl_attention_plain");
+        return 0;
+    }
 #define BL_GO(TT, VEC, NV) attention_plain_kernel<TT, VEC, NV><<<blocks, WARPS * 32, 0, s>>>((const TT*)q, (const TT*)k_cache, \
             (const TT*)v_cache, tok_req, cu_q, ctx_len, block_table, max_pages, (TT*)out, T, H, KV, dh, dv, \
             page_size, window, scale, sinks, sink_dtype, gate, ld_gate, gate_dim, softcap)

@@ -658,3 +658,41 @@ def test_32_bit_product_on_tensor_cores_of_infinities_and_extremes():
     cols = [n for n in range(N) if n not in (40, 41)]
     assert torch.equal(out[keep][:, cols], plainly[keep][:, cols])
     o.check_status()
+
+
+@pytest.mark.parametrize("H,KV,dh,dv,page", [(14, 2, 64, 64, 16), (9, 1, 32, 16, 16), (10, 2, 128, 64, 8), (12, 2, 16, 128, 16), (9, 1, 36, 20, 16), (5, 5, 64, 64, 16)])
+@pytest.mark.parametrize("window,extras", [(0, False), (40, True)])
+def test_32_bit_attention_with_several_heads_a_warp(H, KV, dh, dv, page, window, extras):
+    """Many rows (several heads a warp) against the same rows a few at a time (a warp per head), bit for bit; and against 64 bits."""
+    o = ops()
+    ctx_lens, q_lens = [211, 1, 64, 300], [211, 1, 33, 170]
+    s = paged_setup(ctx_lens, q_lens, KV, dh, page, torch.float32, 3)
+    T = s["T"]
+    s["kc"] = data(s["kc"].shape, 1)
+    vc = data(s["kc"].shape[:3] + (dv,), 2)
+    q = data((T, H * dh), 3)
+    sinks, gate = (data((H,), 4), data((T, H * dv), 5)) if extras else (None, None)
+    cap = 20.0 if extras else 0.0
+
+    def run(t0, t1):
+        out = torch.full((t1 - t0, H * dv), float("nan"), device=DEV)
+        o.attention_plain(q[t0:t1].contiguous(), s["kc"], vc, s["tok_req"][t0:t1].contiguous(), s["cu_q"] - t0, s["ctx_len"], s["table"], out, H, window,
+                          0.3, sinks, None if gate is None else gate[t0:t1], softcap=cap, gate_dim=dv if extras else 0)
+        return out
+    got = run(0, T)
+    few = torch.cat([run(t, min(t + 40, T)) for t in range(0, T, 40)])
+    assert T * H >= 2048 > 40 * H and torch.equal(got, few)
+    for t in (0, 100, 211, 212, 244, T - 1):
+        r, pos = int(s["tok_req_np"][t]), int(s["positions_np"][t])
+        j = np.arange(max(0, pos - window + 1) if window else 0, pos + 1)
+        pages = torch.from_numpy(s["table_np"][r, j // page]).long().to(DEV)
+        k64, v64 = (c[pages, :, torch.from_numpy(j % page).to(DEV)].double() for c in (s["kc"], vc))
+        for h in (0, H - 1):
+            g = h // (H // KV)
+            sc = k64[:, g] @ q[t, h * dh:(h + 1) * dh].double() * 0.3
+            if extras:
+                sc = torch.cat([cap * torch.tanh(sc / cap), sinks[h:h + 1].double()])
+            want = torch.softmax(sc, 0)[:len(j)] @ v64[:, g]
+            if extras:
+                want = want * torch.sigmoid(gate[t, h * dv:(h + 1) * dv].double())
+            close(got[t, h * dv:(h + 1) * dv], want, torch.float32, f"token {t} head {h}")
