@@ -126,6 +126,91 @@ int launch_out(const void* x, const void* w, const void* bias, int bias_dtype, v
     BL_FAIL("bl_gemm_plain: unknown output dtype %d", out_dtype);
 }
 
+// ---- products with a short K (the second factor of a low-rank pair) --------------------------------------------------------
+// The same sums (one accumulator an output, ascending k) for 32-bit x and 32-bit results with K up to RANK_MAX: a thread holds a
+// row of W in registers and goes down the rows of x, which the block has brought to shared memory (a broadcast each). W is on its
+// way before the kernel before has finished. Tiles of 64 x 64 gave a decode step 16 blocks and no early start (8 rows of 1,024 x
+// 16 in a decode step's chain 9.6 us, and 1,840 rows 15 us).
+constexpr int RANK_MAX = 64, RANK_THREADS = 128;
+
+template <typename TW, int EPI, int KM>
+__global__ void __launch_bounds__(RANK_THREADS)
+gemm_rank_kernel(const float* __restrict__ x, const TW* __restrict__ w, const void* __restrict__ bias, int bias_dtype, float* __restrict__ out,
+                 int M, int N, int K, int ldx, const float* __restrict__ coef, int group, float sign, int x_tanh, int rows) {
+    extern __shared__ __align__(16) float xrow[];                 // [rows][K]
+    bl_pdl_trigger();
+    const int n = blockIdx.x * RANK_THREADS + threadIdx.x, m0 = blockIdx.y * rows;
+    float wr[KM];
+#pragma unroll
+    for (int k = 0; k < KM; k += 4) {
+        if (n < N && k < K) {                                     // K is a multiple of four
+            if constexpr (sizeof(TW) == 4) {
+                const float4 f = *reinterpret_cast<const float4*>(w + (size_t)n * K + k);
+                wr[k] = f.x; wr[k + 1] = f.y; wr[k + 2] = f.z; wr[k + 3] = f.w;
+            } else {
+                const uint2 u = *reinterpret_cast<const uint2*>(w + (size_t)n * K + k);
+                const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+                wr[k] = a.x; wr[k + 1] = a.y; wr[k + 2] = b.x; wr[k + 3] = b.y;
+            }
+        } else {
+            wr[k] = wr[k + 1] = wr[k + 2] = wr[k + 3] = 0.f;
+        }
+    }
+    const float bn = bias != nullptr && n < N ? bl_load_any(bias, bias_dtype, n) : 0.f;
+    const float cn = EPI == BL_EPI_DECAY && n < N ? coef[n / group] : 0.f;
+    bl_pdl_wait();
+    const int here = min(rows, M - m0), k4 = K >> 2;
+    for (int c = threadIdx.x; c < here * k4; c += RANK_THREADS) {
+        float4 f = *reinterpret_cast<const float4*>(x + (size_t)(m0 + c / k4) * ldx + (c % k4) * 4);
+        if (EPI == BL_EPI_DECAY_EXP && x_tanh) f = make_float4(tanhf(f.x), tanhf(f.y), tanhf(f.z), tanhf(f.w));
+        *reinterpret_cast<float4*>(xrow + 4 * c) = f;
+    }
+    __syncthreads();
+    if (n >= N) return;
+#pragma unroll 2
+    for (int i = 0; i < here; ++i) {
+        float acc = 0.f;
+#pragma unroll
+        for (int k = 0; k < KM; k += 4) {
+            if (k < K) {
+                const float4 f = *reinterpret_cast<const float4*>(xrow + i * K + k);
+                acc = fmaf(f.x, wr[k], acc); acc = fmaf(f.y, wr[k + 1], acc); acc = fmaf(f.z, wr[k + 2], acc); acc = fmaf(f.w, wr[k + 3], acc);
+            }
+        }
+        float v = acc;
+        if (EPI != BL_EPI_NONE && bias) v += bn;
+        if (EPI == BL_EPI_DECAY) {
+            const float u = sign * v;
+            v = expf(-cn * (u > 20.f ? u : log1pf(expf(u))));
+        }
+        if (EPI == BL_EPI_DECAY_EXP) v = expf(-expf(v));
+        out[(size_t)(m0 + i) * N + n] = v;
+    }
+}
+
+template <typename TW, int EPI>
+int launch_rank(const float* x, const TW* w, const void* bias, int bias_dtype, float* out, int M, int N, int K, int ldx, cudaStream_t s,
+                const float* coef, int group, float sign, int x_tanh) {
+    // rows a block: up to 16, fewer where the launch would not give every SM four blocks
+    const int across = (N + RANK_THREADS - 1) / RANK_THREADS;
+    int rows = 16;
+    while (rows > 1 && (long long)across * ((M + rows - 1) / rows) < 4 * 148) rows >>= 1;
+    const dim3 grid(across, (M + rows - 1) / rows);
+    const size_t bytes = (size_t)rows * K * sizeof(float);
+#define BL_GO(KM) BL_CUDA(bl_launch_dependent(gemm_rank_kernel<TW, EPI, KM>, grid, dim3(RANK_THREADS), bytes, s, x, w, bias, bias_dtype, out, \
+        M, N, K, ldx, coef, group, sign, x_tanh, rows))
+    if (K <= 16) BL_GO(16); else if (K <= 32) BL_GO(32); else BL_GO(64);
+#undef BL_GO
+    BL_CHECK_LAUNCH("bl_gemm_plain (short K)");
+    return 0;
+}
+
+// Short K, whole 16-byte pieces of x and four values of W (the sums are the same either way).
+template <typename TW>
+bool rank_fits(const float* x, const TW* w, int M, int K, int ldx) {
+    return K <= RANK_MAX && K % 4 == 0 && ldx % 4 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)w & (4 * sizeof(TW) - 1)) == 0 && M <= 65535;
+}
+
 // ---- the 32-bit product with tiles in flight ---------------------------------------------------------------------------
 // The same sums (one accumulator an output, ascending k, so the same bits as the kernel above and independent of the tile)
 // for 32-bit x and W whose rows are whole 16-byte pieces: BK values of k of a tile's rows come by cp.async into a ring of
@@ -324,6 +409,13 @@ extern "C" int bl_gemm_plain_ld(const void* x, int x_dtype, int ldx, const void*
         return launch_out<float, float>(x, w, bias, bias_dtype, out, out_dtype, M, N, K, ldx, epilogue, s);
     if (x_dtype == BL_BF16 && w_dtype == BL_BF16)
         return launch_out<__nv_bfloat16, __nv_bfloat16>(x, w, bias, bias_dtype, out, out_dtype, M, N, K, ldx, epilogue, s);
+    if (x_dtype == BL_F32 && w_dtype == BL_BF16 && out_dtype == BL_F32 && (epilogue == BL_EPI_NONE || epilogue == BL_EPI_BIAS) &&
+        rank_fits((const float*)x, (const __nv_bfloat16*)w, M, K, ldx)) {
+        const float* xf = (const float*)x;
+        const __nv_bfloat16* wb = (const __nv_bfloat16*)w;
+        if (epilogue == BL_EPI_NONE) return launch_rank<__nv_bfloat16, BL_EPI_NONE>(xf, wb, nullptr, 0, (float*)out, M, N, K, ldx, s, nullptr, 1, 1.f, 0);
+        return launch_rank<__nv_bfloat16, BL_EPI_BIAS>(xf, wb, bias, bias_dtype, (float*)out, M, N, K, ldx, s, nullptr, 1, 1.f, 0);
+    }
     if (x_dtype == BL_F32 && w_dtype == BL_BF16)
         return launch_out<float, __nv_bfloat16>(x, w, bias, bias_dtype, out, out_dtype, M, N, K, ldx, epilogue, s);
     BL_FAIL("bl_gemm_plain: unsupported input dtypes x=%d w=%d", x_dtype, w_dtype);
@@ -337,7 +429,11 @@ extern "C" int bl_gemm_plain_decay(const float* x, int ldx, const void* w, int w
     if (N <= 0 || K <= 0 || ldx < K || group <= 0 || N % group != 0 || coef == nullptr)
         BL_FAIL("bl_gemm_plain_decay: bad sizes N=%d K=%d ldx=%d group=%d", N, K, ldx, group);
     cudaStream_t s = (cudaStream_t)stream;
+    if (w_dtype == BL_F32 && rank_fits(x, (const float*)w, M, K, ldx))
+        return launch_rank<float, BL_EPI_DECAY>(x, (const float*)w, bias, bias_dtype, out, M, N, K, ldx, s, coef, group, sign, 0);
     if (w_dtype == BL_F32) return launch_epi<float, float, float>(x, w, bias, bias_dtype, out, M, N, K, ldx, BL_EPI_DECAY, s, coef, group, sign);
+    if (w_dtype == BL_BF16 && rank_fits(x, (const __nv_bfloat16*)w, M, K, ldx))
+        return launch_rank<__nv_bfloat16, BL_EPI_DECAY>(x, (const __nv_bfloat16*)w, bias, bias_dtype, out, M, N, K, ldx, s, coef, group, sign, 0);
     if (w_dtype == BL_BF16) return launch_epi<float, __nv_bfloat16, float>(x, w, bias, bias_dtype, out, M, N, K, ldx, BL_EPI_DECAY, s, coef, group, sign);
     BL_FAIL("bl_gemm_plain_decay: unknown matrix dtype %d", w_dtype);
 }
@@ -349,7 +445,11 @@ extern "C" int bl_gemm_plain_decay_exp(const float* x, int ldx, int x_tanh, cons
     if (M <= 0) return 0;
     if (N <= 0 || K <= 0 || ldx < K) BL_FAIL("bl_gemm_plain_decay_exp: bad sizes N=%d K=%d ldx=%d", N, K, ldx);
     cudaStream_t s = (cudaStream_t)stream;
+    if (w_dtype == BL_F32 && rank_fits(x, (const float*)w, M, K, ldx))
+        return launch_rank<float, BL_EPI_DECAY_EXP>(x, (const float*)w, bias, bias_dtype, out, M, N, K, ldx, s, nullptr, 1, 1.f, x_tanh);
     if (w_dtype == BL_F32) return launch_epi<float, float, float>(x, w, bias, bias_dtype, out, M, N, K, ldx, BL_EPI_DECAY_EXP, s, nullptr, 1, 1.f, x_tanh);
+    if (w_dtype == BL_BF16 && rank_fits(x, (const __nv_bfloat16*)w, M, K, ldx))
+        return launch_rank<__nv_bfloat16, BL_EPI_DECAY_EXP>(x, (const __nv_bfloat16*)w, bias, bias_dtype, out, M, N, K, ldx, s, nullptr, 1, 1.f, x_tanh);
     if (w_dtype == BL_BF16) return launch_epi<float, __nv_bfloat16, float>(x, w, bias, bias_dtype, out, M, N, K, ldx, BL_EPI_DECAY_EXP, s, nullptr, 1, 1.f, x_tanh);
     BL_FAIL("bl_gemm_plain_decay_exp: unknown matrix dtype %d", w_dtype);
 }

@@ -696,3 +696,27 @@ def test_32_bit_attention_with_several_heads_a_warp(H, KV, dh, dv, page, window,
             if extras:
                 want = want * torch.sigmoid(gate[t, h * dv:(h + 1) * dv].double())
             close(got[t, h * dv:(h + 1) * dv], want, torch.float32, f"token {t} head {h}")
+
+
+@pytest.mark.parametrize("K", [4, 16, 20, 36, 64])
+@pytest.mark.parametrize("M,N", [(1, 1), (8, 130), (37, 256), (700, 100)])
+def test_products_with_a_short_k(M, N, K):
+    """Every epilogue, both kinds of W, rows of x in a wider matrix; the same bits for a row alone."""
+    o = ops()
+    x = data((M, K + 8), 1)[:, :K]
+    coef, bias = data((N,), 4).abs() + 0.1, data((N,), 3)
+    for wd in (torch.float32, BF):
+        w = (data((N, K), 2) * 0.3).to(wd)
+        z = x.double() @ w.double().T
+        out, one = torch.empty(M, N, device=DEV), torch.empty(1, N, device=DEV)
+        o.gemm_plain_decay(x, w, bias, coef, 1, -1.0, out)
+        close(out, torch.exp(-coef.double() * torch.nn.functional.softplus(-(z + bias.double()))), torch.float32, "decay")
+        o.gemm_plain_decay(x[M // 2:M // 2 + 1], w, bias, coef, 1, -1.0, one)
+        assert torch.equal(one[0], out[M // 2])
+        o.gemm_plain_decay_exp(x, w, None, out, x_tanh=True)
+        close(out, torch.exp(-torch.exp(torch.tanh(x.double()) @ w.double().T)), torch.float32, "decay of exp")
+        if wd == BF:
+            o.gemm_plain(x, w, out)
+            close(out, z, torch.float32, "product")
+            o.gemm_plain(x, w, out, bias, o.EPI_BIAS)
+            close(out, z + bias.double(), torch.float32, "bias")
