@@ -720,3 +720,22 @@ def test_products_with_a_short_k(M, N, K):
             close(out, z, torch.float32, "product")
             o.gemm_plain(x, w, out, bias, o.EPI_BIAS)
             close(out, z + bias.double(), torch.float32, "bias")
+
+
+@pytest.mark.parametrize("d", [4, 508, 516, 1028, 2052, 4096])
+def test_layer_end_chain_of_many_rows(d):
+    """More rows than run at once with every operand in registers against the same rows a few at a time, bit for bit."""
+    o = ops()
+    rows, n = 303, 5
+    whole = data((n + 1, rows, d), 61) * 2
+    sub, gate, gb = data((rows, d), 62), data((rows, d), 63), data((d,), 64).to(BF)
+    pw, pb, tw, tb = ((data((d,), 65 + i) * 0.25 + 1).to(BF) for i in range(4))
+    c = data((n,), 70)
+    parts = [whole[:, i:i + 100].contiguous() for i in range(0, rows, 100)]
+    ys = []
+    for i, s in enumerate([whole] + parts):
+        r = slice(0, rows) if i == 0 else slice(100 * (i - 1), min(100 * i, rows))
+        y = torch.empty(s.shape[1], d, dtype=BF, device=DEV)
+        o.norm_chain(s[n - 1], sub[r], gate[r], gb, (pw, pb, 1e-6), streams=s, coeffs=c, n=n, mix_out=s[n], then=(tw, tb, 1e-5), y=y)
+        ys.append(y)
+    assert torch.equal(whole, torch.cat(parts, dim=1)) and torch.equal(ys[0], torch.cat(ys[1:]))
