@@ -116,7 +116,7 @@ qk_norm_rope_write_kernel(const float* proj, int ld, int off_k, int off_v, const
     }
 }
 
-// The same four values at a time, for rows, heads and rotated parts that are multiples of four and rotation in halves: the
+// The same four values at a time, for rows, heads and rotated parts that are multiples of four, pairs in halves or neighbours: the
 // token's q and k rows are read once, into shared memory, with both sums of squares on the way; positions, angles and page
 // numbers are worked out before the kernel's predecessor has finished.
 constexpr int FAST_THREADS = 512;
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(FAST_THREADS)
 qk_norm_rope_write4_kernel(const float* proj, int ld, int off_k, int off_v, const void* __restrict__ qw, int qw_dtype,
                            const void* __restrict__ kw, int kw_dtype, float eps, const int* __restrict__ positions,
                            const int* __restrict__ tok_req, const int* __restrict__ block_table, int max_pages,
-                           const float* __restrict__ inv_freq, int rot_half, TT* __restrict__ q_out,
+                           const float* __restrict__ inv_freq, int rot_half, int neighbours, TT* __restrict__ q_out,
                            TT* __restrict__ k_cache, TT* __restrict__ v_cache, int H, int KV, int dk, int dv, int page_size,
                            int per_head, const float* __restrict__ q_head_scale, BlBlendArgs bl) {
     bl_pdl_trigger();
@@ -225,7 +225,14 @@ qk_norm_rope_write4_kernel(const float* proj, int ld, int off_k, int off_v, cons
         const float4 m = *reinterpret_cast<const float4*>(x + e);
         const float4 mw = weights4(w, wd, wbase + d);
         float v[4] = {m.x * inv * mw.x, m.y * inv * mw.y, m.z * inv * mw.z, m.w * inv * mw.w};
-        if (d < 2 * rot_half) {
+        if (d < 2 * rot_half && neighbours) {          // two pairs in the four values
+            const float2 c = *reinterpret_cast<const float2*>(cs + d / 2), s2 = *reinterpret_cast<const float2*>(sn + d / 2);
+            const float a0 = v[0], a1 = v[2];
+            v[0] = a0 * c.x - v[1] * s2.x;
+            v[1] = v[1] * c.x + a0 * s2.x;
+            v[2] = a1 * c.y - v[3] * s2.y;
+            v[3] = v[3] * c.y + a1 * s2.y;
+        } else if (d < 2 * rot_half) {
             const bool first = d < rot_half;
             const int od = first ? d + rot_half : d - rot_half, j = first ? d : d - rot_half;
             const float4 o = *reinterpret_cast<const float4*>(x + hh * dk + od);
@@ -293,7 +300,7 @@ extern "C" int bl_qk_norm_rope_write_ext(const float* proj, int ld, int off_k, i
     const BlBlendArgs bl{norm_q, norm_k, v_first, ld_first, first_dv, first_places, dv_real, lambda, lambda_dtype, same};
     cudaStream_t s = (cudaStream_t)stream;
     const size_t smem4 = (size_t)(2 * rot_half + (H + KV) * dk + (per_head ? H + KV : 0)) * sizeof(float);
-    const bool fours = (pair_layout == BL_PAIRS_HALVES || rot_half == 0) && dk % 4 == 0 && dv % 4 == 0 && rot_half % 4 == 0 && ld % 4 == 0 &&
+    const bool fours = dk % 4 == 0 && dv % 4 == 0 && rot_half % 4 == 0 && ld % 4 == 0 &&
                        off_k % 4 == 0 && off_v % 4 == 0 && smem4 <= 48 * 1024 &&
                        (((uintptr_t)proj | (uintptr_t)q_norm_w | (uintptr_t)k_norm_w | (uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0;
     if (fours) {
@@ -302,7 +309,7 @@ extern "C" int bl_qk_norm_rope_write_ext(const float* proj, int ld, int off_k, i
         if (threads > most) threads = most;
 #define BL_GO(TT) BL_CUDA(bl_launch_dependent(qk_norm_rope_write4_kernel<TT>, dim3(T), dim3(threads), smem4, s, proj, ld, off_k, off_v, \
         q_norm_w, qw_dtype, k_norm_w, kw_dtype, eps, positions, tok_req, block_table, max_pages, inv_freq, rot_half, \
-        (TT*)q_out, (TT*)k_cache, (TT*)v_cache, H, KV, dk, dv, page_size, per_head, q_head_scale, bl))
+        pair_layout == BL_PAIRS_INTERLEAVED ? 1 : 0, (TT*)q_out, (TT*)k_cache, (TT*)v_cache, H, KV, dk, dv, page_size, per_head, q_head_scale, bl))
         if (dtype == BL_F32) BL_GO(float);
         else if (dtype == BL_BF16) BL_GO(__nv_bfloat16);
         else BL_FAIL("bl_qk_norm_rope_write: unknown dtype %d", dtype);

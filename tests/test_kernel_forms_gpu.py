@@ -739,3 +739,33 @@ def test_layer_end_chain_of_many_rows(d):
         o.norm_chain(s[n - 1], sub[r], gate[r], gb, (pw, pb, 1e-6), streams=s, coeffs=c, n=n, mix_out=s[n], then=(tw, tb, 1e-5), y=y)
         ys.append(y)
     assert torch.equal(whole, torch.cat(parts, dim=1)) and torch.equal(ys[0], torch.cat(ys[1:]))
+
+
+@pytest.mark.parametrize("dk,dv,rot_half,per", [(8, 8, 4, 1), (64, 128, 32, 2), (64, 64, 16, 1), (128, 64, 64, 3)])
+def test_rotation_of_neighbouring_pairs_four_values_at_a_time(dk, dv, rot_half, per):
+    """Norms of the q and k rows, neighbours rotated (a part of each head among them), caches written, against 64 bits."""
+    o = ops()
+    T, KV, page = 9, 2, 16
+    H = KV * per
+    off_k, off_v = H * dk + 4, (H + KV) * dk + 8
+    proj = data((T, off_v + KV * dv + 4), 1) * 2
+    qw, kw = data((H * dk,), 2).to(BF), data((KV * dk,), 3)
+    pos = torch.tensor([0, 1, 2, 3, 17, 40, 5, 6, 31], dtype=torch.int32, device=DEV)
+    req = torch.tensor([0, 0, 0, 0, 0, 0, 1, 1, 1], dtype=torch.int32, device=DEV)
+    table = torch.tensor([[3, 0, 5], [1, 4, 2]], dtype=torch.int32, device=DEV)
+    inv = torch.from_numpy((1e4 ** (-np.arange(rot_half) / rot_half)).astype(np.float32)).to(DEV)
+    q = torch.empty(T, H * dk, device=DEV)
+    kc, vc = torch.zeros(6, KV, page, dk, device=DEV), torch.zeros(6, KV, page, dv, device=DEV)
+    o.qk_norm_rope_write(proj, off_k, off_v, qw, kw, 1e-6, pos, req, table, inv, rot_half, 1, q, kc, vc, H, KV, dk, dv)
+    p64 = proj.double()
+    ang = (pos.float()[:, None] * inv).double()[:, None]
+
+    def turned(z, w, heads):
+        z = (z / torch.sqrt((z * z).mean(-1, keepdim=True) + 1e-6) * w.double()).view(T, heads, dk)
+        a, b = z[..., 0:2 * rot_half:2], z[..., 1:2 * rot_half:2]
+        r = torch.stack((a * ang.cos() - b * ang.sin(), b * ang.cos() + a * ang.sin()), -1).flatten(-2)
+        return torch.cat([r, z[..., 2 * rot_half:]], -1)
+    close(q, turned(p64[:, :H * dk], qw, H).reshape(T, -1), torch.float32, "q")
+    pages, rows = table[req.long(), pos.long() // page].long(), pos.long() % page
+    close(kc[pages, :, rows], turned(p64[:, off_k:off_k + KV * dk], kw, KV), torch.float32, "k")
+    assert torch.equal(vc[pages, :, rows], proj[:, off_v:off_v + KV * dv].view(T, KV, dv))
