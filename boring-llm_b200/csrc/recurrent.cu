@@ -738,6 +738,77 @@ conv4_silu_unit_kernel(const float* x, int ld, const float4* __restrict__ taps, 
     }
 }
 
+// The same for many tokens: a block takes CONV_RUN neighbouring tokens, and a thread goes down them with its channels' taps and
+// last inputs in registers. One token a block reads every input four times and the taps (16 bytes a channel, as much as four inputs)
+// once a token, all through L2, which is what it waits for (1,840 tokens of 4,096 channels 39 us, of which 9 are bytes; 2,048 of
+// 1,792 24 us). A request's first tokens fetch the inputs before them from its tail.
+constexpr int CONV_RUN = 4;
+__global__ void __launch_bounds__(CONV4_THREADS)
+conv4_silu_unit_run_kernel(const float* x, int ld, const float4* __restrict__ taps, const float* tail, size_t slot_stride,
+                           const int* __restrict__ slots, const int* __restrict__ tok_req, const int* __restrict__ cu_q, float* y,
+                           int T, int C, int unit_heads, int scaled_heads, int dk, float q_scale, float unit_eps, const void* __restrict__ bias,
+                           int bias_dtype) {
+    bl_pdl_trigger();
+    extern __shared__ __align__(16) float units[];               // [CONV_RUN][unit_heads * dk]
+    const int lane = threadIdx.x & 31, unit_cols = unit_heads * dk;
+    const int t0 = blockIdx.x * CONV_RUN, n = min(CONV_RUN, T - t0);
+    int place[CONV_RUN];                                         // a token's place in its request
+    const float* tl[CONV_RUN];
+#pragma unroll
+    for (int u = 0; u < CONV_RUN; ++u) {
+        const int r = tok_req[t0 + min(u, n - 1)];
+        place[u] = t0 + u - cu_q[r];
+        tl[u] = tail + (size_t)slots[r] * slot_stride;
+    }
+    bl_pdl_wait();
+    for (int ch = threadIdx.x * 4; ch < C; ch += CONV4_THREADS * 4) {
+        float4 tp[4], in[CONV_RUN + 3];                          // in[u + i]: input i of the four that token u sums
+        float b[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) tp[i] = taps[ch + i];        // the four taps of channel ch + i
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {                            // before the first token
+            const int off = place[0] - 3 + i;
+            in[i] = *reinterpret_cast<const float4*>(off >= 0 ? x + ((ptrdiff_t)t0 - 3 + i) * ld + ch : tl[0] + (size_t)(3 + off) * C + ch);
+        }
+#pragma unroll
+        for (int u = 0; u < CONV_RUN; ++u)
+            if (u < n) in[u + 3] = *reinterpret_cast<const float4*>(x + (size_t)(t0 + u) * ld + ch);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) b[e] = bias ? bl_load_any(bias, bias_dtype, ch + e) : 0.f;
+#pragma unroll
+        for (int u = 0; u < CONV_RUN; ++u) {
+            if (u >= n) continue;
+            float4 q[3] = {in[u], in[u + 1], in[u + 2]};
+            if (u > 0 && place[u] < 3 && place[u] <= u) {        // its request begins in this block: what precedes its first token is in the tail
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+                    if (place[u] - 3 + i < 0) q[i] = *reinterpret_cast<const float4*>(tl[u] + (size_t)(place[u] + i) * C + ch);
+            }
+            float acc[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                float a = b[e];
+                a = fmaf(tp[e].x, reinterpret_cast<const float*>(&q[0])[e], a);
+                a = fmaf(tp[e].y, reinterpret_cast<const float*>(&q[1])[e], a);
+                a = fmaf(tp[e].z, reinterpret_cast<const float*>(&q[2])[e], a);
+                a = fmaf(tp[e].w, reinterpret_cast<const float*>(&in[u + 3])[e], a);
+                acc[e] = bl_silu(a);
+            }
+            *reinterpret_cast<float4*>(ch < unit_cols ? units + (size_t)u * unit_cols + ch : y + (size_t)(t0 + u) * C + ch) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        }
+    }
+    __syncthreads();
+    for (int item = threadIdx.x >> 5; item < n * unit_heads; item += CONV4_THREADS / 32) {
+        const int u = item / unit_heads, hh = item % unit_heads;
+        const float* p = units + (size_t)u * unit_cols + (size_t)hh * dk;
+        float ss = 0.f;
+        for (int d = lane; d < dk; d += 32) ss += p[d] * p[d];
+        const float inv = (hh < scaled_heads ? q_scale : 1.f) / sqrtf(bl_warp_sum(ss) + unit_eps);
+        for (int d = lane; d < dk; d += 32) y[(size_t)(t0 + u) * C + (size_t)hh * dk + d] = p[d] * inv;
+    }
+}
+
 // After the step's convolutions have read the tail: the last n_taps - 1 inputs of each request with tokens.
 __global__ void conv_tail_update_kernel(const float* x, int ld, int n_taps, float* tail, size_t slot_stride,
                                         const int* __restrict__ slots, const int* __restrict__ cu_q, int C) {
@@ -1091,6 +1162,14 @@ extern "C" int bl_conv_silu_unit_bias(const float* x, int ld, const float* taps,
     const int unit_cols = unit_heads * dk;
     if (n_taps == 4 && C % 4 == 0 && ld % 4 == 0 && slot_stride % 4 == 0 && unit_cols % 4 == 0 && unit_cols <= 8192 &&
         (((uintptr_t)x | (uintptr_t)taps | (uintptr_t)tail | (uintptr_t)y) & 15) == 0) {
+        // several tokens a block where the launch then still has a block for every SM, and their unit heads fit its 48 KB
+        if (T >= CONV_RUN * 148 && CONV_RUN * unit_cols * (int)sizeof(float) <= 48 * 1024) {
+            BL_CUDA(bl_launch_dependent(conv4_silu_unit_run_kernel, dim3((T + CONV_RUN - 1) / CONV_RUN), dim3(CONV4_THREADS),
+                                        (size_t)CONV_RUN * unit_cols * sizeof(float), (cudaStream_t)stream, x, ld, (const float4*)taps, tail,
+                                        (size_t)slot_stride, slots, tok_req, cu_q, y, T, C, unit_heads, scaled_heads, dk, q_scale, unit_eps, bias, bias_dtype));
+            BL_CHECK_LAUNCH("bl_conv_silu_unit");
+            return 0;
+        }
         BL_CUDA(bl_launch_dependent(conv4_silu_unit_kernel, dim3(T), dim3(CONV4_THREADS), (size_t)unit_cols * sizeof(float),
                                     (cudaStream_t)stream, x, ld, (const float4*)taps, tail, (size_t)slot_stride, slots, tok_req, cu_q, y, C,
                                     unit_heads, scaled_heads, dk, q_scale, unit_eps, bias, bias_dtype));

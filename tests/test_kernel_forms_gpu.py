@@ -769,3 +769,30 @@ def test_rotation_of_neighbouring_pairs_four_values_at_a_time(dk, dv, rot_half, 
     pages, rows = table[req.long(), pos.long() // page].long(), pos.long() % page
     close(kc[pages, :, rows], turned(p64[:, off_k:off_k + KV * dk], kw, KV), torch.float32, "k")
     assert torch.equal(vc[pages, :, rows], proj[:, off_v:off_v + KV * dv].view(T, KV, dv))
+
+
+@pytest.mark.parametrize("unit,dk,C", [(3, 16, 96), (4, 64, 260), (0, 16, 36), (24, 128, 3100)])
+def test_short_convolution_of_many_tokens(unit, dk, C):
+    """Several tokens a block against a token a block, bit for bit: requests that begin, end and have one token anywhere in a block."""
+    o = ops()
+    lens = [5, 1, 1, 1, 0, 2, 400, 3, 2, 1, 190, 6]
+    T, R = sum(lens), len(lens)
+    x, tail = data((T, C + 4), 3), data((R, 3 * C + 4), 5)
+    w, bias = data((C, 4), 7), data((C,), 8)
+    slots = torch.arange(R, dtype=torch.int32, device=DEV).flip(0).contiguous()
+    cu = torch.tensor([0] + lens, device=DEV).cumsum(0).to(torch.int32)
+    req = torch.repeat_interleave(torch.arange(R), torch.tensor(lens)).to(torch.int32).to(DEV)
+    assert T >= 592
+    y = torch.full((T, C), float("nan"), device=DEV)
+    o.conv_silu_unit(x, w, tail, slots, req, cu, y, unit, min(unit, 1), dk, 0.25, 1e-6, bias=bias)
+    few = torch.full((T, C), float("nan"), device=DEV)
+    for r in range(R):                                 # a request by itself
+        lo, hi = int(cu[r]), int(cu[r + 1])
+        if lo == hi:
+            continue
+        part = torch.full((hi - lo, C), float("nan"), device=DEV)
+        one = torch.tensor([0, hi - lo], dtype=torch.int32, device=DEV)
+        o.conv_silu_unit(x[lo:hi], w, tail, slots[r:r + 1].contiguous(), torch.zeros(hi - lo, dtype=torch.int32, device=DEV), one, part, unit,
+                         min(unit, 1), dk, 0.25, 1e-6, bias=bias)
+        few[lo:hi] = part
+    assert torch.equal(y, few)
