@@ -796,3 +796,21 @@ def test_short_convolution_of_many_tokens(unit, dk, C):
                          min(unit, 1), dk, 0.25, 1e-6, bias=bias)
         few[lo:hi] = part
     assert torch.equal(y, few)
+
+
+@pytest.mark.parametrize("H,dv", [(1, 4), (3, 128), (2, 132), (5, 256), (2, 512)])
+@pytest.mark.parametrize("gate", [None, "GATE_SILU", "GATE_SIGMOID"])
+def test_norm_of_heads_in_groups_of_four(H, dv, gate):
+    o = ops()
+    T = 7
+    x, g, w, wh = data((T, H * dv), 3) * 2, data((T, H * dv + 4), 4), data((dv,), 5).to(BF), data((H * dv,), 6)
+    x64 = x.double().view(T, H, dv)
+    n64 = x64 / torch.sqrt((x64 * x64).mean(-1, keepdim=True) + 1e-5)
+    gv = None if gate is None else g[:, :H * dv]
+    f = 1.0 if gate is None else torch.sigmoid(gv.double()) * (gv.double() if gate == "GATE_SILU" else 1.0)
+    for dtype in (torch.float32, BF):
+        out = torch.empty(T, H * dv, dtype=dtype, device=DEV)
+        o.head_norm_gate(x, w, gv, getattr(o, gate or "GATE_SILU"), 1e-5, out, H, dv)
+        close(out, (n64 * w.double()).reshape(T, -1) * f, dtype, "shared weight")
+        o.head_norm_gate_ext(x, wh, gv, getattr(o, gate or "GATE_SILU"), 1e-5, out, H, dv)
+        close(out, n64.reshape(T, -1) * wh.double() * f, dtype, "weight per head")
