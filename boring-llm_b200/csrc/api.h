@@ -523,6 +523,12 @@ int bl_latent_attention_mma(const void* q_lat, const void* q_rot, const void* ca
                             const int* block_table, int max_pages, const int* work, int n_work, int single, void* out, int H, int Tp,
                             int rank, int rot, int page_size, int window, float scale, const void* sinks, int sink_dtype, int n_splits,
                             float* part_o, float* part_ml, void* stream);
+// Products of up to 64 rows by large matrices (a decode step's; gemm_tcgen05_few.cu): W streams once as the M side of the MMA,
+// clusters cut K where W has few tiles. out 32-bit (no epilogue, bias, residual) or, with the gated epilogue, bfloat16.
+int bl_gemm_tc_few_supported(int M, int N, int K);
+int bl_gemm_tc_few(const void* x, const void* w, const void* bias, int bias_dtype, void* out, int out_dtype, int M, int N, int K,
+                   int epilogue, void* stream);
+int bl_gemm_tc_few_status(int* status);
 // Every head's own keys and values made for the step. bl_latent_rows: rows 16 i .. 16 i + 15 of latent [., rank] and shared [., 64]
 // (its first `rot` columns) = the cached rows of the 16 keys from work[i][1] on of request work[i][0], zeros where there are none (latent.cu).
 // bl_attention_rows_tc: the tcgen05 attention (attention_tcgen05.cu) over q [T, H, own + rot], kv [L, H * own + H * dv] (all heads'

@@ -601,6 +601,20 @@ def gemm_tc_splitk(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Op
           M, N, K, epilogue, _stream())
 
 
+def gemm_tc_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
+                epilogue: int = EPI_NONE) -> None:
+    """out = epilogue(x @ w.T) for up to 64 rows by a large matrix, on the tcgen05 kernel that streams W once, with clusters that
+    cut K where W has few tiles. out 32-bit; with EPI_SWIGLU (w with twice the rows) bfloat16."""
+    M, K = x.shape
+    N = out.shape[1]
+    rows_w = 2 * N if epilogue == EPI_SWIGLU else N
+    _need(x, "x", torch.bfloat16); _need(w, "w", torch.bfloat16, (rows_w, K)); _need(out, "out", None, (M, N))
+    if bias is not None:
+        _need_bias(bias, N, epilogue)
+    _call(_lib().bl_gemm_tc_few, _p(x), _p(w), _p(bias), _dt(bias) if bias is not None else 0, _p(out), _dt(out), M, N, K, epilogue,
+          _stream())
+
+
 _splitk_split = {}
 
 
@@ -645,7 +659,8 @@ SPLITK_FEW_ROWS_K = 8192              # ... or, from 9 rows, this long (9 and 16
                                       # 1,024 10.8 and 10.9 against 9.3 and 11.0, 8,192 by 256 6.8 against 5.6 and 6.6; 16 rows of 4,864 by 896 7.1 against 4.8),
 SPLITK_MORE_ROWS_K = 4096             # ... or, from 17 rows, this long (17 and 31 rows of 4,864 by 896: 7.1 and 7.3 us against 9.9 and 12.0, of 4,096 by 2,048 8.0
                                       # and 8.3 against 8.4 and 10.4, by 136 5.2 and 5.3 against 6.0 and 7.8; 24 rows of 2,048 by 2,048 7.4 against 5.4)
-STREAM_MIN_BYTES = 128 << 20          # matrices from this size on stream faster through TMA and tcgen05 than through registers, at any number of rows
+STREAM_MIN_BYTES = 64 << 20           # matrices from this size on stream faster through TMA and tcgen05 than through registers, at any number of rows
+                                      # (90 MB of gate and up rows, K 2,048: 1, 8 and 16 rows 21.1, 21.4 and 21.8 us against 26.2, 28.0 and 47.4)
 SPLITK_LONG_K = 2048                  # ... when K is long (measured: K 4,864 by N 896 gains 2x at 128 rows, 1.25x at 512; K 896 gains only up to 128 rows)
 
 
@@ -655,12 +670,44 @@ def gemm_streams_better(w: torch.Tensor) -> bool:
     return w.numel() * w.element_size() >= STREAM_MIN_BYTES
 
 
+def gemm_few_better(M: int, N: int, w: torch.Tensor, epilogue: int) -> bool:
+    """Whether a product of up to 64 rows runs on the kernel that streams W once as the M side of the MMA (`gemm_tc_few`). A small W
+    is left to the kernels without its 4 us of set-up; where the line lies depends on what stands on the other side. Microseconds,
+    the kernel before and this one, cold matrices, launches in a row:
+
+    gated epilogue, up to 31 rows: 18,944 + 18,944 x 3,584 1 row 61.5 / 42.1, 16 61.5 / 43.2, 24 44.9 / 43.5; 11,008 + 11,008 x 2,048
+        8 rows 28.0 / 21.4, 24 34.9 / 22.6, but 32 20.5 / 22.9 and 64 21.1 / 25.4;
+    up to 8 rows by bytes: 8 rows of 8,208 x 2,048 11.4 / 8.4, 3,584 x 3,584 9.0 / 7.9, 6,224 x 2,048 8.7 / 8.0, 2,048 x 11,008 14.4 / 12.3, one
+        row of 3,584 x 18,944 38.6 / 27.1, 11,008 x 2,048 11.5 / 10.8; but 2,560 x 2,048 5.1 / 5.8;
+    9 to 16 rows, smaller ones if they have columns: 16 rows of 4,864 x 896 6.5 / 5.3, 2,560 x 2,048 6.8 / 5.9, 3,584 x 3,584 12.0 / 8.0; but
+        2,048 x 2,048 3.8 / 5.7, 896 x 4,864 5.2 / 5.4;
+    17 to 32 rows: 896 x 4,864 7.2 / 5.6, 3,600 x 896 5.4 / 5.0, 4,608 x 3,584 10.3 / 10.0; but 24 rows of 2,048 x 2,048 4.6 / 5.5;
+    33 to 64 rows: 64 rows of 2,048 x 2,048 7.5 / 7.0, 3,584 x 3,584 11.4 / 9.5, 8,208 x 2,048 11.3 / 10.5, 3,600 x 896 10.9 / 5.6; but
+        11,008 x 2,048 12.1 / 12.9, 4,864 x 896 6.4 / 6.7, 2,048 x 11,008 14.2 / 14.5, 1,152 x 896 3.1 / 5.6."""
+    rows_w, K = w.shape
+    nbytes = 2 * rows_w * K
+    if M > 64 or N >= TC_MIN_COLUMNS_VERY_FEW_ROWS:
+        return False
+    if epilogue == EPI_SWIGLU:
+        return M < 32 and nbytes >= STREAM_MIN_BYTES
+    if M <= 8:
+        return nbytes >= 24e6
+    if M <= 16:
+        return nbytes >= 20e6 or (N >= 2560 and nbytes >= 8.5e6)
+    if M <= 32:
+        return nbytes >= 8.5e6 or (N >= 2560 and nbytes >= 6e6)
+    if N > 4096 and (K <= 1024 or N >= 10240) or N <= 2048 and K >= 8192:
+        return False
+    return nbytes >= 8e6 or (N >= 2560 and nbytes >= 6e6)
+
+
 def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
          epilogue: int = EPI_NONE, fast: bool = True) -> None:
     """out = epilogue(x @ w.T) by the kernel that suits the operands: float32 operands, operands the tensor-core
     kernels cannot take, and `fast=False` run the plain CUDA-core kernel; bfloat16 operands a tensor-core kernel
     chosen by the number of rows (and, for few rows, of columns)."""
-    kind = gemm_kernel(x, w, out.shape[1], bias, epilogue, fast)
+    few = out.dtype == (torch.bfloat16 if epilogue == EPI_SWIGLU else torch.float32) and out.data_ptr() % 16 == 0
+    kind = gemm_kernel(x, w, out.shape[1], bias, epilogue, fast, few=few)
     if kind == "plain":
         gemm_plain(x, w, out, bias, epilogue)
     elif kind == "cols":
@@ -669,19 +716,24 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[tor
         gemm_tc_splitk(x, w, out, bias, epilogue)
     elif kind == "skinny":
         gemm_skinny(x, w, out, bias, epilogue)
+    elif kind == "few":
+        gemm_tc_few(x, w, out, bias, epilogue)
     elif kind == "tc":
         gemm_tc(x, w, out, bias, epilogue)
     else:
         gemm_tc_pair(x, w, out, bias, epilogue)
 
 
-def gemm_kernel(x: torch.Tensor, w: torch.Tensor, N: int, bias: Optional[torch.Tensor], epilogue: int, fast: bool = True) -> str:
-    """Which kernel `gemm` runs this product on: "plain", "cols" (an output head at decode time: W streams once, as the
+def gemm_kernel(x: torch.Tensor, w: torch.Tensor, N: int, bias: Optional[torch.Tensor], epilogue: int, fast: bool = True, few: bool = True) -> str:
+    """Which kernel `gemm` runs this product on: "plain", "few" (up to 64 rows by a large matrix, see `gemm_few_better`; `few` False: the
+    result is of a type that this kernel does not have, or an RMS norm links the product to the one before or behind), "cols" (an output head at decode time: W streams once, as the
     M side of the product), "splitk" (few tiles and a long K, a down projection: clusters cut K among their blocks),
     "skinny" (few rows: W streams through registers), "tc" or "pair" (tcgen05 tiles on one SM, on pairs of SMs)."""
     if not (fast and gemm_skinny_supported(x, w)):
         return "plain"
     M, K = x.shape
+    if few and gemm_few_better(M, N, w, epilogue):
+        return "few"
     few_rows_tc = ((M > 16 and N >= TC_MIN_COLUMNS_FEW_ROWS) or (M > 8 and N >= TC_MIN_COLUMNS_VERY_FEW_ROWS)
                    or gemm_streams_better(w))
     if ((N >= TC_MIN_COLUMNS_VERY_FEW_ROWS or (N >= COLS_MIN_COLUMNS and M <= 32)) and bias is None and epilogue == EPI_NONE
@@ -713,7 +765,7 @@ def gemm_skinny_links_norm(x: torch.Tensor, w: torch.Tensor, N: int, epilogue: i
     """Whether `gemm` would run this product on the register-streaming kernel at a row count where that kernel's
     epilogues begin an RMS norm (`gemm_skinny_residual_norm`) and finish one (`gemm_skinny_scaled`)."""
     return (SKINNY_LINK_MIN_ROWS <= x.shape[0] <= SKINNY_LINK_MAX_ROWS and -(-N // 16) <= SKINNY_LINK_MAX_BLOCKS
-            and gemm_kernel(x, w, N, None, epilogue, fast) == "skinny")
+            and gemm_kernel(x, w, N, None, epilogue, fast, few=False) == "skinny")
 
 
 def gemm_skinny_residual_norm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, norm_w: torch.Tensor,
@@ -788,7 +840,7 @@ def check_status() -> None:
     for name, fn in (("bl_gemm_tc", _lib().bl_gemm_tc_status), ("bl_gemm_f32_tc", _lib().bl_gemm_f32_tc_status), ("bl_gemm_tc_pair", _lib().bl_gemm_tc_pair_status),
                      ("bl_attention_prefill_tc", _lib().bl_attention_prefill_tc_status),
                      ("bl_gemm_tc_cols", _lib().bl_gemm_tc_cols_status),
-                     ("bl_gemm_tc_splitk", _lib().bl_gemm_tc_splitk_status),
+                     ("bl_gemm_tc_splitk", _lib().bl_gemm_tc_splitk_status), ("bl_gemm_tc_few", _lib().bl_gemm_tc_few_status),
                      ("bl_attention_decode_tma", _lib().bl_attention_decode_tma_status)):
         v = ctypes.c_int(0)
         _call(fn, ctypes.byref(v))

@@ -814,3 +814,40 @@ def test_norm_of_heads_in_groups_of_four(H, dv, gate):
         close(out, (n64 * w.double()).reshape(T, -1) * f, dtype, "shared weight")
         o.head_norm_gate_ext(x, wh, gv, getattr(o, gate or "GATE_SILU"), 1e-5, out, H, dv)
         close(out, n64.reshape(T, -1) * wh.double() * f, dtype, "weight per head")
+@pytest.mark.parametrize("M,N,K", [(1, 130, 72), (16, 896, 4864), (17, 2048, 1096), (33, 257, 200), (64, 1024, 136), (9, 19204, 72), (40, 19101, 128)])
+def test_few_rows_with_w_streamed_once(M, N, K):
+    """Clusters of every size and tiles in rounds (two accumulators taking turns), remainders of rows, columns and k, each epilogue."""
+    o = ops()
+    x, w, b = (data((M, K), 1) * 0.5).to(BF), (data((N, K), 2) * 0.2).to(BF), data((N,), 3)
+    z = x.double() @ w.double().T
+    out = torch.empty(M, N, device=DEV)
+    o.gemm_tc_few(x, w, out)
+    close(out, z, torch.float32, "product")
+    o.gemm_tc_few(x, w, out, b, o.EPI_BIAS)
+    close(out, z + b.double(), torch.float32, "bias")
+    res = data((M, N), 4)
+    want = res.double() + z + b.double()
+    o.gemm_tc_few(x, w, res, b, o.EPI_RESIDUAL)
+    close(res, want, torch.float32, "residual")
+    n = N // 2
+    act = torch.empty(M, n, dtype=BF, device=DEV)
+    o.gemm_tc_few(x, w[:2 * n].contiguous(), act, None, o.EPI_SWIGLU)
+    close(act, plain.silu(z[:, :n]) * z[:, n:2 * n], BF, "swiglu")
+    o.gemm_tc_few(x, w[:2 * n].contiguous(), act, o.glu_args(o.GLU_CLAMPED, 0.5, DEV), o.EPI_SWIGLU)
+    g, u = z[:, :n].clamp(max=0.5), z[:, n:2 * n].clamp(-0.5, 0.5)
+    close(act, g * torch.sigmoid(1.702 * g) * (u + 1), BF, "clamped")
+    o.check_status()
+
+
+def test_few_rows_go_by_the_bytes_of_w():
+    """The kernel on either side of its lines, and that a product that an RMS norm links to another stays where the norm is."""
+    o = ops()
+    m = lambda *s: torch.empty(*s, dtype=BF, device=DEV)
+    kinds = [(8, 8208, 2048, o.EPI_NONE, "few"), (8, 2560, 2048, o.EPI_BIAS, "skinny"), (16, 2560, 2048, o.EPI_BIAS, "few"), (16, 2048, 2048, o.EPI_RESIDUAL, "skinny"),
+             (17, 896, 4864, o.EPI_RESIDUAL, "few"), (64, 3600, 896, o.EPI_NONE, "few"), (64, 1152, 896, o.EPI_BIAS, "skinny"), (64, 11008, 2048, o.EPI_NONE, "tc"),
+             (16, 11008, 2048, o.EPI_SWIGLU, "few"), (32, 11008, 2048, o.EPI_SWIGLU, "tc"), (65, 8208, 2048, o.EPI_NONE, "splitk")]
+    for M, N, K, epi, kind in kinds:
+        b = torch.empty(N, device=DEV) if epi == o.EPI_BIAS else None
+        assert o.gemm_kernel(m(M, K), m(2 * N if epi == o.EPI_SWIGLU else N, K), N, b, epi) == kind, (M, N, K)
+    x, w = m(8, 11008), m(2048, 11008)
+    assert o.gemm_kernel(x, w, 2048, None, o.EPI_RESIDUAL) == "few" and o.gemm_skinny_links_norm(x, w, 2048, o.EPI_RESIDUAL)
