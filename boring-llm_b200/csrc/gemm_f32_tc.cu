@@ -7,20 +7,25 @@
 // in registers, rounded to nearest, in ascending k: 28 rounded additions for K = 896 where a chain of FMAs makes 896.
 // Errors against 64 bits are no larger than such a chain's (the test of this kernel has both).
 //
-// W is the M side of the MMA (128 rows of W a tile; with SWIGLU 64 units, 16 gate rows and the 16 up rows that match in turn) and
-// NT rows of x its N side. A block: 8 warps fetch rows of W and x (16-byte loads, DEPTH segments ahead in registers), split
-// them and store both halves where the MMAs read them (128-byte swizzle); a thread of the first of them issues the 12 MMAs of the
-// segment before, into one of two accumulators (a warp of its own for that would leave 96 registers a thread, and spills); 4 or 8 warps
-// add the other one to their registers. At the end the tile passes through shared memory to the
-// epilogue. Products of few tiles cut K over the blocks of a cluster (f32_tc_spans), whose totals are added in ascending k through
-// distributed shared memory. What a result is computed from, and in which order, depends on N and K only: it is the same whatever
-// rows stand beside a row and however wide a tile is (the same promise that the kernels in gemm_plain.cu make, which keep the
-// small products).
+// W is the M side of the MMA (128 rows of W a tile; with SWIGLU 64 gate rows and the 64 up rows that match) and NT rows of x its
+// N side. A block: TMA brings 32 values of k of the tile's rows into a ring; 8 warps split them and store both halves where the MMAs
+// read them (128-byte swizzle), one thread of the first of them issues the segment's 12 MMAs into one of two accumulators, one of the
+// second refills the ring; 4 or 8 warps add the other accumulator to their registers. (Rows fetched ahead into the splitters' own
+// registers cannot be: the fence that shows their stores to the tensor cores waits for every load under way, 1,600 cycles a
+// segment.) At the end the tile passes through shared memory to the epilogue. Products of few tiles cut K over the blocks of a
+// cluster (f32_tc_spans), whose totals are added in ascending k through distributed shared memory. What a result is computed from, and
+// in which order, depends on N and K only: it is the same whatever rows stand beside a row and however wide a tile is (the same promise
+// that the kernels in gemm_plain.cu make, which keep the small products).
 // A sum that is not finite (an infinity or NaN among the inputs, whose halves are NaN, or an overflow) is worked out again as
 // a chain of FMAs over the inputs themselves.
 //
-// Bound by shared memory: a segment of a 128 x 128 tile stores 64 KB and its MMAs read 96 KB, 1,280 cycles of the SM's
-// port against 830 of the tensor cores.
+// Bound by the splitting (every 4 bytes of W are read from shared memory once, stored twice, and read three times by the MMAs) and,
+// for many rows, the tensor cores (12 MMAs a segment, 830 cycles for 128 x 128). Microseconds, before (FMAs) -> now:
+//   rows                          1             16            128           366           2,048
+//   1,152 x 896, bias             7.8 -> 8.3    8.7 -> 8.4    19.7 -> 19.0   31 -> 25     118 -> 71
+//   896 x 896, residual           7.7 -> 8.2    8.8 -> 8.5    17.8 -> 10.7   33 -> 14     110 -> 62
+//   9,728 + 9,728 x 896, gated   13.6 -> 24.0    25 -> 24.3     71 -> 38    178 -> 75     876 -> 335
+//   896 x 4,864, residual          55 -> 31      48 -> 31.6     84 -> 36    158 -> 47     557 -> 203
 // Every wait on an mbarrier is bounded; when a bound runs out the block records a code in a status word and stops computing, but
 // still meets its cluster, frees its tensor memory and returns (bl_gemm_f32_tc_status).
 #include "tcgen05.cuh"
@@ -29,6 +34,7 @@
 namespace {
 
 constexpr int BM = 128;                    // rows of W a tile
+constexpr int MAX_COLUMNS = 1 << 15;       // more: an output head
 constexpr int BK = 32;                     // values of k a segment: one 128-byte row of the swizzled operand tiles
 constexpr int SPLITTERS = 256, ADDERS = 256, THREADS = SPLITTERS + ADDERS;
 constexpr int TMEM_COLS = 256;             // two accumulators of up to 128 columns
@@ -36,15 +42,15 @@ constexpr uint32_t WAIT_LIMIT = 1u << 22;
 
 template <int NT>
 struct Tile {
-    static constexpr int W_BYTES = BM * 128, X_BYTES = NT * 128, STAGE_BYTES = 2 * (W_BYTES + X_BYTES);     // hi and lo of both
-    static constexpr int STAGES = NT >= 64 ? 3 : 5;
-    static constexpr int DEPTH = NT >= 64 ? 2 : 3;                        // segments that a splitter has in flight
+    static constexpr int W_BYTES = BM * 128, X_BYTES = NT * 128, RAW_BYTES = W_BYTES + X_BYTES, PAIR_BYTES = 2 * RAW_BYTES;     // as they came; hi and lo
+    static constexpr int PAIRS = NT >= 64 ? 2 : 3;                        // stages of halves
+    static constexpr int RAWS = NT == 128 ? 2 : NT >= 64 ? 3 : 5;         // stages of the ring
     static constexpr int HALVES = NT >= 64 ? 2 : 1;                       // the columns are dealt to one or two groups of four adder warps
     static constexpr int COLS = NT / HALVES;
     static constexpr int CHUNKS = 4 + (NT + 31) / 32;                     // 16-byte pieces of a segment a splitter
-    static constexpr int OFF_BARS = STAGES * STAGE_BYTES;
+    static constexpr int OFF_RAW = PAIRS * PAIR_BYTES, OFF_BARS = OFF_RAW + RAWS * RAW_BYTES;
     static constexpr int SMEM_BYTES = OFF_BARS + 256 + 1024;
-    static_assert(NT % 16 == 0 && COLS % 16 == 0 && BM * NT * 4 <= STAGES * STAGE_BYTES && SMEM_BYTES <= 227 * 1024, "tile");
+    static_assert(NT % 16 == 0 && COLS % 16 == 0 && BM * NT * 4 <= OFF_RAW && SMEM_BYTES <= 227 * 1024, "tile");
 };
 
 __device__ int g_status = 0;               // 0 = fine; else the code of the first wait that ran out
@@ -58,6 +64,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     *give_up = 1;
     atomicCAS(&g_status, 0, code);
     return false;
+}
+// Bounded wait that does not look at the give-up flag (a block that has given up waits for its own copies).
+__device__ __forceinline__ void mbar_wait_plain(uint32_t bar, uint32_t parity) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < WAIT_LIMIT; ++i)
+        if (mbar_try_wait(bar, parity)) return;
 }
 __device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}"
@@ -92,18 +104,21 @@ __device__ __noinline__ float plain_dot(const float* x, const float* w, int K) {
 
 template <int EPI, int NT>
 __global__ void __launch_bounds__(THREADS, 1)
-gemm_f32_tc_kernel(const float* __restrict__ x, const float* __restrict__ w, const void* __restrict__ bias, int bias_dtype,
-                   float* __restrict__ out, int M, int N, int K, int ldx, int spans, int m_tiles) {
+gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const float* __restrict__ x,
+                   const float* __restrict__ w, const void* __restrict__ bias, int bias_dtype, float* __restrict__ out, int M, int N, int K,
+                   int ldx, int spans, int m_tiles) {
     using T = Tile<NT>;
     constexpr bool GLU = EPI == BL_EPI_SWIGLU;
     constexpr int UNITS = GLU ? BM / 2 : BM;                              // outputs of a row of x a tile
-    constexpr int STAGES = T::STAGES, DEPTH = T::DEPTH, CHUNKS = T::CHUNKS;
+    constexpr int PAIRS = T::PAIRS, RAWS = T::RAWS;
     // D 32-bit, A and B tf32 and K-major, N >> 3 at bit 17, M >> 4 at bit 24
     constexpr uint32_t IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
     extern __shared__ unsigned char smem_raw[];
+    if (threadIdx.x == 0) { tma_prefetch_map(&map_x); tma_prefetch_map(&map_w); }
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     unsigned char* smem = smem_raw + (base - smem_u32(smem_raw));
-    const uint32_t full0 = base + T::OFF_BARS, empty0 = full0 + 8 * STAGES, sum0 = empty0 + 8 * STAGES, taken0 = sum0 + 16;
+    const uint32_t raw_full0 = base + T::OFF_BARS, raw_read0 = raw_full0 + 8 * RAWS, full0 = raw_read0 + 8 * RAWS, empty0 = full0 + 8 * PAIRS,
+                   sum0 = empty0 + 8 * PAIRS, taken0 = sum0 + 16;
     volatile int* give_up = reinterpret_cast<volatile int*>(smem + T::OFF_BARS + 192);
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + T::OFF_BARS + 200);
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
@@ -114,10 +129,25 @@ gemm_f32_tc_kernel(const float* __restrict__ x, const float* __restrict__ w, con
     const int first = min(span * each, all), steps = min(each, all - first);
     if (threadIdx.x == 0) {
         *give_up = 0;
-        for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, SPLITTERS / 32); mbar_init(empty0 + 8 * s, 1); }
+        for (int s = 0; s < RAWS; ++s) { mbar_init(raw_full0 + 8 * s, 1); mbar_init(raw_read0 + 8 * s, SPLITTERS / 32); }
+        for (int s = 0; s < PAIRS; ++s) { mbar_init(full0 + 8 * s, SPLITTERS / 32); mbar_init(empty0 + 8 * s, 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(sum0 + 8 * b, 1); mbar_init(taken0 + 8 * b, 4 * T::HALVES); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    __syncthreads();
+    auto load_w = [&](int s) {                                             // and announce the segment's bytes
+        const uint32_t bar = raw_full0 + 8 * (s % RAWS), dst = base + T::OFF_RAW + s % RAWS * T::RAW_BYTES;
+        mbar_expect_tx(bar, T::RAW_BYTES);
+        tma_load_2d(dst, &map_w, bar, (first + s) * BK, n0);
+        if (GLU) tma_load_2d(dst + T::W_BYTES / 2, &map_w, bar, (first + s) * BK, N + n0);
+    };
+    auto load_x = [&](int s) {
+        tma_load_2d(base + T::OFF_RAW + s % RAWS * T::RAW_BYTES + T::W_BYTES, &map_x, raw_full0 + 8 * (s % RAWS), (first + s) * BK, m0);
+    };
+    const int early = min(RAWS, steps);
+    if (warp == 9 && elect_one())                                          // W does not depend on the kernel before this one
+        for (int s = 0; s < early; ++s) load_w(s);
+    __syncwarp();
     if (warp == 8) {
         __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -130,119 +160,108 @@ gemm_f32_tc_kernel(const float* __restrict__ x, const float* __restrict__ w, con
     const uint32_t tmem = *tmem_slot;
     bool ok = true;
     float* sums = reinterpret_cast<float*>(smem);                          // in the end: [column][row of the tile]
+    bl_pdl_wait();
+    bl_pdl_trigger();
 
     if (warp >= 8) {
         // ================= splitters: thread (row t / 8 + 32 i, piece t % 8) of W (i < 4) and of x (i >= 4)
         const int t = threadIdx.x - ADDERS, row = t >> 3, piece = t & 7;
-        const int unit = GLU ? n0 + (row & 15) : n0 + row;
-        constexpr int W_STEP = GLU ? 16 : 32;                              // units from one of a thread's rows of W to the next
-        const float* wp = w + (size_t)(unit + (GLU && row >= 16 ? N : 0)) * K + (size_t)first * BK + piece * 4;
-        const float* xp = x + (size_t)(m0 + row) * ldx + (size_t)first * BK + piece * 4;
-        float4 v[DEPTH][CHUNKS];
-        auto fetch = [&](int d, int i0, int i1, int step) {                // pieces i0 .. i1 of segment `step`
-            const int k = (first + step) * BK + piece * 4;
-#pragma unroll
-            for (int i = 0; i < CHUNKS; ++i) {
-                if (i < i0 || i >= i1) continue;
-                const bool is_w = i < 4;
-                bool have = step < steps && k < K;
-                if (is_w) have = have && unit + W_STEP * i < N;
-                else have = have && row + 32 * (i - 4) < NT && m0 + row + 32 * (i - 4) < M;
-                const float* p = is_w ? wp + (size_t)(W_STEP * i) * K : xp + (size_t)(32 * (i - 4)) * ldx;
-                v[d][i] = have ? *reinterpret_cast<const float4*>(p + (size_t)step * BK) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-        };
-#pragma unroll
-        for (int d = 0; d < DEPTH; ++d) fetch(d, 0, 4, d);                 // W does not depend on the kernel before this one
-        bl_pdl_wait();
-        bl_pdl_trigger();
-#pragma unroll
-        for (int d = 0; d < DEPTH; ++d) fetch(d, 4, CHUNKS, d);
-        // the MMAs of segment s, by one thread of the first splitter warp
-        auto issue = [&](int s) {
-            if (warp != 8) return;
-            const int st = s % STAGES, b = s & 1;
-            ok = mbar_wait(full0 + 8 * st, (uint32_t)((s / STAGES) & 1), give_up, 2);
-            if (ok && s >= 2) ok = mbar_wait(taken0 + 8 * b, (uint32_t)((s / 2 - 1) & 1), give_up, 2);
+        int issued = early;
+        if (warp == 9 && elect_one())
+            for (int s = 0; s < early; ++s) load_x(s);
+        __syncwarp();
+        const uint32_t from = base + T::OFF_RAW + (uint32_t)row * 128 + (uint32_t)piece * 16;
+        const uint32_t to = base + (uint32_t)row * 128 + (uint32_t)((piece ^ (row & 7)) << 4);       // (rows 32 apart swizzle alike)
+        for (int s = 0; s < steps; ++s) {
+            const int rs = s % RAWS, st = s % PAIRS, b = s & 1;
+            ok = mbar_wait(raw_full0 + 8 * rs, (uint32_t)((s / RAWS) & 1), give_up, 1);
             ok = __all_sync(0xffffffffu, ok);
-            if (ok && elect_one()) {
-                fence_after_sync();
-                const uint32_t stage = base + st * T::STAGE_BYTES, d = tmem + b * 128;
-                const uint64_t wh = smem_desc(stage), wl = smem_desc(stage + T::W_BYTES);
-                const uint64_t xh = smem_desc(stage + 2 * T::W_BYTES), xl = smem_desc(stage + 2 * T::W_BYTES + T::X_BYTES);
+            if (!ok) break;
+            float4 v[T::CHUNKS];
 #pragma unroll
-                for (int k = 0; k < BK / 8; ++k) {                         // the small products first
-                    umma_tf32(d, wl + 2 * k, xh + 2 * k, IDESC, k != 0);
-                    umma_tf32(d, wh + 2 * k, xl + 2 * k, IDESC, 1);
-                }
-#pragma unroll
-                for (int k = 0; k < BK / 8; ++k) umma_tf32(d, wh + 2 * k, xh + 2 * k, IDESC, 1);
-                umma_commit(empty0 + 8 * st);
-                umma_commit(sum0 + 8 * b);
+            for (int i = 0; i < T::CHUNKS; ++i) {
+                if (i >= 4 && row + 32 * (i - 4) >= NT) continue;
+                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[i].x), "=f"(v[i].y), "=f"(v[i].z), "=f"(v[i].w)
+                             : "r"(from + rs * T::RAW_BYTES + i * 4096) : "memory");
             }
-            __syncwarp();
-        };
-        const uint32_t at = base + (uint32_t)row * 128 + (uint32_t)((piece ^ (row & 7)) << 4);       // (rows 32 apart swizzle alike)
-        for (int s0 = 0; ok && s0 < steps; s0 += DEPTH) {
-#pragma unroll
-            for (int d = 0; d < DEPTH; ++d) {
-                const int s = s0 + d;
-                if (s >= steps || !ok) break;
-                const int st = s % STAGES;
-                if (s >= STAGES) {
-                    ok = mbar_wait(empty0 + 8 * st, (uint32_t)((s / STAGES - 1) & 1), give_up, 1);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
-                }
-#pragma unroll
-                for (int i = 0; i < CHUNKS; ++i) {
-                    if (i >= 4 && row + 32 * (i - 4) >= NT) continue;
-                    const float4 a = v[d][i];
-                    const float4 h = make_float4(first_half(a.x), first_half(a.y), first_half(a.z), first_half(a.w));
-                    const float4 l = make_float4(second_half(a.x, h.x), second_half(a.y, h.y), second_half(a.z, h.z), second_half(a.w, h.w));
-                    const uint32_t to = at + st * T::STAGE_BYTES + (i < 4 ? i * 4096 : 2 * T::W_BYTES + (i - 4) * 4096);
-                    const uint32_t to_lo = to + (i < 4 ? T::W_BYTES : T::X_BYTES);
-                    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" :: "r"(to), "f"(h.x), "f"(h.y), "f"(h.z), "f"(h.w) : "memory");
-                    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" :: "r"(to_lo), "f"(l.x), "f"(l.y), "f"(l.z), "f"(l.w) : "memory");
-                }
-                fetch(d, 0, CHUNKS, s + DEPTH);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(full0 + 8 * st);
-                if (s > 0) issue(s - 1);
-            }
-        }
-        if (ok && steps > 0) issue(steps - 1);
-    } else {
-        // ================= adders
-        bl_pdl_wait();
-        bl_pdl_trigger();
-        const uint32_t t_at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * T::COLS;
-        if (warp < 4 * T::HALVES) {
-            float acc[T::COLS];                                            // row 32 (warp & 3) + lane of the tile, COLS of its columns
-#pragma unroll
-            for (int j = 0; j < T::COLS; ++j) acc[j] = 0.f;
-            for (int s = 0; ok && s < steps; ++s) {
-                const int b = s & 1;
-                ok = mbar_wait(sum0 + 8 * b, (uint32_t)((s >> 1) & 1), give_up, 3);
+            if (s >= PAIRS) {
+                ok = mbar_wait(empty0 + 8 * st, (uint32_t)((s / PAIRS - 1) & 1), give_up, 1);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                fence_after_sync();
-#pragma unroll
-                for (int c = 0; c < T::COLS; c += 16) {
-                    uint32_t r[16];
-                    tmem_ld16(t_at + b * 128 + c, r);
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) acc[c + j] += __uint_as_float(r[j]);
-                }
-                fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(taken0 + 8 * b);
             }
-            // the last segment's MMAs have read the operand tiles, which make room for the sums
 #pragma unroll
-            for (int j = 0; j < T::COLS; ++j) sums[((warp >> 2) * T::COLS + j) * BM + (warp & 3) * 32 + lane] = acc[j];
+            for (int i = 0; i < T::CHUNKS; ++i) {
+                if (i >= 4 && row + 32 * (i - 4) >= NT) continue;
+                const float4 a = v[i];
+                const float4 h = make_float4(first_half(a.x), first_half(a.y), first_half(a.z), first_half(a.w));
+                const float4 l = make_float4(second_half(a.x, h.x), second_half(a.y, h.y), second_half(a.z, h.z), second_half(a.w, h.w));
+                const uint32_t at = to + st * T::PAIR_BYTES + (i < 4 ? i * 4096 : 2 * T::W_BYTES + (i - 4) * 4096);
+                const uint32_t at_lo = at + (i < 4 ? T::W_BYTES : T::X_BYTES);
+                asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" :: "r"(at), "f"(h.x), "f"(h.y), "f"(h.z), "f"(h.w) : "memory");
+                asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" :: "r"(at_lo), "f"(l.x), "f"(l.y), "f"(l.z), "f"(l.w) : "memory");
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) { mbar_arrive(full0 + 8 * st); mbar_arrive(raw_read0 + 8 * rs); }
+            if (warp == 8) {                                               // the segment's MMAs
+                ok = mbar_wait(full0 + 8 * st, (uint32_t)((s / PAIRS) & 1), give_up, 2);
+                if (ok && s >= 2) ok = mbar_wait(taken0 + 8 * b, (uint32_t)((s / 2 - 1) & 1), give_up, 2);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                if (elect_one()) {
+                    fence_after_sync();
+                    const uint32_t stage = base + st * T::PAIR_BYTES, d = tmem + b * 128;
+                    const uint64_t wh = smem_desc(stage), wl = smem_desc(stage + T::W_BYTES);
+                    const uint64_t xh = smem_desc(stage + 2 * T::W_BYTES), xl = smem_desc(stage + 2 * T::W_BYTES + T::X_BYTES);
+#pragma unroll
+                    for (int k = 0; k < BK / 8; ++k) {                     // the small products first
+                        umma_tf32(d, wl + 2 * k, xh + 2 * k, IDESC, k != 0);
+                        umma_tf32(d, wh + 2 * k, xl + 2 * k, IDESC, 1);
+                    }
+#pragma unroll
+                    for (int k = 0; k < BK / 8; ++k) umma_tf32(d, wh + 2 * k, xh + 2 * k, IDESC, 1);
+                    umma_commit(empty0 + 8 * st);
+                    umma_commit(sum0 + 8 * b);
+                }
+                __syncwarp();
+            }
+            if (warp == 9 && s + RAWS < steps) {                           // the ring's stage takes the segment RAWS on
+                ok = mbar_wait(raw_read0 + 8 * rs, (uint32_t)((s / RAWS) & 1), give_up, 1);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                if (elect_one()) { load_w(s + RAWS); load_x(s + RAWS); }
+                __syncwarp();
+                issued = s + RAWS + 1;
+            }
         }
+        if (warp == 9 && *give_up)                                         // let our own copies land before leaving
+            for (int s = max(0, issued - RAWS); s < issued; ++s) mbar_wait_plain(raw_full0 + 8 * (s % RAWS), (uint32_t)((s / RAWS) & 1));
+    } else if (warp < 4 * T::HALVES) {
+        // ================= adders: row 32 (warp & 3) + lane of the tile, COLS of its columns
+        const uint32_t t_at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * T::COLS;
+        float acc[T::COLS];
+#pragma unroll
+        for (int j = 0; j < T::COLS; ++j) acc[j] = 0.f;
+        for (int s = 0; s < steps; ++s) {
+            const int b = s & 1;
+            ok = mbar_wait(sum0 + 8 * b, (uint32_t)((s >> 1) & 1), give_up, 3);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            fence_after_sync();
+#pragma unroll
+            for (int c = 0; c < T::COLS; c += 16) {
+                uint32_t r[16];
+                tmem_ld16(t_at + b * 128 + c, r);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) acc[c + j] += __uint_as_float(r[j]);
+            }
+            fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(taken0 + 8 * b);
+        }
+        // the last segment's MMAs have read the halves, which make room for the sums
+#pragma unroll
+        for (int j = 0; j < T::COLS; ++j) sums[((warp >> 2) * T::COLS + j) * BM + (warp & 3) * 32 + lane] = acc[j];
     }
     if (spans > 1) cluster_sync(); else __syncthreads();
     const BlGluArgs glu = bl_glu_args(GLU ? bias : nullptr);
@@ -251,17 +270,17 @@ gemm_f32_tc_kernel(const float* __restrict__ x, const float* __restrict__ w, con
         const int u = e % UNITS, col = e / UNITS;
         const int m = m0 + col, n = n0 + u;
         if (m >= M || n >= N) continue;
-        const uint32_t mine = base + (uint32_t)(col * BM + (GLU ? (u >> 4) * 32 + (u & 15) : u)) * 4;
+        const uint32_t mine = base + (uint32_t)(col * BM + u) * 4;       // (the up sums of a gated tile are its rows 64 on)
         float s = 0.f, up = 0.f;
         if (spans == 1) {
             s = *reinterpret_cast<const float*>(smem + (mine - base));
-            if (GLU) up = *reinterpret_cast<const float*>(smem + (mine - base) + 64);
+            if (GLU) up = *reinterpret_cast<const float*>(smem + (mine - base) + 4 * UNITS);
         } else {
             for (int r = 0; r < spans; ++r) {                              // ascending k
                 uint32_t peer;
                 asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(mine), "r"(r));
                 s = r == 0 ? ld_cluster(peer) : s + ld_cluster(peer);
-                if (GLU) up = r == 0 ? ld_cluster(peer + 64) : up + ld_cluster(peer + 64);
+                if (GLU) up = r == 0 ? ld_cluster(peer + 4 * UNITS) : up + ld_cluster(peer + 4 * UNITS);
             }
         }
         if (!isfinite(s)) s = plain_dot(x + (size_t)m * ldx, w + (size_t)n * K, K);
@@ -294,6 +313,20 @@ int device_sms() {
     return sms;
 }
 
+// A row-major matrix of 32-bit numbers, rows `ld` apart, as a tensor map with boxes of box_rows rows of BK values as they lie.
+int make_map(CUtensorMap* map, const float* p, long long rows, long long cols, long long ld, int box_rows) {
+    BlEncodeTiled enc = bl_tensor_map_encoder();
+    if (enc == nullptr) BL_FAIL("bl_gemm_f32_tc: cuTensorMapEncodeTiled is not available from the driver");
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+    cuuint32_t box[2] = {BK, (cuuint32_t)box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) BL_FAIL("bl_gemm_f32_tc: cuTensorMapEncodeTiled failed with code %d (rows %lld, columns %lld)", (int)r, rows, cols);
+    return 0;
+}
+
 template <int EPI, int NT>
 int launch(const float* x, const float* w, const void* bias, int bias_dtype, float* out, int M, int N, int K, int ldx, int spans, cudaStream_t s) {
     static std::atomic<bool> allowed{false};
@@ -303,13 +336,16 @@ int launch(const float* x, const float* w, const void* bias, int bias_dtype, flo
     }
     const int units = EPI == BL_EPI_SWIGLU ? BM / 2 : BM;
     const int m_tiles = (M + NT - 1) / NT;
+    CUtensorMap mx, mw;
+    if (make_map(&mx, x, M, K, ldx, NT)) return 1;
+    if (make_map(&mw, w, EPI == BL_EPI_SWIGLU ? 2LL * N : N, K, K, units)) return 1;
     const dim3 grid((unsigned)((long long)((N + units - 1) / units) * m_tiles * spans));
     if (spans > 1) {
         BL_CUDA(bl_launch_dependent_clusters(gemm_f32_tc_kernel<EPI, NT>, grid, dim3(THREADS), (size_t)Tile<NT>::SMEM_BYTES, s, (unsigned)spans,
-                                             x, w, bias, bias_dtype, out, M, N, K, ldx, spans, m_tiles));
+                                             mx, mw, x, w, bias, bias_dtype, out, M, N, K, ldx, spans, m_tiles));
     } else {
         BL_CUDA(bl_launch_dependent(gemm_f32_tc_kernel<EPI, NT>, grid, dim3(THREADS), (size_t)Tile<NT>::SMEM_BYTES, s,
-                                    x, w, bias, bias_dtype, out, M, N, K, ldx, spans, m_tiles));
+                                    mx, mw, x, w, bias, bias_dtype, out, M, N, K, ldx, spans, m_tiles));
     }
     BL_CHECK_LAUNCH("bl_gemm_f32_tc");
     return 0;
@@ -317,8 +353,8 @@ int launch(const float* x, const float* w, const void* bias, int bias_dtype, flo
 
 template <int EPI>
 int launch_width(const float* x, const float* w, const void* bias, int bias_dtype, float* out, int M, int N, int K, int ldx, int spans, cudaStream_t s) {
-    // The width of a tile: the least of rounds of blocks times a segment's cycles of the shared-memory port (16 KB and NT rows
-    // stored twice, 12 MMAs that read 128 and NT rows of 32 bytes).
+    // The width of a tile: the least of rounds of blocks times a segment's cycles (linear in the rows of W and x that pass through
+    // shared memory).
     const int units = EPI == BL_EPI_SWIGLU ? BM / 2 : BM;
     const long long n_tiles = (N + units - 1) / units;
     const int slots = spans > 1 ? device_sms() / spans - (spans > 2 ? 1 : 0) : device_sms();       // tiles under way at once
@@ -349,8 +385,12 @@ int f32_tc_spans(int N, int K, int epi) {
 
 }  // namespace
 
-// Whether the tensor cores take a product of these sizes (rows of whole 16-byte pieces): by N and K alone, see above.
-extern "C" int bl_gemm_f32_tc_supported(int N, int K, int ldx) { return N >= 128 && K >= 256 && K % 4 == 0 && ldx % 4 == 0; }
+// Whether the tensor cores take a product of these sizes (rows of whole 16-byte pieces): by N and K alone, see above. Products of
+// more columns are output heads: mostly a row or a few of them, which FMAs stream faster than W can be split (151,936 x 896: one
+// row 104 us against 208, 16 rows 150 and 210, 33 rows 448 and 265).
+extern "C" int bl_gemm_f32_tc_supported(int N, int K, int ldx) {
+    return N >= 128 && N <= MAX_COLUMNS && K >= 256 && K % 4 == 0 && ldx % 4 == 0;
+}
 
 extern "C" int bl_gemm_f32_tc(const float* x, int ldx, const float* w, const void* bias, int bias_dtype, float* out, int M, int N, int K,
                               int epilogue, void* stream) {

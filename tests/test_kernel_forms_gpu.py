@@ -585,7 +585,7 @@ def test_attention_over_keys_made_of_latents(H, own, rot, dv, rank, window, gate
             close(out[t, h * dv:(h + 1) * dv], want, BF, f"request {r} head {h}")
 
 
-@pytest.mark.parametrize("N,K", [(128, 256), (130, 260), (896, 896), (1152, 900), (4160, 512), (896, 4864)])
+@pytest.mark.parametrize("N,K", [(128, 256), (130, 260), (896, 896), (1152, 900), (4160, 512), (896, 4864), (32772, 256)])
 @pytest.mark.parametrize("M", [1, 16, 33, 97, 366])
 def test_32_bit_product_on_tensor_cores(M, N, K):
     """Spans of K and none, widths of 16 to 128 rows, remainders of rows, columns and segments, every epilogue: no further from 64
