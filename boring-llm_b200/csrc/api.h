@@ -228,6 +228,18 @@ int bl_attention_decode_tma_cap(const void* q, const void* k_cache, const void* 
                                 int n_splits, void* out, int H, int KV, int dh, int page_size, int window, float scale,
                                 int early, const void* sinks, int sink_dtype, const float* gate, int ld_gate, int gate_dim, float softcap,
                                 void* stream);
+// A step's prompts and its single tokens side by side: bl_attention_decode_tma_started directly behind a bl_attention_prefill_tc_started
+// with the same word (0 before) starts on the kernels before that one and ends after it; the word is 0 again then.
+int bl_attention_prefill_tc_started(const void* q, const void* k_cache, const void* v_cache, const int* cu_q,
+                                    const int* ctx_len, const int* block_table, int max_pages, const int* tiles, int n_tiles,
+                                    void* out, int T, int n_pages, int H, int KV, int dh, int page_size, int window, float scale,
+                                    const void* sinks, int sink_dtype, const float* gate, int ld_gate, int gate_dim, float softcap,
+                                    int* started, void* stream);
+int bl_attention_decode_tma_started(const void* q, const void* k_cache, const void* v_cache, int n_pages, const int* cu_q,
+                                    const int* ctx_len, const int* block_table, int max_pages, const int* reqs, int n,
+                                    int n_splits, void* out, int H, int KV, int dh, int page_size, int window, float scale,
+                                    int early, const void* sinks, int sink_dtype, const float* gate, int ld_gate, int gate_dim, float softcap,
+                                    int* started, void* stream);
 int bl_attention_decode_cap(const void* q, const void* k_cache, const void* v_cache, const int* cu_q,
                             const int* ctx_len, const int* block_table, int max_pages, const int* reqs, int n,
                             int n_splits, float* scratch, int* counters, void* out, int H, int KV, int dh, int page_size,

@@ -34,6 +34,7 @@
 // Every wait on an mbarrier is bounded. When a bound runs out the warp records a code in a status word, waits
 // (bounded again) for the copies it has in flight, and goes on to the barriers that its cluster expects of it; the
 // host reads the status word (bl_attention_decode_tma_status) and discards the launch.
+#include <type_traits>
 #include "tcgen05.cuh"
 
 namespace {
@@ -76,6 +77,7 @@ struct Params {
     int H, KV, window; float scale_log2;
     BlAttnTail tail;              // a sink per head and a gate per (token, head), or nulls
     float cap_log2;               // > 0: a cap c on the scaled scores, s <- c tanh(s / c), here times log2 e (0: none)
+    int* started;                 // null, or the word of the prefill attention in front of this launch (see the wait)
 };
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
@@ -247,7 +249,7 @@ __device__ __forceinline__ void unit_step(uint32_t stage, const uint32_t (&koff)
     }
 }
 
-template <int DH, int NH, bool CAP = false>
+template <int DH, int NH, bool CAP = false, bool SIDE = false>
 __global__ void __launch_bounds__(THREADS)
 attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const Params p) {
     using S = Shape<DH>;
@@ -322,7 +324,22 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         koff[j] = (uint32_t)((ri + 8 * (mi & 1)) * 128 + (((2 * j + (mi >> 1)) ^ ri) << 4));   // keys: rows 0-7 / 8-15, then the next 8 dimensions
         voff[j] = (uint32_t)((ri + 8 * (mi >> 1)) * 128 + (((2 * j + (mi & 1)) ^ ri) << 4));   // values: 8 dimensions on, then keys 8-15
     }
-    bl_pdl_wait();                                                // q and the newest key and value come from the kernel before
+    // q and the newest key and value come from the kernel before. SIDE: in a step of prompts beside single tokens that is not the kernel
+    // directly in front, the prefill attention, whose results this one does not read: that one sets `started` once it has seen the end
+    // of the kernel before it, and lets this one start behind that. Read as 1 with acquire semantics, q and the rows are there (for the
+    // copy engine, too, behind the proxy fence) and the two run side by side; read as anything else, the wait is the ordinary one.
+    // The launch then waits for the prefill attention at its END, so that whoever waits for this launch has both. 512 tokens of a prompt
+    // beside 63 contexts of 2,000 tokens (0.5B sizes): 17 and 14 us a layer one behind the other, the step 2,080 -> 1,921 us. (A build
+    // of its own: asking for the word in every launch cost a decode step of eight requests 0.2 us a layer.)
+    int before_done = 0;
+    if constexpr (SIDE) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(before_done) : "l"(p.started) : "memory");
+    if (before_done == 1) asm volatile("fence.proxy.async;" ::: "memory");
+    else bl_pdl_wait();
+    auto leave = [&]() {
+        if constexpr (!SIDE) return;
+        bl_pdl_wait();
+        if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) *p.started = 0;      // (blocks that have not looked yet wait)
+    };
     while (issued < S::STAGES && issued < n_mine) {
         issue(issued, tab);
         ++issued;
@@ -438,7 +455,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
             }
         }
     }
-    if (n_splits == 1) return;
+    if (n_splits == 1) { leave(); return; }
     // ---- the slices' partial results of the rows this block owns --------------------------------------------
     if (rows_owned > 0 && q_len > 0 && wait_bounded<true>(recv_bar, 0u, 3)) {
         const float* rv = reinterpret_cast<const float*>(gen + S::OFF_RECV);
@@ -463,17 +480,18 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         }
     }
     cluster_sync_all();                                           // nobody leaves while a store to its shared memory may be in flight
+    leave();
 }
 
-template <int DH, int NH, bool CAP = false>
+template <int DH, int NH, bool CAP = false, bool SIDE = false>
 int configure(int* smem_bytes) {
     static bool done = false;
     *smem_bytes = Shape<DH>::SMEM_BYTES;
     if (!done) {
-        BL_CUDA(cudaFuncSetAttribute(attention_decode_kernel<DH, NH, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<DH>::SMEM_BYTES));
-        BL_CUDA(bl_same_carveout(attention_decode_kernel<DH, NH, CAP>));
+        BL_CUDA(cudaFuncSetAttribute(attention_decode_kernel<DH, NH, CAP, SIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<DH>::SMEM_BYTES));
+        BL_CUDA(bl_same_carveout(attention_decode_kernel<DH, NH, CAP, SIDE>));
         // clusters of more than 8 blocks need the kernel's consent; a device that refuses it keeps 8
-        if (cudaFuncSetAttribute(attention_decode_kernel<DH, NH, CAP>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+        if (cudaFuncSetAttribute(attention_decode_kernel<DH, NH, CAP, SIDE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
             (void)cudaGetLastError();
         done = true;
     }
@@ -484,10 +502,10 @@ int configure(int* smem_bytes) {
 // its copies of the cached keys and values under the predecessor's tail. Large clusters of a launch with more blocks
 // than SMs are better launched late: placed while the predecessor's blocks still hold SMs, they pile up two to an SM
 // beside SMs that stay empty, and a long context then runs at the pace of the doubly loaded SMs.
-template <int DH, int NH, bool CAP = false>
+template <int DH, int NH, bool CAP = false, bool SIDE = false>
 int launch(const CUtensorMap& mk, const CUtensorMap& mv, const Params& p, dim3 grid, bool early, cudaStream_t s) {
     int bytes = 0;
-    if (configure<DH, NH, CAP>(&bytes)) return 1;
+    if (configure<DH, NH, CAP, SIDE>(&bytes)) return 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = (size_t)bytes; cfg.stream = s;
     cudaLaunchAttribute attr[2];
@@ -496,7 +514,7 @@ int launch(const CUtensorMap& mk, const CUtensorMap& mv, const Params& p, dim3 g
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = p.n_splits; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = p.n_splits > 1 ? 2 : 1;
-    BL_CUDA(cudaLaunchKernelEx(&cfg, attention_decode_kernel<DH, NH, CAP>, mk, mv, p));
+    BL_CUDA(cudaLaunchKernelEx(&cfg, attention_decode_kernel<DH, NH, CAP, SIDE>, mk, mv, p));
     BL_CHECK_LAUNCH(WHO);
     return 0;
 }
@@ -574,6 +592,16 @@ extern "C" int bl_attention_decode_tma_cap(const void* q, const void* k_cache, c
                                            int n_splits, void* out, int H, int KV, int dh, int page_size, int window,
                                            float scale, int early, const void* sinks, int sink_dtype, const float* gate,
                                            int ld_gate, int gate_dim, float softcap, void* stream) {
+    return bl_attention_decode_tma_started(q, k_cache, v_cache, n_pages, cu_q, ctx_len, block_table, max_pages, reqs, n, n_splits, out, H, KV,
+                                           dh, page_size, window, scale, early, sinks, sink_dtype, gate, ld_gate, gate_dim, softcap, nullptr, stream);
+}
+
+// ... directly behind a bl_attention_prefill_tc_started with the same word `started`.
+extern "C" int bl_attention_decode_tma_started(const void* q, const void* k_cache, const void* v_cache, int n_pages, const int* cu_q,
+                                               const int* ctx_len, const int* block_table, int max_pages, const int* reqs, int n,
+                                               int n_splits, void* out, int H, int KV, int dh, int page_size, int window,
+                                               float scale, int early, const void* sinks, int sink_dtype, const float* gate,
+                                               int ld_gate, int gate_dim, float softcap, int* started, void* stream) {
     if (n <= 0) return 0;
     if (!(softcap >= 0.f)) BL_FAIL("%s: a cap on the scores must not be negative, got %g", WHO, (double)softcap);
     if (!(scale > 0.f)) BL_FAIL("%s: the scale of the scores must be positive (got %g)", WHO, (double)scale);
@@ -589,6 +617,7 @@ extern "C" int bl_attention_decode_tma_cap(const void* q, const void* k_cache, c
     p.tail = BlAttnTail{sinks, sink_dtype, gate, ld_gate, gate_dim};
     if (!bl_channel_gate_ok(gate, ld_gate, gate_dim, H, dh)) BL_FAIL("%s: a gate of %d channels a head in rows of %d does not fit %d heads of %d in 16-byte pieces", WHO, gate_dim, ld_gate, H, dh);
     p.cap_log2 = softcap * 1.4426950408889634f;
+    p.started = started;
     CUtensorMap mk, mv;
     if (bl_make_map_bf16(WHO, &mk, k_cache, (long long)n_pages * KV * PAGE, dh, PAGE, 64)) return 1;
     if (bl_make_map_bf16(WHO, &mv, v_cache, (long long)n_pages * KV * PAGE, dh, PAGE, 64)) return 1;
@@ -596,12 +625,16 @@ extern "C" int bl_attention_decode_tma_cap(const void* q, const void* k_cache, c
     const bool two = G > 8;
     const dim3 grid(n_splits, KV * ((G + (two ? 16 : 8) - 1) / (two ? 16 : 8)), n);
     cudaStream_t s = (cudaStream_t)stream;
-    if (softcap > 0.f) {                                          // a second build of the kernel: without a cap it is the code it was
-        if (dh == 64) return two ? launch<64, 2, true>(mk, mv, p, grid, early != 0, s) : launch<64, 1, true>(mk, mv, p, grid, early != 0, s);
-        return two ? launch<128, 2, true>(mk, mv, p, grid, early != 0, s) : launch<128, 1, true>(mk, mv, p, grid, early != 0, s);
-    }
-    if (dh == 64) return two ? launch<64, 2>(mk, mv, p, grid, early != 0, s) : launch<64, 1>(mk, mv, p, grid, early != 0, s);
-    return two ? launch<128, 2>(mk, mv, p, grid, early != 0, s) : launch<128, 1>(mk, mv, p, grid, early != 0, s);
+    // builds of their own for a cap and for a launch beside the prefill attention: without them it is the code it was
+    auto run = [&](auto cap, auto side) {
+        constexpr bool C = decltype(cap)::value, B = decltype(side)::value;
+        if (dh == 64) return two ? launch<64, 2, C, B>(mk, mv, p, grid, early != 0, s) : launch<64, 1, C, B>(mk, mv, p, grid, early != 0, s);
+        return two ? launch<128, 2, C, B>(mk, mv, p, grid, early != 0, s) : launch<128, 1, C, B>(mk, mv, p, grid, early != 0, s);
+    };
+    const std::true_type yes;
+    const std::false_type no;
+    if (started != nullptr) return softcap > 0.f ? run(yes, yes) : run(no, yes);
+    return softcap > 0.f ? run(yes, no) : run(no, no);
 }
 
 // Reads and clears the status word: 0 when no warp has given up on a wait since the last call. 1: a stage's keys

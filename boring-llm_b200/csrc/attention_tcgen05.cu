@@ -84,6 +84,7 @@ struct Params {
     int H, KV, window; float scale_log2;
     BlAttnTail tail;                   // a sink per head and a gate per (token, head), or nulls
     float cap_log2;                    // the kernel with a cap on the scores: the cap times log2 e (s <- cap tanh(s / cap) on the scaled score)
+    int* started;                      // null, or a word that says to the next kernel that the one before this has finished
     const int* key_row;                // keys in matrices: the row of a request's key 0 (its key j is row key_row[r] + j)
 };
 
@@ -262,6 +263,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // q, the newest keys and values and the output buffer belong to the kernels before this one until here; the block's
     // preamble above may run while they finish
     bl_pdl_wait();
+    if (p.started != nullptr && blockIdx.x == 0) {                       // (see attention_decode.cu: that kernel need not wait for this one then)
+        if (threadIdx.x == 0) asm volatile("st.release.gpu.global.s32 [%0], 1;" :: "l"(p.started) : "memory");
+        __syncthreads();
+    }
     bl_pdl_trigger();                                                    // the next kernel may start its own preamble (it waits before it touches data)
     // tensor memory: scores of block i in columns 128 (i % 3) .., its P over the upper 64 of them, its share of the
     // output in columns 384 + 64 (i & 1) .. (head size 128: 384 ..)
@@ -763,6 +768,17 @@ extern "C" int bl_attention_prefill_tc_cap(const void* q, const void* k_cache, c
                                            int n_tiles, void* out, int T, int n_pages, int H, int KV, int dh, int page_size,
                                            int window, float scale, const void* sinks, int sink_dtype, const float* gate,
                                            int ld_gate, int gate_dim, float softcap, void* stream) {
+    return bl_attention_prefill_tc_started(q, k_cache, v_cache, cu_q, ctx_len, block_table, max_pages, tiles, n_tiles, out, T, n_pages, H, KV,
+                                           dh, page_size, window, scale, sinks, sink_dtype, gate, ld_gate, gate_dim, softcap, nullptr, stream);
+}
+
+// ... and a word `started` (0 before the launch; null: none) that becomes 1 when the kernel before this one has finished, for a
+// bl_attention_decode_tma_started that follows directly.
+extern "C" int bl_attention_prefill_tc_started(const void* q, const void* k_cache, const void* v_cache, const int* cu_q,
+                                               const int* ctx_len, const int* block_table, int max_pages, const int* tiles,
+                                               int n_tiles, void* out, int T, int n_pages, int H, int KV, int dh, int page_size,
+                                               int window, float scale, const void* sinks, int sink_dtype, const float* gate,
+                                               int ld_gate, int gate_dim, float softcap, int* started, void* stream) {
     if (n_tiles <= 0) return 0;
     if (!(softcap >= 0.f)) BL_FAIL("bl_attention_prefill_tc: a cap on the scores must not be negative, got %g", (double)softcap);
     if ((dh != 64 && dh != 128) || page_size != PAGE)
@@ -779,6 +795,7 @@ extern "C" int bl_attention_prefill_tc_cap(const void* q, const void* k_cache, c
     p.tail = BlAttnTail{sinks, sink_dtype, gate, ld_gate, gate_dim};
     if (!bl_channel_gate_ok(gate, ld_gate, gate_dim, H, dh)) BL_FAIL("%s: a gate of %d channels a head in rows of %d does not fit %d heads of %d in 16-byte pieces", "bl_attention_prefill_tc", gate_dim, ld_gate, H, dh);
     p.cap_log2 = softcap * 1.4426950408889634f;
+    p.started = started;
     if (softcap > 0.f) {
         if (dh == 64) return launch<Shape<64, 2>, true>(q, k_cache, v_cache, p, n_tiles, T, n_pages, (cudaStream_t)stream);
         return launch<Shape<128, 1>, true>(q, k_cache, v_cache, p, n_tiles, T, n_pages, (cudaStream_t)stream);

@@ -379,8 +379,9 @@ def attention_prefill_tc_supported(dtype: torch.dtype, dh: int, page_size: int) 
 
 def attention_prefill_tc(q, k_cache, v_cache, cu_q, ctx_len, block_table, tiles, out, H: int, window: int,
                          scale: float, sinks: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None,
-                         softcap: float = 0.0, gate_dim: int = 0) -> None:
-    """The tcgen05 form of `attention_prefill` (head size 64, pages of 16). tiles: int32 [n, 2] = (request,
+                         softcap: float = 0.0, gate_dim: int = 0, started: Optional[torch.Tensor] = None) -> None:
+    """The tcgen05 form of `attention_prefill` (head size 64, pages of 16). `started`: a word (int32, 0 before) for an
+    `attention_decode_tma` that follows directly with the same one and runs beside this launch. tiles: int32 [n, 2] = (request,
     first token of a tile of 128 among the request's new tokens); the last entries are launched first. `softcap` c > 0:
     scaled scores pass c tanh(s / c) (a second build of the kernel; without a cap the kernel is the one it was)."""
     T = q.shape[0]
@@ -389,7 +390,12 @@ def attention_prefill_tc(q, k_cache, v_cache, cu_q, ctx_len, block_table, tiles,
     _need(v_cache, "v_cache", torch.bfloat16, k_cache.shape); _need(out, "out", torch.bfloat16, (T, H * dh))
     _need(cu_q, "cu_q", torch.int32); _need(ctx_len, "ctx_len", torch.int32); _need(block_table, "block_table", torch.int32)
     _need(tiles, "tiles", torch.int32, (tiles.shape[0], 2))
-    if softcap > 0 or gate_dim:
+    if started is not None:
+        _need(started, "started", torch.int32, (1,))
+        _call(_lib().bl_attention_prefill_tc_started, _p(q), _p(k_cache), _p(v_cache), _p(cu_q), _p(ctx_len), _p(block_table),
+          block_table.shape[1], _p(tiles), tiles.shape[0], _p(out), T, n_pages, H, KV, dh, page_size, window,
+          ctypes.c_float(scale), *_tail(T, H, sinks, gate, gate_dim), gate_dim, ctypes.c_float(softcap), _p(started), _stream())
+    elif softcap > 0 or gate_dim:
         _call(_lib().bl_attention_prefill_tc_cap, _p(q), _p(k_cache), _p(v_cache), _p(cu_q), _p(ctx_len), _p(block_table),
           block_table.shape[1], _p(tiles), tiles.shape[0], _p(out), T, n_pages, H, KV, dh, page_size, window,
           ctypes.c_float(scale), *_tail(T, H, sinks, gate, gate_dim), gate_dim, ctypes.c_float(softcap), _stream())
@@ -458,7 +464,7 @@ def attention_decode_tma_supported(dtype: torch.dtype, dh: int, page_size: int) 
 
 def attention_decode_tma(q, k_cache, v_cache, cu_q, ctx_len, block_table, reqs, n_splits: int, out, H: int, window: int,
                          scale: float, sinks: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None,
-                         softcap: float = 0.0, gate_dim: int = 0) -> None:
+                         softcap: float = 0.0, gate_dim: int = 0, started: Optional[torch.Tensor] = None) -> None:
     """`attention_decode` for head sizes 64 and 128 with keys and values streamed by TMA into per-warp rings and the
     query heads of a key/value head as the columns of the MMAs; 1 to `DECODE_CLUSTER_SPLITS` slices, which are the
     blocks of one cluster and send their partial rows to the blocks that finish them."""
@@ -475,7 +481,12 @@ def attention_decode_tma(q, k_cache, v_cache, cu_q, ctx_len, block_table, reqs, 
     G = H // KV
     blocks = n * KV * (-(-G // (8 if G <= 8 else 16))) * n_splits
     early = not (n_splits >= DECODE_TMA_LATE_CLUSTER and blocks > _sms())
-    if softcap > 0 or gate_dim:              # (a cap on the scaled scores: a second build of the kernel)
+    if started is not None:                  # beside the prefill attention that was launched directly before (see there)
+        _need(started, "started", torch.int32, (1,))
+        _call(_lib().bl_attention_decode_tma_started, _p(q), _p(k_cache), _p(v_cache), n_pages, _p(cu_q), _p(ctx_len), _p(block_table),
+          block_table.shape[1], _p(reqs), n, n_splits, _p(out), H, KV, dh, page_size, window, ctypes.c_float(scale),
+          1, *_tail(T, H, sinks, gate, gate_dim), gate_dim, ctypes.c_float(softcap), _p(started), _stream())
+    elif softcap > 0 or gate_dim:            # (a cap on the scaled scores: a second build of the kernel)
         _call(_lib().bl_attention_decode_tma_cap, _p(q), _p(k_cache), _p(v_cache), n_pages, _p(cu_q), _p(ctx_len), _p(block_table),
           block_table.shape[1], _p(reqs), n, n_splits, _p(out), H, KV, dh, page_size, window, ctypes.c_float(scale),
           1 if early else 0, *_tail(T, H, sinks, gate, gate_dim), gate_dim, ctypes.c_float(softcap), _stream())

@@ -87,10 +87,17 @@ def paged_attention(ctx, q, k_cache, v_cache, table, out, H: int, KV: int, dh: i
         plan.arrays = {k: torch.from_numpy(v).to(ctx.device) for k, v in plan.arrays.items()}
         ctx.plans[PLAN_KEY] = plan
     tiles64, tiles128, singles = plan.arrays["tiles64"], plan.arrays["tiles128"], plan.arrays["singles"]
+    started = None
+    if (tiles128.shape[0] and singles.shape[0] and ops.attention_prefill_tc_supported(q.dtype, dh, k_cache.shape[2])
+            and ops.attention_decode_tma_supported(q.dtype, dh, k_cache.shape[2])):
+        # prompts and single tokens: the two launches run side by side, through a word that is 0 between them
+        started = ctx.memo.get("attention started")
+        if started is None:
+            started = ctx.memo["attention started"] = torch.zeros(1, dtype=torch.int32, device=ctx.device)
     if tiles64.shape[0]:
         if tiles128.shape[0] and ops.attention_prefill_tc_supported(q.dtype, dh, k_cache.shape[2]):
             ops.attention_prefill_tc(q, k_cache, v_cache, ctx.cu_q, ctx.ctx_len, table, tiles128, out, H, window, scale, sinks, gate,
-                                     softcap=softcap, gate_dim=gate_dim)
+                                     softcap=softcap, gate_dim=gate_dim, started=started)
         else:
             ops.attention_prefill(q, k_cache, v_cache, ctx.cu_q, ctx.ctx_len, table, tiles64, out, H, window, scale, sinks, gate,
                                   softcap=softcap, gate_dim=gate_dim)
@@ -105,7 +112,7 @@ def paged_attention(ctx, q, k_cache, v_cache, table, out, H: int, KV: int, dh: i
             # head sizes 64 and 128: the TMA-fed kernel, which knows how many slices pay for this many requests
             n_splits = ops.attention_decode_tma_splits(n, KV, G, dh, longest)
             ops.attention_decode_tma(q, k_cache, v_cache, ctx.cu_q, ctx.ctx_len, table, singles, n_splits, out, H, window, scale,
-                                     sinks, gate, softcap=softcap, gate_dim=gate_dim)
+                                     sinks, gate, softcap=softcap, gate_dim=gate_dim, started=started)
             return
         groups = KV * (-(-G // 16))
         resident = ops.attention_decode_resident_blocks(dh)

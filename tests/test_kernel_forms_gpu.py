@@ -851,3 +851,43 @@ def test_few_rows_go_by_the_bytes_of_w():
         assert o.gemm_kernel(m(M, K), m(2 * N if epi == o.EPI_SWIGLU else N, K), N, b, epi) == kind, (M, N, K)
     x, w = m(8, 11008), m(2048, 11008)
     assert o.gemm_kernel(x, w, 2048, None, o.EPI_RESIDUAL) == "few" and o.gemm_skinny_links_norm(x, w, 2048, o.EPI_RESIDUAL)
+
+
+@pytest.mark.parametrize("H,KV,dh,window", [(14, 2, 64, 0), (4, 4, 64, 100), (16, 2, 128, 0)])
+def test_prompts_and_single_tokens_side_by_side(H, KV, dh, window):
+    """The two attention launches of a mixed step with the word between them against the same without it, bit for bit, kernel by
+    kernel and replayed from a graph in which the queries are written before and the results read behind them, layer after layer."""
+    o = ops()
+    ctx_lens, q_lens = [700, 90, 3000, 1, 513, 257, 64], [700, 1, 1, 1, 130, 1, 1]
+    s = paged_setup(ctx_lens, q_lens, KV, dh, 16, BF, 5)
+    s["kc"], s["vc"] = data(s["kc"].shape, 1).to(BF), data(s["vc"].shape, 2).to(BF)
+    T = s["T"]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    tiles = i32([[r, t] for r, n in enumerate(q_lens) if n > 1 for t in range(0, n, 128)])
+    singles = i32([r for r, n in enumerate(q_lens) if n == 1])
+    src = [data((T, H * dh), 3 + i) for i in range(3)]
+    word = torch.zeros(1, dtype=torch.int32, device=DEV)
+    splits = o.attention_decode_tma_splits(singles.shape[0], KV, H // KV, dh, 3000)
+
+    def layers(started):
+        outs, q = [], torch.empty(T, H * dh, dtype=BF, device=DEV)
+        for i in range(6):
+            o.cast_rows(src[i % 3], q)
+            out = torch.full((T, H * dh), float("nan"), dtype=BF, device=DEV) if i == 0 else torch.empty(T, H * dh, dtype=BF, device=DEV)
+            o.attention_prefill_tc(q, s["kc"], s["vc"], s["cu_q"], s["ctx_len"], s["table"], tiles, out, H, window, 0.1, started=started)
+            o.attention_decode_tma(q, s["kc"], s["vc"], s["cu_q"], s["ctx_len"], s["table"], singles, splits, out, H, window, 0.1, started=started)
+            outs.append(out.float())
+        return outs
+    want = layers(None)
+    assert all(torch.isfinite(w).all() for w in want)
+    for _ in range(3):
+        assert all(torch.equal(a, b) for a, b in zip(layers(word), want)) and word.item() == 0
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = layers(word)
+    for _ in range(5):
+        for g in got:
+            g.zero_()
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(got, want)) and word.item() == 0
+    o.check_status()
