@@ -42,6 +42,23 @@ __device__ __forceinline__ void cp_async16(float* smem, const float* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" :: "r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+// Two 32-bit numbers in one register pair, for the instructions that work on both at once.
+__device__ __forceinline__ uint64_t f2_pack(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_unpack(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" :: "n"(N)); }
 
 // The tokens of a request pass through shared memory in chunks of `chunk` tokens, two buffers taking turns: while the
@@ -207,20 +224,27 @@ __device__ __forceinline__ int scan_cut_place(const int* __restrict__ cu_q, int 
 // four blocks fit an SM and hide each other's latencies. The order of every sum is the same in both.
 // CUT: portions may be cut. A launch of few blocks that cuts nothing (decode steps of a few requests) goes without the code for it:
 // its set-up counts there (8 requests, 7 heads of 64 x 128: 3.9 -> 3.5 us, delta rule 4.2 -> 3.5).
+// NC: columns a lane holds, 1 or 4 neighbours. A token's q, k and decays come from shared memory once for all of them: with one column
+// a warp's 12 loads of 16 bytes feed 48 multiplications a lane, and where many warps walk side by side the SM's shared-memory port is
+// what they wait for (48 cycles a token and warp); with four a warp takes longer over a token, which a launch of few warps would feel.
 // QUIET: the first pass over a portion that was cut: no read-out. With four blocks an SM, up to 32 parts instead of 16 and
 // the folds' loads in flight, a Fezopel prefill of 2,048 tokens (0.5B sizes, six recurrent layers) 2,629 -> 2,090 us.
-template <int RULE, int RK4, bool DENSE, bool QUIET, bool CUT>
-__global__ void __launch_bounds__(WARPS * 32, DENSE ? 4 : 1)
+// KSC: the number of lanes that share a column where the build is for one (0: any, an argument).
+// Two neighbouring rows go through the instructions that work on a pair of 32-bit numbers (each rounded as the scalar instruction
+// rounds it): a token's time is its instructions and their latencies.
+template <int RULE, int RK4, int NC, int KSC, bool DENSE, bool QUIET, bool CUT>
+__global__ void __launch_bounds__(WARPS * 32, NC > 1 ? 3 : DENSE ? 4 : 1)
 recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, const float* z, int ldz,
                           const float* beta, int ldb, float q_scale,
                           float* state, size_t slot_stride, const int* __restrict__ slots, const int* __restrict__ cu_q,
-                          float* out, int H, int G, int dk, int dv, int KS, int chunk, int vec,
+                          float* out, int H, int G, int dk, int dv, int lanes, int chunk, int vec,
                           int nc, int n_cut, int* places, float* part_s, float* part_p, const float* part_start) {
     bl_pdl_trigger();
     bl_pdl_wait();
     extern __shared__ __align__(16) float sm[];
     constexpr bool DELTA = RULE == BL_RULE_DELTA, BONUS = RULE == BL_RULE_BONUS;
-    constexpr int RK = RK4 * 4;
+    constexpr int RK = RK4 * 4, RP = RK / 2;                     // rows a lane holds, pairs of them
+    const int KS = KSC ? KSC : lanes;
     // A long portion of a request may be cut into nc parts that run side by side (the recurrence is linear in S). First pass
     // (QUIET): every part from a ZERO state, leaving its own contribution S_part and its transition P (a product of decays a
     // row; of the delta rule a matrix). Between the passes a fold (S <- P S + S_part) leaves every part's start state in
@@ -248,9 +272,9 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
     const int t0 = cu_q[r] + t_first, n = (split ? (int)((long long)(part + 1) * n_all / nc) : n_all) - t_first;
     const int gh = h / (H / G);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int CW = 32 / KS, cols_blk = WARPS * CW;
+    const int CW = 32 / KS, cols_blk = WARPS * CW * NC;          // CW: lanes side by side along the columns
     const int s = lane / CW, cc = lane % CW;
-    const int c = (blockIdx.x * WARPS + warp) * CW + cc;
+    const int c = ((blockIdx.x * WARPS + warp) * CW + cc) * NC;  // the lane's first column (NC 4: dv and dk are multiples of 4)
     // The delta rule's transition over a part is a key x key matrix: pass 1 makes it in dk further columns that start as
     // the identity and see values of zero (column dv + j ends as the part's transition applied to unit vector j).
     const int n_cols = dv + (DELTA && QUIET ? dk : 0);
@@ -282,6 +306,12 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
                 }
             }
             const float* gv = v + tok * ldv + h * dv + col0;
+            if (NC > 1) {
+                for (int j = lane * 4; j < cols_blk; j += 128) {
+                    if (col0 + j < dv) cp_async16(dst + 3 * dk + j, gv + j);
+                    else *reinterpret_cast<float4*>(dst + 3 * dk + j) = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            } else
             for (int j = lane; j < cols_blk; j += 32) {
                 if (col0 + j < dv) cp_async4(dst + 3 * dk + j, gv + j);
                 else dst[3 * dk + j] = 0.f;
@@ -292,77 +322,161 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
     };
 
     issue(0, sm);
-    float st[RK], pr[QUIET && !DELTA ? RK : 1];
+    uint64_t st[NC][RP], pr[QUIET && !DELTA ? RP : 1];           // a column's rows in pairs
     const size_t part_base = ((size_t)place * nc) * H + h;       // + p * H for part p
+    auto read_row = [&](const float* p, float (&x)[NC]) {        // the lane's columns of a row
+        if constexpr (NC == 4) {
+            const float4 f = *reinterpret_cast<const float4*>(p);
+            x[0] = f.x; x[1] = f.y; x[2] = f.z; x[3] = f.w;
+        } else {
+            x[0] = *p;
+        }
+    };
+    auto write_row = [&](float* p, const float (&x)[NC]) {
+        if constexpr (NC == 4) *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
+        else *p = x[0];
+    };
+    const float* start = split ? part_start + ((part_base + (size_t)part * H) * dk + row0) * dv + c : S + (size_t)row0 * dv + c;
 #pragma unroll
-    for (int i = 0; i < RK; ++i) {
-        if (QUIET) st[i] = (DELTA && c >= dv && row0 + i == c - dv) ? 1.f : 0.f;
-        else if (split) st[i] = col_ok ? part_start[((part_base + (size_t)part * H) * dk + row0 + i) * dv + c] : 0.f;
-        else st[i] = col_ok ? S[(size_t)(row0 + i) * dv + c] : 0.f;
-        if (QUIET && !DELTA) pr[QUIET && !DELTA ? i : 0] = 1.f;
+    for (int i = 0; i < RP; ++i) {
+        float a[NC], b[NC];
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
+            a[j] = QUIET && DELTA && c + j >= dv && row0 + 2 * i == c + j - dv ? 1.f : 0.f;
+            b[j] = QUIET && DELTA && c + j >= dv && row0 + 2 * i + 1 == c + j - dv ? 1.f : 0.f;
+        }
+        if (!QUIET && col_ok) { read_row(start + (size_t)(2 * i) * dv, a); read_row(start + (size_t)(2 * i + 1) * dv, b); }
+#pragma unroll
+        for (int j = 0; j < NC; ++j) st[j][i] = f2_pack(a[j], b[j]);
+        if (QUIET && !DELTA) pr[QUIET && !DELTA ? i : 0] = f2_pack(1.f, 1.f);
     }
-    const int v_off = 3 * dk + warp * CW + cc, b_off = 3 * dk + cols_blk;
+    // the lane's columns of its rows, to `p` with rows dv (or dk) apart
+    auto write_state = [&](float* p, int ld) {
+#pragma unroll
+        for (int i = 0; i < RP; ++i) {
+            float a[NC], b[NC];
+#pragma unroll
+            for (int j = 0; j < NC; ++j) f2_unpack(st[j][i], a[j], b[j]);
+            write_row(p + (size_t)(2 * i) * ld, a);
+            write_row(p + (size_t)(2 * i + 1) * ld, b);
+        }
+    };
+    const int v_off = 3 * dk + (warp * CW + cc) * NC, b_off = 3 * dk + cols_blk;
     const int dk4 = dk >> 2;
 
-    struct Tok { float4 q[QUIET ? 1 : RK4], k[RK4], d[RK4]; float v, b; };
+    struct Tok { ulonglong2 q[QUIET ? 1 : RK4], k[RK4], d[RK4]; float v[NC], b; };
     auto fetch = [&](const float* tokp, Tok& t) {
-        const float4* p4 = reinterpret_cast<const float4*>(tokp + row0);
+        const ulonglong2* p4 = reinterpret_cast<const ulonglong2*>(tokp + row0);
 #pragma unroll
         for (int j = 0; j < RK4; ++j) {
             if (!QUIET) t.q[QUIET ? 0 : j] = p4[j];
             t.k[j] = p4[dk4 + j]; t.d[j] = p4[2 * dk4 + j];
         }
-        t.v = tokp[v_off];
+        if constexpr (NC == 4) {
+            const float4 x = *reinterpret_cast<const float4*>(tokp + v_off);
+            t.v[0] = x.x; t.v[1] = x.y; t.v[2] = x.z; t.v[3] = x.w;
+        } else {
+            t.v[0] = tokp[v_off];
+        }
         t.b = (DELTA || BONUS) ? tokp[b_off] : 0.f;
     };
+    // The sums of a column's rows over the KS lanes that hold them, always in the order of the butterfly. With four columns a
+    // lane gives the sums away that it does not go on with: two after the first exchange, one after the second; it ends with `kept`
+    // of them, from column `mine` on.
+    const int kept = NC == 1 || KS == 1 ? NC : KS == 2 ? 2 : 1;
+    const int mine = NC == 1 || KS == 1 ? 0 : KS == 2 ? (lane >> 4) * 2 : (lane >> 4) * 2 + ((lane >> 3) & 1);
+    const bool speaks = NC == 1 ? s == 0 : KS <= 4 || (s & (KS / 4 - 1)) == 0;       // of the lanes that end with equal sums, one writes them
+    auto column_sums = [&](float (&o)[NC]) {
+        if constexpr (NC == 1) {
+            for (int x = 16; x >= CW; x >>= 1) o[0] += __shfl_xor_sync(0xffffffffu, o[0], x);
+        } else if (KS > 1) {
+            const bool up = (lane & 16) != 0;
+            const float g0 = __shfl_xor_sync(0xffffffffu, up ? o[0] : o[2], 16), g1 = __shfl_xor_sync(0xffffffffu, up ? o[1] : o[3], 16);
+            o[0] = (up ? o[2] : o[0]) + g0;
+            o[1] = (up ? o[3] : o[1]) + g1;
+            if (KS > 2) {
+                const bool up2 = (lane & 8) != 0;
+                const float g = __shfl_xor_sync(0xffffffffu, up2 ? o[0] : o[1], 8);
+                o[0] = (up2 ? o[1] : o[0]) + g;
+                for (int x = 4; x >= CW; x >>= 1) o[0] += __shfl_xor_sync(0xffffffffu, o[0], x);
+            }
+        }
+    };
+    auto kept_of = [&](const float (&a)[NC], int j) {            // a[mine + j], without an index that is not known
+        if constexpr (NC == 1) return a[0];
+        else if (KS == 1) return a[j];
+        else if (KS == 2) return mine ? a[2 + (j & 1)] : a[j & 1];
+        else return mine & 2 ? (mine & 1 ? a[3] : a[2]) : (mine & 1 ? a[1] : a[0]);
+    };
     auto step = [&](const Tok& t, size_t tok) {
-        const float* tq = reinterpret_cast<const float*>(t.q);
-        const float* tk = reinterpret_cast<const float*>(t.k);
-        const float* td = reinterpret_cast<const float*>(t.d);
-        float o;
+        auto q2 = [&](int i) { return i & 1 ? t.q[QUIET ? 0 : i >> 1].y : t.q[QUIET ? 0 : i >> 1].x; };
+        auto k2 = [&](int i) { return i & 1 ? t.k[i >> 1].y : t.k[i >> 1].x; };
+        auto d2 = [&](int i) { return i & 1 ? t.d[i >> 1].y : t.d[i >> 1].x; };
+        const uint64_t zero = f2_pack(0.f, 0.f);
+        auto both = [](uint64_t x) { float a, b; f2_unpack(x, a, b); return a + b; };
+        float o[NC], u[NC];
         if (!DELTA) {
-            float o0 = 0.f, o1 = 0.f;
 #pragma unroll
-            for (int i = 0; i < RK; i += 2) {
-                if (BONUS && !QUIET) { o0 = fmaf(st[i], tq[i], o0); o1 = fmaf(st[i + 1], tq[i + 1], o1); }       // the state before the write
-                st[i] = fmaf(td[i], st[i], tk[i] * t.v);
-                st[i + 1] = fmaf(td[i + 1], st[i + 1], tk[i + 1] * t.v);
-                if (!BONUS && !QUIET) { o0 = fmaf(st[i], tq[i], o0); o1 = fmaf(st[i + 1], tq[i + 1], o1); }
+            for (int j = 0; j < NC; ++j) {
+                const uint64_t v2 = f2_pack(t.v[j], t.v[j]);
+                uint64_t o2 = zero;
+#pragma unroll
+                for (int i = 0; i < RP; ++i) {
+                    if (BONUS && !QUIET) o2 = f2_fma(st[j][i], q2(i), o2);                       // the state before the write
+                    st[j][i] = f2_fma(d2(i), st[j][i], f2_mul(k2(i), v2));
+                    if (!BONUS && !QUIET) o2 = f2_fma(st[j][i], q2(i), o2);
+                }
+                o[j] = both(o2);
             }
             if (QUIET) {
 #pragma unroll
-                for (int i = 0; i < (QUIET && !DELTA ? RK : 1); ++i) pr[i] *= td[i];
+                for (int i = 0; i < (QUIET && !DELTA ? RP : 1); ++i) pr[i] = f2_mul(pr[i], d2(i));
                 return;
             }
-            o = o0 + o1;
-            for (int x = 16; x >= CW; x >>= 1) o += __shfl_xor_sync(0xffffffffu, o, x);
-            if (BONUS) o = fmaf(t.b, t.v, o);
+            column_sums(o);
         } else {
-            float sk0 = 0.f, sk1 = 0.f, sq0 = 0.f, sq1 = 0.f, kq0 = 0.f, kq1 = 0.f;
+            float sk[NC], sq[NC];
+            uint64_t kq2 = zero;
 #pragma unroll
-            for (int i = 0; i < RK; i += 2) {
-                st[i] *= td[i];
-                st[i + 1] *= td[i + 1];
-                sk0 = fmaf(st[i], tk[i], sk0); sk1 = fmaf(st[i + 1], tk[i + 1], sk1);
-                if (!QUIET) {
-                    sq0 = fmaf(st[i], tq[i], sq0); sq1 = fmaf(st[i + 1], tq[i + 1], sq1);
-                    kq0 = fmaf(tk[i], tq[i], kq0); kq1 = fmaf(tk[i + 1], tq[i + 1], kq1);
-                }
-            }
-            float sk_ = sk0 + sk1, sq_ = sq0 + sq1, kq = kq0 + kq1;
-            for (int x = 16; x >= CW; x >>= 1) {
-                sk_ += __shfl_xor_sync(0xffffffffu, sk_, x);
-                if (!QUIET) {
-                    sq_ += __shfl_xor_sync(0xffffffffu, sq_, x);
-                    kq += __shfl_xor_sync(0xffffffffu, kq, x);
-                }
-            }
-            const float u = t.b * (t.v - sk_);
+            for (int j = 0; j < NC; ++j) {
+                uint64_t sk2 = zero, sq2 = zero;
 #pragma unroll
-            for (int i = 0; i < RK; ++i) st[i] = fmaf(tk[i], u, st[i]);
-            o = fmaf(kq, u, sq_);
+                for (int i = 0; i < RP; ++i) {
+                    st[j][i] = f2_mul(st[j][i], d2(i));
+                    sk2 = f2_fma(st[j][i], k2(i), sk2);
+                    if (!QUIET) {
+                        sq2 = f2_fma(st[j][i], q2(i), sq2);
+                        if (j == 0) kq2 = f2_fma(k2(i), q2(i), kq2);
+                    }
+                }
+                sk[j] = both(sk2); sq[j] = both(sq2);
+            }
+            float kq = both(kq2);
+            for (int x = 16; x >= CW; x >>= 1) {                 // every lane needs the columns' S^T k
+#pragma unroll
+                for (int j = 0; j < NC; ++j) sk[j] += __shfl_xor_sync(0xffffffffu, sk[j], x);
+                if (!QUIET) kq += __shfl_xor_sync(0xffffffffu, kq, x);
+            }
+            if (!QUIET) column_sums(sq);
+#pragma unroll
+            for (int j = 0; j < NC; ++j) u[j] = t.b * (t.v[j] - sk[j]);
+#pragma unroll
+            for (int j = 0; j < NC; ++j) {
+                const uint64_t u2 = f2_pack(u[j], u[j]);
+#pragma unroll
+                for (int i = 0; i < RP; ++i) st[j][i] = f2_fma(k2(i), u2, st[j][i]);
+            }
+            if (!QUIET) {
+#pragma unroll
+                for (int j = 0; j < NC; ++j) o[j] = j < kept ? fmaf(kq, kept_of(u, j), sq[j]) : 0.f;
+            }
         }
-        if (!QUIET && s == 0 && col_ok) out[tok * H * dv + h * dv + c] = o * q_scale;
+        if (!QUIET && speaks && col_ok) {
+            float* dst = out + tok * H * dv + h * dv + c + mine;
+#pragma unroll
+            for (int j = 0; j < NC; ++j)
+                if (j < kept) dst[j] = (BONUS ? fmaf(t.b, kept_of(t.v, j), o[j]) : o[j]) * q_scale;
+        }
     };
 
     int which = 0;
@@ -405,25 +519,24 @@ recurrent_scan_vec_kernel(const float* q, int ldq, const float* k, int ldk, cons
         if (QUIET && DELTA) {
             float* ps = part_s + (part_base + (size_t)part * H) * dk * dv;
             float* pm = part_p + (part_base + (size_t)part * H) * dk * dk;      // [row][unit vector]
-#pragma unroll
-            for (int i = 0; i < RK; ++i) {
-                if (c < dv) ps[(size_t)(row0 + i) * dv + c] = st[i];
-                else if (col_ok) pm[(size_t)(row0 + i) * dk + (c - dv)] = st[i];
-            }
+            if (c < dv) write_state(ps + (size_t)row0 * dv + c, dv);
+            else if (col_ok) write_state(pm + (size_t)row0 * dk + (c - dv), dk);
         } else if (QUIET) {
             float* ps = part_s + (part_base + (size_t)part * H) * dk * dv;
             float* pp = part_p + (part_base + (size_t)part * H) * dk;
+            if (col_ok) write_state(ps + (size_t)row0 * dv + c, dv);
+            if (blockIdx.x == 0 && warp == 0 && cc == 0) {
 #pragma unroll
-            for (int i = 0; i < RK; ++i) {
-                if (col_ok) ps[(size_t)(row0 + i) * dv + c] = st[i];
-                if (blockIdx.x == 0 && warp == 0 && cc == 0) pp[row0 + i] = pr[QUIET && !DELTA ? i : 0];
+                for (int i = 0; i < (QUIET && !DELTA ? RP : 1); ++i) {
+                    float a, b;
+                    f2_unpack(pr[i], a, b);
+                    pp[row0 + 2 * i] = a; pp[row0 + 2 * i + 1] = b;
+                }
             }
         }
         return;                                        // the slot is written by the fold
     }
-#pragma unroll
-    for (int i = 0; i < RK; ++i)
-        if (col_ok) S[(size_t)(row0 + i) * dv + c] = st[i];
+    if (col_ok) write_state(S + (size_t)row0 * dv + c, dv);
 }
 
 // Between the two passes of a cut portion of the delta rule: start[0] = the slot's state, start[p + 1] = P_p start[p] +
@@ -472,6 +585,91 @@ scan_fold_matrix_kernel(float* state, size_t slot_stride, const int* __restrict_
             }
         }
         __syncthreads();
+    }
+}
+
+// The same for values in groups of four: a thread holds the TPR-th part of a row of P (up to 64 values) in registers, the next part's
+// on its way while it multiplies this one's, and 4 GROUPS columns of the state, which all rows read from shared memory as broadcasts. The
+// kernel above asks for a part's P when the part before it is done, a trip to L2 (or two) a part, and reads the state a value
+// at a time. Sums in its order (two halves of a row, where there are two, added at the end).
+template <int TPR, int GROUPS>
+__global__ void __launch_bounds__(TPR == 1 ? 64 : 256)
+scan_fold_matrix4_kernel(float* state, size_t slot_stride, const int* __restrict__ slots, const int* __restrict__ cu_q,
+                         const int* places, const float* part_s, const float* part_pm, float* part_start, int H, int dk, int dv, int nc) {
+    bl_pdl_trigger();
+    bl_pdl_wait();
+    constexpr int PIECES = 16;                          // of four values of P a thread
+    __shared__ float4 cur[2][FOLD_MAX_DK][GROUPS];
+    const int r = blockIdx.z, h = blockIdx.y, c0 = blockIdx.x * 4 * GROUPS;
+    if (cu_q[r + 1] - cu_q[r] < SCAN_SPLIT_MIN) return;
+    const int place = places ? places[r] : r;
+    if (place < 0) return;
+    float* S = state + (size_t)slots[r] * slot_stride + (size_t)h * dk * dv;
+    const size_t base = ((size_t)place * nc) * H + h;
+    const int row = threadIdx.x / TPR, half = threadIdx.x % TPR, k0 = half * 4 * PIECES;
+    const int pieces = min(PIECES, (dk - k0) >> 2);     // dk is a multiple of 4
+    float4 pa[PIECES], pb[PIECES], sa[GROUPS], sb[GROUPS];
+    auto fetch = [&](int p, float4 (&m)[PIECES], float4 (&a)[GROUPS]) {
+        if (p >= nc) return;
+        const float4* pm = reinterpret_cast<const float4*>(part_pm + ((base + (size_t)p * H) * dk + row) * dk + k0);
+#pragma unroll
+        for (int j = 0; j < PIECES; ++j)
+            if (j < pieces) m[j] = pm[j];
+        const float4* ps = reinterpret_cast<const float4*>(part_s + ((base + (size_t)p * H) * dk + row) * dv + c0);
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g)
+            a[g] = half == 0 && c0 + 4 * g < dv ? ps[g] : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto part = [&](int p, const float4 (&m)[PIECES], const float4 (&a)[GROUPS]) {
+        const int w = p & 1;
+        float4 acc[GROUPS];
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g) acc[g] = a[g];
+#pragma unroll
+        for (int j = 0; j < PIECES; ++j) {
+            if (j >= pieces) continue;
+            const float e[4] = {m[j].x, m[j].y, m[j].z, m[j].w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int g = 0; g < GROUPS; ++g) {
+                    const float4 c = cur[w][k0 + 4 * j + i][g];
+                    acc[g].x = fmaf(e[i], c.x, acc[g].x); acc[g].y = fmaf(e[i], c.y, acc[g].y);
+                    acc[g].z = fmaf(e[i], c.z, acc[g].z); acc[g].w = fmaf(e[i], c.w, acc[g].w);
+                }
+        }
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g) {
+            if (TPR == 2) {
+                acc[g].x += __shfl_xor_sync(0xffffffffu, acc[g].x, 1); acc[g].y += __shfl_xor_sync(0xffffffffu, acc[g].y, 1);
+                acc[g].z += __shfl_xor_sync(0xffffffffu, acc[g].z, 1); acc[g].w += __shfl_xor_sync(0xffffffffu, acc[g].w, 1);
+            }
+            if (half == 0) {
+                cur[w ^ 1][row][g] = acc[g];
+                if (c0 + 4 * g < dv) {
+                    float* to = p + 1 < nc ? part_start + ((base + (size_t)(p + 1) * H) * dk + row) * dv : S + (size_t)row * dv;
+                    *reinterpret_cast<float4*>(to + c0 + 4 * g) = acc[g];
+                }
+            }
+        }
+        __syncthreads();
+    };
+    fetch(0, pa, sa);
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g) {
+        if (half != 0) continue;
+        const bool ok = c0 + 4 * g < dv;
+        const float4 x = ok ? *reinterpret_cast<const float4*>(S + (size_t)row * dv + c0 + 4 * g) : make_float4(0.f, 0.f, 0.f, 0.f);
+        cur[0][row][g] = x;
+        if (ok) *reinterpret_cast<float4*>(part_start + (base * dk + row) * dv + c0 + 4 * g) = x;
+    }
+    __syncthreads();
+    for (int p = 0; p < nc; p += 2) {
+        fetch(p + 1, pb, sb);
+        part(p, pa, sa);
+        if (p + 1 >= nc) break;
+        fetch(p + 2, pa, sa);
+        part(p + 1, pb, sb);
     }
 }
 
@@ -1049,17 +1247,27 @@ extern "C" int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const 
     for (int ks = 1; ks <= 32 && rk4 == 0; ks *= 2)
         if (dk % (4 * ks) == 0 && dk / ks <= SCAN_VEC_ROWS) { KS = ks; rk4 = dk / (4 * ks); }
     if (rk4 == 0 && dk % (4 * KS) == 0) rk4 = dk / (4 * KS);
-    const int CW = 32 / KS, cols_blk = WARPS * CW;
-    const size_t per_token = (size_t)(3 * dk + cols_blk + 4) * sizeof(float);
-    int chunk = (int)(SCAN_SMEM_BYTES / (2 * per_token));
-    chunk = chunk < 1 ? 1 : (chunk > 16 ? 16 : chunk);
-    const size_t smem = 2 * per_token * chunk;
-    if (smem > 48 * 1024) BL_FAIL("bl_recurrent_scan: %d key channels need %zu bytes of shared memory a token", dk, per_token);
+    const int CW = 32 / KS;
+    struct Walk { int cols_blk, chunk; size_t smem; };
+    auto walk_of = [&](int columns) {                  // of lanes with so many columns
+        Walk k;
+        k.cols_blk = WARPS * CW * columns;
+        const size_t per_token = (size_t)(3 * dk + k.cols_blk + 4) * sizeof(float);
+        k.chunk = (int)(SCAN_SMEM_BYTES / (2 * per_token));
+        k.chunk = k.chunk < 1 ? 1 : (k.chunk > 16 ? 16 : k.chunk);
+        k.smem = 2 * per_token * k.chunk;
+        return k;
+    };
+    const Walk one = walk_of(1), four = walk_of(4);
+    const int cols_blk = one.cols_blk, chunk = one.chunk;
+    const size_t smem = one.smem;
+    if (smem > 48 * 1024) BL_FAIL("bl_recurrent_scan: %d key channels need %zu bytes of shared memory a token", dk, smem / (2 * chunk));
     // 16-byte copies where every row of q, k and z starts on a 16-byte boundary
     const int vec = dk % 4 == 0 && ldq % 4 == 0 && ldk % 4 == 0 && ldz % 4 == 0 &&
                     (((uintptr_t)q | (uintptr_t)k | (uintptr_t)z) & 15) == 0;
     dim3 grid((dv + cols_blk - 1) / cols_blk, H, R * nc);
-    const dim3 grid_wide((dv + dk + cols_blk - 1) / cols_blk, H, R * nc);     // the delta rule's first pass
+    // four columns a lane: where values and states are whole 16-byte pieces, too
+    const bool fours = rk4 == 4 && vec && dv % 4 == 0 && ldv % 4 == 0 && slot_stride % 4 == 0 && (((uintptr_t)v | (uintptr_t)state) & 15) == 0 && four.smem <= 48 * 1024;
     cudaStream_t s = (cudaStream_t)stream;
     if (rule != BL_RULE_GLA && rule != BL_RULE_DELTA && rule != BL_RULE_BONUS) BL_FAIL("bl_recurrent_scan: unknown rule %d", rule);
     if (rk4 > 0) {                                     // a lane's rows are whole groups of four
@@ -1073,18 +1281,36 @@ extern "C" int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const 
         // tokens beside a long portion that leave at once (2,000 tokens beside 31 running requests, in one piece: 7 heads of
         // 64 x 128 640 us counted by all, 507 so; 8 of 128 x 256 1,115 and 824; the delta rule 778 and 613, 1,215 and 934).
         const int two_an_sm = 2 * scan_sms();
+        // Four columns a lane from four blocks of one column an SM on, when a second round of those would begin: 8 single tokens of 8
+        // heads of 128 x 256 9.4 -> 6.3 us, 64 of them 56 -> 23; prompts of 401 to 57 tokens 249 -> 177 (delta rule 315 -> 238); 2,048
+        // tokens in 32 parts of 7 heads of 64 x 128 103 -> 78. Below, a fourth of the blocks is too few: 8 single tokens of 7 heads of
+        // 64 x 128 3.3 us against 4.1, 8 x 250 tokens 79 against 97.
+        const long long fours_from = 4LL * scan_sms();
         const long long at_once[2] = {(long long)n_cut * nc, nc > 1 ? (long long)n_cut * nc + (busy > n_cut ? busy - n_cut : 0) : busy};
-#define BL_SCAN_Q(D, R4, DENSE, QUIET, CUT, GRID) BL_CUDA(bl_launch_dependent(recurrent_scan_vec_kernel<D, R4, DENSE, QUIET, CUT>, GRID, dim3(WARPS * 32), smem, s, \
-        q, ldq, k, ldk, v, ldv, z, ldz, beta, ldb, q_scale, state, (size_t)slot_stride, slots, cu_q, out, H, G, dk, dv, KS, chunk, vec, nc, n_cut, places, \
-        part_s, part_p, (const float*)part_start))
+#define BL_SCAN_Q(D, R4, NC, KSC, DENSE, QUIET, CUT, GRID) BL_CUDA(bl_launch_dependent(recurrent_scan_vec_kernel<D, R4, NC, KSC, DENSE, QUIET, CUT>, GRID, \
+        dim3(WARPS * 32), NC == 4 ? four.smem : smem, s, q, ldq, k, ldk, v, ldv, z, ldz, beta, ldb, q_scale, state, (size_t)slot_stride, slots, cu_q, out, H, G, \
+        dk, dv, KS, NC == 4 ? four.chunk : chunk, vec, nc, n_cut, places, part_s, part_p, (const float*)part_start))
+#define BL_SCAN_4(D, KSC, PASS, GRID) do { if (PASS == 1) BL_SCAN_Q(D, 4, 4, KSC, true, true, true, GRID); else BL_SCAN_Q(D, 4, 4, KSC, true, false, true, GRID); } while (0)
 #define BL_SCAN(D, R4, PASS) do { \
-        const dim3 g = (D == BL_RULE_DELTA && PASS == 1) ? grid_wide : grid; \
-        const bool dense = at_once[PASS - 1] * g.x * g.y > two_an_sm; \
-        if (PASS == 1) { if (dense) BL_SCAN_Q(D, R4, true, true, true, g); else BL_SCAN_Q(D, R4, false, true, true, g); } \
-        else if (dense) BL_SCAN_Q(D, R4, true, false, true, g); \
-        else if (nc > 1) BL_SCAN_Q(D, R4, false, false, true, g); else BL_SCAN_Q(D, R4, false, false, false, g); } while (0)
+        const int cols = D == BL_RULE_DELTA && PASS == 1 ? dv + dk : dv;         /* the delta rule's first pass makes its transition in dk more */ \
+        const dim3 g((cols + cols_blk - 1) / cols_blk, H, R * nc), g4((cols + four.cols_blk - 1) / four.cols_blk, H, R * nc); \
+        const long long blocks = at_once[PASS - 1] * g.x * g.y; \
+        const bool dense = blocks > two_an_sm; \
+        if (fours && blocks >= fours_from) { \
+            if (KS == 4) BL_SCAN_4(D, 4, PASS, g4); else if (KS == 8) BL_SCAN_4(D, 8, PASS, g4); else BL_SCAN_4(D, 0, PASS, g4); } \
+        else if (PASS == 1) { if (dense) BL_SCAN_Q(D, R4, 1, 0, true, true, true, g); else BL_SCAN_Q(D, R4, 1, 0, false, true, true, g); } \
+        else if (dense) BL_SCAN_Q(D, R4, 1, 0, true, false, true, g); \
+        else if (nc > 1) BL_SCAN_Q(D, R4, 1, 0, false, false, true, g); else BL_SCAN_Q(D, R4, 1, 0, false, false, false, g); } while (0)
         for (int pass = (nc > 1 ? 1 : 2); pass <= 2; ++pass) {
-            if (pass == 2 && nc > 1 && dl)
+            if (pass == 2 && nc > 1 && dl && dv % 4 == 0 && slot_stride % 4 == 0 && (((uintptr_t)state | (uintptr_t)scratch) & 15) == 0) {
+                // rows of up to 64 values a thread; 8 columns a block where P is large (every block of a head reads all of it)
+                const bool wide = dk > 64;
+                const dim3 g((dv + (wide ? 8 : 4) - 1) / (wide ? 8 : 4), H, R);
+                if (wide) BL_CUDA(bl_launch_dependent(scan_fold_matrix4_kernel<2, 2>, g, dim3(2 * dk), 0, s, state, (size_t)slot_stride, slots, cu_q,
+                                                      (const int*)places, (const float*)part_s, (const float*)part_p, part_start, H, dk, dv, nc));
+                else BL_CUDA(bl_launch_dependent(scan_fold_matrix4_kernel<1, 1>, g, dim3(dk), 0, s, state, (size_t)slot_stride, slots, cu_q,
+                                                 (const int*)places, (const float*)part_s, (const float*)part_p, part_start, H, dk, dv, nc));
+            } else if (pass == 2 && nc > 1 && dl)
                 BL_CUDA(bl_launch_dependent(scan_fold_matrix_kernel, dim3((dv + FOLD_COLS - 1) / FOLD_COLS, H, R), dim3(256), 0, s, state,
                                             (size_t)slot_stride, slots, cu_q, (const int*)places, (const float*)part_s, (const float*)part_p, part_start,
                                             H, dk, dv, nc));
@@ -1102,6 +1328,7 @@ extern "C" int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const 
             }
         }
 #undef BL_SCAN
+#undef BL_SCAN_4
 #undef BL_SCAN_Q
         BL_CHECK_LAUNCH("bl_recurrent_scan");
         return 0;

@@ -1077,22 +1077,46 @@ def _scan_cost(rule: int, H: int, dk: int, dv: int, n_long: int, tokens: int, pa
     return tokens / parts * token * (_scan_rounds(first_blocks * n_long * parts) + _scan_rounds(blocks * n_long * parts)) + between
 
 
+SCAN_FOUR_TOKENS = 2048           # portions from which the four-column build decides the number of parts ...
+SCAN_FOUR_BLOCKS_PER_SM = 3       # ... of whose blocks an SM holds so many
+SCAN_FOUR_MAX_PARTS = 64
+
+
+def _scan_parts_of_fours(rule: int, H: int, dk: int, dv: int, n_long: int, tokens: int):
+    """(parts, microseconds) when the passes run with four columns a lane: a token's chain is twice that of one column, 0.58 us, but a
+    fourth of the blocks walks the same columns, so that the most parts whose blocks are all under way are the best. None where that
+    build is not there (key sizes of 16 times a power of two) or not measured to pay: short portions, and the delta rule up to 64 key
+    channels, which is kept at its number of parts."""
+    ks = dk // 16
+    if tokens < SCAN_FOUR_TOKENS or dk % 16 or ks & (ks - 1) or not 1 <= ks <= 32 or dv % 4 or (rule == RULE_DELTA and dk <= 64):
+        return None
+    columns = dv + (dk if rule == RULE_DELTA else 0)
+    blocks = H * -(-columns // (512 // ks)) * n_long                   # of one part's first pass
+    parts = min(SCAN_FOUR_MAX_PARTS, SCAN_FOUR_BLOCKS_PER_SM * _sms() // blocks)
+    if parts < 2:
+        return None
+    between = 9.0 + parts * 16.0 * H * n_long * dk * dv / 3e6
+    if rule == RULE_DELTA:
+        between += 2.2 * parts * (dk / 64) ** 2 * max(1.0, H * n_long * -(-dv // 8) / _sms())
+    return parts, 2 * tokens / parts * 0.58 + between
+
+
 @functools.lru_cache(maxsize=1024)                    # (asked by every layer of every step)
 def recurrent_scan_parts(rule: int, H: int, dk: int, dv: int, n_long: int, tokens: int = 1024) -> int:
     """How many parts `recurrent_scan` should cut the portions of a step's `n_long` long requests into (1: none), the longest of
     about `tokens` tokens (a power of two: the number of parts names captured steps). Cutting
     runs every token twice, on `parts` times the blocks; the delta rule's first pass has as many columns more as the key size
-    (its transition over a part is a matrix). It pays while a request's blocks leave much of the device idle: the fewest parts
-    within 2 % of the least time by `_scan_cost`, if that is 0.9 of the walk in one piece or less. Microseconds in one piece
+    (its transition over a part is a matrix). Portions of 2,048 tokens: see `_scan_parts_of_fours` (7 heads of 64 x 128 in 63 parts 85 ->
+    54 us, 8 heads of 128 x 256 in 13 parts 445 -> 183, the delta rule at that size in 9 parts 853 -> 460). Otherwise it pays while a request's blocks leave much of the device
+    idle: the fewest parts within 2 % of the least time by `_scan_cost`, if that is 0.9 of the walk in one piece or less. Microseconds in one piece
     and as chosen, one portion of 2,048 / 1,024 / 256 tokens:
         linear attention, 7 heads of  64 x 128    520 / 260 / 68    21 parts   85 /  50 / 24
                           8 heads of 128 x 256    770 / 389 / 99     9 parts  445 / 235 / 78   (23 parts 454 / 249 / 97)
         the delta rule,   7 heads of  64 x 128    626 / 314 / 81    14, 10 and 6 parts 242 / 134 / 61   (14 parts 242 / 174 / 122)
                           8 heads of 128 x 256    886 / 445 / 114   6 parts 901, one piece     (3 parts 894 / 492 / 189)
-    and four portions of 512 tokens: linear attention, 7 heads of 64 x 128, 150 in one piece, 88 in 5 parts. (Alone. Between the
-    other kernels of a model 14 parts are the better ones for 2,048 tokens of the delta rule, 2,055 us a step against 2,069 in 10:
-    they fill the device, so no later launch's blocks wait where the fold's would run. So are 6 parts at the larger size: 6,687 us
-    a step against 6,813 in one piece.)"""
+    and four portions of 512 tokens: linear attention, 7 heads of 64 x 128, 150 in one piece, 88 in 5 parts. (Alone, one column a
+    lane. Between the other kernels of a model 14 parts are the better ones for 2,048 tokens of the delta rule, 2,055 us a step
+    against 2,069 in 10: they fill the device, so no later launch's blocks wait where the fold's would run.)"""
     if n_long <= 0:
         return 1
     first = int(library.load().bl_recurrent_scan_can_split(rule, H, dk, dv))
@@ -1102,6 +1126,9 @@ def recurrent_scan_parts(rule: int, H: int, dk: int, dv: int, n_long: int, token
     cost = {p: _scan_cost(rule, H, dk, dv, n_long, tokens, p, first, blocks) for p in range(1, SCAN_MAX_PARTS + 1)}
     least = min(cost[p] for p in cost if p > 1)
     best = min(p for p in cost if p > 1 and cost[p] <= 1.02 * least)
+    fours = _scan_parts_of_fours(rule, H, dk, dv, n_long, tokens)
+    if fours is not None and fours[1] <= 0.9 * min(cost[1], cost[best]):
+        return fours[0]
     return best if cost[best] <= 0.9 * cost[1] else 1
 
 

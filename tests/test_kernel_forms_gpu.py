@@ -853,6 +853,35 @@ def test_few_rows_go_by_the_bytes_of_w():
     assert o.gemm_kernel(x, w, 2048, None, o.EPI_RESIDUAL) == "few" and o.gemm_skinny_links_norm(x, w, 2048, o.EPI_RESIDUAL)
 
 
+@pytest.mark.parametrize("rule", ["RULE_GLA", "RULE_DELTA", "RULE_BONUS"])
+@pytest.mark.parametrize("H,dk,dv", [(1, 16, 36), (2, 32, 132), (1, 64, 128), (1, 48, 20), (2, 128, 68), (1, 256, 32), (1, 512, 24)])
+def test_scan_with_four_columns_a_lane(rule, H, dk, dv):
+    """Many requests side by side (four columns a lane) against the same taken as few (one column), bit for bit, over the numbers of
+    lanes that share a column; columns that end within a block; and against 64 bits."""
+    o = ops()
+    rule = getattr(o, rule)
+    lens = [3, 1, 2, 0, 5, 17] * 100
+    T, R = sum(lens), len(lens)
+    q, k, v, b = data((T, H * dk), 1) * 0.3, data((T, H * dk), 2) * 0.1, data((T, H * dv), 3), data((T, H), 4)
+    a = torch.sigmoid(data((T, H * dk), 5) + 3.0)
+    cu = torch.tensor([0] + lens, device=DEV).cumsum(0).to(torch.int32)
+    got = []
+    for busy in (1, R):
+        st, out = data((R, H * dk * dv), 6), torch.full((T, H * dv), float("nan"), device=DEV)
+        o.recurrent_scan(rule, q, k, v, a, None if rule == o.RULE_GLA else b, 0.5, st, torch.arange(R, dtype=torch.int32, device=DEV), cu, out,
+                         H, H, dk, dv, busy=busy)
+        got.append((out, st))
+    assert all(torch.equal(x, y) for x, y in zip(*got))
+    out, st = got[1]
+    first = data((R, H * dk * dv), 6)
+    for r in (0, 5, R - 1):
+        lo, hi = int(cu[r]), int(cu[r + 1])
+        S = first[r].double().view(H, dk, dv)
+        w = _scan64(rule, *(x[lo:hi].double().view(hi - lo, H, -1) for x in (q, k, v, a)), b[lo:hi].double(), 0.5, S, H)
+        close(out[lo:hi], w.reshape(hi - lo, -1), torch.float32, f"outputs of request {r}")
+        close(st[r], S.reshape(-1), torch.float32, f"state of request {r}")
+
+
 @pytest.mark.parametrize("H,KV,dh,window", [(14, 2, 64, 0), (4, 4, 64, 100), (16, 2, 128, 0)])
 def test_prompts_and_single_tokens_side_by_side(H, KV, dh, window):
     """The two attention launches of a mixed step with the word between them against the same without it, bit for bit, kernel by
