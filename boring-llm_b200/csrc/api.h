@@ -482,6 +482,14 @@ int bl_moe_combine_rows_some(const float* y, const int* pos, const float* wts, f
 // (bl_gather_rows, bfloat16 rows of a multiple of 8 values), bl_gemm_tc_grouped multiplies every tile of 128 rows by its
 // expert's matrix (gemm_tcgen05.cu), and bl_moe_combine_rows adds up a token's rows y[pos[t * top + k]].
 int bl_moe_plan(const int* ids, int P, int E, int tile, int max_tiles, int* pos, int* row_src, int* tile_expert, void* stream);
+// For routed experts the rows lie in tiles of 16 and are multiplied in chunks of one expert (gemm_tcgen05_experts.cu): x [M, K], w
+// [n_experts, N or 2 N, K], chunks as bl_moe_plan_chunks writes them, of chunk_rows (64 or 256) rows at most; out bfloat16 with the gated
+// epilogue (`act` as for bl_gemm_tc_grouped), 32-bit without one.
+int bl_moe_plan_chunks(const int* ids, int P, int E, int chunk_rows, int max_tiles, int max_chunks, int* pos, int* row_src, int* chunks,
+                       void* stream);
+int bl_gemm_tc_experts(const void* x, const void* w, void* out, int out_dtype, int M, int N, int K, int epilogue, int n_experts,
+                       const int* chunks, int max_chunks, int chunk_rows, const float* act, void* stream);
+int bl_gemm_tc_experts_status(int* status);
 int bl_gather_rows(const void* x, const int* row_src, int div, void* dst, int rows, int cols, void* stream);
 // A weight per pair on what the pair's expert READS (instead of on its result): the gathered row of pair p times wts[p]
 // (null: 1), or, for the plain products, dst [T * top, d] = x[p / top, :] * wts[p]. bl_moe_combine and its variants add the

@@ -171,27 +171,41 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const float* __r
 constexpr int PLAN_THREADS = 1024;
 __global__ void __launch_bounds__(PLAN_THREADS)
 moe_plan_kernel(const int* __restrict__ ids, int P, int E, int tile, int max_tiles, int* __restrict__ pos, int* __restrict__ row_src,
-                int* __restrict__ tile_expert) {
+                int* __restrict__ tile_expert, int4* __restrict__ chunks, int chunk_tiles) {
     bl_pdl_trigger();
     bl_pdl_wait();
-    extern __shared__ int sh[];                        // counts [E], first tile [E + 1]
+    extern __shared__ int sh[];                        // counts [E], first tile [E + 1], first chunk [E]
     int* counts = sh;
     int* first = sh + E;
+    int* first_chunk = sh + 2 * E + 1;
     for (int e = threadIdx.x; e < E; e += PLAN_THREADS) counts[e] = 0;
-    for (int i = threadIdx.x; i < max_tiles; i += PLAN_THREADS) tile_expert[i] = -1;
+    for (int i = threadIdx.x; tile_expert && i < max_tiles; i += PLAN_THREADS) tile_expert[i] = -1;
     for (int i = threadIdx.x; i < max_tiles * tile; i += PLAN_THREADS) row_src[i] = -1;
     __syncthreads();
     for (int p = threadIdx.x; p < P; p += PLAN_THREADS)                                              // the pair's rank in its expert
         pos[p] = ids[p] < E ? atomicAdd(&counts[ids[p]], 1) : -1;                                    // (an identity expert: no row)
     __syncthreads();
     if (threadIdx.x == 0) {
-        int t = 0;
-        for (int e = 0; e < E; ++e) { first[e] = t; t += (counts[e] + tile - 1) / tile; }
+        int t = 0, c = 0;
+        for (int e = 0; e < E; ++e) {
+            const int n = (counts[e] + tile - 1) / tile;
+            first[e] = t;
+            t += n;
+            if (chunks) { first_chunk[e] = c; c += (n + chunk_tiles - 1) / chunk_tiles; }
+        }
         first[E] = t;
+        if (chunks) chunks[0] = make_int4(c, 0, 0, 0);
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < E; e += PLAN_THREADS)
-        for (int i = first[e]; i < first[e + 1]; ++i) tile_expert[i] = e;
+    for (int e = threadIdx.x; e < E; e += PLAN_THREADS) {
+        const int t0 = first[e], n = first[e + 1] - t0;
+        for (int i = 0; tile_expert && i < n; ++i) tile_expert[t0 + i] = e;
+        const int nc = chunks ? (n + chunk_tiles - 1) / chunk_tiles : 0;
+        for (int i = 0; i < nc; ++i) {                                         // chunks of even size
+            const int a = i * n / nc, b = (i + 1) * n / nc;
+            chunks[1 + first_chunk[e] + i] = make_int4((t0 + a) * tile, (b - a) * tile, e, 0);
+        }
+    }
     for (int p = threadIdx.x; p < P; p += PLAN_THREADS) {
         if (ids[p] >= E) continue;
         const int row = first[ids[p]] * tile + pos[p];
@@ -374,8 +388,24 @@ extern "C" int bl_moe_plan(const int* ids, int P, int E, int tile, int max_tiles
     const size_t smem = (size_t)(2 * E + 1) * sizeof(int);
     if (smem > 48 * 1024) BL_FAIL("bl_moe_plan: %d experts are too many for shared memory", E);
     BL_CUDA(bl_launch_dependent(moe_plan_kernel, dim3(1), dim3(PLAN_THREADS), smem, (cudaStream_t)stream, ids, P, E, tile, max_tiles, pos,
-                                row_src, tile_expert));
+                                row_src, tile_expert, (int4*)nullptr, 0));
     BL_CHECK_LAUNCH("bl_moe_plan");
+    return 0;
+}
+
+// The same in tiles of 16 rows, with each expert's run of rows cut into chunks of even size, `chunk_rows` rows at most: chunks [1 +
+// max_chunks][4] = {how many}, then {first row, rows, expert, 0} each. max_tiles >= ceil(P / 16) + E, max_chunks >= ceil(P / chunk_rows) + E.
+extern "C" int bl_moe_plan_chunks(const int* ids, int P, int E, int chunk_rows, int max_tiles, int max_chunks, int* pos, int* row_src,
+                                  int* chunks, void* stream) {
+    if (P <= 0) return 0;
+    if (E <= 0 || chunk_rows <= 0 || chunk_rows % 16 != 0 || max_tiles < (P + 15) / 16 + E || max_chunks < (P + chunk_rows - 1) / chunk_rows + E ||
+        ((uintptr_t)chunks & 15))
+        BL_FAIL("bl_moe_plan_chunks: %d pairs, %d experts, %d tiles, %d chunks of %d rows", P, E, max_tiles, max_chunks, chunk_rows);
+    const size_t smem = (size_t)(3 * E + 1) * sizeof(int);
+    if (smem > 48 * 1024) BL_FAIL("bl_moe_plan_chunks: %d experts are too many for shared memory", E);
+    BL_CUDA(bl_launch_dependent(moe_plan_kernel, dim3(1), dim3(PLAN_THREADS), smem, (cudaStream_t)stream, ids, P, E, 16, max_tiles, pos,
+                                row_src, (int*)nullptr, (int4*)chunks, chunk_rows / 16));
+    BL_CHECK_LAUNCH("bl_moe_plan_chunks");
     return 0;
 }
 

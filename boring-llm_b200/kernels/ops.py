@@ -852,6 +852,7 @@ def check_status() -> None:
                      ("bl_attention_prefill_tc", _lib().bl_attention_prefill_tc_status),
                      ("bl_gemm_tc_cols", _lib().bl_gemm_tc_cols_status),
                      ("bl_gemm_tc_splitk", _lib().bl_gemm_tc_splitk_status), ("bl_gemm_tc_few", _lib().bl_gemm_tc_few_status),
+                     ("bl_gemm_tc_experts", _lib().bl_gemm_tc_experts_status),
                      ("bl_attention_decode_tma", _lib().bl_attention_decode_tma_status)):
         v = ctypes.c_int(0)
         _call(fn, ctypes.byref(v))
@@ -1543,6 +1544,54 @@ def moe_plan(ids: torch.Tensor, n_experts: int):
     tile_expert = torch.empty(tiles, dtype=torch.int32, device=ids.device)
     _call(_lib().bl_moe_plan, _p(ids), P, n_experts, GROUPED_TILE, tiles, _p(pos), _p(row_src), _p(tile_expert), _stream())
     return pos, row_src, tile_expert
+
+
+EXPERT_TILE = 16           # rows of x that one expert's share of them is padded to (see `moe_chunks`)
+EXPERT_CHUNK, EXPERT_CHUNK_FEW = 256, 64     # the most rows of an expert that are multiplied together ...
+EXPERT_FEW_PAIRS = 32      # ... the second up to this many pairs an expert on average
+EXPERT_LARGE = 1 << 22     # values of one of an expert's matrices from which chunks are the faster form for many rows, too
+
+
+def experts_in_chunks(pairs: int, n_experts: int, dim: int, hidden: int) -> bool:
+    """Whether routed experts run in chunks with W as the M side (`moe_chunks`, `gemm_experts`) or in tiles of 128 rows (`moe_plan`,
+    `gemm_grouped`). Chunks pad nothing, but a work item is up to 256 rows by 128 of W, and small matrices make few of those for the
+    device. Both products, 16 experts of which a token has two, microseconds in tiles and in chunks:
+        tokens                                8           64           256          1,000       2,000
+        2,048 wide, 2,752 hidden values   79 / 72     110 / 89     110 / 92     135 / 117    190 / 166
+        896 wide, 1,216 hidden values     23 / 19      33 / 25      33 / 27                   48 / 57"""
+    return pairs <= EXPERT_FEW_PAIRS * n_experts or dim * hidden >= EXPERT_LARGE
+
+
+def moe_chunks(ids: torch.Tensor, n_experts: int):
+    """The layout of the pairs (token, chosen expert) for `gemm_experts`: (pos [P] the row of each pair, row_src [rows] the
+    pair of each row or -1, (chunks, chunk rows)); every expert's rows start a new tile of 16. Otherwise as `moe_plan`."""
+    P = ids.numel()
+    chunk = EXPERT_CHUNK_FEW if P <= EXPERT_FEW_PAIRS * n_experts else EXPERT_CHUNK
+    tiles, n_chunks = -(-P // EXPERT_TILE) + n_experts, -(-P // chunk) + n_experts
+    _need(ids, "ids", torch.int32)
+    pos = torch.empty(P, dtype=torch.int32, device=ids.device)
+    row_src = torch.empty(tiles * EXPERT_TILE, dtype=torch.int32, device=ids.device)
+    chunks = torch.empty((1 + n_chunks, 4), dtype=torch.int32, device=ids.device)
+    _call(_lib().bl_moe_plan_chunks, _p(ids), P, n_experts, chunk, tiles, n_chunks, _p(pos), _p(row_src), _p(chunks), _stream())
+    return pos, row_src, (chunks, chunk)
+
+
+def gemm_experts(x: torch.Tensor, w: torch.Tensor, chunks, out: torch.Tensor, epilogue: int = EPI_NONE,
+                 act: Optional[torch.Tensor] = None) -> None:
+    """out = epilogue(x @ w[expert of the row].T) on tcgen05, rows laid out by `moe_chunks`: x [rows, K] bfloat16, w [E, N, K],
+    out 32-bit; with EPI_SWIGLU w [E, 2N, K] (gate rows then up rows), out bfloat16 and `act` as for `gemm_grouped`."""
+    if act is not None:
+        if epilogue != EPI_SWIGLU:
+            raise KernelError("an activation goes with the gated epilogue only")
+        _need(act, "act", torch.float32, (2,))
+    M, K = x.shape
+    N = out.shape[1]
+    E = w.shape[0]
+    table, chunk = chunks
+    _need(x, "x", torch.bfloat16); _need(w, "w", torch.bfloat16, (E, 2 * N if epilogue == EPI_SWIGLU else N, K))
+    _need(out, "out", torch.bfloat16 if epilogue == EPI_SWIGLU else torch.float32, (M, N)); _need(table, "chunks", torch.int32)
+    _call(_lib().bl_gemm_tc_experts, _p(x), _p(w), _p(out), _dt(out), M, N, K, epilogue, E, _p(table), table.shape[0] - 1, chunk, _p(act),
+          _stream())
 
 
 def gather_rows(x: torch.Tensor, row_src: torch.Tensor, div: int, out: torch.Tensor, wts: Optional[torch.Tensor] = None) -> None:

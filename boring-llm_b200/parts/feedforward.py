@@ -381,14 +381,16 @@ class RoutedExperts(FeedForward):
         ids, wts = self.route(ctx, h)
         scale, left = (wts, None) if self.weight_input else (None, wts)
         if ctx.fast and ops.grouped_gemm_supported(h, self.w_gate_up) and self.hidden % 8 == 0:
-            # tensor cores: the pairs lie expert by expert in tiles of 128 rows, each tile multiplied by its expert's matrices
-            pos, row_src, tile_expert = ops.moe_plan(ids, self.E)
+            # tensor cores: the pairs lie expert by expert, each run of rows multiplied by its expert's matrices
+            in_chunks = ops.experts_in_chunks(ids.numel(), self.E, self.dim, self.hidden)
+            pos, row_src, runs = ops.moe_chunks(ids, self.E) if in_chunks else ops.moe_plan(ids, self.E)
+            product = ops.gemm_experts if in_chunks else ops.gemm_grouped
             rows = ctx.empty((row_src.numel(), self.dim))
             ops.gather_rows(h, row_src, self.top, rows, scale)
             act = ctx.empty((row_src.numel(), self.hidden))
-            ops.gemm_grouped(rows, self.w_gate_up, tile_expert, act, EPI_SWIGLU, self.act_args)
+            product(rows, self.w_gate_up, runs, act, EPI_SWIGLU, self.act_args)
             y = ctx.empty((row_src.numel(), self.dim), torch.float32)
-            ops.gemm_grouped(act, self.w_down, tile_expert, y, EPI_NONE)
+            product(act, self.w_down, runs, y, EPI_NONE)
             return y, pos, left, ids
         rows, per = h, self.top
         if scale is not None:

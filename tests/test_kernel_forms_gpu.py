@@ -920,3 +920,43 @@ def test_prompts_and_single_tokens_side_by_side(H, KV, dh, window):
         graph.replay()
         assert all(torch.equal(a, b) for a, b in zip(got, want)) and word.item() == 0
     o.check_status()
+
+
+@pytest.mark.parametrize("K, N", [(256, 192), (200, 72), (8, 8), (1216, 100)])
+@pytest.mark.parametrize("T, E, top, spread", [(1, 3, 2, "even"), (50, 4, 2, "even"), (300, 4, 1, "one"), (700, 3, 2, "skewed"), (1030, 16, 2, "even")])
+def test_products_of_routed_experts_in_chunks(K, N, T, E, top, spread):
+    """`gemm_experts` behind `moe_chunks`, gated and plain, against float64: experts without rows, one expert with all (several chunks),
+    shares of every size modulo 16, inner sizes and columns that are not multiples of a tile. A 32-bit sum of K products of bfloat16
+    values is off by at most K eps times the sum of their sizes; the gated result is rounded to bfloat16 (2^-8) once more."""
+    o = ops()
+    g = torch.Generator().manual_seed(T + K)
+    if spread == "one":
+        ids = torch.full((T, 1), 2, dtype=torch.int32)
+    else:
+        p = torch.ones(E) if spread == "even" else torch.tensor([0.9, 0.09, 0.01][:E])
+        ids = torch.stack([torch.multinomial(p, top, generator=g) for _ in range(T)]).int()
+    x = (torch.randn(T, K, generator=g) * 0.5).bfloat16()
+    w = (torch.randn(E, 2 * N, K, generator=g) * 0.2).bfloat16()
+    pos, row_src, chunks = o.moe_chunks(ids.to(DEV), E)
+    assert row_src.numel() == (-(-T * top // 16) + E) * 16
+    at = pos.long().cpu()
+    assert torch.equal(row_src.cpu()[at], torch.arange(T * top, dtype=torch.int32)) and int((row_src >= 0).sum()) == T * top
+    rows = torch.empty((row_src.numel(), K), dtype=BF, device=DEV)
+    o.gather_rows(x.to(DEV), row_src, top, rows)
+    e, t = ids.flatten().long(), torch.arange(T).repeat_interleave(top)
+    full = torch.empty(T * top, 2 * N, dtype=torch.float64)
+    size = torch.empty(T * top, 2 * N, dtype=torch.float64)
+    for k in range(E):
+        mine = e == k
+        full[mine] = x[t[mine]].double() @ w[k].double().T
+        size[mine] = x[t[mine]].double().abs() @ w[k].double().abs().T
+    off = K * 2.0 ** -23 * size
+    y = torch.empty((row_src.numel(), 2 * N), dtype=torch.float32, device=DEV)
+    o.gemm_experts(rows, w.to(DEV), chunks, y)
+    assert ((y[pos.long()].double().cpu() - full).abs() <= off + 1e-30).all()
+    act = torch.empty((row_src.numel(), N), dtype=BF, device=DEV)
+    o.gemm_experts(rows, w.to(DEV), chunks, act, o.EPI_SWIGLU)
+    want = full[:, :N] * torch.sigmoid(full[:, :N]) * full[:, N:]
+    slack = 1.1 * off[:, :N] * full[:, N:].abs() + full[:, :N].abs() * off[:, N:] + 1e-5 * want.abs()     # |silu'| <= 1.1; the sigmoid's own error
+    assert ((act[pos.long()].double().cpu() - want).abs() <= slack + 2.0 ** -8 * want.abs() + 1e-30).all()
+    o.check_status()
