@@ -844,7 +844,7 @@ def test_few_rows_go_by_the_bytes_of_w():
     o = ops()
     m = lambda *s: torch.empty(*s, dtype=BF, device=DEV)
     kinds = [(8, 8208, 2048, o.EPI_NONE, "few"), (8, 2560, 2048, o.EPI_BIAS, "skinny"), (16, 2560, 2048, o.EPI_BIAS, "few"), (16, 2048, 2048, o.EPI_RESIDUAL, "skinny"),
-             (17, 896, 4864, o.EPI_RESIDUAL, "few"), (64, 3600, 896, o.EPI_NONE, "few"), (64, 1152, 896, o.EPI_BIAS, "skinny"), (64, 11008, 2048, o.EPI_NONE, "tc"),
+             (17, 896, 4864, o.EPI_RESIDUAL, "few"), (64, 896, 4864, o.EPI_RESIDUAL, "splitk"), (64, 3600, 896, o.EPI_NONE, "few"), (64, 1152, 896, o.EPI_BIAS, "skinny"), (64, 11008, 2048, o.EPI_NONE, "tc"),
              (16, 11008, 2048, o.EPI_SWIGLU, "few"), (32, 11008, 2048, o.EPI_SWIGLU, "tc"), (65, 8208, 2048, o.EPI_NONE, "splitk")]
     for M, N, K, epi, kind in kinds:
         b = torch.empty(N, device=DEV) if epi == o.EPI_BIAS else None
