@@ -1,31 +1,38 @@
 // The 32-bit product on the fifth-generation tensor cores: out[M, N] = epilogue(x[M, K] . W[N, K]^T), 32-bit operands and results.
 //
-// A 32-bit number v is split into hi, its first 11 significant bits (tf32), and lo = v - hi rounded to tf32: hi + lo is v to
-// 2^-22. A product is then hi hi' + (lo hi' + hi lo'), whose missing lo lo' is 2^-20 of it at most, 2^-22 on average. The tensor cores add
-// into a 32-bit accumulator, but they cut bits off where a register's addition rounds, an error that has a sign and grows with
-// the number of additions. So they sum 32 values of k at a time, the small products first, and threads add these segments' sums up
-// in registers, rounded to nearest, in ascending k: 28 rounded additions for K = 896 where a chain of FMAs makes 896.
-// Errors against 64 bits are no larger than such a chain's (the test of this kernel has both).
+// A 32-bit number has 24 significant bits. It is split into three bfloat16 numbers of 8 (each the rest so far rounded to nearest;
+// Henry, Tang and Heinecke, "Leveraging the bfloat16 artificial intelligence datatype for higher-precision computations", 2019), whose
+// sum IS the number. Of the nine products of two such triples all but the last (2^-32 of the whole at most) are made, each exact.
+// The tensor cores add into a 32-bit accumulator, but they cut bits off where a register's addition rounds, an error that has a sign
+// and grows with the number of additions. So the first parts' products have an accumulator of their own, which holds one of them exactly,
+// for 32 values of k at a time: threads add such segments up in registers, rounded to nearest, in ascending k. The other products,
+// 2^-8 of those, stay in a second accumulator, which is added at the end. A product alone is then rounded as an FMA rounds it, and
+// K = 896 makes 29 rounded additions where a chain of FMAs makes 896. Errors against 64 bits are no larger than such a chain's, of
+// rows with a few numbers as of full ones (the tests of this kernel have both).
 //
 // W is the M side of the MMA (128 rows of W a tile; with SWIGLU 64 gate rows and the 64 up rows that match) and NT rows of x its
-// N side. A block: TMA brings 32 values of k of the tile's rows into a ring; 8 warps split them and store both halves where the MMAs
-// read them (128-byte swizzle), one thread of the first of them issues the segment's 12 MMAs into one of two accumulators, one of the
-// second refills the ring; 4 or 8 warps add the other accumulator to their registers. (Rows fetched ahead into the splitters' own
+// N side. A block: TMA brings 32 values of k of the tile's rows into a ring; 8 warps split them and store the parts where the MMAs
+// read them (64-byte swizzle); a warp of its own issues the segment's MMAs into one of two accumulators (and the one of the small
+// products) and refills the ring; 4 or 8 warps add the other accumulator to their registers. (Rows fetched ahead into the splitters' own
 // registers cannot be: the fence that shows their stores to the tensor cores waits for every load under way, 1,600 cycles a
 // segment.) At the end the tile passes through shared memory to the epilogue. Products of few tiles cut K over the blocks of a
 // cluster (f32_tc_spans), whose totals are added in ascending k through distributed shared memory. What a result is computed from, and
 // in which order, depends on N and K only: it is the same whatever rows stand beside a row and however wide a tile is (the same promise
 // that the kernels in gemm_plain.cu make, which keep the small products).
-// A sum that is not finite (an infinity or NaN among the inputs, whose halves are NaN, or an overflow) is worked out again as
-// a chain of FMAs over the inputs themselves.
+// A sum that is not finite (an infinity or NaN among the inputs, or an overflow) is worked out again as a chain of FMAs over the
+// inputs themselves. So is a small one, |sum| < 2^-48, of a row of x or of W with an operand other than 0 below 2^-50: the parts of such
+// operands may lie below bfloat16's smallest numbers (an operand from 2^-110 on loses nothing, a smaller one 2^-134 at most), and
+// products of them below 32-bit ones. With the other operand under 2^40 (else the row's every sum is worked out again) that is
+// less than 2^-24 of any larger sum.
 //
-// Bound by the splitting (every 4 bytes of W are read from shared memory once, stored twice, and read three times by the MMAs) and,
-// for many rows, the tensor cores (12 MMAs a segment, 830 cycles for 128 x 128). Microseconds, before (FMAs) -> now:
+// Bound by shared memory: a segment's bytes are written and read once as they come, its parts (6 bytes a number) written once and read
+// by the eight MMAs of each 16 values of k. Issued by a warp that splits as well, the MMAs held up the next segment's splitting (4,864 +
+// 4,864 x 896: 1 row 27.3 us, 366 rows 89). Microseconds, FMAs (gemm_plain.cu) -> this:
 //   rows                          1             16            128           366           2,048
-//   1,152 x 896, bias             7.8 -> 8.3    8.7 -> 8.4    19.7 -> 19.0   31 -> 25     118 -> 71
-//   896 x 896, residual           7.7 -> 8.2    8.8 -> 8.5    17.8 -> 10.7   33 -> 14     110 -> 62
-//   9,728 + 9,728 x 896, gated   13.6 -> 24.0    25 -> 24.3     71 -> 38    178 -> 75     876 -> 335
-//   896 x 4,864, residual          55 -> 31      48 -> 31.6     84 -> 36    158 -> 47     557 -> 203
+//   1,152 x 896, bias             7.8 -> 7.7    8.7 -> 8.1    19.7 -> 18.8   31 -> 26     118 -> 75
+//   896 x 896, residual           7.7 -> 7.8    8.8 -> 8.1    17.8 -> 10.5   33 -> 15     110 -> 64
+//   4,864 + 4,864 x 896, gated   13.6 -> 23.7    25 -> 24.2     71 -> 36    178 -> 69     876 -> 308
+//   896 x 4,864, residual          55 -> 31      48 -> 31.3     84 -> 34    158 -> 42     557 -> 179
 // Every wait on an mbarrier is bounded; when a bound runs out the block records a code in a status word and stops computing, but
 // still meets its cluster, frees its tensor memory and returns (bl_gemm_f32_tc_status).
 #include "tcgen05.cuh"
@@ -35,22 +42,26 @@ namespace {
 
 constexpr int BM = 128;                    // rows of W a tile
 constexpr int MAX_COLUMNS = 1 << 15;       // more: an output head
-constexpr int BK = 32;                     // values of k a segment: one 128-byte row of the swizzled operand tiles
-constexpr int SPLITTERS = 256, ADDERS = 256, THREADS = SPLITTERS + ADDERS;
-constexpr int TMEM_COLS = 256;             // two accumulators of up to 128 columns
+constexpr int BK = 32;                     // values of k a segment: rows of 128 bytes as they come, 64 bytes a part
+constexpr int SPLITTERS = 256, ADDERS = 256, THREADS = SPLITTERS + ADDERS + 32;    // the last warp issues
+constexpr float SMALL_SUM = 3.5527136788005009e-15f;          // 2^-48
+constexpr uint32_t SMALL_OPERAND = (127u - 50u) << 24;         // 2^-50, its bits without the sign, doubled
+constexpr float HUGE_OPERAND = 1099511627776.f;                // 2^40
 constexpr uint32_t WAIT_LIMIT = 1u << 22;
 
 template <int NT>
 struct Tile {
-    static constexpr int W_BYTES = BM * 128, X_BYTES = NT * 128, RAW_BYTES = W_BYTES + X_BYTES, PAIR_BYTES = 2 * RAW_BYTES;     // as they came; hi and lo
-    static constexpr int PAIRS = NT >= 64 ? 2 : 3;                        // stages of halves
-    static constexpr int RAWS = NT == 128 ? 2 : NT >= 64 ? 3 : 5;         // stages of the ring
+    static constexpr int RAW_W = BM * 128, RAW_BYTES = RAW_W + NT * 128;  // a segment as it comes
+    static constexpr int W_BYTES = BM * 64, X_BYTES = NT * 64, PART_BYTES = 3 * (W_BYTES + X_BYTES);     // and in parts: W's three, x's three
+    static constexpr int PARTS = NT >= 64 ? 2 : 3;                        // stages of parts
+    static constexpr int RAWS = NT == 128 ? 3 : NT >= 64 ? 4 : 5;         // stages of the ring
+    static constexpr int TMEM_COLS = NT >= 96 ? 512 : 4 * NT;             // three accumulators of NT columns
     static constexpr int HALVES = NT >= 64 ? 2 : 1;                       // the columns are dealt to one or two groups of four adder warps
     static constexpr int COLS = NT / HALVES;
     static constexpr int CHUNKS = 4 + (NT + 31) / 32;                     // 16-byte pieces of a segment a splitter
-    static constexpr int OFF_RAW = PAIRS * PAIR_BYTES, OFF_BARS = OFF_RAW + RAWS * RAW_BYTES;
-    static constexpr int SMEM_BYTES = OFF_BARS + 256 + 1024;
-    static_assert(NT % 16 == 0 && COLS % 16 == 0 && BM * NT * 4 <= OFF_RAW && SMEM_BYTES <= 227 * 1024, "tile");
+    static constexpr int OFF_RAW = PARTS * PART_BYTES, OFF_BARS = OFF_RAW + RAWS * RAW_BYTES, OFF_MARKS = OFF_BARS + 256;
+    static constexpr int SMEM_BYTES = OFF_MARKS + BM + NT + 1024;
+    static_assert(NT % 16 == 0 && COLS % 16 == 0 && 2 * BM * NT * 4 <= OFF_BARS && SMEM_BYTES <= 227 * 1024, "tile");
 };
 
 __device__ int g_status = 0;               // 0 = fine; else the code of the first wait that ran out
@@ -71,9 +82,11 @@ __device__ __forceinline__ void mbar_wait_plain(uint32_t bar, uint32_t parity) {
     for (uint32_t i = 0; i < WAIT_LIMIT; ++i)
         if (mbar_try_wait(bar, parity)) return;
 }
-__device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}"
-                 :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+// Operand tile of rows of 64 bytes (32 bfloat16 values of k) with 64-byte swizzle: groups of 8 rows 512 bytes apart.
+__device__ __forceinline__ uint64_t smem_desc64(uint32_t addr) {
+    const uint32_t lo = ((addr >> 4) & 0x3FFFu) | (1u << 16);
+    const uint32_t hi = (512u >> 4) | (1u << 14) | (4u << 29);
+    return ((uint64_t)hi << 32) | lo;
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -83,10 +96,14 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
                    "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                  : "r"(taddr) : "memory");
 }
-// The halves of a number: its first 11 significant bits, and the rest rounded to 11. Integer arithmetic: the conversion instruction
-// runs at a fraction of its rate. (The first half of an infinity or a NaN is one, too.)
-__device__ __forceinline__ float first_half(float v) { return __uint_as_float(__float_as_uint(v) & 0xffffe000u); }
-__device__ __forceinline__ float second_half(float v, float first) { return __uint_as_float((__float_as_uint(v - first) + 0x1000u) & 0xffffe000u); }
+// The next parts of two numbers as a pair, and what is left of them.
+__device__ __forceinline__ uint32_t next_parts(float& a, float& b) {
+    const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
+    const uint32_t u = *reinterpret_cast<const uint32_t*>(&p);
+    a -= __uint_as_float(u << 16);
+    b -= __uint_as_float(u & 0xffff0000u);
+    return u;
+}
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -110,17 +127,19 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     using T = Tile<NT>;
     constexpr bool GLU = EPI == BL_EPI_SWIGLU;
     constexpr int UNITS = GLU ? BM / 2 : BM;                              // outputs of a row of x a tile
-    constexpr int PAIRS = T::PAIRS, RAWS = T::RAWS;
-    // D 32-bit, A and B tf32 and K-major, N >> 3 at bit 17, M >> 4 at bit 24
-    constexpr uint32_t IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+    constexpr int PARTS = T::PARTS, RAWS = T::RAWS;
+    // D 32-bit, A and B bfloat16 and K-major, N >> 3 at bit 17, M >> 4 at bit 24
+    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
     extern __shared__ unsigned char smem_raw[];
     if (threadIdx.x == 0) { tma_prefetch_map(&map_x); tma_prefetch_map(&map_w); }
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     unsigned char* smem = smem_raw + (base - smem_u32(smem_raw));
-    const uint32_t raw_full0 = base + T::OFF_BARS, raw_read0 = raw_full0 + 8 * RAWS, full0 = raw_read0 + 8 * RAWS, empty0 = full0 + 8 * PAIRS,
-                   sum0 = empty0 + 8 * PAIRS, taken0 = sum0 + 16;
+    const uint32_t raw_full0 = base + T::OFF_BARS, raw_read0 = raw_full0 + 8 * RAWS, full0 = raw_read0 + 8 * RAWS, empty0 = full0 + 8 * PARTS,
+                   sum0 = empty0 + 8 * PARTS, taken0 = sum0 + 16;
     volatile int* give_up = reinterpret_cast<volatile int*>(smem + T::OFF_BARS + 192);
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + T::OFF_BARS + 200);
+    int* any_small = reinterpret_cast<int*>(smem + T::OFF_BARS + 208);    // whether a row of the tile has a small operand
+    unsigned char* marks = smem + T::OFF_MARKS;                           // of the tile's rows of W and then of x: 1 a small operand, 2 a huge one
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     // a cluster is the spans of one tile; the tiles of rows are neighbours, so that a tile of W is fetched from memory once
     const int span = blockIdx.x % spans, tile = blockIdx.x / spans;
@@ -129,8 +148,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     const int first = min(span * each, all), steps = min(each, all - first);
     if (threadIdx.x == 0) {
         *give_up = 0;
+        *any_small = 0;
         for (int s = 0; s < RAWS; ++s) { mbar_init(raw_full0 + 8 * s, 1); mbar_init(raw_read0 + 8 * s, SPLITTERS / 32); }
-        for (int s = 0; s < PAIRS; ++s) { mbar_init(full0 + 8 * s, SPLITTERS / 32); mbar_init(empty0 + 8 * s, 1); }
+        for (int s = 0; s < PARTS; ++s) { mbar_init(full0 + 8 * s, SPLITTERS / 32); mbar_init(empty0 + 8 * s, 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(sum0 + 8 * b, 1); mbar_init(taken0 + 8 * b, 4 * T::HALVES); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -139,19 +159,19 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         const uint32_t bar = raw_full0 + 8 * (s % RAWS), dst = base + T::OFF_RAW + s % RAWS * T::RAW_BYTES;
         mbar_expect_tx(bar, T::RAW_BYTES);
         tma_load_2d(dst, &map_w, bar, (first + s) * BK, n0);
-        if (GLU) tma_load_2d(dst + T::W_BYTES / 2, &map_w, bar, (first + s) * BK, N + n0);
+        if (GLU) tma_load_2d(dst + T::RAW_W / 2, &map_w, bar, (first + s) * BK, N + n0);
     };
     auto load_x = [&](int s) {
-        tma_load_2d(base + T::OFF_RAW + s % RAWS * T::RAW_BYTES + T::W_BYTES, &map_x, raw_full0 + 8 * (s % RAWS), (first + s) * BK, m0);
+        tma_load_2d(base + T::OFF_RAW + s % RAWS * T::RAW_BYTES + T::RAW_W, &map_x, raw_full0 + 8 * (s % RAWS), (first + s) * BK, m0);
     };
     const int early = min(RAWS, steps);
-    if (warp == 9 && elect_one())                                          // W does not depend on the kernel before this one
+    if (warp == 16 && elect_one())                                         // W does not depend on the kernel before this one
         for (int s = 0; s < early; ++s) load_w(s);
     __syncwarp();
     if (warp == 8) {
         __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     :: "r"(smem_u32((const void*)tmem_slot)), "r"(TMEM_COLS) : "memory");
+                     :: "r"(smem_u32((const void*)tmem_slot)), "r"(T::TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     fence_before_sync();
@@ -159,21 +179,62 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     fence_after_sync();
     const uint32_t tmem = *tmem_slot;
     bool ok = true;
-    float* sums = reinterpret_cast<float*>(smem);                          // in the end: [column][row of the tile]
+    float* sums = reinterpret_cast<float*>(smem);                          // in the end: [first products, small ones][column][row of the tile]
     bl_pdl_wait();
     bl_pdl_trigger();
 
-    if (warp >= 8) {
-        // ================= splitters: thread (row t / 8 + 32 i, piece t % 8) of W (i < 4) and of x (i >= 4)
-        const int t = threadIdx.x - ADDERS, row = t >> 3, piece = t & 7;
+    if (warp == 16) {
+        // ================= the segments' MMAs and copies
         int issued = early;
-        if (warp == 9 && elect_one())
+        if (elect_one())
             for (int s = 0; s < early; ++s) load_x(s);
         __syncwarp();
-        const uint32_t from = base + T::OFF_RAW + (uint32_t)row * 128 + (uint32_t)piece * 16;
-        const uint32_t to = base + (uint32_t)row * 128 + (uint32_t)((piece ^ (row & 7)) << 4);       // (rows 32 apart swizzle alike)
         for (int s = 0; s < steps; ++s) {
-            const int rs = s % RAWS, st = s % PAIRS, b = s & 1;
+            const int rs = s % RAWS, st = s % PARTS, b = s & 1;
+            ok = mbar_wait(full0 + 8 * st, (uint32_t)((s / PARTS) & 1), give_up, 2);
+            if (ok && s >= 2) ok = mbar_wait(taken0 + 8 * b, (uint32_t)((s / 2 - 1) & 1), give_up, 2);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            if (elect_one()) {
+                fence_after_sync();
+                const uint32_t stage = base + st * T::PART_BYTES, sum = tmem + b * NT, rest = tmem + 2 * NT;
+                const uint64_t w1 = smem_desc64(stage), w2 = smem_desc64(stage + T::W_BYTES), w3 = smem_desc64(stage + 2 * T::W_BYTES);
+                const uint64_t x1 = smem_desc64(stage + 3 * T::W_BYTES), x2 = smem_desc64(stage + 3 * T::W_BYTES + T::X_BYTES),
+                               x3 = smem_desc64(stage + 3 * T::W_BYTES + 2 * T::X_BYTES);
+#pragma unroll
+                for (int k = 0; k < BK / 8; k += 2) {                  // 16 values of k, two 16-byte units of a descriptor
+                    umma_bf16(sum, w1 + k, x1 + k, IDESC, k != 0);
+                    umma_bf16(rest, w1 + k, x2 + k, IDESC, (s | k) != 0);
+                    umma_bf16(rest, w1 + k, x3 + k, IDESC, 1);
+                    umma_bf16(rest, w2 + k, x1 + k, IDESC, 1);
+                    umma_bf16(rest, w2 + k, x2 + k, IDESC, 1);
+                    umma_bf16(rest, w2 + k, x3 + k, IDESC, 1);
+                    umma_bf16(rest, w3 + k, x1 + k, IDESC, 1);
+                    umma_bf16(rest, w3 + k, x2 + k, IDESC, 1);
+                }
+                umma_commit(empty0 + 8 * st);
+                umma_commit(sum0 + 8 * b);
+            }
+            __syncwarp();
+            if (s + RAWS < steps) {                                        // the ring's stage takes the segment RAWS on
+                ok = mbar_wait(raw_read0 + 8 * rs, (uint32_t)((s / RAWS) & 1), give_up, 2);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                if (elect_one()) { load_w(s + RAWS); load_x(s + RAWS); }
+                __syncwarp();
+                issued = s + RAWS + 1;
+            }
+        }
+        if (*give_up)                                                      // let our own copies land before leaving
+            for (int s = max(0, issued - RAWS); s < issued; ++s) mbar_wait_plain(raw_full0 + 8 * (s % RAWS), (uint32_t)((s / RAWS) & 1));
+    } else if (warp >= 8) {
+        // ================= splitters: thread (row t / 8 + 32 i, piece t % 8) of W (i < 4) and of x (i >= 4)
+        const int t = threadIdx.x - ADDERS, row = t >> 3, piece = t & 7;
+        const uint32_t from = base + T::OFF_RAW + (uint32_t)row * 128 + (uint32_t)piece * 16;
+        const uint32_t to = base + (uint32_t)row * 64 + (uint32_t)(((piece >> 1) ^ ((row >> 1) & 3)) << 4) + (piece & 1) * 8;       // (rows 32 apart swizzle alike)
+        uint32_t held = 0;                                                 // two bits of each of the thread's rows: a small operand, a huge one
+        for (int s = 0; s < steps; ++s) {
+            const int rs = s % RAWS, st = s % PARTS;
             ok = mbar_wait(raw_full0 + 8 * rs, (uint32_t)((s / RAWS) & 1), give_up, 1);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
@@ -184,58 +245,38 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[i].x), "=f"(v[i].y), "=f"(v[i].z), "=f"(v[i].w)
                              : "r"(from + rs * T::RAW_BYTES + i * 4096) : "memory");
             }
-            if (s >= PAIRS) {
-                ok = mbar_wait(empty0 + 8 * st, (uint32_t)((s / PAIRS - 1) & 1), give_up, 1);
+            if (s >= PARTS) {
+                ok = mbar_wait(empty0 + 8 * st, (uint32_t)((s / PARTS - 1) & 1), give_up, 1);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
             }
 #pragma unroll
             for (int i = 0; i < T::CHUNKS; ++i) {
                 if (i >= 4 && row + 32 * (i - 4) >= NT) continue;
-                const float4 a = v[i];
-                const float4 h = make_float4(first_half(a.x), first_half(a.y), first_half(a.z), first_half(a.w));
-                const float4 l = make_float4(second_half(a.x, h.x), second_half(a.y, h.y), second_half(a.z, h.z), second_half(a.w, h.w));
-                const uint32_t at = to + st * T::PAIR_BYTES + (i < 4 ? i * 4096 : 2 * T::W_BYTES + (i - 4) * 4096);
-                const uint32_t at_lo = at + (i < 4 ? T::W_BYTES : T::X_BYTES);
-                asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" :: "r"(at), "f"(h.x), "f"(h.y), "f"(h.z), "f"(h.w) : "memory");
-                asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" :: "r"(at_lo), "f"(l.x), "f"(l.y), "f"(l.z), "f"(l.w) : "memory");
+                float4 a = v[i];
+                const uint32_t least = min(min(2 * __float_as_uint(a.x) - 1, 2 * __float_as_uint(a.y) - 1), min(2 * __float_as_uint(a.z) - 1, 2 * __float_as_uint(a.w) - 1));   // 0 is the largest
+                const float most = fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w)));
+                if (least < SMALL_OPERAND - 1) held |= 1u << (2 * i);
+                if (most >= HUGE_OPERAND) held |= 2u << (2 * i);
+                const uint32_t at = to + st * T::PART_BYTES + (i < 4 ? i * 2048 : 3 * T::W_BYTES + (i - 4) * 2048);
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    const uint32_t lo = next_parts(a.x, a.y), hi = next_parts(a.z, a.w);
+                    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(at + j * (i < 4 ? T::W_BYTES : T::X_BYTES)), "r"(lo), "r"(hi) : "memory");
+                }
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) { mbar_arrive(full0 + 8 * st); mbar_arrive(raw_read0 + 8 * rs); }
-            if (warp == 8) {                                               // the segment's MMAs
-                ok = mbar_wait(full0 + 8 * st, (uint32_t)((s / PAIRS) & 1), give_up, 2);
-                if (ok && s >= 2) ok = mbar_wait(taken0 + 8 * b, (uint32_t)((s / 2 - 1) & 1), give_up, 2);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                if (elect_one()) {
-                    fence_after_sync();
-                    const uint32_t stage = base + st * T::PAIR_BYTES, d = tmem + b * 128;
-                    const uint64_t wh = smem_desc(stage), wl = smem_desc(stage + T::W_BYTES);
-                    const uint64_t xh = smem_desc(stage + 2 * T::W_BYTES), xl = smem_desc(stage + 2 * T::W_BYTES + T::X_BYTES);
-#pragma unroll
-                    for (int k = 0; k < BK / 8; ++k) {                     // the small products first
-                        umma_tf32(d, wl + 2 * k, xh + 2 * k, IDESC, k != 0);
-                        umma_tf32(d, wh + 2 * k, xl + 2 * k, IDESC, 1);
-                    }
-#pragma unroll
-                    for (int k = 0; k < BK / 8; ++k) umma_tf32(d, wh + 2 * k, xh + 2 * k, IDESC, 1);
-                    umma_commit(empty0 + 8 * st);
-                    umma_commit(sum0 + 8 * b);
-                }
-                __syncwarp();
-            }
-            if (warp == 9 && s + RAWS < steps) {                           // the ring's stage takes the segment RAWS on
-                ok = mbar_wait(raw_read0 + 8 * rs, (uint32_t)((s / RAWS) & 1), give_up, 1);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                if (elect_one()) { load_w(s + RAWS); load_x(s + RAWS); }
-                __syncwarp();
-                issued = s + RAWS + 1;
-            }
         }
-        if (warp == 9 && *give_up)                                         // let our own copies land before leaving
-            for (int s = max(0, issued - RAWS); s < issued; ++s) mbar_wait_plain(raw_full0 + 8 * (s % RAWS), (uint32_t)((s / RAWS) & 1));
+#pragma unroll
+        for (int d = 1; d < 8; d *= 2) held |= __shfl_xor_sync(0xffffffffu, held, d);          // the row's eight threads
+        if (piece == 0) {
+#pragma unroll
+            for (int i = 0; i < T::CHUNKS; ++i)
+                if (i < 4 || row + 32 * (i - 4) < NT) marks[row + 32 * i] = (unsigned char)(held >> (2 * i) & 3);
+            if (held & 0x55555555u) *any_small = 1;
+        }
     } else if (warp < 4 * T::HALVES) {
         // ================= adders: row 32 (warp & 3) + lane of the tile, COLS of its columns
         const uint32_t t_at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * T::COLS;
@@ -251,7 +292,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 #pragma unroll
             for (int c = 0; c < T::COLS; c += 16) {
                 uint32_t r[16];
-                tmem_ld16(t_at + b * 128 + c, r);
+                tmem_ld16(t_at + b * NT + c, r);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) acc[c + j] += __uint_as_float(r[j]);
             }
@@ -259,32 +300,62 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             __syncwarp();
             if (lane == 0) mbar_arrive(taken0 + 8 * b);
         }
-        // the last segment's MMAs have read the halves, which make room for the sums
+        // the last segment's MMAs have read the parts, which make room for the sums, and for those of the small products
+        const int at = (warp >> 2) * T::COLS * BM + (warp & 3) * 32 + lane;
 #pragma unroll
-        for (int j = 0; j < T::COLS; ++j) sums[((warp >> 2) * T::COLS + j) * BM + (warp & 3) * 32 + lane] = acc[j];
+        for (int j = 0; j < T::COLS; ++j) sums[at + j * BM] = acc[j];
+#pragma unroll
+        for (int c = 0; c < T::COLS; c += 16) {
+            uint32_t r[16] = {};
+            if (ok && steps > 0) tmem_ld16(t_at + 2 * NT + c, r);          // (the warps agree on ok, and the last segment's barrier has been waited for)
+#pragma unroll
+            for (int j = 0; j < 16; ++j) sums[BM * NT + at + (c + j) * BM] = __uint_as_float(r[j]);
+        }
     }
     if (spans > 1) cluster_sync(); else __syncthreads();
     const BlGluArgs glu = bl_glu_args(GLU ? bias : nullptr);
+    auto peer_byte = [&](const void* at, int r) {                          // a byte of the shared memory of block r of the cluster
+        if (spans == 1) return (int)*reinterpret_cast<const unsigned char*>(at);
+        uint32_t peer, v;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(smem_u32(at)), "r"(r));
+        asm volatile("ld.shared::cluster.u8 %0, [%1];" : "=r"(v) : "r"(peer) : "memory");
+        return (int)v;
+    };
+    int small_tile = 0;
+    for (int r = 0; r < spans; ++r) small_tile |= peer_byte(any_small, r);
+    // Whether the sum of row `col` of the tile's x and row `u` of its W is worked out again: by what these two rows hold, nothing else.
+    auto again = [&](float sum, int u, int col) {
+        if (!isfinite(sum)) return true;
+        if (!small_tile) return false;
+        int mark = 0;
+        for (int r = 0; r < spans; ++r) mark |= peer_byte(marks + u, r) | peer_byte(marks + BM + col, r);
+        return (mark & 1) != 0 && ((mark & 2) != 0 || fabsf(sum) < SMALL_SUM);
+    };
     // the outputs of the tile, neighbours along n in neighbouring threads; a cluster's blocks take a share each
     for (int e = span * THREADS + threadIdx.x; e < NT * UNITS; e += spans * THREADS) {
         const int u = e % UNITS, col = e / UNITS;
         const int m = m0 + col, n = n0 + u;
         if (m >= M || n >= N) continue;
-        const uint32_t mine = base + (uint32_t)(col * BM + u) * 4;       // (the up sums of a gated tile are its rows 64 on)
+        const uint32_t mine = base + (uint32_t)(col * BM + u) * 4, small = BM * NT * 4;      // (the up sums of a gated tile are its rows 64 on)
         float s = 0.f, up = 0.f;
         if (spans == 1) {
-            s = *reinterpret_cast<const float*>(smem + (mine - base));
-            if (GLU) up = *reinterpret_cast<const float*>(smem + (mine - base) + 4 * UNITS);
+            const float* at = reinterpret_cast<const float*>(smem + (mine - base));
+            s = at[0] + at[BM * NT];
+            if (GLU) up = at[UNITS] + at[BM * NT + UNITS];
         } else {
+            float rest = 0.f, up_rest = 0.f;
             for (int r = 0; r < spans; ++r) {                              // ascending k
                 uint32_t peer;
                 asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(mine), "r"(r));
-                s = r == 0 ? ld_cluster(peer) : s + ld_cluster(peer);
-                if (GLU) up = r == 0 ? ld_cluster(peer + 4 * UNITS) : up + ld_cluster(peer + 4 * UNITS);
+                s += ld_cluster(peer);
+                rest += ld_cluster(peer + small);
+                if (GLU) { up += ld_cluster(peer + 4 * UNITS); up_rest += ld_cluster(peer + small + 4 * UNITS); }
             }
+            s += rest;
+            up += up_rest;
         }
-        if (!isfinite(s)) s = plain_dot(x + (size_t)m * ldx, w + (size_t)n * K, K);
-        if (GLU && !isfinite(up)) up = plain_dot(x + (size_t)m * ldx, w + (size_t)(N + n) * K, K);
+        if (again(s, u, col)) s = plain_dot(x + (size_t)m * ldx, w + (size_t)n * K, K);
+        if (GLU && again(up, UNITS + u, col)) up = plain_dot(x + (size_t)m * ldx, w + (size_t)(N + n) * K, K);
         float* dst = out + (size_t)m * N + n;
         if (EPI == BL_EPI_BIAS) s += bl_load_any(bias, bias_dtype, n);
         if (EPI == BL_EPI_RESIDUAL) {
@@ -301,7 +372,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     if (spans > 1) cluster_sync(); else __syncthreads();                   // no block leaves while another may still read its sums
     if (warp == 8) {
         fence_after_sync();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(T::TMEM_COLS) : "memory");
     }
 }
 
@@ -410,7 +481,7 @@ extern "C" int bl_gemm_f32_tc(const float* x, int ldx, const float* w, const voi
     }
 }
 
-// Reads and clears the status word: 0 when no block has given up on a wait (1 a splitter, 2 the issuer, 3 an adder). Synchronises.
+// Reads and clears the status word: 0 when no block has given up on a wait (1 a splitter, 2 the issuing warp, 3 an adder). Synchronises.
 extern "C" int bl_gemm_f32_tc_status(int* status) {
     int v = 0, zero = 0;
     BL_CUDA(cudaMemcpyFromSymbol(&v, g_status, sizeof(int)));

@@ -660,6 +660,81 @@ def test_32_bit_product_on_tensor_cores_of_infinities_and_extremes():
     o.check_status()
 
 
+def fma_chain(x, w):
+    """fmaf in ascending k: the 48-bit product is exact in 64 bits, the sum rounded to 32."""
+    acc = torch.zeros(x.shape[0], w.shape[0], device=x.device)
+    for k in range(x.shape[1]):
+        acc = (acc.double() + x[:, k:k + 1].double() * w[:, k].double()).float()
+    return acc
+
+
+@pytest.mark.parametrize("N,K", [(128, 256), (896, 900), (512, 2048)])
+@pytest.mark.parametrize("M", [1, 20, 200])
+def test_32_bit_product_of_rows_with_few_numbers(M, N, K):
+    """A row of one 1 gives a column of W as it is. Rows of 1, 4 and 16 numbers and full ones: every single result within what a chain of
+    as many FMAs is off by at most (half a last place of the sum of magnitudes each; 2 % for the products left out and what follows),
+    and the rows' error together no larger than the chain's."""
+    o = ops()
+    g = torch.Generator().manual_seed(M * 31 + N + K)
+    w = (torch.randn(N, K, generator=g) * 0.3).to(DEV)
+    out = torch.empty(M, N, device=DEV)
+    at = torch.randint(0, K, (M,), generator=g)
+    one = torch.zeros(M, K)
+    one[torch.arange(M), at] = 1.0
+    o.gemm(one.to(DEV), w, out)
+    assert torch.equal(out, w[:, at.to(DEV)].T)
+    for n in (1, 4, 16, K):
+        keep = torch.rand(M, K, generator=g).argsort(dim=1) < n
+        x = (torch.randn(M, K, generator=g) * keep).to(DEV)
+        o.gemm(x, w, out)
+        want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+        assert ((out.double() - want).abs() <= 1.02 * n * 2.0 ** -24 * size).all()
+        assert (out.double() - want).norm() <= 1.02 * (fma_chain(x, w).double() - want).norm()
+    o.check_status()
+
+
+def test_32_bit_product_of_tiny_numbers():
+    """Operands down to the smallest 32-bit numbers (with large ones on the other side, too) lose no more than in a chain of FMAs, and a
+    row's bits are the same beside such rows as without them."""
+    o = ops()
+    g = torch.Generator().manual_seed(9)
+    M, N, K = 40, 256, 512
+    x, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    before = torch.empty(M, N, device=DEV)
+    o.gemm(x, w, before)
+    y, v = x.clone(), w.clone()
+    scales = {3: 2.0 ** -60, 4: 2.0 ** -112, 5: 2.0 ** -120, 6: 2.0 ** -126, 7: 2.0 ** -140}
+    for r, scale in scales.items():
+        y[r] *= scale
+        v[r] *= scale
+    y[8] = 0.0
+    y[8, 100] = 2.0 ** -120                            # one number: 2^-120 times a column of W
+    y[9] = 0.0
+    y[9, 101], y[9, 102] = 2.0 ** -125, 2.0 ** 50      # tiny and huge in one row
+    v[10] = 0.0
+    v[10, 101] = 2.0 ** 100
+    y[11, ::7] = 2.0 ** -130                           # tiny numbers among ordinary ones
+    y[12] *= 2.0 ** 45
+    out = torch.empty(M, N, device=DEV)
+    o.gemm(y, v, out)
+    want, chain = y.double() @ v.double().T, fma_chain(y, v)
+    # a chain's results are rounded to multiples of 2^-149 where they are that small: what both sides are held to
+    size = y.double().abs() @ v.double().abs().T
+    for r in [*scales, 8, 9, 11, 12]:
+        for c in ([n for n in range(N) if n not in scales], list(scales)):
+            err, limit = (out[r, c].double() - want[r, c]).norm(), (chain[r, c].double() - want[r, c]).norm()
+            assert err <= 1.02 * limit + 2.0 ** -30 * size[r, c].norm() / K ** 0.5, (r, len(c), err.item(), limit.item())
+    assert torch.equal(out[8], chain[8])
+    plain_rows = [r for r in range(M) if r not in scales and not 8 <= r <= 12]
+    plain_cols = [n for n in range(N) if n not in scales and n != 10]
+    assert torch.equal(out[plain_rows][:, plain_cols], before[plain_rows][:, plain_cols])
+    alone = torch.empty(1, N, device=DEV)
+    for r in (0, 4, 9, 11):
+        o.gemm(y[r:r + 1].contiguous(), v, alone)
+        assert torch.equal(alone[0], out[r]), r
+    o.check_status()
+
+
 @pytest.mark.parametrize("H,KV,dh,dv,page", [(14, 2, 64, 64, 16), (9, 1, 32, 16, 16), (10, 2, 128, 64, 8), (12, 2, 16, 128, 16), (9, 1, 36, 20, 16), (5, 5, 64, 64, 16)])
 @pytest.mark.parametrize("window,extras", [(0, False), (40, True)])
 def test_32_bit_attention_with_several_heads_a_warp(H, KV, dh, dv, page, window, extras):
