@@ -12,7 +12,7 @@ DTYPES = ("bfloat16", "float32")
 
 @dataclass
 class EngineOptions:
-    dtype: str = "bfloat16"             # "bfloat16": serving kernels; "float32": true 32-bit everywhere
+    dtype: str = "bfloat16"             # "bfloat16": serving kernels; "float32": 32-bit numbers and sums everywhere
     page_size: int = 16                 # tokens per cache page
     max_tokens: int = 0                 # cache capacity in tokens (0: ctx_size * max_num_seqs)
     ctx_size: int = 4096                # prompt + reply limit of one request (-c, src/main.br:638-639)

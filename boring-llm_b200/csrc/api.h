@@ -23,9 +23,10 @@ int bl_rmsnorm(const float* x, const int* row_idx, const void* w, int w_dtype, v
 // out[M, N] = epilogue(x[M, K] . W[N, K]^T). For BL_EPI_SWIGLU W has 2N rows (gate, then up), and `bias`, which that epilogue
 // does not add, may point to two 32-bit numbers {kind, limit} on the device that name the gated activation (BL_GLU_* of
 // common.cuh; null: SiLU). The same holds for every product below that takes a bias and this epilogue.
-// 32-bit operands and results of 128 to 32,768 columns and a long K (bl_gemm_f32_tc_supported, by N and K alone) run on the tensor cores
-// instead (gemm_f32_tc.cu: numbers in two halves, 32-bit sums of 32 values of k added up in ascending k), with the same promise:
-// what an output is depends on its row of x and its row of W only.
+// bl_gemm_f32_tc: the same for 32-bit operands and results of 128 to 32,768 columns and a long K (bl_gemm_f32_tc_supported) on the tensor
+// cores (gemm_f32_tc.cu: numbers in three exact parts, 32-bit sums of 32 values of k added up in ascending k), with the same promise:
+// what an output is depends on its row of x and its row of W only. It asks for W before the kernel in front of it on the stream has
+// finished: W must not be a result of that kernel.
 int bl_gemm_f32_tc_supported(int N, int K, int ldx);
 int bl_gemm_f32_tc(const float* x, int ldx, const float* w, const void* bias, int bias_dtype, float* out, int M, int N, int K,
                    int epilogue, void* stream);

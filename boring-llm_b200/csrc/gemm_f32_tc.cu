@@ -18,7 +18,8 @@
 // segment.) At the end the tile passes through shared memory to the epilogue. Products of few tiles cut K over the blocks of a
 // cluster (f32_tc_spans), whose totals are added in ascending k through distributed shared memory. What a result is computed from, and
 // in which order, depends on N and K only: it is the same whatever rows stand beside a row and however wide a tile is (the same promise
-// that the kernels in gemm_plain.cu make, which keep the small products).
+// that the kernels in gemm_plain.cu make, which keep the small products, rows that are no whole 16-byte pieces, and steps that are
+// asked to do without tensor cores).
 // A sum that is not finite (an infinity or NaN among the inputs, or an overflow) is worked out again as a chain of FMAs over the
 // inputs themselves. So is a small one, |sum| < 2^-48, of a row of x or of W with an operand other than 0 below 2^-50: the parts of such
 // operands may lie below bfloat16's smallest numbers (an operand from 2^-110 on loses nothing, a smaller one 2^-134 at most), and
@@ -469,6 +470,7 @@ extern "C" int bl_gemm_f32_tc(const float* x, int ldx, const float* w, const voi
     if (N <= 0 || K <= 0 || ldx < K || !bl_gemm_f32_tc_supported(N, K, ldx) || (((uintptr_t)x | (uintptr_t)w) & 15))
         BL_FAIL("bl_gemm_f32_tc: N=%d K=%d ldx=%d is not what this kernel takes", N, K, ldx);
     if (epilogue == BL_EPI_BIAS && bias == nullptr) BL_FAIL("bl_gemm_f32_tc: bias epilogue without a bias");
+    if (epilogue == BL_EPI_BIAS && bias_dtype != BL_F32 && bias_dtype != BL_BF16) BL_FAIL("bl_gemm_f32_tc: unknown bias dtype %d", bias_dtype);
     const int spans = f32_tc_spans(N, K, epilogue);
     if ((long long)((N + 63) / 64) * ((M + 15) / 16) * spans > 0x7fffffffLL) BL_FAIL("bl_gemm_f32_tc: too many blocks");
     cudaStream_t s = (cudaStream_t)stream;

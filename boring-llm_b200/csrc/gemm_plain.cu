@@ -2,8 +2,8 @@
 // as in the reference's `linear` (src/math.br:66-82) and its tiled GPU kernel LinearKernel
 // (src/math_gpu.br:82-135). Every output element accumulates its products in ascending k in one
 // 32-bit accumulator, whatever the number of rows, so results do not depend on how a batch is cut.
-// This is the whole-model 32-bit path's product and the twin that the tensor-core kernels are
-// checked against.
+// This is the product of the 32-bit path where gemm_f32_tc.cu does not take it, and the twin that the
+// tensor-core kernels are checked against.
 #include "common.cuh"
 #include "api.h"
 
@@ -401,8 +401,6 @@ extern "C" int bl_gemm_plain_ld(const void* x, int x_dtype, int ldx, const void*
     if (epilogue == BL_EPI_BIAS && bias_dtype != BL_F32 && bias_dtype != BL_BF16)
         BL_FAIL("bl_gemm_plain: unknown bias dtype %d", bias_dtype);
     cudaStream_t s = (cudaStream_t)stream;
-    if (x_dtype == BL_F32 && w_dtype == BL_F32 && f32_tiles_fit(x, w, K, ldx, epilogue, out_dtype) && bl_gemm_f32_tc_supported(N, K, ldx))
-        return bl_gemm_f32_tc((const float*)x, ldx, (const float*)w, bias, bias_dtype, (float*)out, M, N, K, epilogue, stream);
     if (x_dtype == BL_F32 && w_dtype == BL_F32 && f32_tiles_fit(x, w, K, ldx, epilogue, out_dtype))
         return launch_f32_tiles((const float*)x, (const float*)w, bias, bias_dtype, (float*)out, M, N, K, ldx, epilogue, s);
     if (x_dtype == BL_F32 && w_dtype == BL_F32)

@@ -606,7 +606,7 @@ class ModelRunner:
         ctx.plans = _plans_on_device(plans, {k: take(int(arr.size)).view(arr.shape) for k, arr in plan_items})
         logits = self.model.forward(ctx)
         if self.dtype == torch.float32:               # products on tensor cores; single tokens are looked at now and then, as replays are
-            self._waits_unchecked = self._waits_unchecked or T > R or self.steps % 256 == 0
+            self._waits_unchecked = self._waits_unchecked or self.fast and (T > R or self.steps % 256 == 0)
         else:
             self._waits_unchecked = self.fast
         return logits

@@ -181,9 +181,8 @@ def _need_bias(bias: torch.Tensor, N: int, epilogue: int) -> None:
 
 def gemm_plain(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
                epilogue: int = EPI_NONE) -> None:
-    """out = epilogue(x @ w.T) on CUDA cores with 32-bit accumulation (32-bit operands with a long K: on the tensor cores, to the same
-    precision, see gemm_f32_tc.cu); a row's result does not depend on the rows beside it. x may be a range of columns of a wider
-    row-major matrix (its rows `x.stride(0)` values apart)."""
+    """out = epilogue(x @ w.T) on CUDA cores with 32-bit accumulation; a row's result does not depend on the rows beside it. x may be
+    a range of columns of a wider row-major matrix (its rows `x.stride(0)` values apart)."""
     M, K = x.shape
     N = out.shape[1]
     rows_w = 2 * N if epilogue == EPI_SWIGLU else N
@@ -194,6 +193,30 @@ def gemm_plain(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Option
         _need_bias(bias, N, epilogue)
     _call(_lib().bl_gemm_plain_ld, _p(x), _dt(x), x.stride(0), _p(w), _dt(w), _p(bias), _dt(bias) if bias is not None else 0,
           _p(out), _dt(out), M, N, K, epilogue, _stream())
+
+
+def gemm_f32_tc_supported(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
+    """Whether `gemm_f32_tc` takes this product: 32-bit numbers, rows of whole 16-byte pieces, and of the sizes N and K alone."""
+    return (x.dtype == w.dtype == out.dtype == torch.float32 and x.dim() == 2 and x.stride(1) == 1 and w.is_contiguous()
+            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+            and bool(library.load().bl_gemm_f32_tc_supported(out.shape[1], x.shape[1], x.stride(0))))
+
+
+def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
+                epilogue: int = EPI_NONE) -> None:
+    """`gemm_plain` of 32-bit numbers on the tensor cores, as precise (numbers in three exact parts). w is a weight: it is read before
+    the kernel in front has finished."""
+    M, K = x.shape
+    N = out.shape[1]
+    if not x.is_cuda or x.stride(1) != 1 or x.stride(0) < K:
+        raise KernelError("x: must be a CUDA matrix whose rows are contiguous")
+    if x.dtype != torch.float32:
+        raise KernelError(f"x: dtype {x.dtype} is not float32")
+    _need(w, "w", torch.float32, (2 * N if epilogue == EPI_SWIGLU else N, K)); _need(out, "out", torch.float32, (M, N))
+    if bias is not None:
+        _need_bias(bias, N, epilogue)
+    _call(_lib().bl_gemm_f32_tc, _p(x), x.stride(0), _p(w), _p(bias), _dt(bias) if bias is not None else 0, _p(out), M, N, K, epilogue,
+          _stream())
 
 
 def rope_kv_write(qkv: torch.Tensor, positions: torch.Tensor, tok_req: torch.Tensor,
@@ -715,13 +738,17 @@ def gemm_few_better(M: int, N: int, w: torch.Tensor, epilogue: int) -> bool:
 
 def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
          epilogue: int = EPI_NONE, fast: bool = True) -> None:
-    """out = epilogue(x @ w.T) by the kernel that suits the operands: float32 operands, operands the tensor-core
-    kernels cannot take, and `fast=False` run the plain CUDA-core kernel; bfloat16 operands a tensor-core kernel
-    chosen by the number of rows (and, for few rows, of columns)."""
+    """out = epilogue(x @ w.T) by the kernel that suits the operands: operands the tensor-core kernels cannot take and
+    `fast=False` run the plain CUDA-core kernel; float32 operands the tensor-core kernel that keeps 32 bits (by columns and K
+    alone, so that a row's result does not depend on the rows beside it); bfloat16 operands a tensor-core kernel chosen by the
+    number of rows (and, for few rows, of columns)."""
     few = out.dtype == (torch.bfloat16 if epilogue == EPI_SWIGLU else torch.float32) and out.data_ptr() % 16 == 0
     kind = gemm_kernel(x, w, out.shape[1], bias, epilogue, fast, few=few)
     if kind == "plain":
-        gemm_plain(x, w, out, bias, epilogue)
+        if fast and gemm_f32_tc_supported(x, w, out):
+            gemm_f32_tc(x, w, out, bias, epilogue)
+        else:
+            gemm_plain(x, w, out, bias, epilogue)
     elif kind == "cols":
         gemm_tc_cols(x, w, out)
     elif kind == "splitk":

@@ -2,8 +2,9 @@
 
 W is stored (outputs x inputs) row-major, as in the reference (src/math.br:66-68) and in
 checkpoints, so nothing is transposed at load. Which kernel runs is the kernel library's business
-(`ops.gemm`): float32 operands always take the plain CUDA-core kernel (true 32-bit), bfloat16
-operands a tensor-core kernel chosen by the product's shape.
+(`ops.gemm`): float32 operands take a tensor-core kernel that keeps all their bits, or the plain
+CUDA-core kernel where the product is small, bfloat16 operands a tensor-core kernel chosen by the
+product's shape.
 """
 from __future__ import annotations
 

@@ -597,34 +597,28 @@ def test_32_bit_product_on_tensor_cores(M, N, K):
     full, w, w2, b = rnd(M, K + 4), rnd(N, K) * 0.3, rnd(2 * N, K) * 0.3, rnd(N)
     x = full[:, :K]
 
-    def chain(x, w):                                   # fmaf in ascending k: the 48-bit product is exact in 64 bits, the sum rounded to 32
-        acc = torch.zeros(x.shape[0], w.shape[0], device=DEV)
-        for k in range(x.shape[1]):
-            acc = (acc.double() + x[:, k:k + 1].double() * w[:, k].double()).float()
-        return acc.double()
-
     def rel(got, want):
         return ((got.double() - want).norm() / want.norm()).item()
 
     out = torch.empty(M, N, device=DEV)
     for x_, w_ in ((x, w), (full.abs()[:, :K], w.abs())):
-        o.gemm_plain(x_, w_, out)
+        o.gemm(x_, w_, out)
         want = x_.double() @ w_.double().T
-        assert rel(out, want) <= rel(chain(x_, w_), want)
+        assert rel(out, want) <= rel(fma_chain(x_, w_), want)
         close(out, want, torch.float32, "product")
     one = torch.empty(1, N, device=DEV)
-    o.gemm_plain(x, w, out, b, o.EPI_BIAS)
-    o.gemm_plain(x[M // 2:M // 2 + 1].contiguous(), w, one, b, o.EPI_BIAS)
+    o.gemm(x, w, out, b, o.EPI_BIAS)
+    o.gemm(x[M // 2:M // 2 + 1].contiguous(), w, one, b, o.EPI_BIAS)
     assert torch.equal(one[0], out[M // 2])
     res = rnd(M, N)
     want = res.double() + x.double() @ w.double().T
-    o.gemm_plain(x, w, res, None, o.EPI_RESIDUAL)
+    o.gemm(x, w, res, None, o.EPI_RESIDUAL)
     close(res, want, torch.float32, "residual")
-    o.gemm_plain(x, w2, out, None, o.EPI_SWIGLU)
+    o.gemm(x, w2, out, None, o.EPI_SWIGLU)
     gu = x.double() @ w2.double().T
     close(out, plain.silu(gu[:, :N]) * gu[:, N:], torch.float32, "swiglu")
     one = torch.empty(1, N, device=DEV)
-    o.gemm_plain(x[M - 1:], w2, one, None, o.EPI_SWIGLU)
+    o.gemm(x[M - 1:], w2, one, None, o.EPI_SWIGLU)
     assert torch.equal(one[0], out[M - 1])
     o.check_status()
 
@@ -636,7 +630,7 @@ def test_32_bit_product_on_tensor_cores_of_infinities_and_extremes():
     M, N, K = 70, 256, 512
     x, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
     plainly = torch.empty(M, N, device=DEV)
-    o.gemm_plain(x, w, plainly)
+    o.gemm(x, w, plainly)
     y = x.clone()
     y[3, 7], y[5, 9], y[8, 0], y[11, 500] = float("inf"), float("nan"), -float("inf"), 3.4028234e38
     y[20] *= 1e-30
@@ -645,7 +639,7 @@ def test_32_bit_product_on_tensor_cores_of_infinities_and_extremes():
     v[40, 7] = 0.0                                     # infinity times zero
     v[41] = w[41].bfloat16().float()                   # numbers whose second half is zero
     out = torch.empty(M, N, device=DEV)
-    o.gemm_plain(y, v, out)
+    o.gemm(y, v, out)
     want = (y.double() @ v.double().T)
     for r in (3, 8):
         torch.testing.assert_close(out[r].double(), want[r], rtol=0, atol=0, equal_nan=True)
@@ -666,6 +660,45 @@ def fma_chain(x, w):
     for k in range(x.shape[1]):
         acc = (acc.double() + x[:, k:k + 1].double() * w[:, k].double()).float()
     return acc
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 256), (33, 896, 896), (200, 132, 512)])
+def test_32_bit_product_without_tensor_cores(M, N, K):
+    """`fast=False` and `gemm_plain` are the chain of FMAs, bit for bit, at sizes that the tensor cores take, too; those give other bits."""
+    o = ops()
+    g = torch.Generator().manual_seed(M + N + K)
+    x, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    want = fma_chain(x, w)
+    out = torch.empty(M, N, device=DEV)
+    assert o.gemm_f32_tc_supported(x, w, out)
+    o.gemm(x, w, out, fast=False)
+    assert torch.equal(out, want)
+    out.zero_()
+    o.gemm_plain(x, w, out)
+    assert torch.equal(out, want)
+    o.gemm(x, w, out)
+    assert not torch.equal(out, want)
+    close(out, x.double() @ w.double().T, torch.float32, "product")
+    o.check_status()
+
+
+@pytest.mark.parametrize("fast", [True, False])
+def test_32_bit_steps_with_and_without_tensor_cores(fast, tmp_path):
+    """A float32 model at sizes that the tensor cores take: both ways against the plain implementation, and only the fast one asks for
+    the status words."""
+    import boring_llm_b200 as b
+    cfg = b.Qwen2Config.from_dict(dict(
+        architectures=["Qwen2ForCausalLM"], num_hidden_layers=2, hidden_size=256, num_attention_heads=4, num_key_value_heads=2,
+        intermediate_size=384, vocab_size=300, rope_theta=10000.0, rms_norm_eps=1e-6, tie_word_embeddings=True, max_position_embeddings=128))
+    b.write_random_model(str(tmp_path), cfg, 3, "float32", 0.05)
+    eng = b.Engine(str(tmp_path), dtype="float32", ctx_size=96, max_num_seqs=2, max_tokens=192)
+    eng.runner.fast = fast
+    toks = np.random.default_rng(0).integers(0, 300, 70).tolist()
+    got = eng.runner.step([b.StepEntry("a", toks, list(range(len(toks))))]).double().cpu()
+    assert eng.runner._waits_unchecked == fast
+    eng.runner.check_kernels()
+    want = torch.as_tensor(plain.forward(*plain.read_model_folder(str(tmp_path)), toks)).double()
+    assert ((got - want).norm() / want.norm()) < 2e-6      # sums of up to 384 in 32 bits, two layers
 
 
 @pytest.mark.parametrize("N,K", [(128, 256), (896, 900), (512, 2048)])
