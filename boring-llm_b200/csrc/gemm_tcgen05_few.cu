@@ -150,7 +150,7 @@ gemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             for (int j = 0; j < 4; ++j) {
                 float g = v[j], up = u[j];
                 if (glu.bias && n + j < N) { g += glu.bias[n + j]; up += glu.bias[N + n + j]; }
-                v[j] = bl_glu_fast(glu.kind, g, up, glu.limit);
+                v[j] = bl_glu(glu.kind, g, up, glu.limit);                     // (the exponential and division of the kernel for few rows beside this one)
             }
         }
         if (EPI == BL_EPI_BIAS || (EPI == BL_EPI_RESIDUAL && bias != nullptr)) {

@@ -947,6 +947,23 @@ def test_few_rows_with_w_streamed_once(M, N, K):
     o.check_status()
 
 
+@pytest.mark.parametrize("kind", ["silu", "gelu", "clamped"])
+def test_gated_activation_of_few_rows_is_the_same_in_both_kernels(kind):
+    """Sums that are one number of W each (rows of one 1): the two kernels that a gated product of few rows may run on round the same
+    activation, bit for bit."""
+    o = ops()
+    K, N = 256, 4096
+    x = torch.zeros(16, K, dtype=BF, device=DEV)
+    x[torch.arange(16), torch.arange(16) * 9] = 1.0
+    w = (data((2 * N, K), 2) * 8).to(BF)
+    act = {"silu": None, "gelu": o.glu_args(o.GLU_GELU_TANH, 0.0, DEV), "clamped": o.glu_args(o.GLU_CLAMPED, 7.0, DEV)}[kind]
+    a, b = torch.empty(16, N, dtype=BF, device=DEV), torch.empty(16, N, dtype=BF, device=DEV)
+    o.gemm_tc_few(x, w, a, act, o.EPI_SWIGLU)
+    o.gemm_skinny(x, w, b, act, o.EPI_SWIGLU)
+    o.check_status()
+    assert torch.equal(a, b)
+
+
 def test_few_rows_go_by_the_bytes_of_w():
     """The kernel on either side of its lines, and that a product that an RMS norm links to another stays where the norm is."""
     o = ops()
