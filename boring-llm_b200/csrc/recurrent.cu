@@ -1266,12 +1266,14 @@ extern "C" int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const 
     const int vec = dk % 4 == 0 && ldq % 4 == 0 && ldk % 4 == 0 && ldz % 4 == 0 &&
                     (((uintptr_t)q | (uintptr_t)k | (uintptr_t)z) & 15) == 0;
     dim3 grid((dv + cols_blk - 1) / cols_blk, H, R * nc);
-    // four columns a lane: where values and states are whole 16-byte pieces, too
-    const bool fours = rk4 == 4 && vec && dv % 4 == 0 && ldv % 4 == 0 && slot_stride % 4 == 0 && (((uintptr_t)v | (uintptr_t)state) & 15) == 0 && four.smem <= 48 * 1024;
+    // four columns a lane: where values, states and the parts' states between the passes are whole 16-byte pieces, too
+    const bool fours = rk4 == 4 && vec && dv % 4 == 0 && ldv % 4 == 0 && slot_stride % 4 == 0 &&
+                       (((uintptr_t)v | (uintptr_t)state | (uintptr_t)scratch) & 15) == 0 && four.smem <= 48 * 1024;
     cudaStream_t s = (cudaStream_t)stream;
     if (rule != BL_RULE_GLA && rule != BL_RULE_DELTA && rule != BL_RULE_BONUS) BL_FAIL("bl_recurrent_scan: unknown rule %d", rule);
     if (rk4 > 0) {                                     // a lane's rows are whole groups of four
         const bool dl = rule == BL_RULE_DELTA;
+        if (dl && nc > 1 && ((uintptr_t)scratch & 15)) BL_FAIL("bl_recurrent_scan_parts: the delta rule's scratch must be 16-byte aligned (its folds read the transitions in such pieces)");
         int* places = n_cut < R ? reinterpret_cast<int*>(scratch) : nullptr;     // [R], up to a multiple of 16 bytes; null: r is r's place
         float* part_s = scratch ? scratch + (R + 3) / 4 * 4 : nullptr;           // [n_cut, nc, H, dk, dv]
         float* part_p = scratch ? part_s + (size_t)n_cut * nc * H * dk * dv : nullptr;   // [n_cut, nc, H, dk] or, delta rule, [n_cut, nc, H, dk, dk]

@@ -1007,6 +1007,38 @@ def test_scan_with_four_columns_a_lane(rule, H, dk, dv):
         close(st[r], S.reshape(-1), torch.float32, f"state of request {r}")
 
 
+@pytest.mark.parametrize("rule", ["RULE_GLA", "RULE_DELTA", "RULE_BONUS"])
+def test_cut_scan_with_scratch_that_is_not_aligned(rule):
+    """The parts' states at an address that is no multiple of 16: served by the build that reads them a value at a time, or refused (the
+    delta rule, whose folds read transitions in pieces of 16 bytes)."""
+    import ctypes
+    o = ops()
+    rule = getattr(o, rule)
+    H, dk, dv, T, parts = 8, 64, 128, 2100, 60
+    q, k, v, b = data((T, H * dk), 1) * 0.3, data((T, H * dk), 2) * 0.1, data((T, H * dv), 3), data((T, H), 4)
+    a = torch.sigmoid(data((T, H * dk), 5) + 3.0)
+    cu, slots = torch.tensor([0, T], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    beta = None if rule == o.RULE_GLA else b
+    lib = o._lib()
+    lib.bl_recurrent_scan_parts_scratch.restype = ctypes.c_longlong
+    n = int(lib.bl_recurrent_scan_parts_scratch(rule, 1, 1, parts, H, dk, dv))
+    got = []
+    for off in (0, 1):
+        st, out = data((1, H * dk * dv), 6), torch.full((T, H * dv), float("nan"), device=DEV)
+        room = torch.empty(n + 4, device=DEV)[off:]
+        call = lambda: o._call(lib.bl_recurrent_scan_parts, rule, o._p(q), H * dk, o._p(k), H * dk, o._p(v), H * dv, o._p(a), H * dk, o._p(beta),
+                H if beta is not None else 0, ctypes.c_float(0.5), o._p(st), ctypes.c_longlong(H * dk * dv), o._p(slots), o._p(cu), 1, o._p(out),
+                H, H, dk, dv, parts, 1, 1, ctypes.c_void_p(room.data_ptr()), o._stream())
+        if off and rule == o.RULE_DELTA:
+            with pytest.raises(o.KernelError, match="aligned"):
+                call()
+            return
+        call()
+        got.append((out, st))
+    for x, y in zip(*got):
+        assert ((x - y).norm() / x.norm()) < 1e-5
+
+
 @pytest.mark.parametrize("H,KV,dh,window", [(14, 2, 64, 0), (4, 4, 64, 100), (16, 2, 128, 0)])
 def test_prompts_and_single_tokens_side_by_side(H, KV, dh, window):
     """The two attention launches of a mixed step with the word between them against the same without it, bit for bit, kernel by
