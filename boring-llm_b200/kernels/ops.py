@@ -1109,6 +1109,7 @@ def _scan_cost(rule: int, H: int, dk: int, dv: int, n_long: int, tokens: int, pa
 SCAN_FOUR_TOKENS = 2048           # portions from which the four-column build decides the number of parts ...
 SCAN_FOUR_BLOCKS_PER_SM = 3       # ... of whose blocks an SM holds so many
 SCAN_FOUR_MAX_PARTS = 64
+SCAN_MAX_PORTIONS = 65535         # requests times parts that one launch takes
 
 
 def _scan_parts_of_fours(rule: int, H: int, dk: int, dv: int, n_long: int, tokens: int):

@@ -43,6 +43,7 @@ class _StateMixer(Mixer):
         portions are under way for most of the scan (the tokens over those of the longest)."""
         n_long = sum(1 for n in q_lens if n >= ops.SCAN_PART_MIN_TOKENS)
         parts = ops.recurrent_scan_parts(self.RULE, self.H, self.dk, self._value_columns(), n_long, 1 << round(math.log2(max(q_lens)))) if n_long else 1
+        parts = max(1, min(parts, ops.SCAN_MAX_PORTIONS // len(q_lens)))
         return {"parts": parts, "n_long": n_long if parts > 1 else 0, "busy": max(1, round(sum(q_lens) / max(1, max(q_lens))))}
 
     def _value_columns(self) -> int:

@@ -170,3 +170,19 @@ def test_command_line_lists_the_configuration_and_tensors(tmp_path, capsys):
     assert cli.main(["--model", d, "--dump-metadata"]) == 0
     out = capsys.readouterr().out
     assert "architecture = Fezopel" in out and "tensor l2.mix.q.conv [8, 3] matrix" in out and "tensor l0.dwa [2] norm" in out
+
+
+@pytest.mark.parametrize("requests", [1, 31, 1040, 1041, 2000, 3121, 32768, 70000])
+def test_scans_of_many_requests_are_cut_into_what_a_launch_takes(requests, monkeypatch):
+    """A launch has a row of blocks for every request and part, 65,535 at most: the parts that a long portion is cut into leave room for
+    all requests beside it (63 parts beside 1,041 are more than that)."""
+    from boring_llm_b200.kernels import ops
+    from boring_llm_b200.parts.recurrent import GatedLinearAttention
+    asked = []
+    monkeypatch.setattr(ops, "recurrent_scan_parts", lambda *a: asked.append(a) or 63)
+    m = GatedLinearAttention.__new__(GatedLinearAttention)
+    m.H, m.dk, m.dv = 7, 64, 128
+    cut = m._cut([2048] + [1] * (requests - 1))
+    assert asked and cut["parts"] == max(1, min(63, 65535 // requests))
+    assert cut["parts"] * requests <= max(65535, requests) and cut["n_long"] == (1 if cut["parts"] > 1 else 0)
+    assert m._cut([1] * requests)["parts"] == 1
