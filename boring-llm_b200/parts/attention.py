@@ -275,6 +275,9 @@ class GQAAttention(Mixer):
         self.project_out(ctx, attn, x)
         return True
 
+    def plan_key(self):
+        return PLAN_KEY
+
     def plan_step(self, q_lens, ctx_lens, filler=None):
         return PLAN_KEY, attention_plan(q_lens, ctx_lens, filler)
 
@@ -405,6 +408,9 @@ class GatedSinkAttention(Mixer):
     def cache_spec(self):
         return PagedKVSpec(self.KV, self.pk, self.window, 0 if self.pv == self.pk else self.pv)
 
+    def plan_key(self):
+        return PLAN_KEY
+
     def plan_step(self, q_lens, ctx_lens, filler=None):
         return PLAN_KEY, attention_plan(q_lens, ctx_lens, filler)
 
@@ -513,6 +519,9 @@ class ChunkedTalkingAttention(Mixer):
 
     def cache_spec(self):
         return PagedKVSpec(self.KV, self.dk, self.window, 0 if self.dv == self.dk else self.dv, self.chunk)
+
+    def plan_key(self):
+        return PLAN_KEY
 
     def plan_step(self, q_lens, ctx_lens, filler=None):
         return PLAN_KEY, attention_plan(q_lens, ctx_lens, filler)
@@ -643,6 +652,9 @@ class MixedScoreAttention(Mixer):
         return (ops.SKINNY_LINK_MIN_ROWS <= rows <= ops.SKINNY_LINK_MAX_ROWS and self.w_in is not None
                 and self.w_in.dtype == torch.bfloat16 and -(-self.n_in // 16) <= ops.SKINNY_LINK_MAX_BLOCKS
                 and not ops.gemm_streams_better(self.w_in))
+
+    def plan_key(self):
+        return PLAN_KEY
 
     def plan_step(self, q_lens, ctx_lens, filler=None):
         return PLAN_KEY, attention_plan(q_lens, ctx_lens, filler)

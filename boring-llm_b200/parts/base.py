@@ -63,10 +63,15 @@ class Part:
         filler, and everything that decides a launch must come from `shape` alone."""
         return None
 
+    def plan_key(self) -> Optional[str]:
+        """The key of `plan_step`'s plan where it does not depend on the batch: a layer whose plan another has made is not asked."""
+        return None
+
     def collect_plans(self, q_lens, ctx_lens, filler=None, into: Optional[dict] = None) -> dict:
         """The plans of this part and of the parts inside it, one per key."""
         into = {} if into is None else into
-        got = self.plan_step(q_lens, ctx_lens, filler)
+        key = self.plan_key()
+        got = self.plan_step(q_lens, ctx_lens, filler) if key is None or key not in into else None
         if got is not None and got[0] not in into:
             into[got[0]] = got[1]
         for c in self.children():

@@ -16,6 +16,29 @@ from .rotary import RotaryTable
 
 
 KEY_BLOCK = 128                # keys that the tcgen05 attention reads at a time
+OWN_KEYS_MAX_BYTES = 128 << 20     # of a layer's keys and values in one step (the other way's queries and results: twice 32 MB for
+                                   # 2,048 tokens of 16 heads over 512 latent values)
+
+
+def _page_bucket(pages: int) -> int:
+    """Up to a multiple of 8, from 64 on to one of four lengths an octave: the portions of a long prompt, whose contexts grow, then come to
+    few shapes of captured steps."""
+    step = max(8, 1 << max(0, (pages - 1).bit_length() - 3))
+    return -(-pages // step) * step
+
+
+def _own_keys_pay(pairs: float, tokens: int, rows: int, sizes) -> bool:
+    """Whether a step with so many (query, key) pairs and new tokens runs faster on keys and values of their own, made of so many rows,
+    than on the cached rows. In microseconds: the cached rows cost 143 TFLOP/s over 2 (2 rank + shared) operations a (query, key, head)
+    and 150 in the products with Uk and Uv before and behind; keys and values of their own 300 over 2 (own + shared + values), and their
+    product over all rows at 700; 6 us more of launches.
+    A step of one prompt over eight layers, cached rows and own keys: 16 heads of 128 + 64 over a rank of 512, 160 tokens 1,873 and
+    1,788 us, 256 1,944 and 1,826, 512 2,311 and 2,037, 2,000 6,306 and 3,671; 14 heads of 64 + 32 over 256, 512 1,234 and 1,043,
+    1,000 1,650 and 1,236, 2,000 2,610 and 1,560."""
+    H, dn, dr, dv, rank = sizes
+    cached = pairs * H * (4 * rank + 2 * dr) / 143e6 + tokens * H * rank * 2.0 * (dn + dv) / 150e6
+    own = pairs * H * 2.0 * (dn + dr + dv) / 300e6 + rows * H * rank * 2.0 * (dn + dv) / 700e6 + 6.0
+    return own < cached
 
 
 def latent_keys_plan(q_lens, ctx_lens, filler, window: int, sizes) -> Optional[StepPlan]:
@@ -24,48 +47,45 @@ def latent_keys_plan(q_lens, ctx_lens, filler, window: int, sizes) -> Optional[S
     go to rows 16 i .. of the step's matrices; `key_row` [requests]: the row of a request's key 0 (key blocks start at multiples of
     128, so every block that is read lies in the request's own rows or past its last key); `tiles` [n, 2]: the 128-token tiles, the
     one with the fewest keys first. Requests with a single token and a long context (decoding beside prompts) would pay for all of
-    their context: such steps stay with the cached rows. The lists of a step that is replayed (`filler` given) are padded to
-    multiples of 8.
-
-    The line between the two, in microseconds (`sizes`: heads, own and shared part of a key, values, rank): the cached rows cost
-    143 TFLOP/s over 2 (2 rank + shared) operations a (query, key, head) and 150 in the products with Uk and Uv before and behind;
-    keys and values of their own 300 over 2 (own + shared + values), and their product over all rows at 700; 6 us more of launches.
-    A step of one prompt over eight layers, cached rows and own keys: 16 heads of 128 + 64 over a rank of 512, 160 tokens 1,873 and
-    1,788 us, 256 1,944 and 1,826, 512 2,311 and 2,037, 2,000 6,306 and 3,671; 14 heads of 64 + 32 over 256, 512 1,234 and 1,043,
-    1,000 1,650 and 1,236, 2,000 2,610 and 1,560."""
-    H, dn, dr, dv, rank = sizes
-    pairs, tokens, at = 0.0, 0, 0
-    key_row = [0] * len(q_lens)
-    work, tiles = [], []
+    their context: such steps stay with the cached rows, and so do steps whose rows would take more than OWN_KEYS_MAX_BYTES. The lists of a
+    step that is replayed (`filler` given) are padded (`_page_bucket`, multiples of 8). Lists are made only once the way is chosen.
+    `sizes`: heads, own and shared part of a key, values, rank."""
+    H, dn, _, dv, _ = sizes
+    pairs, tokens, pages = 0.0, 0, 0
+    spans = []                                       # (request, new tokens, keys, first key, pages before, pages)
     for r, (n, c) in enumerate(zip(q_lens, ctx_lens)):
         if n == 0:
             continue
         if n == 1 and c > KEY_BLOCK:
             return None
         start = max(0, c - n - window + 1) // KEY_BLOCK * KEY_BLOCK if window > 0 else 0
-        key_row[r] = at - start
-        pages = -(-(c - start) // 16)
-        work += [[r, start + 16 * i] for i in range(pages)]
-        at += 16 * pages
-        seen = min(window, c - 0.5 * n) if window > 0 else c - 0.5 * n
-        pairs += n * seen
+        spans.append((r, n, c, start, pages, -(-(c - start) // 16)))
+        pages += spans[-1][-1]
+        pairs += n * (min(window, c - 0.5 * n) if window > 0 else c - 0.5 * n)
         tokens += n
+    padded = pages if filler is None else _page_bucket(pages)
+    if 16 * padded * 2 * H * (dn + dv) > OWN_KEYS_MAX_BYTES:
+        return None
+    if not _own_keys_pay(pairs, tokens, 16 * padded, sizes):
+        return None
+    work = np.empty((padded, 2), dtype=np.int32)
+    work[pages:] = (filler or 0, 0)
+    key_row = np.zeros(len(q_lens), dtype=np.int32)
+    tiles = []
+    for r, n, c, start, at, count in spans:
+        key_row[r] = 16 * at - start
+        work[at:at + count, 0] = r
+        work[at:at + count, 1] = np.arange(start, start + 16 * count, 16, dtype=np.int32)
         for t0 in range(0, n, KEY_BLOCK):
             first = c - n + t0
             lo = max(0, first - window + 1) if window > 0 else 0
             tiles.append([min(first + KEY_BLOCK, c) // KEY_BLOCK - lo // KEY_BLOCK, r, t0])
-    cached = pairs * H * (4 * rank + 2 * dr) / 143e6 + tokens * H * rank * 2.0 * (dn + dv) / 150e6
-    own = pairs * H * 2.0 * (dn + dr + dv) / 300e6 + at * H * rank * 2.0 * (dn + dv) / 700e6 + 6.0
-    if own >= cached:
-        return None
     tiles.sort()
     tiles = [t[1:] for t in tiles]
     if filler is not None:
-        work = work + [[filler, 0]] * (-len(work) % 8)
         tiles = [[filler, 0]] * (-len(tiles) % 8) + tiles                # the front of this list is launched last
-    return StepPlan(arrays={"work": np.asarray(work, dtype=np.int32), "key_row": np.asarray(key_row, dtype=np.int32),
-                            "tiles": np.asarray(tiles, dtype=np.int32)},
-                    host={}, shape=("keys", len(work), len(key_row), len(tiles)))
+    return StepPlan(arrays={"work": work, "key_row": key_row, "tiles": np.asarray(tiles, dtype=np.int32)},
+                    host={}, shape=("keys", padded, len(key_row), len(tiles)))
 
 
 class LatentAttention(Mixer):
@@ -184,7 +204,7 @@ class LatentAttention(Mixer):
                 and self.w_in.dtype == torch.bfloat16 and -(-self.n_in // 16) <= ops.SKINNY_LINK_MAX_BLOCKS
                 and not ops.gemm_streams_better(self.w_in))
 
-    def _plan_key(self) -> str:
+    def plan_key(self) -> str:
         """Mixers of equal sizes and window share their plan."""
         return "latent attention, window %d, %d heads, sizes %d %d %d %d" % (self.window, self.H, self.dn, self.dr, self.dv, self.rank)
 
@@ -197,14 +217,14 @@ class LatentAttention(Mixer):
         plan = None
         if self._makes_keys():
             plan = latent_keys_plan(q_lens, ctx_lens, filler, self.window, (self.H, self.dn, self.dr, self.dv, self.rank))
-        return self._plan_key(), plan if plan is not None else attention_plan(q_lens, ctx_lens, filler)
+        return self.plan_key(), plan if plan is not None else attention_plan(q_lens, ctx_lens, filler)
 
     def _plan(self, ctx) -> StepPlan:
-        plan = ctx.plans.get(self._plan_key())
+        plan = ctx.plans.get(self.plan_key())
         if plan is None:                              # a step put together without asking the parts: plan it now
             plan = self.plan_step(ctx.q_lens, ctx.ctx_lens)[1]
             plan.arrays = {k: torch.from_numpy(v).to(ctx.device) for k, v in plan.arrays.items()}
-            ctx.plans[self._plan_key()] = plan
+            ctx.plans[self.plan_key()] = plan
         return plan
 
     # -- the steps of a pass, each one kernel or product ----------------------------------------------------------------
@@ -233,7 +253,7 @@ class LatentAttention(Mixer):
         T, H = cq.shape[0], self.H
         per = self.dn + self.dr
         work = plan.arrays["work"]
-        key = ("latent rows", cache_layer, self._plan_key())
+        key = ("latent rows", cache_layer, self.plan_key())
         if not self.own_kv and key in ctx.memo:       # the layer that wrote the cache has read the same rows back already
             latent, shared = ctx.memo[key]
         else:

@@ -52,16 +52,16 @@ class _StateMixer(Mixer):
     def plan_step(self, q_lens, ctx_lens, filler=None):
         """How the scan is launched: part of what names a captured step."""
         cut = self._cut(q_lens)
-        return self._plan_key(), StepPlan(host=cut, shape=tuple(cut.values()))
+        return self.plan_key(), StepPlan(host=cut, shape=tuple(cut.values()))
 
-    def _plan_key(self) -> str:
+    def plan_key(self) -> str:
         return f"recurrence parts {self.RULE} {self.H}x{self.dk}x{self._value_columns()}"       # layers of equal sizes share the plan
 
     def _step_cut(self, ctx) -> dict:
         """The arguments of `recurrent_scan` that say how it is launched."""
         if not ctx.fast:
             return {}
-        plan = ctx.plans.get(self._plan_key())
+        plan = ctx.plans.get(self.plan_key())
         if plan is not None:
             return plan.host
         return self._cut(ctx.q_lens) if ctx.q_lens else {}       # a step put together without asking the parts

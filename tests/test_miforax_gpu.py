@@ -78,8 +78,16 @@ SHAPES = {
     "D": model(83, 96, 1e-5, 2.0, [
         layer(mixer(35, 8, 8, 8, 40, 272, 45), dense(64)),
         layer(mixer(3, 16, 8, 24, 40, 272, 0, kv_from=0), moe(32, 1.0, 4, 3))]),
+    # heads of 64 + 32 and of 128 + 64 values, for which prompts make keys and values of their own: a window and a layer that reads the
+    # same rows (once through the same window, once through a smaller one with fewer heads), a layer that sees everything and a reader
+    "E": model(300, 128, 1e-6, 8.0, [
+        layer(mixer(6, 64, 32, 64, 48, 160, 150), dense(128)),
+        layer(mixer(6, 64, 32, 64, 64, 160, 150, kv_from=0), dense(128)),
+        layer(mixer(4, 64, 32, 64, 48, 160, 70, kv_from=0), moe(64, 2.0, 4, 2)),
+        layer(mixer(3, 128, 64, 128, 40, 136, 0), dense(128)),
+        layer(mixer(3, 128, 64, 128, 48, 136, 200, kv_from=3), dense(128))]),
 }
-SEEDS = {"A": 31, "B": 32, "C": 33, "D": 34}
+SEEDS = {"A": 31, "B": 32, "C": 33, "D": 34, "E": 35}
 
 
 @pytest.fixture(scope="module")
@@ -198,6 +206,36 @@ def test_wide_shape_on_the_tensor_core_products(folders, dtype):
     check_trace(folder, dtype, reqs, steps, 512, "wide tail").check_kernels()
     steps, peak = helpers.mixed_trace(reqs, seed=3, max_live=2)
     check_trace(folder, dtype, reqs, steps, peak, "wide mixed").check_kernels()
+
+
+def test_prompts_on_keys_and_values_of_their_own(folders, monkeypatch):
+    """Whole models through the way that makes a step's keys and values (asked for at every size): prompts whole, portions behind cached
+    contexts, tails token by token, mixed batches with pages used again, against 64 bits; launched one by one and replayed, bit for bit."""
+    from boring_llm_b200.kernels import ops
+    from boring_llm_b200.parts import latent
+    monkeypatch.setattr(latent, "_own_keys_pay", lambda *a: True)
+    calls = []
+    attend = ops.attention_rows_tc
+    monkeypatch.setattr(ops, "attention_rows_tc", lambda *a, **k: calls.append(a[0].shape[0]) or attend(*a, **k))
+    folder = folders("E", 0.06)
+    reqs = {f"k{i}": helpers.random_tokens(300, n, 700 + i) for i, n in enumerate([300, 143, 90, 17])}
+    traces = {"whole": (solo_steps(reqs, lambda t, i: helpers.cut_whole(t)), 512),
+              "portions": (solo_steps(reqs, lambda t, i: [n for n in ([130, 101, 50, 19] if len(t) == 300 else [len(t) - 9, 9])]), 512),
+              "tail": (solo_steps(reqs, lambda t, i: helpers.cut_tail_singly(t, 10)), 512),
+              "mixed": helpers.mixed_trace(reqs, seed=8, max_live=3)}
+    for what, (steps, room) in traces.items():
+        calls.clear()
+        check_trace(folder, "bfloat16", reqs, steps, room, what).check_kernels()
+        assert calls, what
+        twice = steps + [dict(s, step=s["step"] + len(steps)) for s in steps]
+        replayed, runner = helpers.run_inprocess(folder, "bfloat16", twice, room, step_graph_after=1)
+        one_by_one, _ = helpers.run_inprocess(folder, "bfloat16", steps, room, step_graph_after=10 ** 6, debug_poison=True)
+        assert runner.graph_steps > 0
+        for s in steps:
+            if s["step"] in replayed:
+                np.testing.assert_array_equal(replayed[s["step"]], replayed[s["step"] + len(steps)], err_msg=what)
+                if what in ("whole", "portions"):
+                    np.testing.assert_allclose(replayed[s["step"]], one_by_one[s["step"]], atol=0.06 * np.abs(one_by_one[s["step"]]).max(), err_msg=what)
 
 
 def test_captured_steps_replay_the_same_bits(folders):

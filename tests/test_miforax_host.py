@@ -144,3 +144,79 @@ def test_plain_attention_closed_forms():
     assert abs(one(5.0, 0.0) - 2.0 / (1 + math.exp(-3.404))) < 1e-12
     assert abs(one(-5.0, 9.0) - (-5.0 / (1 + math.exp(8.51)) * 3.0)) < 1e-12
     assert abs(one(1.0, -9.0) - (1.0 / (1 + math.exp(-1.702)) * -1.0)) < 1e-12
+
+
+# ---- latent attention on keys made for the step: its plan -----------------------------------------------------------------
+SIZES_3B = (16, 128, 64, 128, 512)
+
+
+@pytest.mark.parametrize("window", [0, 37, 128, 1024])
+def test_plan_of_own_keys_lists_every_visible_page(window, monkeypatch):
+    """Pages, rows and tiles against lists put together request by request; a replayed step's lists padded with the filler."""
+    from boring_llm_b200.parts import latent
+    monkeypatch.setattr(latent, "_own_keys_pay", lambda *a: True)
+    rng = np.random.default_rng(window)
+    for _ in range(40):
+        q = rng.integers(0, 300, rng.integers(1, 9)).tolist()
+        c = [max(n, 1) + (int(rng.integers(0, 500)) if n > 1 else 0) for n in q]
+        if not any(q):
+            continue
+        work, key_row, tiles, at = [], [], [], 0
+        for r, (n, have) in enumerate(zip(q, c)):
+            start = max(0, have - n - window + 1) // 128 * 128 if window else 0
+            key_row.append(at - start if n else 0)
+            for first in range(start, have, 16) if n else ():
+                work.append([r, first])
+                at += 16
+            for t0 in range(0, n, 128):
+                lo = max(0, have - n + t0 - window + 1) if window else 0
+                tiles.append((min(have - n + t0 + 128, have) // 128 - lo // 128, r, t0))
+        tiles = [list(t[1:]) for t in sorted(tiles)]
+        got = latent.latent_keys_plan(q, c, None, window, SIZES_3B)
+        assert got.arrays["work"].tolist() == work and got.arrays["key_row"].tolist() == key_row and got.arrays["tiles"].tolist() == tiles
+        assert all(a.dtype.name == "int32" for a in got.arrays.values())
+        filler = len(q)
+        got = latent.latent_keys_plan(q + [0], c + [1], filler, window, SIZES_3B)
+        n_work, n_tiles = len(got.arrays["work"]), len(got.arrays["tiles"])
+        assert got.arrays["work"].tolist() == work + [[filler, 0]] * (n_work - len(work)) and n_work % 8 == 0
+        assert got.arrays["tiles"].tolist() == [[filler, 0]] * (n_tiles - len(tiles)) + tiles and n_tiles % 8 == 0
+        assert got.shape == ("keys", n_work, len(q) + 1, n_tiles)
+
+
+def test_plan_of_own_keys_is_bounded_and_left_to_steps_of_prompts():
+    from boring_llm_b200.parts.latent import latent_keys_plan, OWN_KEYS_MAX_BYTES
+    assert latent_keys_plan([2000], [2000], None, 0, SIZES_3B) is not None
+    assert latent_keys_plan([2000, 1], [2000, 129], None, 0, SIZES_3B) is None                  # a token that decodes
+    # short portions behind long contexts: their rows would take gigabytes
+    for portions, tokens, have in ((64, 32, 4096), (4, 512, 32768), (16, 128, 32768)):
+        assert latent_keys_plan([tokens] * portions, [have] * portions, None, 0, SIZES_3B) is None
+    for have in range(512, 40000, 512):
+        plan = latent_keys_plan([512], [have], 1, 0, SIZES_3B)
+        if plan is not None:
+            assert len(plan.arrays["work"]) * 16 * 16 * 256 * 2 <= OWN_KEYS_MAX_BYTES
+
+
+def test_portions_of_a_long_prompt_share_their_captured_steps():
+    """Without a window every portion sees more rows than the one before: four shapes an octave at most."""
+    from boring_llm_b200.parts.latent import latent_keys_plan
+    plans = [latent_keys_plan([512, 0], [have, 1], 1, 0, SIZES_3B) for have in range(512, 16384 + 1, 512)]
+    shapes = {p.shape for p in plans if p is not None}
+    assert sum(p is not None for p in plans) >= 16 and len(shapes) <= 4 * 5 + 1
+
+
+def test_layers_of_one_kind_are_planned_once(monkeypatch):
+    """Eight layers of two kinds and a step of many requests: one plan each, and no lists where the cached rows are the faster."""
+    import boring_llm_b200 as b
+    from boring_llm_b200.parts import latent
+    mixer = {"heads": 14, "dim": 64, "rot_dim": 32, "vdim": 64, "q_rank": 64, "kv_rank": 256, "scale": 0.1, "rot": {"base": 1e4, "dims": 32}}
+    layers = [{"type": "latent_attention", "mixer": dict(mixer, mask={"size": 1024}) if i % 2 else dict(mixer), "mlp": None} for i in range(8)]
+    model = b.build_model(b.MiforaxConfig.from_dict({"architecture": "Miforax", "vocab": 32, "width": 64, "norm": {"eps": 1e-6},
+                                                     "embedding": {"scale": 1.0}, "layers": layers}))
+    asked, made = [], []
+    plan, empty = latent.latent_keys_plan, np.empty
+    monkeypatch.setattr(latent, "latent_keys_plan", lambda *a: asked.append(a) or plan(*a))
+    monkeypatch.setattr(latent.LatentAttention, "_makes_keys", lambda self: True)
+    monkeypatch.setattr(np, "empty", lambda *a, **k: made.append(a) or empty(*a, **k))
+    assert len(model.collect_plans([2] * 64, [4000] * 64)) == 2
+    assert len(asked) == 2 and not made
+    assert len(model.collect_plans([512], [512])) == 2 and len(asked) == 4 and len(made) == 2
