@@ -547,6 +547,7 @@ int bl_latent_attention_mma(const void* q_lat, const void* q_rot, const void* ca
 // Products of up to 64 rows by large matrices (a decode step's; gemm_tcgen05_few.cu): W streams once as the M side of the MMA,
 // clusters cut K where W has few tiles. out 32-bit (no epilogue, bias, residual) or, with the gated epilogue, bfloat16.
 int bl_gemm_tc_few_supported(int M, int N, int K);
+int bl_gemm_tc_few_blocks(int N, int K, int epilogue);
 int bl_gemm_tc_few(const void* x, const void* w, const void* bias, int bias_dtype, void* out, int out_dtype, int M, int N, int K,
                    int epilogue, void* stream);
 int bl_gemm_tc_few_status(int* status);

@@ -363,6 +363,12 @@ int launch_rows(const void* x, const void* w, const void* bias, int bias_dtype, 
 
 }  // namespace
 
+// The blocks of this kernel's launch (the blocks of clusters where tiles are shared, else one a tile, the SMs walk them in rounds).
+extern "C" int bl_gemm_tc_few_blocks(int N, int K, int epilogue) {
+    const int units = epilogue == BL_EPI_SWIGLU ? BN / 2 : BN, n_tiles = (N + units - 1) / units;
+    return n_tiles * split_for(n_tiles, (K + BK - 1) / BK);
+}
+
 extern "C" int bl_gemm_tc_few_supported(int M, int N, int K) { return M >= 1 && M <= 64 && N >= 1 && K >= 8 && K % 8 == 0; }
 
 extern "C" int bl_gemm_tc_few(const void* x, const void* w, const void* bias, int bias_dtype, void* out, int out_dtype, int M, int N, int K,

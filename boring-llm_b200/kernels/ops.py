@@ -693,47 +693,73 @@ SPLITK_FEW_ROWS_K = 8192              # ... or, from 9 rows, this long (9 and 16
                                       # 1,024 10.8 and 10.9 against 9.3 and 11.0, 8,192 by 256 6.8 against 5.6 and 6.6; 16 rows of 4,864 by 896 7.1 against 4.8),
 SPLITK_MORE_ROWS_K = 4096             # ... or, from 17 rows, this long (17 and 31 rows of 4,864 by 896: 7.1 and 7.3 us against 9.9 and 12.0, of 4,096 by 2,048 8.0
                                       # and 8.3 against 8.4 and 10.4, by 136 5.2 and 5.3 against 6.0 and 7.8; 24 rows of 2,048 by 2,048 7.4 against 5.4)
-STREAM_MIN_BYTES = 64 << 20           # matrices from this size on stream faster through TMA and tcgen05 than through registers, at any number of rows
-                                      # (90 MB of gate and up rows, K 2,048: 1, 8 and 16 rows 21.1, 21.4 and 21.8 us against 26.2, 28.0 and 47.4)
+STREAM_TILES_MIN_BYTES = 128 << 20    # matrices from this size on stream faster through TMA in tcgen05 tiles than through registers, at any number of rows;
+                                      # gated ones at 32 rows and more half of it (5,120 by 3,584 + 3,584, 32 and 64 rows: 35 and 61 us -> 21 and 21)
+STREAM_MIN_BYTES = 64 << 20           # ... and from this size on through the kernel made for few rows (90 MB of gate and up rows, K 2,048: 1, 8 and 16 rows
+                                      # 20.8, 21.0 and 21.6 us against 25.5, 27.1 and 46.7), so that a norm is not linked to such a product
 SPLITK_LONG_K = 2048                  # ... when K is long (measured: K 4,864 by N 896 gains 2x at 128 rows, 1.25x at 512; K 896 gains only up to 128 rows)
 
 
 def gemm_streams_better(w: torch.Tensor) -> bool:
-    """Whether a matrix is so large that few rows of x are better served by the TMA-fed tcgen05 kernels than by the
-    kernels that stream W through registers (measured on 272 MB at 8 rows: 4.3 TB/s against 2.6 TB/s)."""
+    """Whether a matrix is so large that few rows of x are better served by the kernels that stream W through TMA (`gemm_few_better`) than by those
+    that stream it through registers and share a norm with their neighbours."""
     return w.numel() * w.element_size() >= STREAM_MIN_BYTES
 
 
-def gemm_few_better(M: int, N: int, w: torch.Tensor, epilogue: int) -> bool:
-    """Whether a product of up to 64 rows runs on the kernel that streams W once as the M side of the MMA (`gemm_tc_few`). A small W
-    is left to the kernels without its 4 us of set-up; where the line lies depends on what stands on the other side. Microseconds,
-    the kernel before and this one, cold matrices, launches in a row:
+@functools.lru_cache(maxsize=4096)
+def _few_fill(N: int, K: int, epilogue: int) -> float:
+    """The share of the device's SMs that `gemm_tc_few` keeps busy: its blocks over whole rounds of SMs."""
+    blocks = int(library.load().bl_gemm_tc_few_blocks(N, K, epilogue))
+    return blocks / (-(-blocks // _sms()) * _sms())
 
-    gated epilogue, up to 31 rows: 18,944 + 18,944 x 3,584 1 row 61.5 / 42.1, 16 61.5 / 43.2, 24 44.9 / 43.5; 11,008 + 11,008 x 2,048
-        8 rows 28.0 / 21.4, 24 34.9 / 22.6, but 32 20.5 / 22.9 and 64 21.1 / 25.4;
-    up to 8 rows by bytes: 8 rows of 8,208 x 2,048 11.4 / 8.4, 3,584 x 3,584 9.0 / 7.9, 6,224 x 2,048 8.7 / 8.0, 2,048 x 11,008 14.4 / 12.3, one
-        row of 3,584 x 18,944 38.6 / 27.1, 11,008 x 2,048 11.5 / 10.8; but 2,560 x 2,048 5.1 / 5.8;
-    9 to 16 rows, smaller ones if they have columns: 16 rows of 4,864 x 896 6.5 / 5.3, 2,560 x 2,048 6.8 / 5.9, 3,584 x 3,584 12.0 / 8.0; but
-        2,048 x 2,048 3.8 / 5.7, 896 x 4,864 5.2 / 5.4;
-    17 to 32 rows: 896 x 4,864 7.2 / 5.6, 3,600 x 896 5.4 / 5.0, 4,608 x 3,584 10.3 / 10.0; but 24 rows of 2,048 x 2,048 4.6 / 5.5;
-    33 to 64 rows: 64 rows of 2,048 x 2,048 7.5 / 7.0, 3,584 x 3,584 11.4 / 9.5, 8,208 x 2,048 11.3 / 10.5, 3,600 x 896 10.9 / 5.6; but
-        11,008 x 2,048 12.1 / 12.9, 4,864 x 896 6.4 / 6.7, 2,048 x 11,008 14.2 / 14.5, 1,152 x 896 3.1 / 5.6, and
-        with 896 x 4,864 a step of 64 requests takes 1,084 / 1,093 (blocks on 112 SMs / 56)."""
+
+def gemm_few_better(M: int, N: int, w: torch.Tensor, epilogue: int, kind: str, sums_only: bool) -> bool:
+    """Whether a product of up to 64 rows runs on the kernel that streams W once as the M side of the MMA (`gemm_tc_few`) instead of on
+    `kind`, the kernel that takes it otherwise. Its time is 4 us and the stream of W at the share of the SMs that its tiles (or
+    clusters of blocks that share one) fill; measured against every other kernel at 1 to 64 rows of 16 numbers of columns by 13 of K
+    (256 to 18,944 by 512 to 14,336), and gated at 10 by 7, cold matrices, launches in a row. Microseconds, the other kernel / this one:
+
+    through registers ("skinny"): small matrices stay there, by bytes. Up to 8 rows from 24 MB (8 rows of 8,192 x 2,048 12.1 / 8.8, one row of
+        11,008 x 3,584 51.7 / 18.4), but not with up to 1,024 columns (14,336 by 1,024 9.1 / 10.9) and, up to 40 MB, not where the other kernel's
+        blocks of 16 columns just fill the SMs (8,192 by 2,048 9.1 / 10.0); 9 to 16 rows from 20 MB or, from 2,560 columns on, 8.5 MB
+        (2,560 x 2,048 7.0 / 6.3), but short K in clusters of three (1,024 by 4,608 5.3 / 6.0); 17 to 32 rows 8.5 and 6 MB; more 8 and 6 MB;
+    K cut over clusters ("splitk"): 4 to 15 % faster up to 4,096 columns, but with more by a long K only where the clusters fill the device (64
+        rows of 6,144 x 14,336 in 96 blocks 40.4 / 43.2, of 8,192 x 14,336 in 128 3 % faster), and not few columns by a very long K (576 x
+        14,336 10.2 / 11.2);
+    the output head's kernel ("cols"): 3 to 9 % faster, but between 512 and 2,048 of K only where the rounds are nearly full (25,000 x 1,024, 196
+        tiles, 11.3 / 12.2; 18,944, 148 tiles, 8.9 / 8.2); so, too, tiles of 128 rows for plain sums of as many columns (32 rows of 25,000 x
+        3,584 33.7 / 38.3);
+    tiles of 128 rows ("tc"): half the time at up to 2,560 of K, but 8 to 16 rows of 11,008 x 11,008, 86 tiles, 50.0 / 55.1;
+    gated, up to 31 rows from 64 MB (24 rows of 11,008 + 11,008 x 2,048 32.7 / 22.3), but with more than 16 rows by a K above 2,560, or 13 to 16 by
+        one above 3,584, only where the rounds are nearly full (24 rows of 3,584 by 11,008 + 11,008, 172 tiles, 31.2 / 38.5, by 18,944 +
+        18,944, 296 tiles, 43.5 / 42.8; 32 rows lose 10 % and more at most sizes)."""
     rows_w, K = w.shape
     nbytes = 2 * rows_w * K
     if M > 64 or N >= TC_MIN_COLUMNS_VERY_FEW_ROWS:
         return False
     if epilogue == EPI_SWIGLU:
-        return M < 32 and nbytes >= STREAM_MIN_BYTES
+        return (M < 32 and nbytes >= STREAM_MIN_BYTES
+                and (kind == "skinny" or M <= 12 or K <= (2560 if M > 16 else 3584) or _few_fill(N, K, epilogue) >= 0.85))
     if M <= 8:
-        return nbytes >= 24e6
-    if M <= 16:
-        return nbytes >= 20e6 or (N >= 2560 and nbytes >= 8.5e6)
-    if M <= 32:
-        return nbytes >= 8.5e6 or (N >= 2560 and nbytes >= 6e6)
-    if N > 4096 and (K <= 1024 or N >= 10240) or N <= 2048 and K > 4096:
+        large = nbytes >= 24e6 and N > 1024 and not (1792 <= N <= 2368 and nbytes < 40e6)
+    elif M <= 16:
+        large = nbytes >= 20e6 or (N >= 2560 and nbytes >= 8.5e6 and not (4096 < N < 5120 and K < 1536))
+    elif M <= 32:
+        large = nbytes >= 8.5e6 or (N >= 2560 and nbytes >= 6e6)
+    else:
+        large = ((nbytes >= 8e6 or (N >= 2560 and nbytes >= 6e6))
+                 and not (N > 4096 and (K <= 1024 or N >= 10240) or N <= 2048 and K > 4096))
+    if not large:
         return False
-    return nbytes >= 8e6 or (N >= 2560 and nbytes >= 6e6)
+    if kind == "splitk":
+        return not (N < 1024 and K > 8192) and (N <= 4096 or K <= 2048 or _few_fill(N, K, epilogue) >= 0.75)
+    if kind == "cols":
+        return not 512 < K < 2048 or _few_fill(N, K, epilogue) >= 0.85
+    if kind == "tc" and sums_only and N >= COLS_MIN_COLUMNS:
+        return _few_fill(N, K, epilogue) >= 0.85
+    if kind == "tc" and 8 <= M <= 16 and K > 8192:
+        return _few_fill(N, K, epilogue) >= 0.6
+    return True
 
 
 def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
@@ -770,11 +796,14 @@ def gemm_kernel(x: torch.Tensor, w: torch.Tensor, N: int, bias: Optional[torch.T
     "skinny" (few rows: W streams through registers), "tc" or "pair" (tcgen05 tiles on one SM, on pairs of SMs)."""
     if not (fast and gemm_skinny_supported(x, w)):
         return "plain"
+    kind = _gemm_kernel_beside_few(x, w, N, bias, epilogue)
+    return "few" if few and gemm_few_better(x.shape[0], N, w, epilogue, kind, bias is None and epilogue == EPI_NONE) else kind
+
+
+def _gemm_kernel_beside_few(x: torch.Tensor, w: torch.Tensor, N: int, bias: Optional[torch.Tensor], epilogue: int) -> str:
     M, K = x.shape
-    if few and gemm_few_better(M, N, w, epilogue):
-        return "few"
     few_rows_tc = ((M > 16 and N >= TC_MIN_COLUMNS_FEW_ROWS) or (M > 8 and N >= TC_MIN_COLUMNS_VERY_FEW_ROWS)
-                   or gemm_streams_better(w))
+                   or w.numel() * w.element_size() >= (STREAM_TILES_MIN_BYTES // 2 if epilogue == EPI_SWIGLU and M >= 32 else STREAM_TILES_MIN_BYTES))
     if ((N >= TC_MIN_COLUMNS_VERY_FEW_ROWS or (N >= COLS_MIN_COLUMNS and M <= 32)) and bias is None and epilogue == EPI_NONE
             and M <= 64 and gemm_tc_cols_supported(x, w)):
         return "cols"
@@ -804,7 +833,7 @@ def gemm_skinny_links_norm(x: torch.Tensor, w: torch.Tensor, N: int, epilogue: i
     """Whether `gemm` would run this product on the register-streaming kernel at a row count where that kernel's
     epilogues begin an RMS norm (`gemm_skinny_residual_norm`) and finish one (`gemm_skinny_scaled`)."""
     return (SKINNY_LINK_MIN_ROWS <= x.shape[0] <= SKINNY_LINK_MAX_ROWS and -(-N // 16) <= SKINNY_LINK_MAX_BLOCKS
-            and gemm_kernel(x, w, N, None, epilogue, fast, few=False) == "skinny")
+            and not gemm_streams_better(w) and gemm_kernel(x, w, N, None, epilogue, fast, few=False) == "skinny")
 
 
 def gemm_skinny_residual_norm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, norm_w: torch.Tensor,

@@ -965,12 +965,16 @@ def test_gated_activation_of_few_rows_is_the_same_in_both_kernels(kind):
 
 
 def test_few_rows_go_by_the_bytes_of_w():
-    """The kernel on either side of its lines, and that a product that an RMS norm links to another stays where the norm is."""
+    """The kernel on either side of its lines (by bytes, and by the share of the device that its blocks fill), and that a product that an RMS norm links to another stays where the norm is."""
     o = ops()
     m = lambda *s: torch.empty(*s, dtype=BF, device=DEV)
     kinds = [(8, 8208, 2048, o.EPI_NONE, "few"), (8, 2560, 2048, o.EPI_BIAS, "skinny"), (16, 2560, 2048, o.EPI_BIAS, "few"), (16, 2048, 2048, o.EPI_RESIDUAL, "skinny"),
              (17, 896, 4864, o.EPI_RESIDUAL, "few"), (64, 896, 4864, o.EPI_RESIDUAL, "splitk"), (64, 3600, 896, o.EPI_NONE, "few"), (64, 1152, 896, o.EPI_BIAS, "skinny"), (64, 11008, 2048, o.EPI_NONE, "tc"),
-             (16, 11008, 2048, o.EPI_SWIGLU, "few"), (32, 11008, 2048, o.EPI_SWIGLU, "tc"), (65, 8208, 2048, o.EPI_NONE, "splitk")]
+             (16, 11008, 2048, o.EPI_SWIGLU, "few"), (32, 11008, 2048, o.EPI_SWIGLU, "tc"), (65, 8208, 2048, o.EPI_NONE, "splitk"),
+             (8, 1024, 14336, o.EPI_RESIDUAL, "skinny"), (8, 2048, 8192, o.EPI_RESIDUAL, "skinny"), (16, 4608, 1024, o.EPI_RESIDUAL, "skinny"),
+             (24, 576, 14336, o.EPI_RESIDUAL, "splitk"), (64, 6144, 14336, o.EPI_RESIDUAL, "splitk"), (64, 8192, 14336, o.EPI_RESIDUAL, "few"),
+             (16, 25000, 1024, o.EPI_NONE, "cols"), (16, 18944, 1024, o.EPI_NONE, "few"), (8, 11008, 11008, o.EPI_RESIDUAL, "tc"),
+             (24, 11008, 3584, o.EPI_SWIGLU, "tc"), (24, 18944, 3584, o.EPI_SWIGLU, "few"), (32, 3584, 5120, o.EPI_SWIGLU, "tc")]
     for M, N, K, epi, kind in kinds:
         b = torch.empty(N, device=DEV) if epi == o.EPI_BIAS else None
         assert o.gemm_kernel(m(M, K), m(2 * N if epi == o.EPI_SWIGLU else N, K), N, b, epi) == kind, (M, N, K)
