@@ -1607,17 +1607,29 @@ def moe_plan(ids: torch.Tensor, n_experts: int):
 EXPERT_TILE = 16           # rows of x that one expert's share of them is padded to (see `moe_chunks`)
 EXPERT_CHUNK, EXPERT_CHUNK_FEW = 256, 64     # the most rows of an expert that are multiplied together ...
 EXPERT_FEW_PAIRS = 32      # ... the second up to this many pairs an expert on average
-EXPERT_LARGE = 1 << 22     # values of one of an expert's matrices from which chunks are the faster form for many rows, too
+EXPERT_LARGE = 1 << 22     # values of one of an expert's matrices from which chunks are the faster form for many rows, too ...
+EXPERT_ROUNDS = 1.7        # ... if the chunks by the tiles of either product make so many rounds of the device
+EXPERT_PLAN_MAX = 4095     # experts whose counts fit the plan's shared memory
 
 
 def experts_in_chunks(pairs: int, n_experts: int, dim: int, hidden: int) -> bool:
     """Whether routed experts run in chunks with W as the M side (`moe_chunks`, `gemm_experts`) or in tiles of 128 rows (`moe_plan`,
-    `gemm_grouped`). Chunks pad nothing, but a work item is up to 256 rows by 128 of W, and small matrices make few of those for the
-    device. Both products, 16 experts of which a token has two, microseconds in tiles and in chunks:
-        tokens                                8           64           256          1,000       2,000
-        2,048 wide, 2,752 hidden values   79 / 72     110 / 89     110 / 92     135 / 117    190 / 166
-        896 wide, 1,216 hidden values     23 / 19      33 / 25      33 / 27                   48 / 57"""
-    return pairs <= EXPERT_FEW_PAIRS * n_experts or dim * hidden >= EXPERT_LARGE
+    `gemm_grouped`). Chunks pad nothing, but a work item is up to 256 rows by 128 of W, and small matrices, or few experts, make few of
+    those for the device. Plan, gather and both products, a token in two experts (in 8 of 64), microseconds in tiles and in chunks:
+        tokens                                            8           64           256          512          1,000        2,000
+        16 experts,  896 wide, 1,216 hidden values    26 / 23      39 / 31      39 / 31      42 / 39      45 / 46      57 / 66
+        16 experts, 1,536 wide, 2,304                 61 / 46      78 / 66      78 / 70      79 / 82      89 / 92     126 / 123
+        16 experts, 2,048 wide, 2,752                 81 / 69     114 / 93     115 / 98     116 / 113    134 / 124    196 / 171
+        16 experts, 4,096 wide, 1,536                 97 / 78     135 / 104    136 / 109    138 / 132    146 / 147    221 / 199
+        64 experts, 2,048 wide, 2,752                288 / 234    399 / 332    402 / 348    406 / 392    477 / 438    707 / 608
+         8 experts, 2,048 wide, 2,752                 65 / 53      68 / 56      73 / 68      76 / 76      93 / 106    150 / 135
+         8 experts, 4,096 wide, 1,536                 70 / 63      70 / 65      71 / 82      83 / 92     112 / 120    176 / 160"""
+    if n_experts > EXPERT_PLAN_MAX:
+        return False
+    if pairs <= EXPERT_FEW_PAIRS * n_experts:
+        return True
+    items = max(n_experts, -(-pairs // EXPERT_CHUNK)) * min(hidden // 64, dim // 128)       # of the product that makes fewer
+    return dim * hidden >= EXPERT_LARGE and items >= EXPERT_ROUNDS * _sms()
 
 
 def moe_chunks(ids: torch.Tensor, n_experts: int):

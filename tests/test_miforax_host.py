@@ -220,3 +220,14 @@ def test_layers_of_one_kind_are_planned_once(monkeypatch):
     assert len(model.collect_plans([2] * 64, [4000] * 64)) == 2
     assert len(asked) == 2 and not made
     assert len(model.collect_plans([512], [512])) == 2 and len(asked) == 4 and len(made) == 2
+
+
+@pytest.mark.parametrize("experts,top,dim,hidden,tokens,chunks", [
+    (16, 2, 2048, 2752, 2000, True), (16, 2, 2048, 2752, 1000, True), (8, 2, 2048, 2752, 1000, False), (8, 2, 2048, 2752, 2000, True),
+    (8, 2, 4096, 1536, 1000, False), (8, 2, 4096, 1536, 128, True), (16, 2, 896, 1216, 2000, False), (16, 2, 896, 1216, 256, True),
+    (4095, 2, 2048, 2752, 1, True), (4096, 2, 2048, 2752, 1, False), (6000, 2, 256, 256, 100, False)])
+def test_who_takes_the_products_of_routed_experts(experts, top, dim, hidden, tokens, chunks, monkeypatch):
+    """Chunks where they were measured to be the faster; more experts than their plan has shared memory for keep the tiles."""
+    from boring_llm_b200.kernels import ops
+    monkeypatch.setattr(ops, "_sms", lambda: 148)
+    assert ops.experts_in_chunks(tokens * top, experts, dim, hidden) == chunks
