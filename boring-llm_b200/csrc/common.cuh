@@ -145,6 +145,15 @@ __device__ __forceinline__ float bl_attn_tail(const BlAttnTail& t, float m_log2,
     return inv;
 }
 
+// The device's SMs (148 where they cannot be asked for).
+inline int bl_device_sms() {
+    static const int sms = [] {
+        int dev = 0, n = 0;
+        return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
+    }();
+    return sms;
+}
+
 // Programmatic dependent launch. A kernel launched with bl_launch_dependent() may start while its predecessor
 // on the stream is still running; whatever it does before bl_pdl_wait() must touch only data that no earlier
 // kernel of the step writes (weights, the step's index arrays). bl_pdl_wait() returns once the predecessor has

@@ -68,34 +68,13 @@ struct Tile {
 __device__ int g_status = 0;               // 0 = fine; else the code of the first wait that ran out
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* give_up, int code) {
-#pragma unroll 1
-    for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (*give_up) return false;
-    }
-    *give_up = 1;
-    atomicCAS(&g_status, 0, code);
-    return false;
-}
-// Bounded wait that does not look at the give-up flag (a block that has given up waits for its own copies).
-__device__ __forceinline__ void mbar_wait_plain(uint32_t bar, uint32_t parity) {
-#pragma unroll 1
-    for (uint32_t i = 0; i < WAIT_LIMIT; ++i)
-        if (mbar_try_wait(bar, parity)) return;
+    return mbar_wait_bounded(bar, parity, WAIT_LIMIT, give_up, &g_status, code);
 }
 // Operand tile of rows of 64 bytes (32 bfloat16 values of k) with 64-byte swizzle: groups of 8 rows 512 bytes apart.
 __device__ __forceinline__ uint64_t smem_desc64(uint32_t addr) {
     const uint32_t lo = ((addr >> 4) & 0x3FFFu) | (1u << 16);
     const uint32_t hi = (512u >> 4) | (1u << 14) | (4u << 29);
     return ((uint64_t)hi << 32) | lo;
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-                 "tcgen05.wait::ld.sync.aligned;"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
 }
 // The next parts of two numbers as a pair, and what is left of them.
 __device__ __forceinline__ uint32_t next_parts(float& a, float& b) {
@@ -104,9 +83,6 @@ __device__ __forceinline__ uint32_t next_parts(float& a, float& b) {
     a -= __uint_as_float(u << 16);
     b -= __uint_as_float(u & 0xffff0000u);
     return u;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ float ld_cluster(uint32_t addr) {
     float v;
@@ -227,7 +203,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             }
         }
         if (*give_up)                                                      // let our own copies land before leaving
-            for (int s = max(0, issued - RAWS); s < issued; ++s) mbar_wait_plain(raw_full0 + 8 * (s % RAWS), (uint32_t)((s / RAWS) & 1));
+            for (int s = max(0, issued - RAWS); s < issued; ++s) mbar_wait_landed(raw_full0 + 8 * (s % RAWS), (uint32_t)((s / RAWS) & 1), WAIT_LIMIT);
     } else if (warp >= 8) {
         // ================= splitters: thread (row t / 8 + 32 i, piece t % 8) of W (i < 4) and of x (i >= 4)
         const int t = threadIdx.x - ADDERS, row = t >> 3, piece = t & 7;
@@ -293,7 +269,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 #pragma unroll
             for (int c = 0; c < T::COLS; c += 16) {
                 uint32_t r[16];
-                tmem_ld16(t_at + b * NT + c, r);
+                tmem_ld16_wait(t_at + b * NT + c, r);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) acc[c + j] += __uint_as_float(r[j]);
             }
@@ -308,12 +284,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 #pragma unroll
         for (int c = 0; c < T::COLS; c += 16) {
             uint32_t r[16] = {};
-            if (ok && steps > 0) tmem_ld16(t_at + 2 * NT + c, r);          // (the warps agree on ok, and the last segment's barrier has been waited for)
+            if (ok && steps > 0) tmem_ld16_wait(t_at + 2 * NT + c, r);          // (the warps agree on ok, and the last segment's barrier has been waited for)
 #pragma unroll
             for (int j = 0; j < 16; ++j) sums[BM * NT + at + (c + j) * BM] = __uint_as_float(r[j]);
         }
     }
-    if (spans > 1) cluster_sync(); else __syncthreads();
+    if (spans > 1) cluster_meet(); else __syncthreads();
     const BlGluArgs glu = bl_glu_args(GLU ? bias : nullptr);
     auto peer_byte = [&](const void* at, int r) {                          // a byte of the shared memory of block r of the cluster
         if (spans == 1) return (int)*reinterpret_cast<const unsigned char*>(at);
@@ -370,19 +346,11 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         *dst = s;
     }
     fence_before_sync();
-    if (spans > 1) cluster_sync(); else __syncthreads();                   // no block leaves while another may still read its sums
+    if (spans > 1) cluster_meet(); else __syncthreads();                   // no block leaves while another may still read its sums
     if (warp == 8) {
         fence_after_sync();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(T::TMEM_COLS) : "memory");
     }
-}
-
-int device_sms() {
-    static const int sms = [] {
-        int dev = 0, n = 0;
-        return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
-    }();
-    return sms;
 }
 
 // A row-major matrix of 32-bit numbers, rows `ld` apart, as a tensor map with boxes of box_rows rows of BK values as they lie.
@@ -429,7 +397,7 @@ int launch_width(const float* x, const float* w, const void* bias, int bias_dtyp
     // shared memory).
     const int units = EPI == BL_EPI_SWIGLU ? BM / 2 : BM;
     const long long n_tiles = (N + units - 1) / units;
-    const int slots = spans > 1 ? device_sms() / spans - (spans > 2 ? 1 : 0) : device_sms();       // tiles under way at once
+    const int slots = spans > 1 ? bl_device_sms() / spans - (spans > 2 ? 1 : 0) : bl_device_sms();       // tiles under way at once
     const int widths[] = {128, 96, 64, 32, 16};
     int best = 0;
     double least = 0.0;

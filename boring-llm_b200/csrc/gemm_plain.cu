@@ -194,7 +194,7 @@ int launch_rank(const float* x, const TW* w, const void* bias, int bias_dtype, f
     // rows a block: up to 16, fewer where the launch would not give every SM four blocks
     const int across = (N + RANK_THREADS - 1) / RANK_THREADS;
     int rows = 16;
-    while (rows > 1 && (long long)across * ((M + rows - 1) / rows) < 4 * 148) rows >>= 1;
+    while (rows > 1 && (long long)across * ((M + rows - 1) / rows) < 4 * bl_device_sms()) rows >>= 1;
     const dim3 grid(across, (M + rows - 1) / rows);
     const size_t bytes = (size_t)rows * K * sizeof(float);
 #define BL_GO(KM) BL_CUDA(bl_launch_dependent(gemm_rank_kernel<TW, EPI, KM>, grid, dim3(RANK_THREADS), bytes, s, x, w, bias, bias_dtype, out, \
@@ -346,19 +346,11 @@ struct F32Tile { int bm, bn; float alone, pace; };
 constexpr F32Tile F32_TILES[] = {{64, 32, 18.5f, 13.2f}, {32, 32, 11.8f, 8.3f}, {16, 64, 12.8f, 9.4f},
                                  {16, 32, 9.3f, 6.4f}, {4, 64, 11.8f, 5.9f}, {4, 16, 6.8f, 1.95f}};
 
-int f32_sms() {
-    static const int sms = [] {
-        int dev = 0, n = 0;
-        return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
-    }();
-    return sms;
-}
-
 int launch_f32_tiles(const float* x, const float* w, const void* bias, int bias_dtype, float* out, int M, int N, int K, int ldx, int epi,
                      cudaStream_t s) {
     int best = 0;
     float best_us = 0.f;
-    const int sms = f32_sms();
+    const int sms = bl_device_sms();
     for (int v = 0; v < (int)(sizeof(F32_TILES) / sizeof(F32_TILES[0])); ++v) {
         const F32Tile& t = F32_TILES[v];
         const int cols = epi == BL_EPI_SWIGLU ? t.bn / 2 : t.bn;

@@ -42,28 +42,7 @@ struct Ring {
 __device__ int g_status = 0;            // 0 = fine; else the code of the first wait that ran out
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* give_up, int code) {
-#pragma unroll 1
-    for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (*give_up) return false;
-    }
-    *give_up = 1;
-    atomicCAS(&g_status, 0, code);
-    return false;
-}
-// Bounded wait that does not look at the give-up flag (a block that has given up waits for its own copies).
-__device__ __forceinline__ void mbar_wait_plain(uint32_t bar, uint32_t parity) {
-#pragma unroll 1
-    for (uint32_t i = 0; i < WAIT_LIMIT; ++i)
-        if (mbar_try_wait(bar, parity)) return;
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-                 "tcgen05.wait::ld.sync.aligned;"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
+    return mbar_wait_bounded(bar, parity, WAIT_LIMIT, give_up, &g_status, code);
 }
 
 // chunks[0].x: how many; chunks[1 + c]: {first row of x, rows (a multiple of 16, up to NT), expert, 0}.
@@ -135,7 +114,7 @@ gemm_tc_experts_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
                 }
             }
             if (*give_up)                                                      // let our own copies land before leaving
-                for (int i = max(0, it - STAGES); i < it; ++i) mbar_wait_plain(full0 + 8 * (i % STAGES), (uint32_t)((i / STAGES) & 1));
+                for (int i = max(0, it - STAGES); i < it; ++i) mbar_wait_landed(full0 + 8 * (i % STAGES), (uint32_t)((i / STAGES) & 1), WAIT_LIMIT);
         }
         __syncwarp();
     } else if (warp == 2) {
@@ -178,7 +157,7 @@ gemm_tc_experts_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
 #pragma unroll 1
             for (int t = 0; t < c.y; t += 16) {
                 uint32_t r[16];
-                tmem_ld16(taddr + t, r);
+                tmem_ld16_wait(taddr + t, r);
                 if (GLU) {
 #pragma unroll
                     for (int j = 0; j < 16; j += 2) {                          // lanes 0..15 gate row t + j, lanes 16..31 row t + j + 1
@@ -206,14 +185,6 @@ gemm_tc_experts_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
     }
 }
 
-int sm_count() {
-    static const int n = [] {
-        int dev = 0, v = 0;
-        return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0 ? v : 148;
-    }();
-    return n;
-}
-
 template <bool GLU, typename TO, int NT>
 int launch(const CUtensorMap& mx, const CUtensorMap& mw, const int4* chunks, const float* act, void* out, int max_chunks, int N, int K, cudaStream_t s) {
     static std::atomic<bool> configured{false};
@@ -223,7 +194,7 @@ int launch(const CUtensorMap& mx, const CUtensorMap& mw, const int4* chunks, con
     }
     const long long items = (long long)max_chunks * ((N + (GLU ? BN / 2 : BN) - 1) / (GLU ? BN / 2 : BN));
     if (items > 0x7fffffffLL) BL_FAIL("bl_gemm_tc_experts: too many tiles");
-    const int blocks = items < sm_count() ? (int)items : sm_count();
+    const int blocks = items < bl_device_sms() ? (int)items : bl_device_sms();
     BL_CUDA(bl_launch_dependent(gemm_tc_experts_kernel<GLU, TO, NT>, dim3((unsigned)blocks), dim3(THREADS), (size_t)Ring<NT>::SMEM_BYTES, s,
                                 mx, mw, chunks, act, (TO*)out, N, K));
     BL_CHECK_LAUNCH("bl_gemm_tc_experts");

@@ -45,31 +45,7 @@ struct Ring {
 __device__ int g_status = 0;            // 0 = fine; else the code of the first wait that ran out
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* give_up, int code) {
-#pragma unroll 1
-    for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (*give_up) return false;
-    }
-    *give_up = 1;
-    atomicCAS(&g_status, 0, code);
-    return false;
-}
-// Bounded wait that does not look at the give-up flag (a block that has given up waits for its own copies).
-__device__ __forceinline__ void mbar_wait_plain(uint32_t bar, uint32_t parity) {
-#pragma unroll 1
-    for (uint32_t i = 0; i < WAIT_LIMIT; ++i)
-        if (mbar_try_wait(bar, parity)) return;
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-                 "tcgen05.wait::ld.sync.aligned;"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    return mbar_wait_bounded(bar, parity, WAIT_LIMIT, give_up, &g_status, code);
 }
 __device__ __forceinline__ float4 ld_cluster4(uint32_t addr) {
     float4 v;
@@ -194,7 +170,7 @@ gemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 issued = it + 1;
             }
             if (*give_up)                                                      // let our own copies land before leaving
-                for (int it = max(0, issued - STAGES); it < issued; ++it) mbar_wait_plain(full0 + 8 * (it % STAGES), (uint32_t)((it / STAGES) & 1));
+                for (int it = max(0, issued - STAGES); it < issued; ++it) mbar_wait_landed(full0 + 8 * (it % STAGES), (uint32_t)((it / STAGES) & 1), WAIT_LIMIT);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -232,7 +208,7 @@ gemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 #pragma unroll
                 for (int c = 0; c < NT; c += 16) {
                     uint32_t r[16];
-                    tmem_ld16(taddr + c, r);
+                    tmem_ld16_wait(taddr + c, r);
 #pragma unroll
                     for (int j = 0; j < 16; ++j) part[(c + j) * PITCH + q * 32 + lane] = __uint_as_float(r[j]);
                 }
@@ -259,7 +235,7 @@ gemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     }
     if (split > 1) {
         __syncwarp();
-        cluster_sync();                                                        // every block's sums are written and visible
+        cluster_meet();                                                        // every block's sums are written and visible
         const uint32_t mine = base + R::OFF_PART;
         const int quads = M * QUADS, e1 = (int)((long long)(rank + 1) * quads / split), n0 = first * UNITS;
         for (int e = (int)((long long)rank * quads / split) + threadIdx.x; e < e1; e += THREADS) {
@@ -281,19 +257,11 @@ gemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     }
     __syncwarp();
     fence_before_sync();
-    if (split > 1) cluster_sync(); else __syncthreads();                       // no block leaves while another may still read its sums
+    if (split > 1) cluster_meet(); else __syncthreads();                       // no block leaves while another may still read its sums
     if (warp == 1) {
         fence_after_sync();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(R::TMEM_COLS) : "memory");
     }
-}
-
-int sm_count() {
-    static const int n = [] {
-        int dev = 0, v = 0;
-        return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0 ? v : 148;
-    }();
-    return n;
 }
 
 // Clusters of each size that the device holds at once with one block of this kernel an SM (clusters live inside one GPC, so fewer
@@ -306,7 +274,7 @@ const int* clusters_at_once() {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<16>::SMEM_BYTES) != cudaSuccess) { (void)cudaGetLastError(); return; }
         for (int sp = 2; sp <= MAX_SPLIT; ++sp) {
             cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(sp * sm_count());
+            cfg.gridDim = dim3(sp * bl_device_sms());
             cfg.blockDim = dim3(THREADS);
             cfg.dynamicSmemBytes = Ring<16>::SMEM_BYTES;
             cudaLaunchAttribute attr[1];
@@ -347,7 +315,7 @@ int launch(const void* x, const void* w, const void* bias, int bias_dtype, void*
         BL_CUDA(bl_launch_dependent_clusters(gemm_tc_few_kernel<EPI, TO, NT>, dim3((unsigned)(n_tiles * split)), dim3(THREADS), (size_t)Ring<NT>::SMEM_BYTES, s,
                                              (unsigned)split, mx, mw, bias, bias_dtype, (TO*)out, M, N, K, split));
     } else {
-        const int blocks = n_tiles < sm_count() ? n_tiles : sm_count();
+        const int blocks = n_tiles < bl_device_sms() ? n_tiles : bl_device_sms();
         BL_CUDA(bl_launch_dependent(gemm_tc_few_kernel<EPI, TO, NT>, dim3((unsigned)blocks), dim3(THREADS), (size_t)Ring<NT>::SMEM_BYTES, s,
                                     mx, mw, bias, bias_dtype, (TO*)out, M, N, K, 1));
     }

@@ -169,7 +169,6 @@ bool rows_fast(int d, const void* a, const void* b2, const void* c, const void* 
 // sublayer's result, its gate and the stream, and the earlier streams are averaged last; the other rows hide the waits. A Fezopel
 // prefill of 2,048 tokens, 16 such launches (3B widths, 8 layers): 5,136 -> 4,791 us, 0.5B widths 2,096 -> 2,031; of 500 tokens 1,020 -> 1,005.
 template <int NV> constexpr int lean_blocks() { return NV <= 1 ? 16 : NV == 2 ? 12 : NV <= 4 ? 8 : 4; }     // an SM
-constexpr int CHAIN_LEAN_ROWS = 300;       // two an SM
 template <typename TY, int NV, bool LEAN>
 __global__ void __launch_bounds__(ROW_THREADS, LEAN ? lean_blocks<NV>() : 0)
 norm_chain_kernel(float* x, const float* sub, const float* gate, int ld_gate, const void* __restrict__ gb, int gb_dtype,
@@ -608,7 +607,8 @@ extern "C" int bl_norm_chain(float* x, const float* sub, const float* gate, int 
 #define BL_CHAIN_FORM(TY, NV, LEAN) BL_CUDA(bl_launch_dependent(norm_chain_kernel<TY, NV, LEAN>, dim3(rows), dim3(ROW_THREADS), 0, s, x, sub, gate, ld_gate, \
         gate_bias, gb_dtype, w, w_dtype, b, b_dtype, eps, streams, (size_t)stride, coeffs, c_dtype, n, mix_out, w2, w2_dtype, \
         b2, b2_dtype, eps2, (TY*)y, d))
-#define BL_CHAIN(TY, NV) do { if (rows > CHAIN_LEAN_ROWS) BL_CHAIN_FORM(TY, NV, true); else BL_CHAIN_FORM(TY, NV, false); } while (0)
+    // (the lean build from two rows an SM on)
+#define BL_CHAIN(TY, NV) do { if (rows > 2 * bl_device_sms()) BL_CHAIN_FORM(TY, NV, true); else BL_CHAIN_FORM(TY, NV, false); } while (0)
 #define BL_CHAIN_NV(TY) do { if (nv <= 1) BL_CHAIN(TY, 1); else if (nv == 2) BL_CHAIN(TY, 2); else if (nv <= 4) BL_CHAIN(TY, 4); else BL_CHAIN(TY, 8); } while (0)
     if (y_dtype == BL_BF16) BL_CHAIN_NV(__nv_bfloat16);
     else if (y_dtype == BL_F32) BL_CHAIN_NV(float);

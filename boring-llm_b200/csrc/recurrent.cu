@@ -1189,14 +1189,6 @@ gated_group_norm_kernel(const float* o, const float* x, int ld_x, const void* __
         bl_store(y + (size_t)t * width + c0 + i, value(c0 + i) * inv * (w ? bl_load_any(w, w_dtype, c0 + i) : 1.f));
 }
 
-int scan_sms() {
-    static const int sms = [] {                                                 // (of the current device at the first call)
-        int dev = 0, n = 0;
-        return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
-    }();
-    return sms;
-}
-
 }  // namespace
 
 extern "C" int bl_recurrent_scan(int rule, const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
@@ -1282,12 +1274,12 @@ extern "C" int bl_recurrent_scan_parts(int rule, const float* q, int ldq, const 
         // Two an SM, or the build for four: by the blocks that work side by side for most of the launch, not by those of a few
         // tokens beside a long portion that leave at once (2,000 tokens beside 31 running requests, in one piece: 7 heads of
         // 64 x 128 640 us counted by all, 507 so; 8 of 128 x 256 1,115 and 824; the delta rule 778 and 613, 1,215 and 934).
-        const int two_an_sm = 2 * scan_sms();
+        const int two_an_sm = 2 * bl_device_sms();
         // Four columns a lane from four blocks of one column an SM on, when a second round of those would begin: 8 single tokens of 8
         // heads of 128 x 256 9.4 -> 6.3 us, 64 of them 56 -> 23; prompts of 401 to 57 tokens 249 -> 177 (delta rule 315 -> 238); 2,048
         // tokens in 32 parts of 7 heads of 64 x 128 103 -> 78. Below, a fourth of the blocks is too few: 8 single tokens of 7 heads of
         // 64 x 128 3.3 us against 4.1, 8 x 250 tokens 79 against 97.
-        const long long fours_from = 4LL * scan_sms();
+        const long long fours_from = 4LL * bl_device_sms();
         const long long at_once[2] = {(long long)n_cut * nc, nc > 1 ? (long long)n_cut * nc + (busy > n_cut ? busy - n_cut : 0) : busy};
 #define BL_SCAN_Q(D, R4, NC, KSC, DENSE, QUIET, CUT, GRID) BL_CUDA(bl_launch_dependent(recurrent_scan_vec_kernel<D, R4, NC, KSC, DENSE, QUIET, CUT>, GRID, \
         dim3(WARPS * 32), NC == 4 ? four.smem : smem, s, q, ldq, k, ldk, v, ldv, z, ldz, beta, ldb, q_scale, state, (size_t)slot_stride, slots, cu_q, out, H, G, \
@@ -1453,7 +1445,7 @@ extern "C" int bl_conv_silu_unit_bias(const float* x, int ld, const float* taps,
     if (n_taps == 4 && C % 4 == 0 && ld % 4 == 0 && slot_stride % 4 == 0 && unit_cols % 4 == 0 && unit_cols <= 8192 &&
         (((uintptr_t)x | (uintptr_t)taps | (uintptr_t)tail | (uintptr_t)y) & 15) == 0) {
         // several tokens a block where the launch then still has a block for every SM, and their unit heads fit its 48 KB
-        if (T >= CONV_RUN * 148 && CONV_RUN * unit_cols * (int)sizeof(float) <= 48 * 1024) {
+        if (T >= CONV_RUN * bl_device_sms() && CONV_RUN * unit_cols * (int)sizeof(float) <= 48 * 1024) {
             BL_CUDA(bl_launch_dependent(conv4_silu_unit_run_kernel, dim3((T + CONV_RUN - 1) / CONV_RUN), dim3(CONV4_THREADS),
                                         (size_t)CONV_RUN * unit_cols * sizeof(float), (cudaStream_t)stream, x, ld, (const float4*)taps, tail,
                                         (size_t)slot_stride, slots, tok_req, cu_q, y, T, C, unit_heads, scaled_heads, dk, q_scale, unit_eps, bias, bias_dtype));

@@ -1,6 +1,6 @@
 // What the tcgen05 kernels share: thin wrappers around the PTX of mbarriers, TMA loads, tcgen05.mma / ld / fences,
-// the shared-memory operand descriptor, and the host side's tensor maps. Each kernel file keeps its own bounded
-// wait (it records into the file's own status word) and its own instruction descriptors.
+// the shared-memory operand descriptor, and the host side's tensor maps. Each kernel file keeps its own status
+// word, into which its bounded waits record, and its own instruction descriptors.
 #pragma once
 #include "common.cuh"
 #include "api.h"
@@ -24,6 +24,30 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
+}
+
+// Bounded wait of a block that goes on after a wait has run out: false when the bound did or another thread of the block has given up;
+// the first such wait leaves `code` in the file's status word.
+__device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, uint32_t limit, volatile int* give_up, int* status, int code) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < limit; ++i) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if (*give_up) return false;
+    }
+    *give_up = 1;
+    atomicCAS(status, 0, code);
+    return false;
+}
+// Bounded wait that does not look at the give-up flag (a block that has given up waits for its own copies).
+__device__ __forceinline__ void mbar_wait_landed(uint32_t bar, uint32_t parity, uint32_t limit) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < limit; ++i)
+        if (mbar_try_wait(bar, parity)) return;
+}
+
+// All blocks of the cluster; what each has written before is visible to the others behind it.
+__device__ __forceinline__ void cluster_meet() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // ---- TMA: one 2-D box into shared memory, its bytes reported to `bar` -----------------------------------------
@@ -73,6 +97,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
                  : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// 16 columns, waited for
+__device__ __forceinline__ void tmem_ld16_wait(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
+}
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
