@@ -34,6 +34,10 @@
 //   896 x 896, residual           7.7 -> 7.8    8.8 -> 8.1    17.8 -> 10.5   33 -> 15     110 -> 64
 //   4,864 + 4,864 x 896, gated   13.6 -> 23.7    25 -> 24.2     71 -> 36    178 -> 69     876 -> 308
 //   896 x 4,864, residual          55 -> 31      48 -> 31.3     84 -> 34    158 -> 42     557 -> 179
+// Up to some ten rows, which FMAs take as fast as W streams, the widest products (from 73 tiles on, whose K is not cut) are slower than
+// before: one row of 11,008 + 11,008 x 2,048 57 -> 104, of 18,944 + 18,944 x 3,584 120 -> 181. The other products of a layer make up for
+// it (a layer's four, one row: 0.5B sizes 83 -> 70, 3B 230 -> 201, 7B 421 -> 366), and one kernel for all numbers of rows is what
+// keeps a row's bits.
 // Every wait on an mbarrier is bounded; when a bound runs out the block records a code in a status word and stops computing, but
 // still meets its cluster, frees its tensor memory and returns (bl_gemm_f32_tc_status).
 #include "tcgen05.cuh"
@@ -416,11 +420,14 @@ int launch_width(const float* x, const float* w, const void* bias, int bias_dtyp
     }
 }
 
-// Into how many spans K is cut, over the blocks of a cluster: four where a row of tiles fills less than a quarter of the device
-// and the spans keep four segments each. By N and K alone: which spans a sum is made of must not depend on the rows.
+// Into how many spans K is cut, over the blocks of a cluster: four where the clusters of a row of tiles fit the device at once (up to 33
+// tiles), two up to 72, if the spans keep four segments each. By N and K alone: which spans a sum is made of must not depend on the rows.
+// Few rows, whose launch is one row of tiles, gain more than many lose in blocks of their own beginning and end. Uncut -> cut, microseconds,
+// 1, 128 and 2,048 rows: 4,224 x 2,048 (33 tiles) 58 -> 18, 55 -> 29, 318 -> 425; 4,608 x 3,584 (36) 86 -> 45, 88 -> 53, 460 -> 495 (FMAs 42,
+// 150, 1,150); 6,144 x 2,048 (48) 55 -> 31, 62 -> 43, 407 -> 443; gated 4,608 + 4,608 x 1,536 (72) 43 -> 23, 48 -> 34, 425 -> 511.
 int f32_tc_spans(int N, int K, int epi) {
-    const int n_tiles = (N + (epi == BL_EPI_SWIGLU ? BM / 2 : BM) - 1) / (epi == BL_EPI_SWIGLU ? BM / 2 : BM);
-    return n_tiles <= 32 && K >= 4 * 4 * BK ? 4 : 1;
+    const int units = epi == BL_EPI_SWIGLU ? BM / 2 : BM, n_tiles = (N + units - 1) / units;
+    return n_tiles <= 33 && K >= 4 * 4 * BK ? 4 : n_tiles <= 72 && K >= 2 * 4 * BK ? 2 : 1;
 }
 
 }  // namespace
