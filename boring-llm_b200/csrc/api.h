@@ -251,7 +251,10 @@ int bl_attention_decode_tma_tail(const void* q, const void* k_cache, const void*
                                  int n_splits, void* out, int H, int KV, int dh, int page_size, int window, float scale,
                                  int early, const void* sinks, int sink_dtype, const float* gate, int ld_gate, void* stream);
 
-// The plain product with rows of x that are `ldx` values apart (a column range of a wider matrix as the input).
+// The plain product with rows of x that are `ldx` values apart (a column range of a wider matrix as the input). Of 32-bit rows by
+// bfloat16 matrices with K up to 64 (and the decays below at any type with such a K) W, bias and coef are weights: they are asked for
+// before the kernel in front on the stream has finished and must not be its results. The same holds for W in every product here that
+// runs on tensor cores.
 int bl_gemm_plain_ld(const void* x, int x_dtype, int ldx, const void* w, int w_dtype, const void* bias, int bias_dtype,
                      void* out, int out_dtype, int M, int N, int K, int epilogue, void* stream);
 

@@ -26,8 +26,8 @@
 // products of them below 32-bit ones. With the other operand under 2^40 (else the row's every sum is worked out again) that is
 // less than 2^-24 of any larger sum.
 //
-// Bound by shared memory: a segment's bytes are written and read once as they come, its parts (6 bytes a number) written once and read
-// by the eight MMAs of each 16 values of k. Issued by a warp that splits as well, the MMAs held up the next segment's splitting (4,864 +
+// Bound by the splitting: 8.5 instructions a number in chains, at 54 % of the issue slots (366 rows below), beside shared memory, which
+// takes a segment as it comes once, its parts (6 bytes a number) once, and gives them to the eight MMAs of each 16 values of k. Issued by a warp that splits as well, the MMAs held up the next segment's splitting (4,864 +
 // 4,864 x 896: 1 row 27.3 us, 366 rows 89). Microseconds, FMAs (gemm_plain.cu) -> this:
 //   rows                          1             16            128           366           2,048
 //   1,152 x 896, bias             7.8 -> 7.7    8.7 -> 8.1    19.7 -> 18.8   31 -> 26     118 -> 75

@@ -129,7 +129,7 @@ int launch_out(const void* x, const void* w, const void* bias, int bias_dtype, v
 // ---- products with a short K (the second factor of a low-rank pair) --------------------------------------------------------
 // The same sums (one accumulator an output, ascending k) for 32-bit x and 32-bit results with K up to RANK_MAX: a thread holds a
 // row of W in registers and goes down the rows of x, which the block has brought to shared memory (a broadcast each). W is on its
-// way before the kernel before has finished. Tiles of 64 x 64 gave a decode step 16 blocks and no early start (8 rows of 1,024 x
+// way before the kernel before has finished (so it must not be that kernel's result: W, bias and coefficients are weights). Tiles of 64 x 64 gave a decode step 16 blocks and no early start (8 rows of 1,024 x
 // 16 in a decode step's chain 9.6 us, and 1,840 rows 15 us).
 constexpr int RANK_MAX = 64, RANK_THREADS = 128;
 

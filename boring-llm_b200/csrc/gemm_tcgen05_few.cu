@@ -9,8 +9,8 @@
 // with two accumulators, so that a tile's epilogue runs under the next one's products. The ring's first round of W is asked for
 // before the dependent-launch wait: W does not depend on the kernel before.
 // SWIGLU: a tile is 64 gate rows of W and the 64 up rows that match.
-// 16 rows, launches in a row on cold matrices: gate/up of 18,944 + 18,944 x 3,584 61.5 -> 43.2 us (6.3 TB/s), 3,584 x 3,584 12.0 -> 8.0,
-// 8,208 x 2,048 14.5 -> 8.8, 11,008 + 11,008 x 2,048 32.3 -> 21.8; one row of 3,584 x 18,944 38.6 -> 27.1.
+// 16 rows, launches in a row on cold matrices: gate/up of 18,944 + 18,944 x 3,584 61.5 -> 42.3 us (6.4 TB/s), 3,584 x 3,584 12.0 -> 8.0,
+// 8,208 x 2,048 14.5 -> 8.8, 11,008 + 11,008 x 2,048 46.7 -> 21.6; one row of 3,584 x 18,944 38.6 -> 27.1.
 // One thread issues the copies, one the MMAs, four warps the epilogue. Every wait on an mbarrier is bounded; when a bound runs out
 // the block records a code in a status word, lets its own copies land, still meets its cluster, frees its tensor memory and returns
 // (bl_gemm_tc_few_status).

@@ -940,8 +940,8 @@ conv_silu_unit_kernel(const float* x, int ld, const float* __restrict__ taps, in
 // The same for four taps, channels in groups of four with 16-byte accesses: the unit heads' values stay in shared memory
 // between the convolution and the norm (the kernel above writes, reads and writes them again, and reads each tap of a
 // channel by itself). Sums in the order of the kernel above. Bound by trips to L2 for few tokens (8 of 4,096 channels
-// 21 -> 5.2 us) and by the rows' bytes for many (2,048 of 1,792 channels 30 -> 19 us; several tokens a block, for their
-// common inputs in L1, are slower: 21).
+// 21 -> 5.2 us) and by the rows' bytes for many (2,048 of 1,792 channels 30 -> 19 us; for that many
+// tokens see the kernel behind this one).
 constexpr int CONV4_THREADS = 256;
 __global__ void __launch_bounds__(CONV4_THREADS)
 conv4_silu_unit_kernel(const float* x, int ld, const float4* __restrict__ taps, const float* tail, size_t slot_stride,

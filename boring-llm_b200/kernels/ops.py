@@ -677,7 +677,8 @@ def gemm_tc_cols(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
 
 
 # Which matrix-product kernel takes a bfloat16 product of M rows by N columns. The thresholds were measured on a
-# B200 (148 SMs) and live here, beside the kernels they choose between, not in the parts that call them.
+# B200 (148 SMs) and live here, beside the kernels they choose between, not in the parts that call them. They choose among the kernels other
+# than the one that streams W once for up to 64 rows (`gemm_tc_few`), which is then weighed against their choice (`gemm_few_better`).
 SKINNY_MAX_ROWS = 64                  # up to here W streams through registers (faster than 128-row tcgen05 tiles at 64 rows)
 TC_MIN_COLUMNS_FEW_ROWS = 4096        # 17..64 rows: wide products have enough 128-column tiles for TMA to stream W at full rate
 TC_MIN_COLUMNS_VERY_FEW_ROWS = 32768  # an output head: up to 64 rows take the kernel made for it; without it 128-row tiles win from 9 rows
@@ -1144,8 +1145,9 @@ SCAN_MAX_PORTIONS = 65535         # requests times parts that one launch takes
 def _scan_parts_of_fours(rule: int, H: int, dk: int, dv: int, n_long: int, tokens: int):
     """(parts, microseconds) when the passes run with four columns a lane: a token's chain is twice that of one column, 0.58 us, but a
     fourth of the blocks walks the same columns, so that the most parts whose blocks are all under way are the best. None where that
-    build is not there (key sizes of 16 times a power of two) or not measured to pay: short portions, and the delta rule up to 64 key
-    channels, which is kept at its number of parts."""
+    build is not there (key sizes of 16 times a power of two), for shorter portions, whose number of parts is left to `_scan_cost` (one
+    column a lane; 1,024 tokens of the delta rule, 8 heads of 128 x 256, would take 292 us in parts of this build and take 517 in one piece),
+    and for the delta rule up to 64 key channels, which is kept at its number of parts."""
     ks = dk // 16
     if tokens < SCAN_FOUR_TOKENS or dk % 16 or ks & (ks - 1) or not 1 <= ks <= 32 or dv % 4 or (rule == RULE_DELTA and dk <= 64):
         return None
